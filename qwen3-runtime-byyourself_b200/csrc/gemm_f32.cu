@@ -2,21 +2,316 @@
 // operands, fmaf accumulation and no tensor-core mode of reduced precision.
 //
 // It replaces the reference's single cublasGemmEx call per projection
-// (src/ops/linear.cpp:165-193) on the 32-bit path only.  Every output element is the
-// sum over k = 0..K-1 in ascending tiles of 16 and ascending order inside a tile,
-// whatever M, N or the tile an element falls in, so a row's result does not depend on
-// which other rows are in the batch.
+// (src/ops/linear.cpp:165-193) on the 32-bit path only.  The order of an element's sum
+// depends on K and on nothing else - not on M, N or the tile it falls in - so a row's
+// result does not depend on which other rows are in the batch, although two kernels share
+// the work.  The order, for rows of whole 16-byte packets:
 //
-// The same kernel with bfloat16 operands (32-bit accumulation, bfloat16 or float output)
-// takes the bfloat16 products whose width is no multiple of 8, which the tensor-core
-// kernels refuse (their 16-byte loads and TMA strides need one).
+//   K is cut into at most 8 ranges (`range_length`); inside a range the even and the odd k
+//   are two ascending chains of fmaf, whose sums are added; the ranges' sums are added in
+//   ascending order.
+//
+// Two chains because fma.rn.f32x2 then takes its operands as they lie in memory; ranges
+// because warps and blocks can share K without changing the sum.  Shorter chains also round
+// less: logits of 4 layers of 8B width are 4.4e-7 away from 64 bits where one chain gave 1.7e-6.
+//
+//   stream_kernel : up to 8 rows (decode).  Bound by reading W once: 5.6 TB/s over the products of a
+//                   decode step of 3 sequences (1.0 ms; tiles of 64 x 64 took 8.9).
+//   tile_kernel   : more rows.  Bound by the CUDA cores' fma: 38 TFLOP/s over the products of 183 rows
+//                   at 8B width (11.1 ms for 4 layers, 31 before).
+//
+// Rows that are not whole packets, and bfloat16 operands of any width (32-bit accumulation,
+// bfloat16 or float output: the products whose width is no multiple of 8, which the
+// tensor-core kernels refuse), go to `gemm_tn_kernel`, one ascending chain.
 #include "common.cuh"
+#include <cooperative_groups.h>
+
+namespace cg = cooperative_groups;
 
 namespace {
 
+constexpr int MAX_RANGES = 8;
+
+// K per range: a multiple of 32 (the kernels' step), at least 256.
+__host__ __device__ __forceinline__ int range_length(int K) {
+    const int even = (K + MAX_RANGES - 1) / MAX_RANGES;
+    return max(256, (even + 31) / 32 * 32);
+}
+
+__device__ __forceinline__ void copy16(uint32_t to, const void* from, bool inside) {
+    // outside: nothing is read, 16 zero bytes are written
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(to), "l"(from), "r"(inside ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int LEFT> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(LEFT) : "memory"); }
+
+// acc = {acc.x + a.x b.x, acc.y + a.y b.y}, each a single rounding (fmaf)
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float both(uint64_t v) {
+    return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
+}
+
+// ---------------------------------------------------------------- few rows
+// A block owns 32 rows of W, a lane one of them; a warp walks one range of K, so X is the same address for all lanes.  A
+// warp stages 32 k of its 32 rows (whole lines) and of X with asynchronous copies in stages of its own, no barrier between
+// warps; the padded row stride (36 words) keeps the lanes' 16-byte reads free of bank conflicts.  The memory's latency at
+// full rate needs about 55 KB in flight an SM: two blocks an SM with two stages, or, when the matrix has no more blocks than
+// there are SMs, one with four.  Sums of ranges meet in shared memory.
+constexpr int S_ROWS = 32, S_WARPS = 8, S_K = 32, S_LD = S_K + 4;
+
+template <int MT> constexpr int stream_stage() { return S_ROWS * S_LD + MT * S_K; }      // floats
+
+template <int MT, int S_STAGES>
+__global__ void __launch_bounds__(S_WARPS * 32)
+stream_kernel(const float* __restrict__ X, const float* __restrict__ W, float* __restrict__ Y, int M, int N, int K, int64_t ldx,
+              int64_t ldw, int64_t ldy) {
+    extern __shared__ __align__(16) float shared[];
+    float* sums = shared + S_WARPS * S_STAGES * stream_stage<MT>();      // [range][MT][32]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n0 = blockIdx.x * S_ROWS;
+    const int length = range_length(K), ranges = (K + length - 1) / length;
+    float* mine = shared + warp * S_STAGES * stream_stage<MT>();
+    const uint32_t mine_at = (uint32_t)__cvta_generic_to_shared(mine);
+    pdl_launch_dependents();
+    pdl_wait();
+
+    const int range = warp;                              // MAX_RANGES == S_WARPS
+    const int k_begin = range * length, k_end = min(K, k_begin + length);
+    const int steps = range < ranges ? (k_end - k_begin + S_K - 1) / S_K : 0;
+    auto fetch = [&](int step) {
+        if (step < steps) {
+            const int k0 = k_begin + step * S_K;
+            const uint32_t at = mine_at + (step % S_STAGES) * (stream_stage<MT>() * 4);
+            const int part = (lane & 7) * 4;             // 8 lanes take a row's 128 bytes
+            const bool in = k0 + part < k_end;
+#pragma unroll
+            for (int i = 0; i < S_ROWS / 4; ++i) {
+                const int row = i * 4 + (lane >> 3);
+                const bool ok = in && n0 + row < N;
+                copy16(at + (row * S_LD + part) * 4, ok ? W + (int64_t)(n0 + row) * ldw + k0 + part : W, ok);
+            }
+#pragma unroll
+            for (int i = 0; i < (MT + 3) / 4; ++i) {
+                const int row = i * 4 + (lane >> 3);
+                const bool ok = in && row < M;
+                if (row < MT) copy16(at + (S_ROWS * S_LD + row * S_K + part) * 4, ok ? X + (int64_t)row * ldx + k0 + part : X, ok);
+            }
+        }
+        copies_commit();          // empty groups past the end keep the count of groups in step
+    };
+    uint64_t acc[MT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) acc[m] = 0;
+#pragma unroll
+    for (int s = 0; s < S_STAGES - 1; ++s) fetch(s);
+    for (int step = 0; step < steps; ++step) {
+        copies_wait<S_STAGES - 2>();
+        __syncwarp();
+        fetch(step + S_STAGES - 1);                     // into the stage that the warp left before the barrier above
+        const float* w = mine + (step % S_STAGES) * stream_stage<MT>() + lane * S_LD;
+        const float* x = mine + (step % S_STAGES) * stream_stage<MT>() + S_ROWS * S_LD;
+#pragma unroll
+        for (int k = 0; k < S_K; k += 4) {
+            const ulonglong2 wv = *reinterpret_cast<const ulonglong2*>(w + k);
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const ulonglong2 xv = *reinterpret_cast<const ulonglong2*>(x + m * S_K + k);
+                fma2(acc[m], xv.x, wv.x);
+                fma2(acc[m], xv.y, wv.y);
+            }
+        }
+    }
+    copies_wait<0>();
+    if (range < ranges) {
+#pragma unroll
+        for (int m = 0; m < MT; ++m) sums[(range * MT + m) * S_ROWS + lane] = both(acc[m]);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < MT * S_ROWS; i += S_WARPS * 32) {
+        const int m = i / S_ROWS, n = n0 + i % S_ROWS;
+        if (m >= M || n >= N) continue;
+        float total = sums[i];
+        for (int r = 1; r < ranges; ++r) total += sums[r * MT * S_ROWS + i];
+        Y[(int64_t)m * ldy + n] = total;
+    }
+}
+
+template <int MT, int STAGES>
+int launch_stream(const float* X, const float* W, float* Y, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldy,
+                  cudaStream_t stream) {
+    static_assert(S_WARPS == MAX_RANGES, "a warp per range");
+    constexpr int SMEM = (S_WARPS * STAGES * stream_stage<MT>() + MAX_RANGES * MT * S_ROWS) * 4;
+    static Q3PerDevice configured;
+    const cudaError_t e = q3_allow_shared_memory(stream_kernel<MT, STAGES>, SMEM, configured);
+    if (e != cudaSuccess) return (int)e;
+    return (int)q3_launch(stream_kernel<MT, STAGES>, dim3((N + S_ROWS - 1) / S_ROWS), dim3(S_WARPS * 32), SMEM, stream, X, W, Y, M,
+                          N, K, ldx, ldw, ldy);
+}
+
+template <int MT>
+int launch_stream(const float* X, const float* W, float* Y, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldy,
+                  cudaStream_t stream) {
+    if ((N + S_ROWS - 1) / S_ROWS <= q3_device_sm_count()) return launch_stream<MT, 4>(X, W, Y, M, N, K, ldx, ldw, ldy, stream);
+    return launch_stream<MT, 2>(X, W, Y, M, N, K, ldx, ldw, ldy, stream);
+}
+
+// ---------------------------------------------------------------- more rows
+// A tile of BM rows of X by 128 rows of W per block, (BM / 16) x 8 elements a thread, both operands staged as they lie in
+// memory (rows of 32 k, padded to 36 words: the 16 rows a warp reads at once fall into different banks) in three stages of
+// asynchronous copies.  Per 4 k a thread makes 4 BM/16 * 8 multiply-adds from BM/16 + 8 16-byte reads.  When there are too
+// few tiles to fill the GPU, the ranges of K are shared out to a cluster's blocks, which leave their sums in shared memory
+// and add a share of the tile each, in the order of the ranges.
+constexpr int T_N = 128, T_K = 32, T_LD = T_K + 4, T_STAGES = 3;
+
+template <int BM> constexpr int tile_stage() { return (BM + T_N) * T_LD; }               // floats
+
+template <int BM>
+__global__ void __launch_bounds__(256, 2)
+tile_kernel(const float* __restrict__ X, const float* __restrict__ W, float* __restrict__ Y, int M, int N, int K, int64_t ldx,
+            int64_t ldw, int64_t ldy, int shares) {
+    extern __shared__ __align__(16) float shared[];
+    constexpr int TM = BM / 16, TN = T_N / 16;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int share = blockIdx.x % shares;
+    const int n0 = (blockIdx.x / shares) * T_N, m0 = blockIdx.y * BM;
+    const int length = range_length(K), ranges = (K + length - 1) / length;
+    const int first = share * ranges / shares, last = (share + 1) * ranges / shares;      // this block's ranges
+    const int k_begin = first * length, k_end = min(K, last * length);
+    const uint32_t shared_at = (uint32_t)__cvta_generic_to_shared(shared);
+    pdl_launch_dependents();
+    pdl_wait();
+
+    const int steps = (k_end - k_begin + T_K - 1) / T_K, per_range = length / T_K;
+    auto fetch = [&](int step) {
+        if (step < steps) {
+            const int k0 = k_begin + step * T_K, part = (tid & 7) * 4;
+            const uint32_t at = shared_at + (step % T_STAGES) * (tile_stage<BM>() * 4);
+            const bool in = k0 + part < k_end;
+#pragma unroll
+            for (int i = 0; i < (BM + 31) / 32; ++i) {
+                const int row = i * 32 + (tid >> 3);
+                const bool ok = in && m0 + row < M;
+                if (row < BM) copy16(at + (row * T_LD + part) * 4, ok ? X + (int64_t)(m0 + row) * ldx + k0 + part : X, ok);
+            }
+#pragma unroll
+            for (int i = 0; i < T_N / 32; ++i) {
+                const int row = i * 32 + (tid >> 3);
+                const bool ok = in && n0 + row < N;
+                copy16(at + ((BM + row) * T_LD + part) * 4, ok ? W + (int64_t)(n0 + row) * ldw + k0 + part : W, ok);
+            }
+        }
+        copies_commit();
+    };
+    uint64_t acc[TM][TN];
+    float total[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0;
+#pragma unroll
+    for (int s = 0; s < T_STAGES - 1; ++s) fetch(s);
+    int done = 0;                                        // ranges that are summed
+    for (int step = 0; step < steps; ++step) {
+        copies_wait<T_STAGES - 2>();
+        __syncthreads();
+        fetch(step + T_STAGES - 1);
+        const float* a = shared + (step % T_STAGES) * tile_stage<BM>() + ty * T_LD;
+        const float* b = shared + (step % T_STAGES) * tile_stage<BM>() + (BM + tx) * T_LD;
+#pragma unroll 2
+        for (int k = 0; k < T_K; k += 4) {
+            ulonglong2 av[TM];
+#pragma unroll
+            for (int i = 0; i < TM; ++i) av[i] = *reinterpret_cast<const ulonglong2*>(a + i * 16 * T_LD + k);
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const ulonglong2 bv = *reinterpret_cast<const ulonglong2*>(b + j * 16 * T_LD + k);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    fma2(acc[i][j], av[i].x, bv.x);
+                    fma2(acc[i][j], av[i].y, bv.y);
+                }
+            }
+        }
+        if ((step + 1) % per_range == 0 || step + 1 == steps) {          // a range is complete
+            if (shares == 1) {
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) {
+                        const float sum = both(acc[i][j]);
+                        total[i][j] = done == 0 ? sum : total[i][j] + sum;
+                        acc[i][j] = 0;
+                    }
+            } else {
+                float* kept = shared + T_STAGES * tile_stage<BM>() + done * BM * T_N;
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) {
+                        kept[(i * 16 + ty) * T_N + j * 16 + tx] = both(acc[i][j]);
+                        acc[i][j] = 0;
+                    }
+            }
+            ++done;
+        }
+    }
+    copies_wait<0>();
+    if (shares == 1) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const int m = m0 + i * 16 + ty;
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const int n = n0 + j * 16 + tx;
+                if (m < M && n < N) Y[(int64_t)m * ldy + n] = total[i][j];
+            }
+        }
+        return;
+    }
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    const float* kept = shared + T_STAGES * tile_stage<BM>();
+    for (int i = share * 256 + tid; i < BM * T_N; i += shares * 256) {
+        const int m = m0 + i / T_N, n = n0 + i % T_N;
+        if (m >= M || n >= N) continue;
+        float sum = 0.0f;
+        for (int c = 0, r = 0; c < shares; ++c) {
+            const float* theirs = cluster.map_shared_rank(kept, c);
+            const int to = (c + 1) * ranges / shares;
+            for (int at = 0; r < to; ++r, ++at) sum = r == 0 ? theirs[i] : sum + theirs[at * BM * T_N + i];
+        }
+        Y[(int64_t)m * ldy + n] = sum;
+    }
+    cluster.sync();                                      // a block's sums stay until all have read them
+}
+
+template <int BM>
+int launch_tiles(const float* X, const float* W, float* Y, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldy,
+                 cudaStream_t stream) {
+    const int length = range_length(K), ranges = (K + length - 1) / length;
+    const int64_t tiles = (int64_t)((N + T_N - 1) / T_N) * ((M + BM - 1) / BM);
+    if ((M + BM - 1) / BM > 65535) return Q3_ERR_TOO_LARGE;
+    // two blocks are resident on an SM; K is shared while that leaves some of the room empty
+    int shares = 1;
+    while (shares * 2 <= ranges && tiles * shares * 2 <= 2 * (int64_t)q3_device_sm_count()) shares *= 2;
+    const int kept = shares > 1 ? (ranges + shares - 1) / shares * BM * T_N : 0;
+    constexpr int MOST = (T_STAGES * tile_stage<BM>() + MAX_RANGES / 2 * BM * T_N) * 4;
+    static Q3PerDevice configured;
+    const cudaError_t e = q3_allow_shared_memory(tile_kernel<BM>, MOST, configured);
+    if (e != cudaSuccess) return (int)e;
+    const int smem = (T_STAGES * tile_stage<BM>() + kept) * 4;
+    const dim3 grid((N + T_N - 1) / T_N * shares, (M + BM - 1) / BM);
+    if (shares == 1)
+        return (int)q3_launch(tile_kernel<BM>, grid, dim3(256), smem, stream, X, W, Y, M, N, K, ldx, ldw, ldy, shares);
+    return (int)q3_launch_cluster(tile_kernel<BM>, grid, dim3(256), smem, stream, dim3(shares, 1, 1), X, W, Y, M, N, K, ldx, ldw,
+                                  ldy, shares);
+}
+
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
 
-template <bool VEC4, typename InT, typename OutT>
+template <typename InT, typename OutT>
 __global__ void __launch_bounds__(256)
 gemm_tn_kernel(const InT* __restrict__ X, const InT* __restrict__ W, OutT* __restrict__ Y, int M, int N, int K,
                int64_t ldx, int64_t ldw, int64_t ldy) {
@@ -40,23 +335,13 @@ gemm_tn_kernel(const InT* __restrict__ X, const InT* __restrict__ W, OutT* __res
         const int gm = m0 + lr, gn = n0 + lr, gk = k0 + lk;
         if (gm < M) {
             const InT* p = X + (int64_t)gm * ldx + gk;
-            if (VEC4 && gk + 3 < K) {
-                const float4 t = *reinterpret_cast<const float4*>(p);
-                xv[0] = t.x; xv[1] = t.y; xv[2] = t.z; xv[3] = t.w;
-            } else {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) if (gk + i < K) xv[i] = to_f32<InT>(p[i]);
-            }
+            for (int i = 0; i < 4; ++i) if (gk + i < K) xv[i] = to_f32<InT>(p[i]);
         }
         if (gn < N) {
             const InT* p = W + (int64_t)gn * ldw + gk;
-            if (VEC4 && gk + 3 < K) {
-                const float4 t = *reinterpret_cast<const float4*>(p);
-                wv[0] = t.x; wv[1] = t.y; wv[2] = t.z; wv[3] = t.w;
-            } else {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) if (gk + i < K) wv[i] = to_f32<InT>(p[i]);
-            }
+            for (int i = 0; i < 4; ++i) if (gk + i < K) wv[i] = to_f32<InT>(p[i]);
         }
         __syncthreads();  // the previous tile has been consumed
 #pragma unroll
@@ -96,13 +381,20 @@ Q3_EXPORT int q3_gemm_tn_f32(const float* X, const float* W, float* Y, int M, in
                              int64_t ldy, void* stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return Q3_ERR_BAD_SIZE;
+    const cudaStream_t s = (cudaStream_t)stream;
+    if (aligned16(X) && aligned16(W) && ldx % 4 == 0 && ldw % 4 == 0 && K % 4 == 0) {
+        // the stream kernel's fma rate lasts for 8 rows at the memory's rate, and no longer for 16
+        if (M == 1) return launch_stream<1>(X, W, Y, M, N, K, ldx, ldw, ldy, s);
+        if (M == 2) return launch_stream<2>(X, W, Y, M, N, K, ldx, ldw, ldy, s);
+        if (M <= 4) return launch_stream<4>(X, W, Y, M, N, K, ldx, ldw, ldy, s);
+        if (M <= 8) return launch_stream<8>(X, W, Y, M, N, K, ldx, ldw, ldy, s);
+        if (M <= 16) return launch_tiles<16>(X, W, Y, M, N, K, ldx, ldw, ldy, s);
+        if (M <= 32) return launch_tiles<32>(X, W, Y, M, N, K, ldx, ldw, ldy, s);
+        return launch_tiles<64>(X, W, Y, M, N, K, ldx, ldw, ldy, s);
+    }
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return Q3_ERR_TOO_LARGE;
-    const bool vec = aligned16(X) && aligned16(W) && ldx % 4 == 0 && ldw % 4 == 0;
-    if (vec)
-        return (int)q3_launch(gemm_tn_kernel<true, float, float>, grid, dim3(256), 0, (cudaStream_t)stream, X, W, Y, M, N, K,
-                              ldx, ldw, ldy);
-    return (int)q3_launch(gemm_tn_kernel<false, float, float>, grid, dim3(256), 0, (cudaStream_t)stream, X, W, Y, M, N, K,
+    return (int)q3_launch(gemm_tn_kernel<float, float>, grid, dim3(256), 0, (cudaStream_t)stream, X, W, Y, M, N, K,
                           ldx, ldw, ldy);
 }
 
@@ -114,8 +406,8 @@ Q3_EXPORT int q3_gemm_tn_bf16(const void* X, const void* W, void* Y, int M, int 
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return Q3_ERR_TOO_LARGE;
     if (out_is_f32)
-        return (int)q3_launch(gemm_tn_kernel<false, bf16, float>, grid, dim3(256), 0, (cudaStream_t)stream, (const bf16*)X,
+        return (int)q3_launch(gemm_tn_kernel<bf16, float>, grid, dim3(256), 0, (cudaStream_t)stream, (const bf16*)X,
                               (const bf16*)W, (float*)Y, M, N, K, ldx, ldw, ldy);
-    return (int)q3_launch(gemm_tn_kernel<false, bf16, bf16>, grid, dim3(256), 0, (cudaStream_t)stream, (const bf16*)X,
+    return (int)q3_launch(gemm_tn_kernel<bf16, bf16>, grid, dim3(256), 0, (cudaStream_t)stream, (const bf16*)X,
                           (const bf16*)W, (bf16*)Y, M, N, K, ldx, ldw, ldy);
 }

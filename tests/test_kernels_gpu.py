@@ -105,6 +105,32 @@ def test_gemm_f32_is_true_32_bit(M, N, K):
     assert torch.equal(one[0], out[M - 1])
 
 
+@pytest.mark.parametrize("K", [4, 96, 256, 260, 2048, 2084, 12288])
+@pytest.mark.parametrize("N", [1, 33, 128, 300])
+def test_gemm_f32_same_sums_in_both_kernels(N, K):
+    """Rows of whole packets: the kernel for few rows and the tiled one, at the edges of their tiles, with K shared out to a
+    cluster or not, give the same bits for a row, within the bound of their order of summation."""
+    from qwen3_b200.csrc import ops
+    rng = np.random.default_rng(N + K)
+    x, w = rng.normal(0, 1, (200, K)), rng.normal(0, 1, (N, K))
+    xd, wd = dev(x, "float32"), dev(w, "float32")
+    exact, size = back(xd) @ back(wd).T, np.abs(back(xd)) @ np.abs(back(wd)).T
+    length = max(256, (-(-K // 8) + 31) // 32 * 32)
+    # every term passes through at most a chain of length / 2, the sum of two chains and the sums of the ranges
+    bound = (length // 2 + 1 + -(-K // length)) * 2.0 ** -24 * size * 1.01
+    rows = {}
+    for M in (200, 1, 2, 3, 4, 8, 9, 16, 17, 32, 33, 64, 65):
+        out = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+        ops.gemm_f32(xd[:M].contiguous(), wd, out)
+        assert (np.abs(back(out) - exact[:M]) <= bound[:M]).all(), M
+        whole = rows.setdefault("whole", out)
+        assert torch.equal(out, whole[:M]), M
+    many = torch.full((200, 20000), float("nan"), dtype=torch.float32, device="cuda")        # K in one block
+    wide = torch.cat([wd, torch.zeros(20000 - N, K, device="cuda")])
+    ops.gemm_f32(xd, wide, many)
+    assert torch.equal(many[:, :N], rows["whole"])
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 45, 67), (37, 130, 100), (200, 333, 100), (5, 64, 9)])
 @pytest.mark.parametrize("out_dtype", ["bfloat16", "float32"])
 def test_bf16_product_of_any_width(M, N, K, out_dtype):
