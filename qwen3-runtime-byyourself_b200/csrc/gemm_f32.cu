@@ -32,11 +32,8 @@ namespace {
 
 constexpr int MAX_RANGES = 8;
 
-// K per range: a multiple of 32 (the kernels' step), at least 256.
-__host__ __device__ __forceinline__ int range_length(int K) {
-    const int even = (K + MAX_RANGES - 1) / MAX_RANGES;
-    return max(256, (even + 31) / 32 * 32);
-}
+// K per range: a multiple of 32 (the kernels' step).
+__host__ __device__ __forceinline__ int range_length(int K) { return ((K + MAX_RANGES - 1) / MAX_RANGES + 31) / 32 * 32; }
 
 __device__ __forceinline__ void copy16(uint32_t to, const void* from, bool inside) {
     // outside: nothing is read, 16 zero bytes are written

@@ -115,7 +115,7 @@ def test_gemm_f32_same_sums_in_both_kernels(N, K):
     x, w = rng.normal(0, 1, (200, K)), rng.normal(0, 1, (N, K))
     xd, wd = dev(x, "float32"), dev(w, "float32")
     exact, size = back(xd) @ back(wd).T, np.abs(back(xd)) @ np.abs(back(wd)).T
-    length = max(256, (-(-K // 8) + 31) // 32 * 32)
+    length = (-(-K // 8) + 31) // 32 * 32
     # every term passes through at most a chain of length / 2, the sum of two chains and the sums of the ranges
     bound = (length // 2 + 1 + -(-K // length)) * 2.0 ** -24 * size * 1.01
     rows = {}
