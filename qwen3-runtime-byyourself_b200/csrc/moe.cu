@@ -22,9 +22,9 @@
 //                 the last term for a shared expert that every token uses (may be absent; without shared_w its weight
 //                 is 1).
 //
-// The products accumulate in 32-bit in ascending order of k whatever the tile a pair falls into, so a token's
-// result does not depend on what else is in the step.  Float tiles run on fmaf; bfloat16 tiles on the tensor cores
-// (mma.m16n8k16, see `mma` below) when the widths are multiples of 32, else on fmaf too.
+// The products accumulate in 32-bit.  Float tiles run on fmaf in ascending order of k whatever the tile a pair falls into, so
+// a token's result does not depend on what else is in the step; bfloat16 tiles run on the tensor cores when the widths are
+// multiples of 32 (few tokens per expert: `few` below; more: moe_tcgen05.cu), else on fmaf too.
 #include "common.cuh"
 
 namespace {
@@ -350,168 +350,153 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const T* __restr
     }
 }
 
-// ---------------------------------------------------------------- the same two products on the tensor cores (bfloat16)
-// A block of 8 warps owns 64 pairs x 64 columns (of gate AND up in the first product): warp w works on rows
-// 16 (w % 4) .. + 15 and columns 32 (w / 4) .. + 31 with mma.m16n8k16 (bfloat16 in, 32-bit accumulators).  X rows
-// (gathered through the pairs' token numbers) and W rows arrive as 16-byte asynchronous copies into a ring of four
-// stages of 32 k-values, so a block keeps three stages in flight: with a handful of pairs per expert (a decode step)
-// the kernel streams each chosen expert's weights once.  Widths in steps of 32.
-namespace mma {
-constexpr int BM = 64, BN = 64, BK = 32, STAGES = 4;
-constexpr int ROW = (BK + 8) * 2;                       // bytes of a padded tile row: ldmatrix without bank conflicts
-constexpr int TILE = BM * ROW;                          // one 64 x 32 tile
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
+// ---------------------------------------------------------------- few tokens per expert, on the tensor cores (bfloat16)
+// A decode step: what counts is reading every chosen expert's weights once.  A block owns 16 rows of W (8 of the gate and the
+// 8 of up of the same features) and up to 8 of an expert's pairs; its 8 warps split K.  As in the few-row product of the
+// dense layers a lane reads 16 contiguous bytes of a W row and hands them to mma.m16n8k16 as they come (both operands permute
+// k the same way), four blocks of 32 k in flight a warp and three blocks an SM; the warps' sums are added in warp order.
+// 8 tokens, 16 experts of 2,048 at width 2,048, two per token (276 MB): both products 65 us from cold caches, 181 with tiles of
+// 64 x 64 fed by asynchronous copies of 64 bytes a row, which this replaced.
+namespace few {
+
+constexpr int WARPS = 8, IN_FLIGHT = 4, PAIRS = 8;
+enum Mode { GATED, RELU2, DOWN };
+
+__device__ __forceinline__ uint4 ld_stream16(const void* p) {
+    uint4 v;   // not volatile: the compiler may hoist and batch these loads
+    asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// acc0 (and acc1 with DUAL) [n-tile][4] of this warp: rows quad and quad + 8 of its 16, columns n * 8 + tq * 2, + 1 of its 32.
-template <bool DUAL>
-__device__ __forceinline__ void tile_product(const bf16* __restrict__ X, int64_t x_stride, const int* src_row, const bf16* __restrict__ W0,
-                                             const bf16* __restrict__ W1, int n_cols, int col0, int K, unsigned char* smem,
-                                             float (&acc0)[4][4], float (&acc1)[4][4]) {
-    constexpr int MATS = DUAL ? 3 : 2;                  // tiles per stage: X, W0 (, W1)
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t base = smem_u32(smem);
+// find_tile by a warp: a lane per expert, 32 experts at a time.
+template <int TM>
+__device__ __forceinline__ bool find_tile_warp(const int* __restrict__ offsets, int n_real, int tile, int& expert, int& row0, int& rows) {
+    const int lane = threadIdx.x & 31;
+    int before = 0;
+    for (int e0 = 0; e0 < n_real; e0 += 32) {
+        const int e = e0 + lane;
+        const int begin = offsets[min(e, n_real)], end = offsets[min(e + 1, n_real)];
+        const int tiles = (end - begin + TM - 1) / TM;
+        int upto = tiles;                                   // tiles of this lane's and all earlier experts of the 32
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc0[n][e] = acc1[n][e] = 0.0f;
-    // this thread's copy per tile and stage: row tid / 4, 16-byte chunk tid % 4
-    const int lr = tid >> 2, lc = tid & 3;
-    const bf16* x_src = X + (int64_t)src_row[lr] * x_stride + lc * 8;
-    const int w_row = min(col0 + lr, n_cols - 1);       // a row beyond the matrix reads the last one; its results are dropped
-    const bf16* w0_src = W0 + (int64_t)w_row * K + lc * 8;
-    const bf16* w1_src = DUAL ? W1 + (int64_t)w_row * K + lc * 8 : nullptr;
-    const uint32_t dst = lr * ROW + lc * 16;
-    const int nk = K / BK;
-    auto issue = [&](int kb) {
-        if (kb < nk) {
-            const uint32_t stage = base + (kb % STAGES) * (MATS * TILE) + dst;
-            cp_async16(stage, x_src + kb * BK);
-            cp_async16(stage + TILE, w0_src + kb * BK);
-            if (DUAL) cp_async16(stage + 2 * TILE, w1_src + kb * BK);
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
         }
-        cp_async_commit();
+        const unsigned past = __ballot_sync(0xffffffffu, tile < before + upto);
+        if (past != 0) {
+            const int who = __ffs(past) - 1;
+            const int local = tile - before - (__shfl_sync(0xffffffffu, upto, who) - __shfl_sync(0xffffffffu, tiles, who));
+            expert = e0 + who;
+            row0 = __shfl_sync(0xffffffffu, begin, who) + local * TM;
+            rows = min(TM, __shfl_sync(0xffffffffu, end, who) - row0);
+            return true;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return false;
+}
+
+// X [.., K]: h, a row per token (GATED, RELU2), or act, a row per slot (DOWN); `features` of an expert's output.
+template <int MODE>
+__global__ void __launch_bounds__(WARPS * 32, 3)
+expert_kernel(const bf16* __restrict__ X, const bf16* __restrict__ W, const int* __restrict__ offsets, const int* __restrict__ pair_of_slot,
+              void* __restrict__ out, int n_real, int top, int features, int K, float limit, float alpha, float up_offset) {
+    constexpr int LD = 17, PER_BLOCK = MODE == GATED ? 8 : 16;
+    __shared__ float red[WARPS][PAIRS * LD];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane >> 2, tq = lane & 3;
+    int expert, row0, rows;
+    if (!find_tile_warp<PAIRS>(offsets, n_real, blockIdx.y, expert, row0, rows)) return;
+    const int f0 = blockIdx.x * PER_BLOCK, nkb = (K + 31) >> 5;
+    const int kb_begin = warp * nkb / WARPS, kb_end = (warp + 1) * nkb / WARPS;
+
+    const bf16* wrow[2];
+    bool wok[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int f = MODE == GATED ? f0 + quad : f0 + h * 8 + quad;
+        wok[h] = f < features;
+        const int64_t row = MODE == GATED ? ((int64_t)expert * 2 + h) * features + f : (int64_t)expert * features + f;
+        wrow[h] = W + (wok[h] ? row : 0) * K + tq * 8;
+    }
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    uint4 w[IN_FLIGHT][2], x[IN_FLIGHT];
+    auto load_w = [&](int s, int kb) {
+        const int k = kb * 32;
+        const bool in = kb < kb_end && k + tq * 8 + 8 <= K;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) w[s][h] = in && wok[h] ? ld_stream16(wrow[h] + k) : zero;
     };
 #pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) issue(s);
-    const int m0 = (warp & 3) * 16, n0 = (warp >> 2) * 32;
-    const int krow = (lane & 7) + ((lane >> 4) << 3);
-    for (int kb = 0; kb < nk; ++kb) {
-        cp_async_wait<STAGES - 2>();
-        __syncthreads();                                // stage kb has landed for every thread; stage kb - 1 is free
-        issue(kb + STAGES - 1);
-        const uint32_t xs = base + (kb % STAGES) * (MATS * TILE);
-        const uint32_t ws0 = xs + TILE, ws1 = ws0 + TILE;
+    for (int s = 0; s < IN_FLIGHT; ++s) load_w(s, kb_begin + s);
+    const bool xok = quad < rows;
+    const int slot = row0 + (xok ? quad : 0);
+    const bf16* xrow = X + (int64_t)(MODE == DOWN ? slot : pair_of_slot[slot] / top) * K + tq * 8;
+    auto load_x = [&](int s, int kb) {
+        const int k = kb * 32;
+        const bool in = kb < kb_end && k + tq * 8 + 8 <= K;
+        x[s] = in && xok ? *reinterpret_cast<const uint4*>(xrow + k) : zero;
+    };
 #pragma unroll
-        for (int kt = 0; kt < BK / 16; ++kt) {
-            uint32_t a[4];                              // rows 0-7 and 8-15 of the warp's 16, k 0-7 and 8-15 of the step
-            ldmatrix_x4(a, xs + (m0 + (lane & 15)) * ROW + (kt * 16 + (lane >> 4) * 8) * 2);
+    for (int s = 0; s < IN_FLIGHT; ++s) load_x(s, kb_begin + s);
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int kb = kb_begin; kb < kb_end; kb += IN_FLIGHT) {
 #pragma unroll
-            for (int jp = 0; jp < 2; ++jp) {
-                uint32_t b[4];
-                const uint32_t off = (n0 + jp * 16 + krow) * ROW + (2 * kt + ((lane >> 3) & 1)) * 16;
-                ldmatrix_x4(b, ws0 + off);
-                mma_bf16(acc0[2 * jp], a, b[0], b[1]);
-                mma_bf16(acc0[2 * jp + 1], a, b[2], b[3]);
-                if (DUAL) {
-                    ldmatrix_x4(b, ws1 + off);
-                    mma_bf16(acc1[2 * jp], a, b[0], b[1]);
-                    mma_bf16(acc1[2 * jp + 1], a, b[2], b[3]);
-                }
-            }
+        for (int s = 0; s < IN_FLIGHT; ++s) {
+            mma_bf16(acc, w[s][0].x, w[s][1].x, w[s][0].y, w[s][1].y, x[s].x, x[s].y);
+            mma_bf16(acc, w[s][0].z, w[s][1].z, w[s][0].w, w[s][1].w, x[s].z, x[s].w);
+            load_w(s, kb + s + IN_FLIGHT);           // blocks past the end load zeros, which add nothing
+            load_x(s, kb + s + IN_FLIGHT);
         }
     }
-    cp_async_wait<0>();
-}
-
-template <bool GATE>
-__global__ void __launch_bounds__(256)
-moe_up_kernel(const bf16* __restrict__ h, const bf16* __restrict__ w_gate_up, const int* __restrict__ offsets,
-              const int* __restrict__ pair_of_slot, bf16* __restrict__ act, int n_real, int top, int hidden, int ff, float limit,
-              float alpha, float up_offset) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int src_row[BM];
-    pdl_launch_dependents();
-    pdl_wait();
-    int expert, row0, rows;
-    if (!find_tile<BM>(offsets, n_real, blockIdx.y, expert, row0, rows)) return;
-    if (threadIdx.x < BM) src_row[threadIdx.x] = pair_of_slot[row0 + min((int)threadIdx.x, rows - 1)] / top;
+    float* mine = red[warp] + tq * 2 * LD + quad;
+    mine[0] = acc[0];
+    mine[LD] = acc[1];
+    mine[8] = acc[2];
+    mine[LD + 8] = acc[3];
     __syncthreads();
-    const int col0 = blockIdx.x * BN;
-    const bf16* wg = w_gate_up + (int64_t)expert * (GATE ? 2 : 1) * ff * hidden;
-    float g[4][4], u[4][4];
-    tile_product<GATE>(h, hidden, src_row, wg, GATE ? wg + (int64_t)ff * hidden : nullptr, ff, col0, hidden, smem, g, u);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane >> 2, tq = lane & 3;
+    for (int i = threadIdx.x; i < PER_BLOCK * PAIRS; i += WARPS * 32) {
+        const int r = i / PER_BLOCK, j = i % PER_BLOCK, f = f0 + j;
+        if (r >= rows || f >= features) continue;
+        float a = 0.0f, b = 0.0f;
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int rr = (warp & 3) * 16 + quad + (e >> 1) * 8, c = col0 + (warp >> 2) * 32 + n * 8 + tq * 2 + (e & 1);
-            if (rr < rows && c < ff) {
-                if constexpr (!GATE) {
-                    const float v = fmaxf(g[n][e], 0.0f);
-                    act[(int64_t)(row0 + rr) * ff + c] = __float2bfloat16_rn(v * v);
-                    continue;
-                }
-                const float gv = fminf(g[n][e], limit), uv = fminf(fmaxf(u[n][e], -limit), limit);
-                act[(int64_t)(row0 + rr) * ff + c] = __float2bfloat16_rn(gv / (1.0f + expf(-alpha * gv)) * (uv + up_offset));
-            }
+        for (int v = 0; v < WARPS; ++v) {
+            a += red[v][r * LD + j];
+            if (MODE == GATED) b += red[v][r * LD + j + 8];
         }
+        const int64_t at = (int64_t)(row0 + r) * features + f;
+        if constexpr (MODE == DOWN) {
+            ((float*)out)[at] = a;
+        } else if constexpr (MODE == RELU2) {
+            const float v = fmaxf(a, 0.0f);
+            ((bf16*)out)[at] = __float2bfloat16_rn(v * v);
+        } else {
+            const float gv = fminf(a, limit), uv = fminf(fmaxf(b, -limit), limit);
+            ((bf16*)out)[at] = __float2bfloat16_rn(gv / (1.0f + expf(-alpha * gv)) * (uv + up_offset));
+        }
+    }
 }
 
-__global__ void __launch_bounds__(256)
-moe_down_kernel(const bf16* __restrict__ act, const bf16* __restrict__ w_down, const int* __restrict__ offsets, float* __restrict__ y,
-                int n_real, int hidden, int ff) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int src_row[BM];
-    pdl_launch_dependents();
-    pdl_wait();
-    int expert, row0, rows;
-    if (!find_tile<BM>(offsets, n_real, blockIdx.y, expert, row0, rows)) return;
-    if (threadIdx.x < BM) src_row[threadIdx.x] = row0 + min((int)threadIdx.x, rows - 1);
-    __syncthreads();
-    const int col0 = blockIdx.x * BN;
-    float acc[4][4], unused[4][4];
-    tile_product<false>(act, ff, src_row, w_down + (int64_t)expert * hidden * ff, nullptr, hidden, col0, ff, smem, acc, unused);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane >> 2, tq = lane & 3;
-#pragma unroll
-    for (int n = 0; n < 4; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int rr = (warp & 3) * 16 + quad + (e >> 1) * 8, c = col0 + (warp >> 2) * 32 + n * 8 + tq * 2 + (e & 1);
-            if (rr < rows && c < hidden) y[(int64_t)(row0 + rr) * hidden + c] = acc[n][e];
-        }
-}
-
-int experts_launch(const bf16* h, const bf16* w_gate_up, const bf16* w_down, const int* offsets, const int* pair_of_slot, bf16* act,
-                   float* y, int n_pairs, int n_real, int top, int hidden, int ff, float limit, float alpha, float up_offset, int gated, cudaStream_t stream) {
-    const int tiles = (n_pairs + BM - 1) / BM + n_real;          // an upper bound on the row tiles of all experts together
+int experts_launch(const bf16* h, const bf16* w_gate_up, const bf16* w_down, const int* offsets, const int* pair_of_slot, bf16* act, float* y,
+                   int n_pairs, int n_real, int top, int hidden, int ff, float limit, float alpha, float up_offset, int gated, cudaStream_t stream) {
+    // an upper bound on the row tiles of all experts together
+    const int tiles = n_pairs < n_real ? n_pairs : (n_pairs + PAIRS - 1) / PAIRS + n_real;
     if (tiles > 65535) return Q3_ERR_TOO_LARGE;
-    static Q3PerDevice up_ok, plain_ok, down_ok;
-    const int up_smem = STAGES * (gated ? 3 : 2) * TILE;
-    cudaError_t e = gated ? q3_allow_shared_memory(moe_up_kernel<true>, up_smem, up_ok) : q3_allow_shared_memory(moe_up_kernel<false>, up_smem, plain_ok);
-    if (e == cudaSuccess) e = q3_allow_shared_memory(moe_down_kernel, STAGES * 2 * TILE, down_ok);
-    if (e != cudaSuccess) return (int)e;
-    int code = (int)q3_launch(gated ? moe_up_kernel<true> : moe_up_kernel<false>, dim3((ff + BN - 1) / BN, tiles), dim3(256), up_smem, stream, h,
-                              w_gate_up, offsets, pair_of_slot, act, n_real, top, hidden, ff, limit, alpha, up_offset);
+    int code = gated ? (int)q3_launch(expert_kernel<GATED>, dim3((ff + 7) / 8, tiles), dim3(WARPS * 32), 0, stream, h, w_gate_up, offsets,
+                                      pair_of_slot, (void*)act, n_real, top, ff, hidden, limit, alpha, up_offset)
+                     : (int)q3_launch(expert_kernel<RELU2>, dim3((ff + 15) / 16, tiles), dim3(WARPS * 32), 0, stream, h, w_gate_up, offsets,
+                                      pair_of_slot, (void*)act, n_real, top, ff, hidden, limit, alpha, up_offset);
     if (code != 0) return code;
-    return (int)q3_launch(moe_down_kernel, dim3((hidden + BN - 1) / BN, tiles), dim3(256), STAGES * 2 * TILE, stream, act, w_down,
-                          offsets, y, n_real, hidden, ff);
+    return (int)q3_launch(expert_kernel<DOWN>, dim3((hidden + 15) / 16, tiles), dim3(WARPS * 32), 0, stream, (const bf16*)act, w_down, offsets,
+                          pair_of_slot, (void*)y, n_real, top, hidden, ff, limit, alpha, up_offset);
 }
-}  // namespace mma
+}  // namespace few
 
 template <typename T, int TM>
 int moe_experts_launch(const T* h, const T* w_gate_up, const T* w_down, const int* offsets, const int* pair_of_slot, T* act, float* y,
@@ -570,14 +555,15 @@ Q3_EXPORT int q3_moe_sort(const int* top_ids, int n_pairs, int n_real, int* offs
                           n_pairs, n_real, offsets, slot_of_pair, pair_of_slot);
 }
 
-// bfloat16 with both widths in steps of 32 (and 16-byte aligned rows): the tensor-core tiles; else the fmaf tiles.
+// bfloat16 with both widths in steps of 32 (and 16-byte aligned rows) on the tensor cores: any number of pairs, made for few
+// per expert (q3_moe_experts_tcgen05_bf16 is for more).
 Q3_EXPORT int q3_moe_experts_tc_bf16(const void* h, const void* w_gate_up, const void* w_down, const int* offsets,
                                      const int* pair_of_slot, void* act, float* y, int n_pairs, int n_real, int top, int hidden, int ff,
                                      float limit, float alpha, float up_offset, int gated, void* stream) {
     if (n_pairs <= 0 || n_real <= 0) return 0;
     if (hidden % 32 != 0 || ff % 32 != 0 || hidden <= 0 || ff <= 0) return Q3_ERR_BAD_SIZE;
     if (!aligned16(h) || !aligned16(w_gate_up) || !aligned16(w_down) || !aligned16(act)) return Q3_ERR_MISALIGNED;
-    return mma::experts_launch((const bf16*)h, (const bf16*)w_gate_up, (const bf16*)w_down, offsets, pair_of_slot, (bf16*)act, y, n_pairs,
+    return few::experts_launch((const bf16*)h, (const bf16*)w_gate_up, (const bf16*)w_down, offsets, pair_of_slot, (bf16*)act, y, n_pairs,
                                n_real, top, hidden, ff, limit, alpha, up_offset, gated, (cudaStream_t)stream);
 }
 

@@ -975,22 +975,44 @@ moe_tensor_cores = True      # tests switch it off to run the fmaf tiles in bflo
 
 def moe_experts(h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, offsets: torch.Tensor, pair_of_slot: torch.Tensor,
                 act: torch.Tensor, y: torch.Tensor, n_pairs: int, n_real: int, top: int, ff: int, limit: float, alpha: float,
-                up_offset: float = 1.0, gated: bool = True) -> None:
+                up_offset: float = 1.0, gated: bool = True, rows: Optional[torch.Tensor] = None) -> None:
     """The experts' two products for the sorted pairs: act[slot] = g sigmoid(alpha g) (u + up_offset) with g = min(W_gate x, limit),
     u = clamp(W_up x, -limit, limit) (limit infinity, alpha 1, up_offset 0: SiLU(gate) * up), then y[slot] = W_down act[slot] (float32).  w_gate_up [n_real, 2 ff, hidden] (an
     expert's gate rows, then its up rows), w_down [n_real, hidden, ff].  `gated=False`: act[slot] = max(W_up x, 0)^2 with
-    w_gate_up [n_real, ff, hidden]."""
+    w_gate_up [n_real, ff, hidden].  `rows`: room for the pairs' rows of h [n_pairs, hidden] (allocated if needed and not given)."""
     hidden = h.shape[1]
     if w_gate_up.numel() != n_real * (2 if gated else 1) * ff * hidden or w_down.numel() != n_real * hidden * ff or act.numel() < n_pairs * ff \
             or y.numel() < n_pairs * hidden or y.dtype != torch.float32 or act.dtype != h.dtype or w_gate_up.dtype != h.dtype:
         raise KernelError("moe_experts: shapes do not fit")
     tensor_cores = h.dtype == torch.bfloat16 and hidden % 32 == 0 and ff % 32 == 0 and moe_tensor_cores
+    ptrs = [_dev(h, "h"), _dev(w_gate_up, "w_gate_up"), _dev(w_down, "w_down"), _dev(offsets, "offsets", torch.int32),
+            _dev(pair_of_slot, "pair_of_slot", torch.int32)]
+    numbers = [int(n_pairs), int(n_real), int(top), hidden, int(ff), float(limit), float(alpha), float(up_offset), int(bool(gated))]
+    kinds = [c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int]
+    if tensor_cores and moe_wide(n_pairs, n_real):
+        if rows is None:
+            rows = torch.empty(n_pairs, hidden, dtype=h.dtype, device=h.device)
+        if rows.numel() < n_pairs * hidden or rows.dtype != h.dtype:
+            raise KernelError("moe_experts: rows do not fit")
+        fn = _fn("moe_tcgen05.cu", "q3_moe_experts_tcgen05_bf16", [c_void_p] * 8 + kinds + [c_void_p, c_void_p])
+        _check(fn(*ptrs, _dev(rows, "rows"), _dev(act, "act"), _dev(y, "y"), *numbers, _status_word(h.device).data_ptr(), _stream()), "moe_experts")
+        _count_extra(2)
+        return
     name = "q3_moe_experts_tc_bf16" if tensor_cores else f"q3_moe_experts_{_suffix(h)}"
-    fn = _fn("moe.cu", name, [c_void_p] * 7 + [c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_void_p])
-    _check(fn(_dev(h, "h"), _dev(w_gate_up, "w_gate_up"), _dev(w_down, "w_down"), _dev(offsets, "offsets", torch.int32),
-              _dev(pair_of_slot, "pair_of_slot", torch.int32), _dev(act, "act"), _dev(y, "y"), int(n_pairs), int(n_real), int(top),
-              hidden, int(ff), float(limit), float(alpha), float(up_offset), int(bool(gated)), _stream()), "moe_experts")
+    fn = _fn("moe.cu", name, [c_void_p] * 7 + kinds + [c_void_p])
+    _check(fn(*ptrs, _dev(act, "act"), _dev(y, "y"), *numbers, _stream()), "moe_experts")
     _count_extra(1)
+
+
+def moe_wide(n_pairs: int, n_real: int) -> bool:
+    """Whether the experts' bfloat16 products run on tcgen05 tiles of many tokens (moe_tcgen05.cu) and not on the kernel for a
+    few tokens per expert: from MOE_WIDE_PAIRS pairs per expert on average."""
+    return n_pairs >= MOE_WIDE_PAIRS * n_real
+
+
+# Both forms, 16 experts, microseconds from cold caches (few / wide): 2 pairs per expert 77 / 103 at width 2,048 and 194 / 220 at
+# 4,096; 4 pairs 91 / 103 and 200 / 220; 6 pairs 108 / 103 and 265 / 241; 16 pairs 146 / 106 and 388 / 247.
+MOE_WIDE_PAIRS = 5
 
 
 def moe_combine(y: torch.Tensor, h: torch.Tensor, slot_of_pair: torch.Tensor, top_w: torch.Tensor, id_weight: torch.Tensor,

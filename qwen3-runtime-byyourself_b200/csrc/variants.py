@@ -22,6 +22,7 @@ def all_variants():
         ("lightning.cu", ()),
         ("differential.cu", ()),
         ("moe.cu", ()),
+        ("moe_tcgen05.cu", ()),
         ("attention_capped.cu", ("Q3_HEAD_DIM=64", "Q3_VALUE_DIM=128")),
         ("attention_capped.cu", ("Q3_HEAD_DIM=64", "Q3_VALUE_DIM=64")),
         ("stream_shift.cu", ()),

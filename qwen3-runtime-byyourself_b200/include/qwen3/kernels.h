@@ -319,10 +319,15 @@ int q3_moe_experts_f32(const void* h, const void* w_gate_up, const void* w_down,
 int q3_moe_experts_bf16(const void* h, const void* w_gate_up, const void* w_down, const int* offsets, const int* pair_of_slot,
                         void* act, float* y, int n_pairs, int n_real, int top, int hidden, int ff, float limit, float alpha,
                         float up_offset, int gated, void* stream);
-/* the same on the tensor cores: bfloat16, hidden and ff multiples of 32 */
+/* the same on the tensor cores, made for few pairs per expert: bfloat16, hidden and ff multiples of 32 */
 int q3_moe_experts_tc_bf16(const void* h, const void* w_gate_up, const void* w_down, const int* offsets, const int* pair_of_slot,
                            void* act, float* y, int n_pairs, int n_real, int top, int hidden, int ff, float limit, float alpha,
                            float up_offset, int gated, void* stream);
+/* the same on tcgen05 tiles, for more pairs per expert (moe_tcgen05.cu): hidden and ff multiples of 8; x [n_pairs, hidden]: room for
+   the pairs' rows of h; status: a device int that becomes non-zero if a bounded wait ran out */
+int q3_moe_experts_tcgen05_bf16(const void* h, const void* w_gate_up, const void* w_down, const int* offsets, const int* pair_of_slot,
+                                void* x, void* act, float* y, int n_pairs, int n_real, int top, int hidden, int ff, float limit,
+                                float alpha, float up_offset, int gated, int* status, void* stream);
 /* out[t] = sum_k top_w[t, k] y[slot_of_pair[t, k]] + id_weight[t] h[t] + shared_w[t] shared[t] (shared may be null; shared_w
    null: weight 1) */
 int q3_moe_combine_f32(const float* y, const void* h, const int* slot_of_pair, const float* top_w, const float* id_weight,

@@ -333,6 +333,53 @@ def test_router_scores_groups_choice_and_weights(outputs, real, top, groups, kee
         assert np.isclose(idw[t], sum(w_ for e, w_ in zip(chosen, weights) if e >= real), rtol=1e-5, atol=1e-7)
 
 
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("hidden,ff,counts", [(64, 32, [1]), (96, 160, [0, 3, 8, 9, 0, 1]), (160, 416, [16, 17, 0, 40, 63]),
+                                              (2048, 288, [64, 65, 0, 130, 257, 1]), (320, 128, [256, 300, 513, 0]),
+                                              (64, 64, [1, 0] * 20 + [7] * 30)])
+def test_experts_products_in_tiles_of_unequal_counts(hidden, ff, counts, gated, wide, monkeypatch):
+    """The two tensor-core forms of the experts' products at the edges of their tiles (pairs, features, K), with experts that
+    nobody chose and pairs without a slot, against 64 bits."""
+    import torch
+    from qwen3_b200.csrc import ops
+    monkeypatch.setattr(ops, "MOE_WIDE_PAIRS", 0 if wide else 10 ** 9)
+    rng = np.random.default_rng(hidden + ff)
+    n, top, idle = len(counts), 3, 2
+    slots = sum(counts)
+    pairs = -(-(slots + idle) // top) * top
+    h = torch.from_numpy(rng.standard_normal((pairs // top, hidden))).to("cuda", torch.bfloat16)
+    mats = 2 if gated else 1
+    w_up = torch.from_numpy(rng.standard_normal((n, mats * ff, hidden)) / np.sqrt(hidden)).to("cuda", torch.bfloat16)
+    w_down = torch.from_numpy(rng.standard_normal((n, hidden, ff)) / np.sqrt(ff)).to("cuda", torch.bfloat16)
+    offsets = torch.tensor(np.concatenate([[0], np.cumsum(counts)]), dtype=torch.int32, device="cuda")
+    order = torch.from_numpy(rng.permutation(pairs)[:slots]).to("cuda", torch.int32)
+    pair_of_slot = torch.cat([order, torch.zeros(pairs - slots, dtype=torch.int32, device="cuda")])
+    act = torch.full((pairs + 1, ff), 7.0, dtype=torch.bfloat16, device="cuda")
+    y = torch.full((pairs + 1, hidden), 7.0, dtype=torch.float32, device="cuda")
+    limit, alpha, off = (5.0, 1.702, 1.0) if hidden == 96 else (float("inf"), 1.0, 0.0)
+    ops.moe_experts(h, w_up, w_down, offsets, pair_of_slot, act, y, pairs, n, top, ff, limit, alpha, off, gated=gated)
+    assert ops.tcgen05_status("cuda") == 0
+    assert bool((act[slots:] == 7.0).all()) and bool((y[slots:] == 7.0).all())      # no slot, no row
+    x = h[(order // top).long()].double()
+    eps_up, eps_down = hidden * 2.0 ** -24, ff * 2.0 ** -24                       # sums of K terms in 32-bit, in any order
+    for e, (lo, hi) in enumerate(zip(offsets[:-1].tolist(), offsets[1:].tolist())):
+        if lo == hi:
+            continue
+        w = w_up[e].double()
+        z, dz = x[lo:hi] @ w.t(), eps_up * (x[lo:hi].abs() @ w.abs().t())
+        if gated:
+            g, u = z[:, :ff].clamp(max=limit), z[:, ff:].clamp(-limit, limit)
+            want = g * torch.sigmoid(alpha * g) * (u + off)
+            slack = 1.1 * dz[:, :ff] * (u + off).abs() + (g.abs() + dz[:, :ff]) * dz[:, ff:]
+        else:
+            want, slack = z.clamp(min=0).square(), 2 * z.abs() * dz + dz.square()
+        slack = slack + 2.0 ** -8 * want.abs() + 2.0 ** -20 * want.abs() + 1e-30      # rounded to bfloat16, expf and division
+        assert bool(((act[lo:hi].double() - want).abs() <= slack).all()), e
+        a, wd = act[lo:hi].double(), w_down[e].double()
+        assert bool(((y[lo:hi].double() - a @ wd.t()).abs() <= eps_down * (a.abs() @ wd.abs().t()) + 1e-30).all()), e
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("hidden,ff", [(72, 40), (96, 64)])
 @pytest.mark.parametrize("N", [1, 7, 33, 300])
