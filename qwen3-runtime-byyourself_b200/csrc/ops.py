@@ -1595,14 +1595,17 @@ def side_gate(a: torch.Tensor, ids: torch.Tensor, table: torch.Tensor, out: torc
 
 # ------------------------------------------------------------------ linear attention whose forget gate also writes (HGRN2)
 def gated_scan(proj: torch.Tensor, state: torch.Tensor, low: torch.Tensor, bias: torch.Tensor, seq_start: torch.Tensor,
-               seq_slots: torch.Tensor, out: torch.Tensor, n_seqs: int, heads: int, d: int, vd: int) -> torch.Tensor:
+               seq_slots: torch.Tensor, out: torch.Tensor, n_seqs: int, heads: int, d: int, vd: int,
+               single: bool = False) -> torch.Tensor:
     """f = low + (1 - low) sigmoid(z + bias), S_t = diag(f_t) S_(t-1) + (1 - f_t) v_t^T, o_t = S_t^T SiLU(q_t) over the new
     tokens of every sequence, from and to the state rows [slot, heads, d, vd] (float32).  `proj` [N, heads (2 d + vd)]
-    holds q, z and v head by head; `out` [N, heads * vd] float32."""
+    holds q, z and v head by head; `out` [N, heads * vd] float32.  `single`: no sequence brings more than one token (a kernel of
+    its own, the same bits)."""
     if proj.shape[1] != heads * (2 * d + vd) or tuple(state.shape[1:]) != (heads, d, vd) or out.shape[1] != heads * vd \
             or out.dtype != torch.float32 or low.numel() != heads * d or bias.numel() != heads * d:
         raise KernelError("gated_scan: shapes do not fit")
-    fn = _fn("gated_recurrence.cu", f"q3_gated_scan_{_suffix(proj)}", [c_void_p] * 7 + [c_int, c_int, c_int, c_int, c_void_p])
+    kernel = "step" if single and d % 8 == 0 and vd % 4 == 0 else "scan"
+    fn = _fn("gated_recurrence.cu", f"q3_gated_{kernel}_{_suffix(proj)}", [c_void_p] * 7 + [c_int, c_int, c_int, c_int, c_void_p])
     _check(fn(_dev(proj, "proj"), _dev(state, "state", torch.float32), _dev(low, "low", torch.float32),
               _dev(bias, "bias", torch.float32), _dev(seq_start, "seq_start", torch.int32),
               _dev(seq_slots, "seq_slots", torch.int32), _dev(out, "out"), int(n_seqs), heads, d, vd, _stream()), "gated_scan")

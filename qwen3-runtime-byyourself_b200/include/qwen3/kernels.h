@@ -364,6 +364,11 @@ int q3_gated_scan_f32(const void* proj, float* state, const float* low, const fl
                       const int* seq_slots, float* out, int n_seqs, int heads, int d, int vd, void* stream);
 int q3_gated_scan_bf16(const void* proj, float* state, const float* low, const float* bias, const int* seq_start,
                        const int* seq_slots, float* out, int n_seqs, int heads, int d, int vd, void* stream);
+/* the same for at most one token per sequence: d a multiple of 8, vd of 4 */
+int q3_gated_step_f32(const void* proj, float* state, const float* low, const float* bias, const int* seq_start,
+                      const int* seq_slots, float* out, int n_seqs, int heads, int d, int vd, void* stream);
+int q3_gated_step_bf16(const void* proj, float* state, const float* low, const float* bias, const int* seq_start,
+                       const int* seq_slots, float* out, int n_seqs, int heads, int d, int vd, void* stream);
 /* out = o / sqrt(mean(o^2) + eps) * w over every run of vd values (n_rows runs) */
 int q3_head_rms_norm_f32(const float* o, const float* w, void* out, int64_t n_rows, int vd, float eps, void* stream);
 int q3_head_rms_norm_bf16(const float* o, const float* w, void* out, int64_t n_rows, int vd, float eps, void* stream);

@@ -61,7 +61,8 @@ class GatedRecurrence(Part):
         proj = ctx.scratch.get("recurrence.proj", (N, h * (2 * d + vd)), ctx.dtype)
         linear(x, self.w_in, proj)
         o = ctx.scratch.get("recurrence.o", (N, h * vd), torch.float32)
-        ops.gated_scan(proj, cache.state, self.low, self.bias, ctx.seq_start, ctx.seq_slots, o, ctx.n_seqs, h, d, vd)
+        ops.gated_scan(proj, cache.state, self.low, self.bias, ctx.seq_start, ctx.seq_slots, o, ctx.n_seqs, h, d, vd,
+                       single=ctx.max_new == 1)
         normed = ctx.scratch.get("recurrence.normed", (N, h * vd), ctx.dtype)
         ops.head_rms_norm(o, self.norm_weight, self.eps, normed, vd)
         out = ctx.scratch.get("mixer.out", (N, self.hidden_size), ctx.dtype)

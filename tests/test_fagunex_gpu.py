@@ -195,6 +195,28 @@ def test_gated_recurrence_over_unequal_sequences_and_from_its_state(dtype, heads
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,d,vd,n", [(2, 8, 4, 3), (1, 64, 100, 5), (3, 48, 64, 2), (16, 128, 128, 9), (1, 256, 256, 1), (2, 256, 36, 4)])
+def test_single_tokens_of_the_recurrence_give_the_scan_s_bits(dtype, heads, d, vd, n):
+    """The kernel for steps of single tokens, with partial tiles of columns and groups of rows: outputs and states of the scan, to
+    the bit; a sequence without a token and slots without a sequence stay as they are."""
+    import torch
+    from qwen3_b200.csrc import ops
+    rng = np.random.default_rng(d * vd + n)
+    T = torch_dtype(dtype)
+    low, bias = dev(rng.uniform(0, 0.95, heads * d), torch.float32), dev(rng.standard_normal(heads * d), torch.float32)
+    proj = dev(rng.standard_normal((n, heads * (2 * d + vd))), T)
+    slots = dev(rng.permutation(n + 3)[:n + 1], torch.int32)
+    start = dev(list(range(n)) + [n, n], torch.int32)                         # the last sequence brings nothing
+    first = dev(rng.standard_normal((n + 3, heads, d, vd)), torch.float32)
+    got = []
+    for single in (False, True):
+        state, out = first.clone(), torch.full((n, heads * vd), 9.0, dtype=torch.float32, device="cuda")
+        ops.gated_scan(proj, state, low, bias, start, slots, out, n + 1, heads, d, vd, single=single)
+        got.append((state, out))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("vd", [1, 9, 32, 200])
 def test_unit_rms_per_head_with_one_weight_for_all_heads(dtype, vd):
     import torch
