@@ -34,8 +34,9 @@ class KernelError(RuntimeError):
 # steps of an 8B-sized model, the TMA + tcgen05 products gain 2.5-5 % at batches of 16 to 64 (4.92 -> 4.74 ms a
 # step at batch 16), while the few-row product loses (batch 8: chains of waiting blocks take the room that a kernel's
 # own later waves need) and the decode attention, which asks for its first pages before it waits, gains 0.5 % at batch
-# 16 and 32 and loses 0.3 % at batch 64.  QWEN3_B200_PDL=1 / =0 turns it on / off for all.
-PDL_SOURCES = ("gemm_tcgen05.cu",)
+# 16 and 32 and loses 0.3 % at batch 64; its form for many sequences, which stands between such products, gains 1.5 % at batch 64
+# (1526 -> 1503 us a step of 12 layers).  QWEN3_B200_PDL=1 / =0 turns it on / off for all.
+PDL_SOURCES = ("gemm_tcgen05.cu", "attention_decode_flat.cu")
 _pdl_override = {"1": True, "0": False}.get(os.environ.get("QWEN3_B200_PDL", ""))
 _libs = {}
 
@@ -1232,16 +1233,37 @@ def attention_decode_fused_max_splits(d: int, device) -> int:
 
 def attention_decode_fused(qkv, k_pages, v_pages, out, q_norm_w, k_norm_w, cos, sin, eps: float, token_seq, token_pos,
                            page_table, n_tokens: int, nq: int, nkv: int, d: int, scale: float, window: Optional[int],
-                           n_splits: int, write_kv: bool = True):
+                           n_splits: int, write_kv: bool = True, parts: Optional[torch.Tensor] = None,
+                           counters: Optional[torch.Tensor] = None):
     """The attention of a decode step in one launch: per-head norm and rotation of the new query and key, the
     write of key and value into the cache pages, attention over the pages split over the keys, and the merge of
-    the splits inside a thread-block cluster.  `qkv` is the projection output [tokens, (nq + 2 nkv) * d]."""
+    the splits inside a thread-block cluster.  `qkv` is the projection output [tokens, (nq + 2 nkv) * d].
+
+    With `parts` and `counters` (float32 and int32 [n_tokens * nkv], the latter zero and left zero; head sizes
+    `attention_decode_flat_fits`) the pages of the whole step are shared out evenly over the GPU, `n_splits` aside."""
     if qkv.dtype != torch.bfloat16:
         raise KernelError("attention_decode_fused is a bfloat16 kernel")
     if nq // nkv > 16 or d % 16 != 0 or d > 256 or not 0 < n_splits <= FUSED_DECODE_MAX_SPLITS:
         raise KernelError(f"attention_decode_fused: group of {nq // nkv} heads, head_dim {d} or {n_splits} splits not supported")
     if qkv.shape[-1] != (nq + 2 * nkv) * d or k_pages.shape[1:] != (nkv, PAGE_TOKENS, d) or out.shape[-1] != nq * d:
         raise KernelError("attention_decode_fused: shapes do not fit")
+    if parts is not None:
+        if not attention_decode_flat_fits(d, nq // nkv) or v_pages.shape != k_pages.shape or counters is None or counters.numel() < n_tokens * nkv \
+                or parts.numel() < attention_decode_flat_parts(d, nq // nkv):
+            raise KernelError("attention_decode_fused: head size, pages, parts or counters do not fit")
+        fn = _fn("attention_decode_flat.cu", "q3_attention_decode_flat_bf16",
+                 [c_void_p] * 10 + [c_float] + [c_void_p] * 3 + [c_int, c_int64, c_int64, c_int, c_int, c_float, c_int, c_int, c_int,
+                                                                 c_void_p, c_void_p],
+                 defines=(f"Q3_HEAD_DIM={d}",))
+        _check(fn(_dev(qkv, "qkv"), _dev(k_pages, "k_pages", torch.bfloat16), _dev(v_pages, "v_pages", torch.bfloat16),
+                  _dev(out, "out", torch.bfloat16), _dev(parts, "parts", torch.float32), _dev(counters, "counters", torch.int32),
+                  _ptr(q_norm_w, "q_norm_w", torch.float32), _ptr(k_norm_w, "k_norm_w", torch.float32),
+                  _ptr(cos, "cos", torch.float32), _ptr(sin, "sin", torch.float32), float(eps),
+                  _dev(token_seq, "token_seq", torch.int32), _dev(token_pos, "token_pos", torch.int32),
+                  _dev(page_table, "page_table", torch.int32), page_table.shape[-1], n_tokens, k_pages.shape[0], nq, nkv,
+                  float(scale), int(window or 0), int(bool(write_kv)), _rotary_dim(cos, sin, d),
+                  _status_word(qkv.device).data_ptr(), _stream()), "attention_decode_fused")
+        return out
     fn = _fn("attention_decode.cu", "q3_attention_decode_fused_bf16",
              [c_void_p] * 8 + [c_float] + [c_void_p] * 3 + [c_int, c_int64, c_int, c_int, c_float, c_int, c_int, c_int, c_int,
                                                             c_void_p],
@@ -1253,6 +1275,18 @@ def attention_decode_fused(qkv, k_pages, v_pages, out, q_norm_w, k_norm_w, cos, 
               _dev(page_table, "page_table", torch.int32), page_table.shape[-1], n_tokens, nq, nkv, float(scale),
               int(window or 0), int(n_splits), int(bool(write_kv)), _rotary_dim(cos, sin, d), _stream()), "attention_decode_fused")
     return out
+
+
+def attention_decode_flat_fits(d: int, group: int) -> bool:
+    """Head sizes and query heads per kv head of the form that shares out the pages of a whole step."""
+    return d in (64, 128) and group <= 8
+
+
+def attention_decode_flat_parts(d: int, group: int) -> int:
+    """Float32 elements of the `parts` buffer of `attention_decode_fused`."""
+    fn = _fn_untimed("attention_decode_flat.cu", "q3_attention_decode_flat_parts", [c_int], defines=(f"Q3_HEAD_DIM={d}",))
+    fn.restype = c_int64
+    return int(fn(group))
 
 
 # ------------------------------------------------------------------ bfloat16 weight-streaming product

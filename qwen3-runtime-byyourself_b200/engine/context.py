@@ -39,6 +39,19 @@ class Scratch:
             self._flat[key] = flat
         return flat[:numel].view(*shape)
 
+    def counters(self, name: str, numel: int) -> torch.Tensor:
+        """`numel` int32 that were zero when the buffer was made and that every kernel leaves as it found them."""
+        key = (name, "counters", numel if self.guard else 0)
+        flat = self._flat.get(key)
+        if flat is None or flat.numel() < numel:
+            if self.guard:
+                flat = self._guarded(name, numel, torch.int32)
+                flat.zero_()
+            else:
+                flat = torch.zeros(max(numel, 64), dtype=torch.int32, device=self.device)
+            self._flat[key] = flat
+        return flat[:numel]
+
     def _guarded(self, name: str, numel: int, dtype: torch.dtype) -> torch.Tensor:
         key = (name, dtype, numel)
         flat = self._flat.get(key)

@@ -198,6 +198,16 @@ int q3_attention_decode_fused_bf16(const void* qkv, void* k_pages, void* v_pages
                                    const float* k_norm_w, const float* cos_tab, const float* sin_tab, float eps, const int* token_seq,
                                    const int* token_pos, const int* page_table, int pages_per_seq, int64_t n_tokens, int nq, int nkv,
                                    float scale, int window, int n_splits, int write_kv, int rotary_dim, void* stream);
+/* attention_decode_flat.cu: the same for head sizes 64 and 128 and groups of up to 8 query heads, the pages of the whole step shared
+   out over `blocks` blocks; parts: q3_attention_decode_flat_parts(group) floats; counters: n_tokens * nkv ints, zero before the first
+   launch and left zero; status: a device int that becomes non-zero if a bounded wait ran out */
+int q3_attention_decode_flat_blocks(int group);
+int64_t q3_attention_decode_flat_parts(int group);
+int q3_attention_decode_flat_bf16(const void* qkv, void* k_pages, void* v_pages, void* out, float* parts, int* counters,
+                                  const float* q_norm_w, const float* k_norm_w, const float* cos_tab, const float* sin_tab, float eps,
+                                  const int* token_seq, const int* token_pos, const int* page_table, int pages_per_seq,
+                                  int64_t n_tokens, int64_t n_cache_pages, int nq, int nkv, float scale, int window, int write_kv,
+                                  int rotary_dim, int* status, void* stream);
 
 /* ---- attention_prefill.cu, attention_prefill_tc.cu (-DQ3_HEAD_DIM): prompts, bfloat16 --------------------- */
 int q3_attention_prefill_head_dim(void);

@@ -930,3 +930,52 @@ def test_prefill_attention_tcgen05_kernel(nq, nkv, d):
         want = plain.gqa_attention(qs, ks, vs).reshape(n, nq * d)
         err = np.abs(got[s] - want).max(axis=1)
         assert err.max() <= 2e-2, f"sequence {s}: row {int(err.argmax())} of {n}: max abs err {err.max():.3e}"
+
+
+@pytest.mark.parametrize("nq,nkv,d,lengths,window", [
+    (8, 2, 128, [1], None), (8, 8, 64, [64, 65, 1, 63], None), (8, 1, 128, [130, 700, 20000], None), (10, 2, 128, [3, 2, 1], None),
+    (12, 4, 64, list(range(1, 700, 17)), None), (32, 8, 128, [200 + 61 * i for i in range(9)], None), (8, 2, 128, [5000, 70, 9], 100)])
+def test_decode_attention_with_pages_shared_out(nq, nkv, d, lengths, window):
+    """The pages of a step shared out evenly: rows cut over many blocks, rows of one page, more rows than blocks and fewer,
+    windows.  Each weight enters the second product rounded to bfloat16, which moves it by 2^-8 of itself at most, and the result
+    is rounded once more: within 2^-7 (1 + 2^-8) sum(p |v|) of float64; the same bits when run again, the same cache rows as the form that splits every row alike,
+    and counters that are zero again."""
+    from qwen3_b200.csrc import ops
+    rng = np.random.default_rng(len(lengths) + d)
+    table, kp, vp = paged_case(rng, lengths, nkv, d, "bfloat16")
+    gen = torch.Generator(device="cuda").manual_seed(nq + d)
+    kp.normal_(generator=gen)
+    vp.normal_(generator=gen)
+    B, table_d = len(lengths), torch.as_tensor(table).cuda()
+    qkv = torch.randn(B, (nq + 2 * nkv) * d, generator=gen, device="cuda").to(torch.bfloat16)
+    seq = torch.arange(B, dtype=torch.int32, device="cuda")
+    pos = torch.as_tensor([n - 1 for n in lengths], dtype=torch.int32).cuda()
+    parts = torch.empty(ops.attention_decode_flat_parts(d, nq // nkv), dtype=torch.float32, device="cuda")
+    counters = torch.zeros(B * nkv, dtype=torch.int32, device="cuda")
+    cos, sin = (dev(x, "float32") for x in plain.rope_table(max(lengths), d, 50000.0))
+    norm = torch.ones(d, dtype=torch.float32, device="cuda")
+    for form in ((None, None, None, None), (norm, norm, cos, sin)):
+        args = (*form, 1e-5, seq, pos, table_d, B, nq, nkv, d, d ** -0.5, window)
+        k1, v1, k2, v2 = kp.clone(), vp.clone(), kp.clone(), vp.clone()
+        out = [torch.empty(B, nq * d, dtype=torch.bfloat16, device="cuda") for _ in range(3)]
+        ops.attention_decode_fused(qkv, k1, v1, out[0], *args, 3)
+        for o in out[1:]:
+            ops.attention_decode_fused(qkv, k2, v2, o, *args, 3, parts=parts, counters=counters)
+        assert ops.tcgen05_status("cuda:0") == 0 and not counters.any()
+        assert torch.equal(k1, k2) and torch.equal(v1, v2) and torch.equal(out[1], out[2])
+        kept = torch.full_like(out[0], 7.0)
+        ops.attention_decode_fused(qkv, k1, v1, kept, *args, 3, write_kv=False, parts=parts, counters=counters)
+        assert torch.equal(k1, k2) and torch.equal(kept, out[1])
+        assert float((out[0].float() - out[1].float()).abs().max()) <= 2.5e-2
+        if form[0] is not None:
+            continue
+        for s, n in enumerate(lengths):
+            pages = table_d[s, :-(-n // 64)].long()
+            lo = max(0, n - window) if window else 0
+            ks, vs = (x[pages].double().transpose(1, 2).reshape(-1, nkv, d)[lo:n].transpose(0, 1) for x in (k2, v2))
+            q = qkv[s, :nq * d].double().view(nkv, nq // nkv, d)
+            p = torch.softmax(q @ ks.transpose(1, 2) * d ** -0.5, dim=-1)
+            bound = 2.0 ** -7 * (1 + 2.0 ** -8) * (p @ vs.abs()) + 1e-6
+            assert bool(((out[1][s].double().view(nkv, nq // nkv, d) - p @ vs).abs() <= bound).all()), (s, n)
+    with pytest.raises(ops.KernelError):
+        ops.attention_decode_fused(qkv, k1, v1, kept, *args, 3, parts=parts, counters=counters[:-1])
