@@ -425,6 +425,120 @@ attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_pages,
         if (tid + n * 128 < vd) o[tid + n * 128] = from_f32<T>(acc[n] / l_run);
 }
 
+// The plain form in 32-bit (no cap, chunks, sink, biases, pooled blocks or first keys; values as wide as keys), for heads of
+// up to 256 in steps of 4.  One block per (query head, token) as above, but the eight warps meet once, at the end: LPK
+// lanes hold a key (and a value) in packets of 16 bytes, a warp takes 8 keys of a page, all of whose keys and values are
+// asked for together, and every group of LPK lanes keeps a maximum, a sum and an output of its own.  With one new token a
+// sequence the general form is a chain of about 17 us a page - each key's sum over a warp, three barriers, 64
+// serial steps over the values.  Decode of 3 sequences of up to 157 tokens, 32 heads of 128: 54 us there, 10 here; 4 of
+// up to 76 tokens, 8 heads of 32: 17.9 and 3.0; prompts of 183 tokens in all, 32 heads of 128: 96 and 57.  The order of the sums depends on the position alone, not on the step.
+constexpr int PLAIN_WARPS = 8, PLAIN_KEYS = PAGE / PLAIN_WARPS;      // keys of a page that a warp takes
+
+template <int LPK, int CH>
+__global__ void __launch_bounds__(PLAIN_WARPS * 32)
+attention_plain_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages,
+                       float* __restrict__ out, const int* __restrict__ token_seq, const int* __restrict__ token_pos,
+                       const int* __restrict__ page_table, int pages_per_seq, int nq, int nkv, int d, float scale, int window) {
+    constexpr int SUBS = 32 / LPK, U = PLAIN_KEYS / SUBS, STATES = PLAIN_WARPS * SUBS;
+    static_assert(U >= 1 && U * SUBS == PLAIN_KEYS, "a warp's keys of a page are shared out among its groups of lanes");
+    extern __shared__ __align__(16) float plain_smem[];                  // [STATES][d], then (max, sum) [STATES][2]
+    pdl_launch_dependents();
+    pdl_wait();
+    const int head = blockIdx.x, kvh = head / (nq / nkv);
+    const int64_t t = blockIdx.y;
+    const int pos = token_pos[t], lo = window > 0 ? max(0, pos - window + 1) : 0;
+    const int* pages = page_table + (int64_t)token_seq[t] * pages_per_seq;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / LPK, c = lane % LPK;
+    bool in[CH];
+    float4 q4[CH], acc[CH];
+#pragma unroll
+    for (int n = 0; n < CH; ++n) {
+        in[n] = (c + n * LPK) * 4 < d;
+        q4[n] = in[n] ? *reinterpret_cast<const float4*>(q + (t * nq + head) * (int64_t)d + (c + n * LPK) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        acc[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float m_run = -INFINITY, l_run = 0.0f;
+    for (int pg = lo / PAGE; pg <= pos / PAGE; ++pg) {
+        const int64_t base = ((int64_t)pages[pg] * nkv + kvh) * PAGE * d;
+        const int j0 = warp * PLAIN_KEYS + sub;
+        float4 k4[U][CH], v4[U][CH];
+        bool seen[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int j = j0 + u * SUBS, key = pg * PAGE + j;
+            seen[u] = key >= lo && key <= pos;
+#pragma unroll
+            for (int n = 0; n < CH; ++n) {
+                const int64_t at = base + (int64_t)j * d + (c + n * LPK) * 4;
+                k4[u][n] = seen[u] && in[n] ? *reinterpret_cast<const float4*>(k_pages + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v4[u][n] = seen[u] && in[n] ? *reinterpret_cast<const float4*>(v_pages + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+        float dot[U], m_new = m_run;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            dot[u] = 0.0f;
+#pragma unroll
+            for (int n = 0; n < CH; ++n)
+                dot[u] = fmaf(q4[n].w, k4[u][n].w, fmaf(q4[n].z, k4[u][n].z, fmaf(q4[n].y, k4[u][n].y, fmaf(q4[n].x, k4[u][n].x, dot[u]))));
+#pragma unroll
+            for (int o = LPK / 2; o > 0; o >>= 1) dot[u] += __shfl_xor_sync(0xffffffffu, dot[u], o);
+            dot[u] = seen[u] ? dot[u] * scale : -INFINITY;
+            m_new = fmaxf(m_new, dot[u]);
+        }
+        if (m_new == -INFINITY) continue;                                // these lanes have seen no key yet
+        const float alpha = expf(m_run - m_new);
+        l_run *= alpha;
+#pragma unroll
+        for (int n = 0; n < CH; ++n) { acc[n].x *= alpha; acc[n].y *= alpha; acc[n].z *= alpha; acc[n].w *= alpha; }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const float p = expf(dot[u] - m_new);
+            l_run += p;
+#pragma unroll
+            for (int n = 0; n < CH; ++n) {
+                acc[n].x = fmaf(p, v4[u][n].x, acc[n].x);
+                acc[n].y = fmaf(p, v4[u][n].y, acc[n].y);
+                acc[n].z = fmaf(p, v4[u][n].z, acc[n].z);
+                acc[n].w = fmaf(p, v4[u][n].w, acc[n].w);
+            }
+        }
+        m_run = m_new;
+    }
+    const int mine = warp * SUBS + sub;
+    float* ml = plain_smem + STATES * d;
+#pragma unroll
+    for (int n = 0; n < CH; ++n)
+        if (in[n]) *reinterpret_cast<float4*>(plain_smem + mine * d + (c + n * LPK) * 4) = acc[n];
+    if (c == 0) {
+        ml[2 * mine] = m_run;
+        ml[2 * mine + 1] = l_run;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < d; i += PLAIN_WARPS * 32) {
+        float m = -INFINITY, l = 0.0f, o = 0.0f;
+#pragma unroll
+        for (int w = 0; w < STATES; ++w) m = fmaxf(m, ml[2 * w]);
+#pragma unroll
+        for (int w = 0; w < STATES; ++w) {
+            const float f = expf(ml[2 * w] - m);                         // 0 where no key was seen
+            l = fmaf(f, ml[2 * w + 1], l);
+            o = fmaf(f, plain_smem[w * d + i], o);
+        }
+        out[(t * nq + head) * (int64_t)d + i] = o / l;
+    }
+}
+
+template <int LPK, int CH>
+int attention_plain_launch(const float* q, const float* k_pages, const float* v_pages, float* out, const int* token_seq,
+                           const int* token_pos, const int* page_table, int pages_per_seq, int64_t n_tokens, int nq, int nkv, int d,
+                           float scale, int window, cudaStream_t stream) {
+    constexpr int STATES = PLAIN_WARPS * (32 / LPK);                     // 32 KB at most: heads of 16 in 64 states, of 256 in 8
+    return (int)q3_launch(attention_plain_kernel<LPK, CH>, dim3(nq, (unsigned)n_tokens), dim3(PLAIN_WARPS * 32),
+                          (size_t)(STATES * (d + 2) * 4), stream, q, k_pages, v_pages, out, token_seq, token_pos, page_table,
+                          pages_per_seq, nq, nkv, d, scale, window);
+}
+
 template <typename T>
 int qkv_prepare_launch(const T* qkv, T* q_out, T* k_pages, T* v_pages, const float* q_norm_w, const float* k_norm_w,
                        const float* cos_tab, const float* sin_tab, const int* token_seq, const int* token_pos,
@@ -479,6 +593,21 @@ int attention_generic_launch(const T* q, const T* k_pages, const T* v_pages, T* 
     if (d <= 0 || d > GENERIC_KEY_DIM || vd > GENERIC_VALUE_DIM || nq <= 0 || nkv <= 0 || nq % nkv != 0) return Q3_ERR_BAD_SIZE;
     if ((window > 0 && chunk > 0) || keep_first < 0) return Q3_ERR_BAD_SIZE;
     if (n_tokens > 65535) return Q3_ERR_TOO_LARGE;
+    if constexpr (sizeof(T) == 4) {
+        const bool plain = !(softcap > 0.0f) && chunk <= 0 && !sink && keep_first <= 0 && pool.size == 0 && bias.table == nullptr && vd == d &&
+                           nv == nkv;
+        if (plain && d % 4 == 0 && d <= 256 && aligned16(q) && aligned16(k_pages) && aligned16(v_pages)) {
+#define Q3_PLAIN(LPK, CH)                                                                                                             \
+    return attention_plain_launch<LPK, CH>(q, k_pages, v_pages, out, token_seq, token_pos, page_table, pages_per_seq, n_tokens, nq,   \
+                                           nkv, d, scale, window, stream)
+            if (d <= 16) Q3_PLAIN(4, 1);
+            if (d <= 32) Q3_PLAIN(8, 1);
+            if (d <= 64) Q3_PLAIN(16, 1);
+            if (d <= 128) Q3_PLAIN(32, 1);
+            Q3_PLAIN(32, 2);
+#undef Q3_PLAIN
+        }
+    }
     const dim3 grid(nq, (unsigned)n_tokens);
     return (int)q3_launch(attention_generic_kernel<T>, grid, dim3(128), 0, stream, q, k_pages, v_pages, out, token_seq,
                           token_pos, page_table, pages_per_seq, nq, nkv, d, scale, window, vd, softcap, chunk, sink, nv, out_f32, sink_values,

@@ -979,3 +979,36 @@ def test_decode_attention_with_pages_shared_out(nq, nkv, d, lengths, window):
             assert bool(((out[1][s].double().view(nkv, nq // nkv, d) - p @ vs).abs() <= bound).all()), (s, n)
     with pytest.raises(ops.KernelError):
         ops.attention_decode_fused(qkv, k1, v1, kept, *args, 3, parts=parts, counters=counters[:-1])
+
+
+@pytest.mark.parametrize("nq,nkv,d,lengths,window", [
+    (4, 2, 4, [1, 65], None), (3, 3, 12, [130], None), (8, 1, 32, [76, 21, 45, 13], None), (6, 2, 48, [64, 63], 17), (5, 5, 80, [200], None),
+    (8, 8, 128, [157, 53, 1], None), (2, 1, 132, [129], 64), (4, 2, 256, [300, 2], None)])
+def test_plain_attention_in_32_bit(nq, nkv, d, lengths, window):
+    """The 32-bit attention without options against the general kernel, which runs with biases of zero, and against
+    float64: a few hundred sums of products of size 1, 2^-24 each; a token's output does not depend on the step it is in."""
+    from qwen3_b200.csrc import ops
+    rng = np.random.default_rng(d)
+    table, kp, vp = paged_case(rng, lengths, nkv, d, "float32")
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    kp.normal_(generator=gen)
+    vp.normal_(generator=gen)
+    seq = torch.as_tensor(np.concatenate([np.full(n, s) for s, n in enumerate(lengths)]).astype(np.int32)).cuda()
+    pos = torch.as_tensor(np.concatenate([np.arange(n) for n in lengths]).astype(np.int32)).cuda()
+    N, table_d = len(pos), torch.as_tensor(table).cuda()
+    q = torch.randn(N, nq * d, generator=gen, device="cuda")
+    out, general = torch.empty_like(q), torch.empty_like(q)
+    ops.attention_generic(q, kp, vp, out, seq, pos, table_d, N, nq, nkv, d, d ** -0.5, window)
+    ops.attention_generic(q, kp, vp, general, seq, pos, table_d, N, nq, nkv, d, d ** -0.5, window, bias=torch.zeros(nq, 1, device="cuda"))
+    assert float((out - general).abs().max()) <= 1e-5
+    last = np.cumsum(lengths) - 1
+    for s, n in enumerate(lengths):
+        i, lo = int(last[s]), max(0, n - window) if window else 0
+        pages = table_d[s, :-(-n // 64)].long()
+        ks, vs = (x[pages].double().transpose(1, 2).reshape(-1, nkv, d)[lo:n].transpose(0, 1) for x in (kp, vp))
+        p = torch.softmax(q[i].double().view(nkv, nq // nkv, d) @ ks.transpose(1, 2) * d ** -0.5, dim=-1)
+        assert float((out[i].double().view(nkv, nq // nkv, d) - p @ vs).abs().max()) <= 1e-5
+        one = torch.empty(1, nq * d, device="cuda")
+        ops.attention_generic(q[i:i + 1].contiguous(), kp, vp, one, torch.full((1,), s, dtype=torch.int32, device="cuda"),
+                              pos[i:i + 1].contiguous(), table_d, 1, nq, nkv, d, d ** -0.5, window)
+        assert torch.equal(one[0], out[i])
