@@ -333,6 +333,29 @@ def test_router_scores_groups_choice_and_weights(outputs, real, top, groups, kee
         assert np.isclose(idw[t], sum(w_ for e, w_ in zip(chosen, weights) if e >= real), rtol=1e-5, atol=1e-7)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("hidden,top", [(8, 1), (12, 2), (20, 3), (2048, 2), (4096 + 8, 2)])
+def test_combining_in_packets_and_value_by_value(dtype, hidden, top):
+    """Rows of whole packets and rows that are not, pairs without a slot, tokens with and without an identity weight."""
+    import torch
+    from qwen3_b200.csrc import ops
+    rng = np.random.default_rng(hidden)
+    N, T = 5, torch.float32 if dtype == "float32" else torch.bfloat16
+    y, w, idw, sw = (dev(rng.standard_normal(shape), torch.float32) for shape in ((N * top, hidden), (N * top,), (N,), (N,)))
+    h, shared = dev(rng.standard_normal((N, hidden)), T), dev(rng.standard_normal((N, hidden)), T)
+    slots = dev(rng.permutation(N * top), torch.int32)
+    slots[1], idw[0] = -1, 0.0
+    for has_shared, weighted in ((False, False), (True, False), (True, True)):
+        out = torch.empty_like(h)
+        ops.moe_combine(y, h, slots, w, idw, out, top, shared if has_shared else None, sw if weighted else None)
+        rows = torch.where((slots >= 0)[:, None], y[slots.clamp(min=0).long()].double(), 0.0) * w.double()[:, None]
+        want = rows.view(N, top, hidden).sum(1) + idw.double()[:, None] * h.double()
+        if has_shared:
+            want = want + (sw.double()[:, None] if weighted else 1.0) * shared.double()
+        bound = 2.0 ** -20 * want.abs().max() + (2.0 ** -8 * want.abs() if dtype != "float32" else 0.0)
+        assert bool(((out.double() - want).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("wide", [False, True])
 @pytest.mark.parametrize("gated", [True, False])
 @pytest.mark.parametrize("hidden,ff,counts", [(64, 32, [1]), (96, 160, [0, 3, 8, 9, 0, 1]), (160, 416, [16, 17, 0, 40, 63]),
