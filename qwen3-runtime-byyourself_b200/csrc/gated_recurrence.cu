@@ -16,6 +16,8 @@
 //                   into shared memory between the two barriers of a stage, so a token costs no barrier of its own
 //                   and no wait for global memory.  The launch depends on the sizes only, never on the step: a
 //                   token's output is the same bits however the sequence was cut.  Gate, state and o are 32-bit whatever T.
+//   gated_scan_wide : the same sums to the bit for d and vd multiples of 8: a thread has 8 rows of four columns, two rows
+//                   at a time in the paired 32-bit arithmetic of this architecture.
 //   gated_step    : the same for a step in which every sequence brings one token, with the same sums to the bit.
 //   head_rms_norm : out = T( o / sqrt(mean(o^2) + eps) * w ) over the vd values of every (token, head); one weight
 //                   vector for all heads.
@@ -171,6 +173,209 @@ gated_scan_kernel(const T* __restrict__ proj, float* __restrict__ state, const f
     }
 }
 
+// The scan for states of whole packets.  The tokens of a sequence are a serial chain, so the length of a token's step counts:
+// the threads that walk the state do nothing else, and as many helpers fetch and activate the stage after and add up the
+// outputs of the stage before, with one barrier a stage.  A walker has eight rows of four columns, so that a gate or query
+// value read from shared memory serves four, and takes rows in pairs (fma.rn.f32x2: each half is the scalar operation, so a
+// pair of rows holds the two chains of a column's sum as they are).  The longest sequences start first.
+// Prompts of 2,048 + 911 + 1,203 tokens, 32 heads of 128 x 128: 1,058 us by threads of one column that do everything, 490 here.
+__device__ __forceinline__ uint64_t two(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void one_each(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+constexpr int WIDE_STAGE = 8;     // tokens fetched together
+constexpr int WIDE_PACKETS = 5;   // packets of them a helper holds
+constexpr int WIDE_TILE = 32;     // columns of the state per block
+
+template <typename T>
+__global__ void __launch_bounds__(512)
+gated_scan_wide_kernel(const T* __restrict__ proj, float* __restrict__ state, const float* __restrict__ low, const float* __restrict__ bias,
+                       const int* __restrict__ seq_start, const int* __restrict__ seq_slots, float* __restrict__ out, int H, int d, int vd,
+                       int n_seqs, int walkers) {
+    constexpr int P = Pack<T>::N, VT = WIDE_TILE;
+    extern __shared__ __align__(16) float smem[];
+    __shared__ int which;
+    const int R = d / 8, per_token = 2 * d + VT, stage_floats = WIDE_STAGE * per_token, red_floats = WIDE_STAGE * R * VT;
+    float* red = smem + 2 * stage_floats;              // [2][stage][R][VT]; before it, [2]: q [stage][d], gates [stage][d], v [stage][VT]
+    float* low_s = red + 2 * red_floats;               // [d]
+    float* bias_s = low_s + d;                         // [d]
+    pdl_launch_dependents();
+    const int head = blockIdx.x, col0 = blockIdx.y * VT, tid = threadIdx.x;
+    const int64_t cols = 2 * (int64_t)H * d + (int64_t)H * vd;
+    for (int i = tid; i < d; i += blockDim.x) {
+        low_s[i] = low[head * d + i];
+        bias_s[i] = bias[head * d + i];
+    }
+    pdl_wait();
+    // the blockIdx.z-th longest sequence (of equal ones the earlier first)
+    for (int i = tid; i < n_seqs; i += blockDim.x) {
+        const int mine = seq_start[i + 1] - seq_start[i];
+        int rank = 0;
+        for (int k = 0; k < n_seqs; ++k) {
+            const int n = seq_start[k + 1] - seq_start[k];
+            rank += n > mine || (n == mine && k < i);
+        }
+        if (rank == (int)blockIdx.z) which = i;
+    }
+    __syncthreads();
+    const int seq = which, t_begin = seq_start[seq], n_tokens = seq_start[seq + 1] - t_begin;
+    if (n_tokens == 0) return;
+    const int stages = (n_tokens + WIDE_STAGE - 1) / WIDE_STAGE;
+
+    if (tid >= walkers) {
+        // ---------------- helpers
+        const int id = tid - walkers, n_helpers = blockDim.x - walkers;
+        // a stage's packets: all of q, then all of the gates, then the block's columns of v, so that a warp's are of one kind
+        const int q_packets = WIDE_STAGE * d / P, v_packets = WIDE_STAGE * VT / P;
+        int token[WIDE_PACKETS], kind[WIDE_PACKETS], place[WIDE_PACKETS], channel[WIDE_PACKETS];   // place: of its first value in the stage
+        const T* src[WIDE_PACKETS];                    // in the first token's row of the sequence
+#pragma unroll
+        for (int k = 0; k < WIDE_PACKETS; ++k) {
+            const int x = id + k * n_helpers;
+            kind[k] = x < q_packets ? 0 : x < 2 * q_packets ? 1 : 2;
+            const int y = x - kind[k] * q_packets, width = kind[k] < 2 ? d : VT, i = y * P % width;
+            token[k] = kind[k] < 2 || (y < v_packets && col0 + i < vd) ? y * P / width : WIDE_STAGE;
+            channel[k] = i;
+            place[k] = kind[k] * WIDE_STAGE * d + y * P;
+            const int64_t column = kind[k] == 0 ? (int64_t)head * d + i : kind[k] == 1 ? (int64_t)(H + head) * d + i
+                                                                                       : 2 * (int64_t)H * d + (int64_t)head * vd + col0 + i;
+            src[k] = proj + (int64_t)(t_begin + token[k]) * cols + column;
+        }
+        Pack<T> raw[WIDE_PACKETS];
+        auto fetch = [&](int st) {
+            const int n_stage = min(WIDE_STAGE, n_tokens - st * WIDE_STAGE);
+#pragma unroll
+            for (int k = 0; k < WIDE_PACKETS; ++k)
+                if (token[k] < n_stage) raw[k] = load_pack<T>(src[k] + (int64_t)st * WIDE_STAGE * cols);
+        };
+        auto activate = [&](int st) {
+            const int n_stage = min(WIDE_STAGE, n_tokens - st * WIDE_STAGE);
+#pragma unroll
+            for (int k = 0; k < WIDE_PACKETS; ++k) {
+                if (token[k] >= n_stage) continue;
+                float v[P];
+#pragma unroll
+                for (int e = 0; e < P; ++e) v[e] = raw[k].get(e);
+                if (kind[k] == 0) {
+#pragma unroll
+                    for (int e = 0; e < P; ++e) v[e] *= sigmoid_of<T>(v[e]);
+                } else if (kind[k] == 1) {
+                    float lo[P], b[P];
+#pragma unroll
+                    for (int e = 0; e < P; e += 4) {
+                        const float4 l4 = *reinterpret_cast<const float4*>(low_s + channel[k] + e), b4 = *reinterpret_cast<const float4*>(bias_s + channel[k] + e);
+                        lo[e] = l4.x; lo[e + 1] = l4.y; lo[e + 2] = l4.z; lo[e + 3] = l4.w;
+                        b[e] = b4.x; b[e + 1] = b4.y; b[e + 2] = b4.z; b[e + 3] = b4.w;
+                    }
+#pragma unroll
+                    for (int e = 0; e < P; ++e) v[e] = lo[e] + (1.0f - lo[e]) * sigmoid_of<T>(v[e] + b[e]);
+                }
+                float* to = smem + (st & 1) * stage_floats + place[k];
+#pragma unroll
+                for (int e = 0; e < P; e += 4) *reinterpret_cast<float4*>(to + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+            }
+        };
+        auto add_up = [&](int st) {
+            const int n_stage = min(WIDE_STAGE, n_tokens - st * WIDE_STAGE), col = id % VT;
+            const float* from = red + (st & 1) * red_floats + col;
+            if (col0 + col >= vd) return;
+            for (int tt = id / VT; tt < n_stage; tt += n_helpers / VT) {
+                float o = 0.0f;
+#pragma unroll 8
+                for (int rr = 0; rr < R; ++rr) o += from[(tt * R + rr) * VT];
+                out[((int64_t)(t_begin + st * WIDE_STAGE + tt) * H + head) * vd + col0 + col] = o;
+            }
+        };
+        fetch(0);
+        activate(0);
+        if (stages > 1) fetch(1);
+        __syncthreads();
+        for (int st = 0; st < stages; ++st) {
+            if (st + 1 < stages) activate(st + 1);
+            if (st + 2 < stages) fetch(st + 2);
+            if (st > 0) add_up(st - 1);
+            __syncthreads();
+        }
+        add_up(stages - 1);
+        return;
+    }
+
+    // ---------------- walkers
+    const int c = (tid % (VT / 4)) * 4, r = tid / (VT / 4);
+    const bool live = r < R && col0 + c < vd;
+    uint64_t S[4][4];                                  // rows 2 n and 2 n + 1 of the thread's eight, its four columns
+    float* S_g = state + ((int64_t)seq_slots[seq] * H + head) * d * vd + (int64_t)r * 8 * vd + col0 + c;
+    if (live) {
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            const float4 a = *reinterpret_cast<const float4*>(S_g + (int64_t)(2 * n) * vd), b = *reinterpret_cast<const float4*>(S_g + (int64_t)(2 * n + 1) * vd);
+            S[n][0] = two(a.x, b.x);
+            S[n][1] = two(a.y, b.y);
+            S[n][2] = two(a.z, b.z);
+            S[n][3] = two(a.w, b.w);
+        }
+    }
+    __syncthreads();
+    for (int st = 0; st < stages; ++st) {
+        const int n_stage = min(WIDE_STAGE, n_tokens - st * WIDE_STAGE);
+        if (live) {
+            const float* q_s = smem + (st & 1) * stage_floats + r * 8;
+            const float* f_s = q_s + WIDE_STAGE * d;
+            const float* v_s = smem + (st & 1) * stage_floats + 2 * WIDE_STAGE * d + c;
+            float* to = red + (st & 1) * red_floats + r * VT + c;
+#pragma unroll 2
+            for (int tt = 0; tt < n_stage; ++tt) {
+                const float4 v4 = *reinterpret_cast<const float4*>(v_s + tt * VT);
+                const uint64_t v2[4] = {two(v4.x, v4.x), two(v4.y, v4.y), two(v4.z, v4.z), two(v4.w, v4.w)};
+                const uint64_t nv2[4] = {two(-v4.x, -v4.x), two(-v4.y, -v4.y), two(-v4.z, -v4.z), two(-v4.w, -v4.w)};
+                uint64_t part[4] = {0ull, 0ull, 0ull, 0ull};             // the sums over even and over odd rows
+#pragma unroll
+                for (int n = 0; n < 4; n += 2) {
+                    const ulonglong2 f2 = *reinterpret_cast<const ulonglong2*>(f_s + tt * d + 2 * n);
+                    const ulonglong2 q2 = *reinterpret_cast<const ulonglong2*>(q_s + tt * d + 2 * n);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        S[n][e] = fma2(f2.x, add2(S[n][e], nv2[e]), v2[e]);                      // f S + (1 - f) v
+                        part[e] = fma2(S[n][e], q2.x, part[e]);
+                        S[n + 1][e] = fma2(f2.y, add2(S[n + 1][e], nv2[e]), v2[e]);
+                        part[e] = fma2(S[n + 1][e], q2.y, part[e]);
+                    }
+                }
+                float even[4], odd[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) one_each(part[e], even[e], odd[e]);
+                *reinterpret_cast<float4*>(to + tt * R * VT) = make_float4(even[0] + odd[0], even[1] + odd[1], even[2] + odd[2], even[3] + odd[3]);
+            }
+        }
+        __syncthreads();
+    }
+    if (live) {
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            float4 a, b;
+            one_each(S[n][0], a.x, b.x);
+            one_each(S[n][1], a.y, b.y);
+            one_each(S[n][2], a.z, b.z);
+            one_each(S[n][3], a.w, b.w);
+            *reinterpret_cast<float4*>(S_g + (int64_t)(2 * n) * vd) = a;
+            *reinterpret_cast<float4*>(S_g + (int64_t)(2 * n + 1) * vd) = b;
+        }
+    }
+}
+
 // A step in which every sequence brings one token: bound by reading and writing the state once.  A block takes 64 columns
 // of one head's state (32 where that leaves SMs without a block), a thread 8 neighbouring rows of 4 columns: eight 16-byte
 // loads in flight a thread, whole lines a warp.  The sums are those of the scan, to the bit: 8 rows in two chains, then the
@@ -238,6 +443,17 @@ int gated_scan_launch(const T* proj, float* state, const float* low, const float
                       float* out, int n_seqs, int H, int d, int vd, cudaStream_t stream) {
     if (n_seqs <= 0) return 0;
     if (H <= 0 || d <= 0 || vd <= 0 || d > 256 || vd > 256 || n_seqs > 65535) return Q3_ERR_BAD_SIZE;
+    if (d % 8 == 0 && vd % 8 == 0 && aligned16(proj) && aligned16(state)) {
+        // walkers of 8 rows x 4 columns in whole warps; helpers: 128, or 256 where a stage has more packets than five each
+        const int walkers = ((d / 8) * (WIDE_TILE / 4) + 31) / 32 * 32, packets = WIDE_STAGE * (2 * d + WIDE_TILE) / Pack<T>::N;
+        const int helpers = packets <= WIDE_PACKETS * 128 ? 128 : 256;
+        const size_t bytes = (size_t)(2 * WIDE_STAGE * (2 * d + WIDE_TILE + (d / 8) * WIDE_TILE) + 2 * d) * sizeof(float);   // at most 102 KB
+        static Q3PerDevice configured;
+        const cudaError_t e = q3_allow_shared_memory(gated_scan_wide_kernel<T>, 112 * 1024, configured);
+        if (e != cudaSuccess) return (int)e;
+        return (int)q3_launch(gated_scan_wide_kernel<T>, dim3(H, (vd + WIDE_TILE - 1) / WIDE_TILE, n_seqs), dim3(walkers + helpers), bytes,
+                              stream, proj, state, low, bias, seq_start, seq_slots, out, H, d, vd, n_seqs, walkers);
+    }
     const int vt = min(vd, COL_TILE);
     const int R = (d + MAX_ROWS - 1) / MAX_ROWS;       // threads that share a column: up to 32
     const int need = (d + R - 1) / R;                  // rows a thread: up to 8

@@ -217,6 +217,32 @@ def test_single_tokens_of_the_recurrence_give_the_scan_s_bits(dtype, heads, d, v
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,d,vd", [(2, 8, 8), (1, 64, 72), (3, 48, 40), (40, 128, 128), (1, 256, 96)])
+def test_prompts_through_the_recurrence_give_the_bits_of_single_tokens(dtype, heads, d, vd):
+    """The scan with rows in pairs, with partial tiles of columns and lengths around the tokens that are fetched together: outputs
+    and states as when every token is a step of its own."""
+    import torch
+    from qwen3_b200.csrc import ops
+    rng = np.random.default_rng(d * vd)
+    T = torch_dtype(dtype)
+    low, bias = dev(rng.uniform(0, 0.95, heads * d), torch.float32), dev(rng.standard_normal(heads * d), torch.float32)
+    lengths = [9, 1, 8, 16, 23]
+    start = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    proj = dev(rng.standard_normal((int(start[-1]), heads * (2 * d + vd))), T)
+    slots = dev([3, 0, 5, 1, 2], torch.int32)
+    whole = dev(rng.standard_normal((6, heads, d, vd)), torch.float32)
+    single, out = whole.clone(), torch.full((int(start[-1]), heads * vd), 9.0, dtype=torch.float32, device="cuda")
+    ops.gated_scan(proj, whole, low, bias, dev(start, torch.int32), slots, out, len(lengths), heads, d, vd)
+    for i in range(max(lengths)):
+        rows = [int(start[s]) + i for s, n in enumerate(lengths) if n > i]
+        at = dev(np.concatenate([[0], np.cumsum([n > i for n in lengths])]), torch.int32)
+        one = torch.empty((len(rows), heads * vd), dtype=torch.float32, device="cuda")
+        ops.gated_scan(proj[rows].contiguous(), single, low, bias, at, slots, one, len(lengths), heads, d, vd, single=True)
+        assert torch.equal(one, out[rows])
+    assert torch.equal(whole, single)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("vd", [1, 9, 32, 200])
 def test_unit_rms_per_head_with_one_weight_for_all_heads(dtype, vd):
     import torch
