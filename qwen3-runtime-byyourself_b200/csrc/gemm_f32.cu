@@ -17,8 +17,8 @@
 //
 //   stream_kernel : up to 8 rows (decode).  Bound by reading W once: 5.6 TB/s over the products of a
 //                   decode step of 3 sequences (1.0 ms; tiles of 64 x 64 took 8.9).
-//   tile_kernel   : more rows.  Bound by the CUDA cores' fma: 38 TFLOP/s over the products of 183 rows
-//                   at 8B width (11.1 ms for 4 layers, 31 before).
+//   tile_kernel   : more rows.  Bound by the CUDA cores' fma: 31 TFLOP/s over the products of 183 rows
+//                   at 8B width (9.0 ms for 4 layers; tiles of 64 x 64 by 4 x 4 a thread took 31).
 //
 // Rows that are not whole packets, and bfloat16 operands of any width (32-bit accumulation,
 // bfloat16 or float output: the products whose width is no multiple of 8, which the
@@ -242,7 +242,8 @@ tile_kernel(const float* __restrict__ X, const float* __restrict__ W, float* __r
                         acc[i][j] = 0;
                     }
             } else {
-                float* kept = shared + T_STAGES * tile_stage<BM>() + done * BM * T_N;
+                if (first + done + 1 == last) __syncthreads();           // everybody has left the stages
+                float* kept = first + done + 1 == last ? shared : shared + T_STAGES * tile_stage<BM>() + done * BM * T_N;
 #pragma unroll
                 for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -269,19 +270,42 @@ tile_kernel(const float* __restrict__ X, const float* __restrict__ W, float* __r
     }
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
-    const float* kept = shared + T_STAGES * tile_stage<BM>();
+    static_assert(BM * T_N <= T_STAGES * tile_stage<BM>(), "the last range's sums lie where the stages were");
     for (int i = share * 256 + tid; i < BM * T_N; i += shares * 256) {
         const int m = m0 + i / T_N, n = n0 + i % T_N;
         if (m >= M || n >= N) continue;
         float sum = 0.0f;
         for (int c = 0, r = 0; c < shares; ++c) {
-            const float* theirs = cluster.map_shared_rank(kept, c);
+            const float* theirs = cluster.map_shared_rank(shared, c);
             const int to = (c + 1) * ranges / shares;
-            for (int at = 0; r < to; ++r, ++at) sum = r == 0 ? theirs[i] : sum + theirs[at * BM * T_N + i];
+            for (int at = 0; r < to; ++r, ++at) {
+                const float part = theirs[(r + 1 == to ? 0 : T_STAGES * tile_stage<BM>() + at * BM * T_N) + i];
+                sum = r == 0 ? part : sum + part;
+            }
         }
         Y[(int64_t)m * ldy + n] = sum;
     }
     cluster.sync();                                      // a block's sums stay until all have read them
+}
+
+// Blocks of a cluster that share K.  The time of a block is its ranges; of two on an SM twice that, of one alone 1.3 times (it
+// does not hide its own latencies).
+int tile_shares(int64_t tiles, int ranges, int stages_bytes, int range_bytes) {
+    const int64_t sms = q3_device_sm_count();
+    int best = 1;
+    double least = 1e30;
+    for (int shares = 1; shares <= ranges; shares *= 2) {
+        const int per = (ranges + shares - 1) / shares, bytes = stages_bytes + (shares > 1 ? (per - 1) * range_bytes : 0);
+        if (bytes > 227 * 1024) continue;
+        const bool two = bytes <= 113 * 1024;                            // 114 KB a block, 1 KB of them the system's
+        const int64_t blocks = tiles * shares, slots = two ? 2 * sms : sms, rest = blocks % slots;
+        const double cost = (double)(blocks / slots) * per * (two ? 2.0 : 1.3) + (rest == 0 ? 0.0 : per * (rest > sms ? 2.0 : 1.3));
+        if (cost < least) {
+            least = cost;
+            best = shares;
+        }
+    }
+    return best;
 }
 
 template <int BM>
@@ -290,15 +314,12 @@ int launch_tiles(const float* X, const float* W, float* Y, int M, int N, int K, 
     const int length = range_length(K), ranges = (K + length - 1) / length;
     const int64_t tiles = (int64_t)((N + T_N - 1) / T_N) * ((M + BM - 1) / BM);
     if ((M + BM - 1) / BM > 65535) return Q3_ERR_TOO_LARGE;
-    // two blocks are resident on an SM; K is shared while that leaves some of the room empty
-    int shares = 1;
-    while (shares * 2 <= ranges && tiles * shares * 2 <= 2 * (int64_t)q3_device_sm_count()) shares *= 2;
-    const int kept = shares > 1 ? (ranges + shares - 1) / shares * BM * T_N : 0;
-    constexpr int MOST = (T_STAGES * tile_stage<BM>() + MAX_RANGES / 2 * BM * T_N) * 4;
+    constexpr int STAGES_BYTES = T_STAGES * tile_stage<BM>() * 4, RANGE_BYTES = BM * T_N * 4, MOST = 227 * 1024;
+    const int shares = tile_shares(tiles, ranges, STAGES_BYTES, RANGE_BYTES);
     static Q3PerDevice configured;
     const cudaError_t e = q3_allow_shared_memory(tile_kernel<BM>, MOST, configured);
     if (e != cudaSuccess) return (int)e;
-    const int smem = (T_STAGES * tile_stage<BM>() + kept) * 4;
+    const int smem = STAGES_BYTES + (shares > 1 ? ((ranges + shares - 1) / shares - 1) * RANGE_BYTES : 0);
     const dim3 grid((N + T_N - 1) / T_N * shares, (M + BM - 1) / BM);
     if (shares == 1)
         return (int)q3_launch(tile_kernel<BM>, grid, dim3(256), smem, stream, X, W, Y, M, N, K, ldx, ldw, ldy, shares);
