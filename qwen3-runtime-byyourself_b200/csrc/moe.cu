@@ -31,45 +31,84 @@ namespace {
 
 __device__ __forceinline__ bool aligned16_device(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-constexpr int MAX_OUTPUTS = 1024;
+constexpr int MAX_OUTPUTS = 1024, MANY_OUTPUTS = 256;     // of the router; where four tokens share a block
 
-template <typename T>
-__global__ void __launch_bounds__(256)
-moe_route_kernel(const T* __restrict__ h, const T* __restrict__ w_router, const float* __restrict__ correction,
-                 int* __restrict__ top_ids, float* __restrict__ top_w, float* __restrict__ id_weight, int hidden, int n_out,
-                 int n_real, int top, int group_count, int group_keep, int by_logit, float* __restrict__ gate_out, int group_pair,
-                 float weight_scale) {
-    __shared__ float z[MAX_OUTPUTS];
-    __shared__ float choice[MAX_OUTPUTS];
-    __shared__ float group_best[MAX_OUTPUTS];
-    __shared__ unsigned char group_kept[MAX_OUTPUTS];
-    pdl_launch_dependents();
-    pdl_wait();
-    const int64_t t = blockIdx.x;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const T* x = h + t * hidden;
-    // a warp per router output; 16-byte packets when the rows allow it (the order of the sum is fixed either way)
-    constexpr int VEC = Pack<T>::N;
-    const bool packed = hidden % VEC == 0 && aligned16_device(x) && aligned16_device(w_router);
-    const int n_rows = n_out + (gate_out != nullptr ? 1 : 0);
-    for (int e = warp; e < n_rows; e += 8) {
-        const T* w = w_router + (int64_t)e * hidden;
-        float dot = 0.0f;
-        if (packed) {
-            for (int c = lane * VEC; c < hidden; c += 32 * VEC) {
-                const Pack<T> wv = load_pack<T>(w + c), xv = load_pack<T>(x + c);
-#pragma unroll
-                for (int i = 0; i < VEC; ++i) dot = fmaf(wv.get(i), xv.get(i), dot);
-            }
+// What `choose_by_one` does, for up to 32 outputs in one group: lane e has output e's logit.  The same operations in the same
+// order, a lane's work being one output's.
+__device__ __forceinline__ void choose_by_lanes(float z, const float* __restrict__ correction, int* __restrict__ top_ids, float* __restrict__ top_w,
+                                                float* __restrict__ id_weight, int n_out, int n_real, int top, int by_logit, float weight_scale,
+                                                int64_t t) {
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const bool mine = lane < n_out;
+    float choice;
+    if (by_logit == 1) {
+        if (mine && correction != nullptr) z += correction[lane];
+        choice = z;
+    } else {
+        if (by_logit == 2) {
+            z = 1.0f / (1.0f + expf(-z));
         } else {
-            for (int c = lane; c < hidden; c += 32) dot = fmaf(to_f32<T>(w[c]), to_f32<T>(x[c]), dot);
+            const float m = warp_max(mine ? z : -INFINITY);
+            z = expf(z - m);
+            float sum = 0.0f;
+            for (int e = 0; e < n_out; ++e) sum += __shfl_sync(ALL, z, e);
+            z *= 1.0f / sum;
         }
-        dot = warp_sum(dot);
-        if (lane == 0) z[e] = dot;
+        choice = z + (mine && correction != nullptr ? correction[lane] : 0.0f);
     }
-    __syncthreads();
-    if (tid != 0) return;
-    if (gate_out != nullptr) gate_out[t] = 1.0f / (1.0f + expf(-z[n_out]));
+    if (!mine) choice = -INFINITY;
+    float best_z = 0.0f, sum = 0.0f, idw = 0.0f, w_of_lane = 0.0f;       // w_of_lane: of the place `lane` among the chosen
+    int id_of_lane = 0;
+    for (int k = 0; k < top; ++k) {
+        // the largest choice score, of equal ones the lowest output; none left: output 0
+        float best_c = choice;
+        int best = choice > -INFINITY ? lane : 32;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float c = __shfl_xor_sync(ALL, best_c, o);
+            const int e = __shfl_xor_sync(ALL, best, o);
+            if (e < 32 && (best == 32 || c > best_c || (c == best_c && e < best))) {
+                best_c = c;
+                best = e;
+            }
+        }
+        if (best == 32) best = 0;
+        const float zb = __shfl_sync(ALL, z, best);
+        if (lane == best) choice = -INFINITY;
+        float w;
+        if (by_logit == 1) {
+            if (k == 0) best_z = zb;
+            w = expf(zb - best_z);
+            sum += w;
+        } else {
+            w = zb * weight_scale;
+            if (best >= n_real) idw += w;
+        }
+        if (lane == k) {
+            id_of_lane = best;
+            w_of_lane = w;
+        }
+    }
+    if (by_logit == 1) {
+        w_of_lane *= 1.0f / sum;
+        for (int k = 0; k < top; ++k) {
+            const float w = __shfl_sync(ALL, w_of_lane, k);
+            if (__shfl_sync(ALL, id_of_lane, k) >= n_real) idw += w;
+        }
+    }
+    if (lane < top) {                                    // top <= n_out <= 32
+        top_ids[t * top + lane] = id_of_lane;
+        top_w[t * top + lane] = w_of_lane;
+    }
+    if (lane == 0) id_weight[t] = idw;
+}
+
+// z [n_out]: a token's logits; choice, group_best, group_kept: room for as many.  By one thread.
+__device__ __forceinline__ void choose_by_one(float* z, float* choice, float* group_best, unsigned char* group_kept,
+                                              const float* __restrict__ correction, int* __restrict__ top_ids, float* __restrict__ top_w,
+                                              float* __restrict__ id_weight, int n_out, int n_real, int top, int group_count, int group_keep,
+                                              int by_logit, int group_pair, float weight_scale, int64_t t) {
     if (by_logit == 1) {
         // the largest logits (ties: the lower index), weighted by the softmax over the chosen logits alone
         float best_z = 0.0f, sum = 0.0f;
@@ -155,6 +194,71 @@ moe_route_kernel(const T* __restrict__ h, const T* __restrict__ w_router, const 
         if (best >= n_real) idw += z[best] * weight_scale;
     }
     id_weight[t] = idw;
+}
+
+// The router matrix is read through the L2 once per block, which bounds the kernel for many tokens (one token a block: 140 KB each
+// at width 4,096 and 16 outputs): TOKENS tokens a block share it.  4,162 tokens: 71 us with one a block, 64 with four; 8 tokens
+// of width 2,048: 7.5 us by eight warps, 5.8 by sixteen with eight packets of a row asked for together.
+template <typename T, int TOKENS, int OUTPUTS, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
+moe_route_kernel(const T* __restrict__ h, const T* __restrict__ w_router, const float* __restrict__ correction,
+                 int* __restrict__ top_ids, float* __restrict__ top_w, float* __restrict__ id_weight, int64_t n_tokens, int hidden, int n_out,
+                 int n_real, int top, int group_count, int group_keep, int by_logit, float* __restrict__ gate_out, int group_pair,
+                 float weight_scale) {
+    __shared__ float z[TOKENS][OUTPUTS];
+    __shared__ float choice[TOKENS][OUTPUTS];
+    __shared__ float group_best[TOKENS][OUTPUTS];
+    __shared__ unsigned char group_kept[TOKENS][OUTPUTS];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int64_t t0 = (int64_t)blockIdx.x * TOKENS;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const T* x[TOKENS];                                  // tokens beyond the last read the last one
+#pragma unroll
+    for (int n = 0; n < TOKENS; ++n) x[n] = h + min(t0 + n, n_tokens - 1) * hidden;
+    // a warp per router output; 16-byte packets when the rows allow it (the order of the sum is fixed either way)
+    constexpr int VEC = Pack<T>::N;
+    const bool packed = hidden % VEC == 0 && aligned16_device(h) && aligned16_device(w_router);
+    const int n_rows = n_out + (gate_out != nullptr ? 1 : 0);
+    for (int e = warp; e < n_rows; e += WARPS) {
+        const T* w = w_router + (int64_t)e * hidden;
+        float dot[TOKENS];
+#pragma unroll
+        for (int n = 0; n < TOKENS; ++n) dot[n] = 0.0f;
+        if (packed) {
+#pragma unroll(TOKENS == 1 ? 8 : 2)
+            for (int c = lane * VEC; c < hidden; c += 32 * VEC) {
+                const Pack<T> wv = load_pack<T>(w + c);
+                Pack<T> xv[TOKENS];
+#pragma unroll
+                for (int n = 0; n < TOKENS; ++n) xv[n] = load_pack<T>(x[n] + c);
+#pragma unroll
+                for (int n = 0; n < TOKENS; ++n)
+#pragma unroll
+                    for (int i = 0; i < VEC; ++i) dot[n] = fmaf(wv.get(i), xv[n].get(i), dot[n]);
+            }
+        } else {
+            for (int c = lane; c < hidden; c += 32)
+#pragma unroll
+                for (int n = 0; n < TOKENS; ++n) dot[n] = fmaf(to_f32<T>(w[c]), to_f32<T>(x[n][c]), dot[n]);
+        }
+#pragma unroll
+        for (int n = 0; n < TOKENS; ++n) {
+            const float sum = warp_sum(dot[n]);
+            if (lane == 0) z[n][e] = sum;
+        }
+    }
+    __syncthreads();
+    const int64_t t = t0 + warp;
+    if (warp >= TOKENS || t >= n_tokens) return;
+    if (lane == 0 && gate_out != nullptr) gate_out[t] = 1.0f / (1.0f + expf(-z[warp][n_out]));
+    if (n_out <= 32 && group_count == 1) {
+        choose_by_lanes(lane < n_out ? z[warp][lane] : 0.0f, correction, top_ids, top_w, id_weight, n_out, n_real, top, by_logit, weight_scale, t);
+        return;
+    }
+    if (lane == 0)
+        choose_by_one(z[warp], choice[warp], group_best[warp], group_kept[warp], correction, top_ids, top_w, id_weight, n_out, n_real, top,
+                      group_count, group_keep, by_logit, group_pair, weight_scale, t);
 }
 
 // counts [E + 1] (the last cell: pairs of identity experts), offsets [E + 1]
@@ -567,8 +671,13 @@ int moe_experts_launch(const T* h, const T* w_gate_up, const T* w_down, const in
             group_count <= 0 || n_out % group_count != 0 || group_keep <= 0 || group_keep > group_count ||                \
             n_tokens > 0x7fffffffLL)                                                                                      \
             return Q3_ERR_BAD_SIZE;                                                                                       \
-        return (int)q3_launch(moe_route_kernel<T>, dim3((unsigned)n_tokens), dim3(256), 0, (cudaStream_t)stream,          \
-                              (const T*)h, (const T*)w_router, correction, top_ids, top_w, id_weight, hidden, n_out,      \
+        /* four tokens a block where that leaves every SM two blocks */                                                   \
+        if (n_out < MANY_OUTPUTS && n_tokens >= 8 * (int64_t)q3_device_sm_count())                                        \
+            return (int)q3_launch(moe_route_kernel<T, 4, MANY_OUTPUTS, 8>, dim3((unsigned)((n_tokens + 3) / 4)), dim3(256), 0, (cudaStream_t)stream, \
+                                  (const T*)h, (const T*)w_router, correction, top_ids, top_w, id_weight, n_tokens, hidden, n_out, \
+                                  n_real, top, group_count, group_keep, by_logit, gate_out, group_pair, weight_scale);    \
+        return (int)q3_launch(moe_route_kernel<T, 1, MAX_OUTPUTS, 16>, dim3((unsigned)n_tokens), dim3(512), 0, (cudaStream_t)stream, \
+                              (const T*)h, (const T*)w_router, correction, top_ids, top_w, id_weight, n_tokens, hidden, n_out, \
                               n_real, top, group_count, group_keep, by_logit, gate_out, group_pair, weight_scale);        \
     }                                                                                                                     \
     Q3_EXPORT int q3_moe_experts_##SUFFIX(const void* h, const void* w_gate_up, const void* w_down, const int* offsets,   \

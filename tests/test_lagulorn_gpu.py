@@ -333,6 +333,37 @@ def test_router_scores_groups_choice_and_weights(outputs, real, top, groups, kee
         assert np.isclose(idw[t], sum(w_ for e, w_ in zip(chosen, weights) if e >= real), rtol=1e-5, atol=1e-7)
 
 
+@pytest.mark.parametrize("mode", ["softmax", "sigmoid", "logit"])
+@pytest.mark.parametrize("outputs,real,top,corrected,N", [(2, 1, 2, True, 40), (17, 12, 4, True, 40), (32, 30, 8, False, 1187), (31, 31, 31, True, 40),
+                                                          (40, 33, 5, True, 1186), (300, 290, 4, False, 1185)])
+def test_router_by_lanes_and_with_four_tokens_a_block(outputs, real, top, corrected, N, mode):
+    """Every output a group of its own, all of them kept, one token at a time: the same choice by the one-thread form, to the bit -
+    with equal logits, rows that give infinities and NaN, and as many choices as outputs."""
+    import torch
+    from qwen3_b200.csrc import ops
+    rng = np.random.default_rng(outputs + top)
+    hidden = 24
+    h = dev(rng.standard_normal((N, hidden)), torch.float32)
+    h[3], h[4, 0], h[5, 0] = 0.0, float("inf"), float("nan")
+    w = dev(rng.standard_normal((outputs, hidden)), torch.float32)
+    w[outputs // 2] = w[0]
+    corr = dev(rng.standard_normal(outputs), torch.float32) if corrected else None
+    picked = list(range(20)) + list(range(N - 20, N))
+
+    def route(rows, groups):
+        n = rows.shape[0]
+        ids = torch.full((n * top,), -1, dtype=torch.int32, device="cuda")
+        tw, idw = torch.full((n * top,), 9.0, device="cuda"), torch.full((n,), 9.0, device="cuda")
+        ops.moe_route(rows, w, corr, ids, tw, idw, real, top, groups, groups, by_logit=mode == "logit", sigmoid=mode == "sigmoid", weight_scale=1.5)
+        return ids.view(n, top), tw.view(n, top), idw.view(n, 1)
+
+    finite = torch.isfinite(h[picked]).all(dim=1)
+    got, want = route(h, 1), route(h[picked].contiguous(), outputs)
+    assert torch.equal(got[0][picked], want[0])
+    for x, y in zip(got[1:], want[1:]):
+        assert torch.equal(x[picked][finite], y[finite])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("hidden,top", [(8, 1), (12, 2), (20, 3), (2048, 2), (4096 + 8, 2)])
 def test_combining_in_packets_and_value_by_value(dtype, hidden, top):
