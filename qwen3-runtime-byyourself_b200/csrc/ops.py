@@ -151,8 +151,26 @@ def _check(code: int, name: str):
 _pinned_stream: Optional[int] = None
 
 
+_stream_objects = {}
+
+
+def _raw_stream() -> int:
+    # torch.cuda.current_stream() builds an object and asks for the device in four ways, 4 us a call; a step of generation
+    # asks a few times (a 32-bit model of three layers, 12 tokens for 4 prompts: 2.57 ms with it, 2.37 without)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+def stream_object() -> "torch.cuda.Stream":
+    """The current stream of the current device, as `torch.cuda.current_stream()` (streams are not taken down)."""
+    key = (torch.cuda.current_device(), _raw_stream())
+    stream = _stream_objects.get(key)
+    if stream is None:
+        stream = _stream_objects[key] = torch.cuda.current_stream()
+    return stream
+
+
 def _stream() -> int:
-    return _pinned_stream if _pinned_stream is not None else torch.cuda.current_stream().cuda_stream
+    return _pinned_stream if _pinned_stream is not None else _raw_stream()
 
 
 class on_current_stream:
@@ -162,7 +180,7 @@ class on_current_stream:
     def __enter__(self):
         global _pinned_stream
         self._before = _pinned_stream
-        _pinned_stream = torch.cuda.current_stream().cuda_stream
+        _pinned_stream = _raw_stream()
         return self
 
     def __exit__(self, *exc):

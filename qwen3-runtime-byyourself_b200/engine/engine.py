@@ -85,8 +85,9 @@ class _MetaBuffer:
         turn = self._turn
         self._turn ^= 1
         self.dev[:total].copy_(self._host[turn][:total], non_blocking=True)
+        from ..csrc import ops
         event = torch.cuda.Event()
-        event.record()
+        event.record(ops.stream_object())
         self._events[turn] = event
         self.bytes_last_upload = total * 4
 

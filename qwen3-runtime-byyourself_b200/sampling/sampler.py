@@ -94,7 +94,7 @@ class Sampler:
         host = self._out_hosts[self._turn][:rows]
         host.copy_(ids, non_blocking=True)
         event = torch.cuda.Event()
-        event.record()
+        event.record(ops.stream_object())
         return PendingChoice(ids, host, event)
 
     def choose(self, logits: torch.Tensor, sequence_ids: Sequence[int], steps: Sequence[int]) -> List[int]:
