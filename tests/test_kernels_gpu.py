@@ -131,6 +131,22 @@ def test_gemm_f32_same_sums_in_both_kernels(N, K):
     assert torch.equal(many[:, :N], rows["whole"])
 
 
+@pytest.mark.parametrize("M", [20, 100, 183])
+@pytest.mark.parametrize("N,K", [(2048, 448), (4096, 512), (6144, 448), (6144, 1056), (9000, 2048)])
+def test_gemm_f32_same_sums_whatever_the_cluster(M, N, K):
+    """Enough tiles that one, two, four or eight blocks share K, with whole and uneven numbers of ranges each: the last range's sums
+    lie where the stages were, the others behind them.  The bits of the kernel for few rows."""
+    from qwen3_b200.csrc import ops
+    gen = torch.Generator(device="cuda").manual_seed(N + K)
+    x, w = torch.randn(M, K, generator=gen, device="cuda"), torch.randn(N, K, generator=gen, device="cuda")
+    out = torch.full((M, N), float("nan"), device="cuda")
+    ops.gemm_f32(x, w, out)
+    for lo in range(0, M, 8):
+        few = torch.empty(min(8, M - lo), N, device="cuda")
+        ops.gemm_f32(x[lo:lo + 8].contiguous(), w, few)
+        assert torch.equal(few, out[lo:lo + 8]), lo
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 45, 67), (37, 130, 100), (200, 333, 100), (5, 64, 9)])
 @pytest.mark.parametrize("out_dtype", ["bfloat16", "float32"])
 def test_bf16_product_of_any_width(M, N, K, out_dtype):
