@@ -134,7 +134,11 @@ decode_split_kernel(const bf16* __restrict__ q, const bf16* k_pages, const bf16*
     const int pg_end = min(first_page + n_pages, pg_begin + per_split);
     const int count = max(pg_end - pg_begin, 0);
 
-    // the first pages are asked for before anything else: what follows runs under their flight
+    // The first pages are asked for before anything else: what follows runs under their flight.  The pages and the step's
+    // positions do not depend on the kernel before this one when the new token's key and value are this kernel's own to
+    // write; otherwise they are in the cache once the kernels before are done.
+    const bool writes = FUSED && fused.write_kv;
+    if (!writes) pdl_wait();
     const uint32_t pipe = smem_u32(smem) + warp * (STAGES * 2 * PANEL_BYTES);
     auto issue = [&](int i) {
         if (i < count) {
@@ -147,12 +151,10 @@ decode_split_kernel(const bf16* __restrict__ q, const bf16* k_pages, const bf16*
     };
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) issue(s);
-    // the pages and the step's positions do not depend on the kernel before this one (the new token's key and
-    // value are this kernel's own to write); its output - the projections - is read from here on
-    pdl_wait();
+    if (writes) pdl_wait();      // the projections, the output of the kernel before, are read from here on
 
     // the block that holds the sequence's last page owns the new token's key and value
-    const bool owner = FUSED && fused.write_kv && count > 0 && pg_end == first_page + n_pages;
+    const bool owner = writes && count > 0 && pg_end == first_page + n_pages;
     bf16* prep = reinterpret_cast<bf16*>(smem + SMEM_BYTES);            // [16][D] queries, then the new key, then the new value
     if constexpr (FUSED) {
         const bf16* row = fused.qkv + (int64_t)t * (nq + 2 * nkv) * D;

@@ -166,6 +166,9 @@ decode_flat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     __syncthreads();                             // the barriers are set up
 
     const bool producer = warp == WARPS;
+    // The pages and the step's positions do not depend on the kernel before this one when the new token's key and value are this
+    // kernel's own to write; a layer that reads another layer's cache finds them there once the kernels before are done.
+    if (producer && !a.write_kv) pdl_wait();
     const int quad = lane >> 2, tq = lane & 3;
     int s = 0;                                   // place in the ring
     uint32_t phase = 0;
@@ -220,8 +223,7 @@ decode_flat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                 continue;
             }
 
-            // the pages and the step's positions do not depend on the kernel before this one (the new token's key and
-            // value are this kernel's own to write); its output - the projections - is read from here on
+            // the projections, the output of the kernel before, are read from here on
             if (!waited) pdl_wait();
             else meet();                             // the results of the part before have been read
             waited = true;

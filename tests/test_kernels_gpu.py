@@ -997,6 +997,55 @@ def test_decode_attention_with_pages_shared_out(nq, nkv, d, lengths, window):
         ops.attention_decode_fused(qkv, k1, v1, kept, *args, 3, parts=parts, counters=counters[:-1])
 
 
+@pytest.mark.parametrize("form", ["cluster", "shared out", "split"])
+def test_decode_attention_reads_a_cache_that_another_kernel_writes_after_that_kernel(form):
+    """With dependent launch on, behind a slow kernel and the one that writes the new token's key and value into the pages: the
+    attention that does not write them itself finds them there."""
+    from qwen3_b200.csrc import ops
+    rng = np.random.default_rng(11)
+    nq, nkv, d, lengths = 8, 2, 128, [70, 130, 64]
+    table, kp, vp = paged_case(rng, lengths, nkv, d, "bfloat16")
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    B, table_d = len(lengths), torch.as_tensor(table).cuda()
+    seq = torch.arange(B, dtype=torch.int32, device="cuda")
+    pos = torch.as_tensor([n - 1 for n in lengths], dtype=torch.int32).cuda()
+    qkv = torch.randn(B, (nq + 2 * nkv) * d, generator=gen, device="cuda").to(torch.bfloat16)
+    q = torch.empty(B, nq * d, dtype=torch.bfloat16, device="cuda")
+    out = torch.empty_like(q)
+    parts = torch.empty(ops.attention_decode_flat_parts(d, nq // nkv), dtype=torch.float32, device="cuda")
+    counters = torch.zeros(B * nkv, dtype=torch.int32, device="cuda")
+    scratch = torch.empty(B * nq * 2 * (d + 2), dtype=torch.float32, device="cuda")
+    tokens = 2000                                        # of a recurrence: a few blocks for some hundred microseconds
+    proj = torch.randn(tokens, 3 * 64, generator=gen, device="cuda").to(torch.bfloat16)
+    state, zeros, o = torch.zeros(1, 1, 64, 64, device="cuda"), torch.zeros(64, device="cuda"), torch.empty(tokens, 64, device="cuda")
+    start, slot = torch.tensor([0, tokens], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def run():
+        ops.gated_scan(proj, state, zeros, zeros, start, slot, o, 1, 1, 64, 64)
+        ops.qkv_prepare(qkv, q, kp, vp, None, None, None, None, seq, pos, table_d, B, nq, nkv, d, 0.0)
+        if form == "split":
+            ops.attention_decode(q, kp, vp, out, scratch, seq, pos, table_d, B, nq, nkv, d, d ** -0.5, None, 2)
+        else:
+            extra = dict(parts=parts, counters=counters) if form == "shared out" else {}
+            ops.attention_decode_fused(qkv, kp, vp, out, None, None, None, None, 0.0, seq, pos, table_d, B, nq, nkv, d, d ** -0.5,
+                                       None, 2, write_kv=False, **extra)
+
+    first_k, first_v = torch.randn_like(kp), torch.randn_like(vp)
+    for pdl in (False, True, True, True):
+        kp.copy_(first_k)
+        vp.copy_(first_v)
+        torch.cuda.synchronize()
+        ops.set_pdl(pdl)
+        try:
+            run()
+        finally:
+            ops.set_pdl(None)
+        torch.cuda.synchronize()
+        if not pdl:
+            want = out.clone()
+        assert torch.equal(out, want), pdl
+
+
 @pytest.mark.parametrize("nq,nkv,d,lengths,window", [
     (4, 2, 4, [1, 65], None), (3, 3, 12, [130], None), (8, 1, 32, [76, 21, 45, 13], None), (6, 2, 48, [64, 63], 17), (5, 5, 80, [200], None),
     (8, 8, 128, [157, 53, 1], None), (2, 1, 132, [129], 64), (4, 2, 256, [300, 2], None)])
