@@ -216,6 +216,31 @@ def test_single_tokens_of_the_recurrence_give_the_scan_s_bits(dtype, heads, d, v
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
+def test_prompts_of_many_sequences_take_time_in_proportion():
+    """The scan of 1,536 short sequences against that of 96: sixteen times the work is not a hundred times as slow."""
+    import torch
+    from qwen3_b200.csrc import ops
+    heads, d, vd, tokens = 2, 16, 16, 3
+    low, bias = torch.rand(heads * d, device="cuda"), torch.randn(heads * d, device="cuda")
+
+    def best(n):
+        start = torch.arange(0, n * tokens + 1, tokens, dtype=torch.int32, device="cuda")
+        proj = torch.randn(n * tokens, heads * (2 * d + vd), device="cuda").to(torch.bfloat16)
+        state, slots = torch.zeros(n, heads, d, vd, device="cuda"), torch.arange(n, dtype=torch.int32, device="cuda")
+        out = torch.empty(n * tokens, heads * vd, device="cuda")
+        times = []
+        for _ in range(5):
+            before, after = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            before.record()
+            for _ in range(8):
+                ops.gated_scan(proj, state, low, bias, start, slots, out, n, heads, d, vd)
+            after.record()
+            torch.cuda.synchronize()
+            times.append(before.elapsed_time(after))
+        return min(times)
+    assert best(1536) < 64 * best(96)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads,d,vd", [(2, 8, 8), (1, 64, 72), (3, 48, 40), (40, 128, 128), (1, 256, 96)])
 def test_prompts_through_the_recurrence_give_the_bits_of_single_tokens(dtype, heads, d, vd):
