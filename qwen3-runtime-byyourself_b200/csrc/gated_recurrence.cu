@@ -224,7 +224,7 @@ gated_scan_wide_kernel(const T* __restrict__ proj, float* __restrict__ state, co
     // The blockIdx.z-th longest sequence (of equal ones the earlier first).  Finding it takes every block n_seqs comparisons a
     // thread, and with many sequences blocks enough follow one another to fill the gaps of the longest: beyond WIDE_RANKED they
     // come as they are.  (1,500 sequences of 3 tokens, 32 heads of 128 x 128: 179 ms ranked, 2.3 ms as they come.)
-    const bool ranked = n_seqs <= WIDE_RANKED;
+    const bool ranked = n_seqs > 1 && n_seqs <= WIDE_RANKED;
     if (ranked) {
         for (int i = tid; i < n_seqs; i += blockDim.x) {
             const int mine = seq_start[i + 1] - seq_start[i];
@@ -449,10 +449,17 @@ int gated_scan_launch(const T* proj, float* state, const float* low, const float
                       float* out, int n_seqs, int H, int d, int vd, cudaStream_t stream) {
     if (n_seqs <= 0) return 0;
     if (H <= 0 || d <= 0 || vd <= 0 || d > 256 || vd > 256 || n_seqs > 65535) return Q3_ERR_BAD_SIZE;
-    if (d % 8 == 0 && vd % 8 == 0 && aligned16(proj) && aligned16(state)) {
-        // walkers of 8 rows x 4 columns in whole warps; helpers: 128, or 256 where a stage has more packets than five each
+    // The scan for whole packets, but for small states of many sequences, where its 160 threads a block and more find little to do (512
+    // sequences of 2 tokens, 2 heads of 16 x 16: 3.9 us below, 9.0 there; 64 of 16 and fewer: level), and for 32-bit heads beyond
+    // 128 in fewer blocks than there are SMs, where its helpers hold the walkers up (one sequence of 2,048 tokens, 8 heads of 256 x 256:
+    // 596 us below, 716 there; four of 700 tokens, 256 blocks: ahead there).
+    const int64_t wide_blocks = (int64_t)H * ((vd + WIDE_TILE - 1) / WIDE_TILE) * n_seqs;
+    const bool wide = (d >= 32 || n_seqs <= WIDE_RANKED) && (sizeof(T) == 2 || d <= 128 || wide_blocks >= q3_device_sm_count());
+    if (wide && d % 8 == 0 && vd % 8 == 0 && aligned16(proj) && aligned16(state)) {
+        // walkers of 8 rows x 4 columns in whole warps; helpers: 128, or 256 where a stage has more than three packets each
         const int walkers = ((d / 8) * (WIDE_TILE / 4) + 31) / 32 * 32, packets = WIDE_STAGE * (2 * d + WIDE_TILE) / Pack<T>::N;
-        const int helpers = packets <= WIDE_PACKETS * 128 ? 128 : 256;
+        const int helpers = packets <= 3 * 128 ? 128 : 256;      // (32-bit, 16 heads of 128 x 128, 2,048 tokens: 640 us with 128, 432 with 256)
+        static_assert(WIDE_PACKETS * 256 >= WIDE_STAGE * (2 * 256 + WIDE_TILE) / 4, "a stage's packets of 32-bit values, d = 256");
         const size_t bytes = (size_t)(2 * WIDE_STAGE * (2 * d + WIDE_TILE + (d / 8) * WIDE_TILE) + 2 * d) * sizeof(float);   // at most 102 KB
         static Q3PerDevice configured;
         const cudaError_t e = q3_allow_shared_memory(gated_scan_wide_kernel<T>, 112 * 1024, configured);

@@ -216,6 +216,32 @@ def test_single_tokens_of_the_recurrence_give_the_scan_s_bits(dtype, heads, d, v
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,d,vd,n_seqs", [(2, 16, 16, 64), (2, 16, 16, 65), (2, 32, 16, 65), (1, 256, 256, 1), (20, 256, 256, 1)])
+def test_every_form_of_the_scan_gives_the_bits_of_single_tokens(dtype, heads, d, vd, n_seqs):
+    """On both sides of the sizes at which the scan changes its form: many sequences and few, small states, 32-bit heads beyond 128 in
+    few blocks and in more."""
+    import torch
+    from qwen3_b200.csrc import ops
+    rng = np.random.default_rng(d + n_seqs)
+    T = torch_dtype(dtype)
+    low, bias = dev(rng.uniform(0, 0.95, heads * d), torch.float32), dev(rng.standard_normal(heads * d), torch.float32)
+    lengths = rng.integers(0, 12, n_seqs) if n_seqs > 1 else np.array([19])
+    start = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    proj = dev(rng.standard_normal((int(start[-1]), heads * (2 * d + vd))), T)
+    slots = dev(rng.permutation(n_seqs), torch.int32)
+    whole = dev(rng.standard_normal((n_seqs, heads, d, vd)), torch.float32)
+    single, out = whole.clone(), torch.full((int(start[-1]), heads * vd), 9.0, dtype=torch.float32, device="cuda")
+    ops.gated_scan(proj, whole, low, bias, dev(start, torch.int32), slots, out, n_seqs, heads, d, vd)
+    for i in range(int(lengths.max())):
+        rows = [int(start[s]) + i for s, n in enumerate(lengths) if n > i]
+        at = dev(np.concatenate([[0], np.cumsum([n > i for n in lengths])]), torch.int32)
+        one = torch.empty((len(rows), heads * vd), dtype=torch.float32, device="cuda")
+        ops.gated_scan(proj[rows].contiguous(), single, low, bias, at, slots, one, n_seqs, heads, d, vd, single=True)
+        assert torch.equal(one, out[rows])
+    assert torch.equal(whole, single)
+
+
 def test_prompts_of_many_sequences_take_time_in_proportion():
     """The scan of 1,536 short sequences against that of 96: sixteen times the work is not a hundred times as slow."""
     import torch
