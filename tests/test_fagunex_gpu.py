@@ -242,6 +242,25 @@ def test_every_form_of_the_scan_gives_the_bits_of_single_tokens(dtype, heads, d,
     assert torch.equal(whole, single)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_single_tokens_over_a_state_off_its_16_byte_boundary(dtype):
+    """A step of single tokens whose state rows begin between two boundaries runs, with the bits of the aligned one."""
+    import torch
+    from qwen3_b200.csrc import ops
+    heads, d, vd, n = 2, 16, 16, 3
+    T = torch_dtype(dtype)
+    low, bias = torch.rand(heads * d, device="cuda"), torch.randn(heads * d, device="cuda")
+    proj = torch.randn(n, heads * (2 * d + vd), device="cuda").to(T)
+    start, slots = torch.arange(n + 1, dtype=torch.int32, device="cuda"), torch.arange(n, dtype=torch.int32, device="cuda")
+    aligned = torch.randn(n, heads, d, vd, device="cuda")
+    room = torch.cat([torch.zeros(1, device="cuda"), aligned.flatten()])
+    shifted = room[1:].view_as(aligned)
+    out = [torch.empty(n, heads * vd, device="cuda") for _ in range(2)]
+    for state, o in zip((aligned, shifted), out):
+        ops.gated_scan(proj, state, low, bias, start, slots, o, n, heads, d, vd, single=True)
+    assert torch.equal(out[0], out[1]) and torch.equal(aligned, shifted)
+
+
 def test_prompts_of_many_sequences_take_time_in_proportion():
     """The scan of 1,536 short sequences against that of 96: sixteen times the work is not a hundred times as slow."""
     import torch
