@@ -553,11 +553,14 @@ Q3_EXPORT int q3_sample_f32(const float* logits, int64_t stride, int rows, int v
         cudaError_t e = q3_allow_shared_memory(sample_kernel, PRIVATE_BYTES, configured);
         if (e != cudaSuccess) return (int)e;
     }
-    // blocks per row: as many as keep the clusters of all rows resident at once (one block of 1,024 threads an SM), and
-    // no more than find two logits a thread: below that the meetings of a cluster cost more than the row
+    // Blocks per row: as many as keep the clusters of all rows resident at once (one block of 1,024 threads an SM).  Where the row
+    // ends as a short sorted list, no more than find two logits a thread: below that the meetings of a cluster cost more than the
+    // row (one row of 4,096, top-k 50: 25 us with eight, 15 with one).  Selection by radix passes over the row some ten times and
+    // wants them all (one row of 4,096 without top-k: 92 us with eight, 145 with one; of 16,000 116 and 155).
+    const bool short_list = valid <= SHORT_LIST || (top_k > 0 && top_k < valid && top_k <= S_THREADS);
     const int sms = q3_device_sm_count();
     int n_blocks = S_BLOCKS_MAX;
-    while (n_blocks > 1 && ((int64_t)rows * n_blocks > sms || valid < n_blocks * 2 * S_THREADS)) n_blocks >>= 1;
+    while (n_blocks > 1 && ((int64_t)rows * n_blocks > sms || (short_list && valid < n_blocks * 2 * S_THREADS))) n_blocks >>= 1;
     return (int)q3_launch_cluster(sample_kernel, dim3(rows * n_blocks), dim3(S_THREADS), PRIVATE_BYTES, (cudaStream_t)stream,
                                   dim3(n_blocks, 1, 1), logits, stride, valid, temperature, top_k, top_p, seed, seq_ids,
                                   steps, step_all, out, n_blocks);

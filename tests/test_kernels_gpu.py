@@ -997,6 +997,30 @@ def test_decode_attention_with_pages_shared_out(nq, nkv, d, lengths, window):
         ops.attention_decode_fused(qkv, k1, v1, kept, *args, 3, parts=parts, counters=counters[:-1])
 
 
+@pytest.mark.parametrize("rows", [1, 4])
+def test_sampling_short_rows_without_top_k_takes_no_longer_than_long_ones(rows):
+    """A quarter of the logits, drawn from without top-k, in less time than all of them (medians over several rows of logits)."""
+    from qwen3_b200.csrc import ops
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    ids, out = torch.arange(rows, device="cuda"), torch.empty(rows, dtype=torch.int32, device="cuda")
+
+    def took(logits):
+        before, after = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        before.record()
+        for step in range(16):
+            ops.sample(logits, out, 0.7, 0, 1.0, 5, ids, step)
+        after.record()
+        torch.cuda.synchronize()
+        return before.elapsed_time(after)
+
+    times = {4096: [], 16384: []}
+    for _ in range(9):
+        logits = 3.0 * torch.randn(rows, 16384, generator=gen, device="cuda")
+        for vocab in times:
+            times[vocab].append(took(logits[:, :vocab].contiguous()))
+    assert sorted(times[4096])[4] < 0.95 * sorted(times[16384])[4], times
+
+
 @pytest.mark.parametrize("form", ["cluster", "shared out", "split"])
 def test_decode_attention_reads_a_cache_that_another_kernel_writes_after_that_kernel(form):
     """With dependent launch on, behind a slow kernel and the one that writes the new token's key and value into the pages: the
