@@ -198,7 +198,9 @@ __device__ __forceinline__ void choose_by_one(float* z, float* choice, float* gr
 
 // The router matrix is read through the L2 once per block, which bounds the kernel for many tokens (one token a block: 140 KB each
 // at width 4,096 and 16 outputs): TOKENS tokens a block share it.  4,162 tokens: 71 us with one a block, 64 with four; 8 tokens
-// of width 2,048: 7.5 us by eight warps, 5.8 by sixteen with eight packets of a row asked for together.
+// of width 2,048: 7.5 us by eight warps, 5.8 by sixteen with eight packets of a row asked for together.  Sixteen warps are for steps
+// whose blocks are all resident at once: of more than 32 outputs one thread chooses while the block waits for it, and then blocks an SM
+// count (4,100 tokens of width 96, 300 outputs: 507 us by eight warps, 1,046 by sixteen; 1,000 tokens 243 and 388).
 template <typename T, int TOKENS, int OUTPUTS, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
 moe_route_kernel(const T* __restrict__ h, const T* __restrict__ w_router, const float* __restrict__ correction,
@@ -251,13 +253,14 @@ moe_route_kernel(const T* __restrict__ h, const T* __restrict__ w_router, const 
     __syncthreads();
     const int64_t t = t0 + warp;
     if (warp >= TOKENS || t >= n_tokens) return;
-    if (lane == 0 && gate_out != nullptr) gate_out[t] = 1.0f / (1.0f + expf(-z[warp][n_out]));
+    const int of = TOKENS == 1 ? 0 : warp;               // a number the compiler knows where one token has the block
+    if (lane == 0 && gate_out != nullptr) gate_out[t] = 1.0f / (1.0f + expf(-z[of][n_out]));
     if (n_out <= 32 && group_count == 1) {
-        choose_by_lanes(lane < n_out ? z[warp][lane] : 0.0f, correction, top_ids, top_w, id_weight, n_out, n_real, top, by_logit, weight_scale, t);
+        choose_by_lanes(lane < n_out ? z[of][lane] : 0.0f, correction, top_ids, top_w, id_weight, n_out, n_real, top, by_logit, weight_scale, t);
         return;
     }
     if (lane == 0)
-        choose_by_one(z[warp], choice[warp], group_best[warp], group_kept[warp], correction, top_ids, top_w, id_weight, n_out, n_real, top,
+        choose_by_one(z[of], choice[of], group_best[of], group_kept[of], correction, top_ids, top_w, id_weight, n_out, n_real, top,
                       group_count, group_keep, by_logit, group_pair, weight_scale, t);
 }
 
@@ -676,7 +679,12 @@ int moe_experts_launch(const T* h, const T* w_gate_up, const T* w_down, const in
             return (int)q3_launch(moe_route_kernel<T, 4, MANY_OUTPUTS, 8>, dim3((unsigned)((n_tokens + 3) / 4)), dim3(256), 0, (cudaStream_t)stream, \
                                   (const T*)h, (const T*)w_router, correction, top_ids, top_w, id_weight, n_tokens, hidden, n_out, \
                                   n_real, top, group_count, group_keep, by_logit, gate_out, group_pair, weight_scale);    \
-        return (int)q3_launch(moe_route_kernel<T, 1, MAX_OUTPUTS, 16>, dim3((unsigned)n_tokens), dim3(512), 0, (cudaStream_t)stream, \
+        /* sixteen warps a token while all tokens' blocks are resident at once, else eight */                             \
+        if (n_tokens <= 4 * (int64_t)q3_device_sm_count())                                                                \
+            return (int)q3_launch(moe_route_kernel<T, 1, MAX_OUTPUTS, 16>, dim3((unsigned)n_tokens), dim3(512), 0, (cudaStream_t)stream, \
+                                  (const T*)h, (const T*)w_router, correction, top_ids, top_w, id_weight, n_tokens, hidden, n_out, \
+                                  n_real, top, group_count, group_keep, by_logit, gate_out, group_pair, weight_scale);    \
+        return (int)q3_launch(moe_route_kernel<T, 1, MAX_OUTPUTS, 8>, dim3((unsigned)n_tokens), dim3(256), 0, (cudaStream_t)stream, \
                               (const T*)h, (const T*)w_router, correction, top_ids, top_w, id_weight, n_tokens, hidden, n_out, \
                               n_real, top, group_count, group_keep, by_logit, gate_out, group_pair, weight_scale);        \
     }                                                                                                                     \

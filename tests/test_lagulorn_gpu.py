@@ -364,6 +364,29 @@ def test_router_by_lanes_and_with_four_tokens_a_block(outputs, real, top, correc
         assert torch.equal(x[picked][finite], y[finite])
 
 
+def test_router_of_a_long_prompt_takes_its_share_of_time():
+    """4,100 tokens and 300 outputs against 64 tokens, whose blocks are all resident at once."""
+    import torch
+    from qwen3_b200.csrc import ops
+    hidden, outputs, top = 96, 300, 8
+    w = torch.randn(outputs, hidden, device="cuda").to(torch.bfloat16)
+
+    def best(n):
+        h = torch.randn(n, hidden, device="cuda").to(torch.bfloat16)
+        ids, tw = torch.empty(n * top, dtype=torch.int32, device="cuda"), torch.empty(n * top, device="cuda")
+        idw, took = torch.empty(n, device="cuda"), []
+        for _ in range(5):
+            before, after = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            before.record()
+            for _ in range(8):
+                ops.moe_route(h, w, None, ids, tw, idw, outputs, top)
+            after.record()
+            torch.cuda.synchronize()
+            took.append(before.elapsed_time(after))
+        return min(took)
+    assert best(4100) < 6.3 * best(64)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("hidden,top", [(8, 1), (12, 2), (20, 3), (2048, 2), (4096 + 8, 2)])
 def test_combining_in_packets_and_value_by_value(dtype, hidden, top):
