@@ -17,12 +17,13 @@
 //
 //   stream_kernel : up to 8 rows (decode).  Bound by reading W once: 5.6 TB/s over the products of a
 //                   decode step of 3 sequences (1.0 ms; tiles of 64 x 64 took 8.9).
-//   tile_kernel   : more rows.  Bound by the CUDA cores' fma: 31 TFLOP/s over the products of 183 rows
-//                   at 8B width (9.0 ms for 4 layers; tiles of 64 x 64 by 4 x 4 a thread took 31).
+//   tile_kernel   : more rows.  Bound by the CUDA cores' fma: 41 TFLOP/s in tiles of 128 x 128 that fill the GPU (1,000 rows, K 2,048,
+//                   32,768 wide: 3.25 ms; 3.9 in one ascending chain by tiles of 64 x 64), less where few rows share K over clusters.
+//   gemm_tn_kernel: short K, where the tiles above have too few steps to pay for their start.
 //
 // Rows that are not whole packets, and bfloat16 operands of any width (32-bit accumulation,
 // bfloat16 or float output: the products whose width is no multiple of 8, which the
-// tensor-core kernels refuse), go to `gemm_tn_kernel`, one ascending chain.
+// tensor-core kernels refuse), go to `gemm_tn_kernel` in its other form, one ascending chain.
 #include "common.cuh"
 #include <cooperative_groups.h>
 
@@ -157,15 +158,21 @@ int launch_stream(const float* X, const float* W, float* Y, int M, int N, int K,
 // ---------------------------------------------------------------- more rows
 // A tile of BM rows of X by 128 rows of W per block, (BM / 16) x 8 elements a thread, both operands staged as they lie in
 // memory (rows of 32 k, padded to 36 words: the 16 rows a warp reads at once fall into different banks) in three stages of
-// asynchronous copies.  Per 4 k a thread makes 4 BM/16 * 8 multiply-adds from BM/16 + 8 16-byte reads.  When there are too
-// few tiles to fill the GPU, the ranges of K are shared out to a cluster's blocks, which leave their sums in shared memory
-// and add a share of the tile each, in the order of the ranges.
+// asynchronous copies.  Per 4 k a thread makes 4 BM/16 * 8 multiply-adds from BM/16 + 8 16-byte reads.  The steps of a range are a
+// loop of their own, without the code that puts its sum by (in one loop the tiles of 128 rows took 3.75 us a step, 3.5 apart).  When
+// there are too few tiles to fill the GPU, the ranges of K are shared out to a cluster's blocks, which leave their sums in shared
+// memory and add a share of the tile each, in the order of the ranges.
 constexpr int T_N = 128, T_K = 32, T_LD = T_K + 4, T_STAGES = 3;
 
 template <int BM> constexpr int tile_stage() { return (BM + T_N) * T_LD; }               // floats
+// Shared memory of a block: the stages, and the sums of its ranges but the last, which lie where the stages were (128 rows: the
+// tile's sums).
+int tile_bytes(int rows, int ranges, int shares) {
+    return T_STAGES * (rows + T_N) * T_LD * 4 + (shares > 1 ? (ranges + shares - 1) / shares - 1 : rows == 128 ? 1 : 0) * rows * T_N * 4;
+}
 
 template <int BM>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, BM == 128 ? 1 : 2)
 tile_kernel(const float* __restrict__ X, const float* __restrict__ W, float* __restrict__ Y, int M, int N, int K, int64_t ldx,
             int64_t ldw, int64_t ldy, int shares) {
     extern __shared__ __align__(16) float shared[];
@@ -202,7 +209,6 @@ tile_kernel(const float* __restrict__ X, const float* __restrict__ W, float* __r
         copies_commit();
     };
     uint64_t acc[TM][TN];
-    float total[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -210,116 +216,131 @@ tile_kernel(const float* __restrict__ X, const float* __restrict__ W, float* __r
 #pragma unroll
     for (int s = 0; s < T_STAGES - 1; ++s) fetch(s);
     int done = 0;                                        // ranges that are summed
-    for (int step = 0; step < steps; ++step) {
-        copies_wait<T_STAGES - 2>();
-        __syncthreads();
-        fetch(step + T_STAGES - 1);
-        const float* a = shared + (step % T_STAGES) * tile_stage<BM>() + ty * T_LD;
-        const float* b = shared + (step % T_STAGES) * tile_stage<BM>() + (BM + tx) * T_LD;
+    for (int step = 0; step < steps;) {
+        const int range_end = min(steps, (done + 1) * per_range);
+        for (; step < range_end; ++step) {
+            copies_wait<T_STAGES - 2>();
+            __syncthreads();
+            fetch(step + T_STAGES - 1);
+            const float* a = shared + (step % T_STAGES) * tile_stage<BM>() + ty * T_LD;
+            const float* b = shared + (step % T_STAGES) * tile_stage<BM>() + (BM + tx) * T_LD;
 #pragma unroll 2
-        for (int k = 0; k < T_K; k += 4) {
-            ulonglong2 av[TM];
+            for (int k = 0; k < T_K; k += 4) {
+                ulonglong2 av[TM];
 #pragma unroll
-            for (int i = 0; i < TM; ++i) av[i] = *reinterpret_cast<const ulonglong2*>(a + i * 16 * T_LD + k);
+                for (int i = 0; i < TM; ++i) av[i] = *reinterpret_cast<const ulonglong2*>(a + i * 16 * T_LD + k);
 #pragma unroll
-            for (int j = 0; j < TN; ++j) {
-                const ulonglong2 bv = *reinterpret_cast<const ulonglong2*>(b + j * 16 * T_LD + k);
+                for (int j = 0; j < TN; ++j) {
+                    const ulonglong2 bv = *reinterpret_cast<const ulonglong2*>(b + j * 16 * T_LD + k);
 #pragma unroll
-                for (int i = 0; i < TM; ++i) {
-                    fma2(acc[i][j], av[i].x, bv.x);
-                    fma2(acc[i][j], av[i].y, bv.y);
+                    for (int i = 0; i < TM; ++i) {
+                        fma2(acc[i][j], av[i].x, bv.x);
+                        fma2(acc[i][j], av[i].y, bv.y);
+                    }
                 }
             }
         }
-        if ((step + 1) % per_range == 0 || step + 1 == steps) {          // a range is complete
-            if (shares == 1) {
+        // a range is complete
+        if (shares == 1 && BM == 128) {              // a block an SM: there is room for the sums so far behind the stages
+            float* kept = shared + T_STAGES * tile_stage<BM>() + tid;
 #pragma unroll
-                for (int i = 0; i < TM; ++i)
+            for (int i = 0; i < TM; ++i)
 #pragma unroll
-                    for (int j = 0; j < TN; ++j) {
-                        const float sum = both(acc[i][j]);
-                        total[i][j] = done == 0 ? sum : total[i][j] + sum;
-                        acc[i][j] = 0;
-                    }
-            } else {
-                if (first + done + 1 == last) __syncthreads();           // everybody has left the stages
-                float* kept = first + done + 1 == last ? shared : shared + T_STAGES * tile_stage<BM>() + done * BM * T_N;
+                for (int j = 0; j < TN; ++j) {
+                    const float sum = both(acc[i][j]);
+                    kept[(i * TN + j) * 256] = done > 0 ? kept[(i * TN + j) * 256] + sum : sum;
+                    acc[i][j] = 0;
+                }
+        } else if (shares == 1) {                    // they wait in Y, where they need neither registers nor shared memory
+            float before[TM][TN];
 #pragma unroll
-                for (int i = 0; i < TM; ++i)
+            for (int i = 0; i < TM; ++i)
 #pragma unroll
-                    for (int j = 0; j < TN; ++j) {
-                        kept[(i * 16 + ty) * T_N + j * 16 + tx] = both(acc[i][j]);
-                        acc[i][j] = 0;
-                    }
-            }
-            ++done;
+                for (int j = 0; j < TN; ++j) {
+                    const int m = m0 + i * 16 + ty, n = n0 + j * 16 + tx;
+                    before[i][j] = done > 0 && m < M && n < N ? Y[(int64_t)m * ldy + n] : 0.0f;
+                }
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    const int m = m0 + i * 16 + ty, n = n0 + j * 16 + tx;
+                    const float sum = both(acc[i][j]);
+                    if (m < M && n < N) Y[(int64_t)m * ldy + n] = done > 0 ? before[i][j] + sum : sum;
+                    acc[i][j] = 0;
+                }
+        } else {
+            if (first + done + 1 == last) __syncthreads();           // everybody has left the stages
+            float* kept = first + done + 1 == last ? shared : shared + T_STAGES * tile_stage<BM>() + done * BM * T_N;
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    kept[(i * 16 + ty) * T_N + j * 16 + tx] = both(acc[i][j]);
+                    acc[i][j] = 0;
+                }
         }
+        ++done;
     }
     copies_wait<0>();
     if (shares == 1) {
+        if (BM < 128) return;
+        const float* kept = shared + T_STAGES * tile_stage<BM>() + tid;
 #pragma unroll
-        for (int i = 0; i < TM; ++i) {
-            const int m = m0 + i * 16 + ty;
+        for (int i = 0; i < TM; ++i)
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
-                const int n = n0 + j * 16 + tx;
-                if (m < M && n < N) Y[(int64_t)m * ldy + n] = total[i][j];
+                const int m = m0 + i * 16 + ty, n = n0 + j * 16 + tx;
+                if (m < M && n < N) Y[(int64_t)m * ldy + n] = kept[(i * TN + j) * 256];
             }
-        }
         return;
     }
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
     static_assert(BM * T_N <= T_STAGES * tile_stage<BM>(), "the last range's sums lie where the stages were");
-    for (int i = share * 256 + tid; i < BM * T_N; i += shares * 256) {
+    // four neighbouring sums at a time, all ranges' asked for together
+    for (int i = (share * 256 + tid) * 4; i < BM * T_N; i += shares * 256 * 4) {
         const int m = m0 + i / T_N, n = n0 + i % T_N;
         if (m >= M || n >= N) continue;
-        float sum = 0.0f;
-        for (int c = 0, r = 0; c < shares; ++c) {
-            const float* theirs = cluster.map_shared_rank(shared, c);
-            const int to = (c + 1) * ranges / shares;
-            for (int at = 0; r < to; ++r, ++at) {
-                const float part = theirs[(r + 1 == to ? 0 : T_STAGES * tile_stage<BM>() + at * BM * T_N) + i];
-                sum = r == 0 ? part : sum + part;
+        float4 part[MAX_RANGES];
+        int c = 0, at = 0, to = ranges / shares;         // the share that holds range r, its place there, the share's end
+#pragma unroll
+        for (int r = 0; r < MAX_RANGES; ++r) {
+            part[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (r >= ranges) continue;
+            if (r == to) {
+                at = 0;
+                to = (++c + 1) * ranges / shares;
             }
+            const float* theirs = cluster.map_shared_rank(shared, c);
+            part[r] = *reinterpret_cast<const float4*>(theirs + (r + 1 == to ? 0 : T_STAGES * tile_stage<BM>() + at * BM * T_N) + i);
+            ++at;
         }
-        Y[(int64_t)m * ldy + n] = sum;
+        float4 sum = part[0];
+#pragma unroll
+        for (int r = 1; r < MAX_RANGES; ++r) {
+            if (r >= ranges) continue;
+            sum.x += part[r].x; sum.y += part[r].y; sum.z += part[r].z; sum.w += part[r].w;
+        }
+        float* y = Y + (int64_t)m * ldy + n;
+        y[0] = sum.x;
+        if (n + 1 < N) y[1] = sum.y;
+        if (n + 2 < N) y[2] = sum.z;
+        if (n + 3 < N) y[3] = sum.w;
     }
     cluster.sync();                                      // a block's sums stay until all have read them
 }
 
-// Blocks of a cluster that share K.  The time of a block is its ranges; of two on an SM twice that, of one alone 1.3 times (it
-// does not hide its own latencies).
-int tile_shares(int64_t tiles, int ranges, int stages_bytes, int range_bytes) {
-    const int64_t sms = q3_device_sm_count();
-    int best = 1;
-    double least = 1e30;
-    for (int shares = 1; shares <= ranges; shares *= 2) {
-        const int per = (ranges + shares - 1) / shares, bytes = stages_bytes + (shares > 1 ? (per - 1) * range_bytes : 0);
-        if (bytes > 227 * 1024) continue;
-        const bool two = bytes <= 113 * 1024;                            // 114 KB a block, 1 KB of them the system's
-        const int64_t blocks = tiles * shares, slots = two ? 2 * sms : sms, rest = blocks % slots;
-        const double cost = (double)(blocks / slots) * per * (two ? 2.0 : 1.3) + (rest == 0 ? 0.0 : per * (rest > sms ? 2.0 : 1.3));
-        if (cost < least) {
-            least = cost;
-            best = shares;
-        }
-    }
-    return best;
-}
-
 template <int BM>
-int launch_tiles(const float* X, const float* W, float* Y, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldy,
+int launch_tiles(const float* X, const float* W, float* Y, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldy, int shares,
                  cudaStream_t stream) {
     const int length = range_length(K), ranges = (K + length - 1) / length;
-    const int64_t tiles = (int64_t)((N + T_N - 1) / T_N) * ((M + BM - 1) / BM);
     if ((M + BM - 1) / BM > 65535) return Q3_ERR_TOO_LARGE;
-    constexpr int STAGES_BYTES = T_STAGES * tile_stage<BM>() * 4, RANGE_BYTES = BM * T_N * 4, MOST = 227 * 1024;
-    const int shares = tile_shares(tiles, ranges, STAGES_BYTES, RANGE_BYTES);
+    constexpr int MOST = 227 * 1024;
     static Q3PerDevice configured;
     const cudaError_t e = q3_allow_shared_memory(tile_kernel<BM>, MOST, configured);
     if (e != cudaSuccess) return (int)e;
-    const int smem = STAGES_BYTES + (shares > 1 ? ((ranges + shares - 1) / shares - 1) * RANGE_BYTES : 0);
+    const int smem = tile_bytes(BM, ranges, shares);
     const dim3 grid((N + T_N - 1) / T_N * shares, (M + BM - 1) / BM);
     if (shares == 1)
         return (int)q3_launch(tile_kernel<BM>, grid, dim3(256), smem, stream, X, W, Y, M, N, K, ldx, ldw, ldy, shares);
@@ -327,58 +348,84 @@ int launch_tiles(const float* X, const float* W, float* Y, int M, int N, int K, 
                                   ldy, shares);
 }
 
+// ---------------------------------------------------------------- short rows of K, and rows that are not whole packets
+// Tiles of 64 x 64, 4 x 4 elements a thread, staged through registers.  RANGES: the order of sums of the kernels above, for
+// packets of float; else one ascending chain.
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
 
-template <typename InT, typename OutT>
-__global__ void __launch_bounds__(256)
+// RESIDENT: blocks that an SM must hold (3: at most 80 registers; 0: as the compiler likes, two blocks an SM).
+template <bool RANGES, int RESIDENT, typename InT, typename OutT>
+__global__ void __launch_bounds__(256, RESIDENT)
 gemm_tn_kernel(const InT* __restrict__ X, const InT* __restrict__ W, OutT* __restrict__ Y, int M, int N, int K,
                int64_t ldx, int64_t ldw, int64_t ldy) {
-    __shared__ float Xs[BK][BM + 4];
-    __shared__ float Ws[BK][BN + 4];
+    __shared__ float Xs[2][BK][BM + 4];                  // two tiles: one barrier a tile, the next is fetched under the products of this
+    __shared__ float Ws[2][BK][BN + 4];
     pdl_launch_dependents();
     pdl_wait();
     const int tid = threadIdx.x;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int tx = tid % 16, ty = tid / 16;  // thread tile: rows ty*4.., cols tx*4..
-    float acc[TM][TN];
+    float acc[TM][TN], odd[TM][TN], total[TM][TN];       // RANGES: chains of the even and of the odd k, the ranges before
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
+        for (int j = 0; j < TN; ++j) acc[i][j] = odd[i][j] = total[i][j] = 0.0f;
+    const int length = range_length(K);
 
     // each thread stages 4 consecutive k of one row of X and one row of W
     const int lr = tid / 4, lk = (tid % 4) * 4;
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        float xv[4] = {0.f, 0.f, 0.f, 0.f}, wv[4] = {0.f, 0.f, 0.f, 0.f};
+    alignas(16) float xv[4];
+    alignas(16) float wv[4];
+    auto fetch = [&](int k0) {
         const int gm = m0 + lr, gn = n0 + lr, gk = k0 + lk;
-        if (gm < M) {
-            const InT* p = X + (int64_t)gm * ldx + gk;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) if (gk + i < K) xv[i] = to_f32<InT>(p[i]);
-        }
-        if (gn < N) {
-            const InT* p = W + (int64_t)gn * ldw + gk;
+        for (int i = 0; i < 4; ++i) xv[i] = wv[i] = 0.0f;
+        const InT *px = X + (int64_t)gm * ldx + gk, *pw = W + (int64_t)gn * ldw + gk;
+        if constexpr (RANGES) {
+            if (gm < M && gk < K) *reinterpret_cast<float4*>(xv) = *reinterpret_cast<const float4*>(px);
+            if (gn < N && gk < K) *reinterpret_cast<float4*>(wv) = *reinterpret_cast<const float4*>(pw);
+        } else {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) if (gk + i < K) wv[i] = to_f32<InT>(p[i]);
+            for (int i = 0; i < 4; ++i) {
+                if (gm < M && gk + i < K) xv[i] = to_f32<InT>(px[i]);
+                if (gn < N && gk + i < K) wv[i] = to_f32<InT>(pw[i]);
+            }
         }
-        __syncthreads();  // the previous tile has been consumed
+    };
+    fetch(0);
+    for (int k0 = 0; k0 < K; k0 += BK) {
+        const int at = k0 / BK & 1;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            Xs[lk + i][lr] = xv[i];
-            Ws[lk + i][lr] = wv[i];
+            Xs[at][lk + i][lr] = xv[i];
+            Ws[at][lk + i][lr] = wv[i];
         }
         __syncthreads();
+        if (k0 + BK < K) fetch(k0 + BK);
 #pragma unroll
         for (int kk = 0; kk < BK; ++kk) {
             float a[TM], b[TN];
 #pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = Xs[kk][ty * TM + i];
+            for (int i = 0; i < TM; ++i) a[i] = Xs[at][kk][ty * TM + i];
 #pragma unroll
-            for (int j = 0; j < TN; ++j) b[j] = Ws[kk][tx * TN + j];
+            for (int j = 0; j < TN; ++j) b[j] = Ws[at][kk][tx * TN + j];
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < TN; ++j) {
+                    float& chain = RANGES && (kk & 1) ? odd[i][j] : acc[i][j];
+                    chain = fmaf(a[i], b[j], chain);
+                }
+        }
+        if (RANGES && ((k0 + BK) % length == 0 || k0 + BK >= K)) {       // a range is complete (its length is a multiple of 32)
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    const float sum = acc[i][j] + odd[i][j];
+                    total[i][j] = k0 < length ? sum : total[i][j] + sum;
+                    acc[i][j] = odd[i][j] = 0.0f;
+                }
         }
     }
 #pragma unroll
@@ -388,9 +435,63 @@ gemm_tn_kernel(const InT* __restrict__ X, const InT* __restrict__ W, OutT* __res
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
             const int gn = n0 + tx * TN + j;
-            if (gn < N) Y[(int64_t)gm * ldy + gn] = from_f32<OutT>(acc[i][j]);
+            if (gn < N) Y[(int64_t)gm * ldy + gn] = from_f32<OutT>(RANGES ? total[i][j] : acc[i][j]);
         }
     }
+}
+
+// ---------------------------------------------------------------- which tiles, and how many blocks share K
+struct Form {
+    int rows, shares;             // rows of X of a tile, blocks of a cluster that share K; 0: the 64 x 64 kernel, its blocks of an SM
+};
+
+// The form that should be done first: microseconds of the waves of its blocks, from constants fitted to measured products of 9 to 4,000
+// rows, widths of 16 to 151,936 and K of 64 to 12,288 (within about a tenth).  What they say: few long rows want K shared, K of 64 or 96
+// the small tiles (64 rows of 64 x 64: 4.5 us there, 6.9 in tiles of 64 x 128), and tiles that fill the GPU 128 rows each, whose
+// reads of shared memory weigh half as much (1,000 rows, K 2,048, 32,768 wide: 3.25 ms, 3.67 in tiles of 64, 4.6 in small ones).
+Form choose_form(int M, int N, int K) {
+    struct Cost {
+        int rows;
+        double alone, paired;     // a step of 32 k of a block alone on its SM, of two that share one
+        double range, start;      // the sum of a range put by; start and end of a block
+        double meet;              // start and end where the sums meet in a cluster
+    };
+    constexpr Cost costs[] = {{16, 1.4, 2.55, 0.3, 2.0, 4.2}, {32, 1.5, 2.6, 0.4, 2.0, 4.3}, {64, 2.2, 4.0, 0.93, 1.5, 5.5},
+                              {128, 3.5, 0.0, 0.7, 3.0, 0.0}};
+    const int64_t sms = q3_device_sm_count();
+    const int length = range_length(K), ranges = (K + length - 1) / length;
+    const int64_t small_tiles = (int64_t)((N + BN - 1) / BN) * ((M + BM - 1) / BM);
+    Form best = {0, 2};
+    // small tiles of an SM, two at a time, or three with fewer registers (4,096 wide, 300 rows, K 64: 12.6 and 9.7 us)
+    double least = 1e30;
+    for (int resident = 2; resident <= 3; ++resident) {
+        const double each = small_tiles <= sms ? 1.0 : (double)((small_tiles + resident * sms - 1) / (resident * sms) * resident);
+        const double cost = 1.5 + 0.55 * each + (K + BK - 1) / BK * (each == 1.0 ? 0.75 : 0.575 * each);
+        if (cost < least) {
+            least = cost;
+            best = {0, resident};
+        }
+    }
+    for (const Cost& c : costs) {
+        if (M <= 16 ? c.rows != 16 : M <= 32 ? c.rows != 32 : c.rows < 64 || (c.rows == 128 && M <= 64)) continue;
+        const int64_t tiles = (int64_t)((N + T_N - 1) / T_N) * ((M + c.rows - 1) / c.rows);
+        for (int shares = 1; shares <= ranges && (shares == 1 || c.rows < 128); shares *= 2) {
+            const int bytes = tile_bytes(c.rows, ranges, shares), per = (ranges + shares - 1) / shares;
+            if (bytes > 227 * 1024) continue;
+            const bool two = c.rows < 128 && bytes <= 113 * 1024;        // 114 KB a block, 1 KB of them the system's
+            const double steps = shares == 1 ? (K + T_K - 1) / T_K : per * (length / T_K);
+            const double ends = shares == 1 ? c.start + ranges * c.range : c.meet + (shares < 8 ? 2.0 : 0.0);   // more sums a block
+            const int64_t blocks = tiles * shares, slots = two ? 2 * sms : sms, rest = blocks % slots;
+            const int64_t apart = shares == 8 ? sms * 3 / 4 : sms;       // blocks that find an SM each: clusters of 8 do not fill them all
+            const double cost = (double)(blocks / slots) * (steps * (two ? c.paired : c.alone) + ends) +
+                                (rest == 0 ? 0.0 : steps * (two && rest > apart ? c.paired : c.alone) + ends);
+            if (cost < least) {
+                least = cost;
+                best = {c.rows, shares};
+            }
+        }
+    }
+    return best;
 }
 
 }  // namespace
@@ -406,17 +507,23 @@ Q3_EXPORT int q3_gemm_tn_f32(const float* X, const float* W, float* Y, int M, in
         if (M == 2) return launch_stream<2>(X, W, Y, M, N, K, ldx, ldw, ldy, s);
         if (M <= 4) return launch_stream<4>(X, W, Y, M, N, K, ldx, ldw, ldy, s);
         if (M <= 8) return launch_stream<8>(X, W, Y, M, N, K, ldx, ldw, ldy, s);
-        if (M <= 16) return launch_tiles<16>(X, W, Y, M, N, K, ldx, ldw, ldy, s);
-        if (M <= 32) return launch_tiles<32>(X, W, Y, M, N, K, ldx, ldw, ldy, s);
-        return launch_tiles<64>(X, W, Y, M, N, K, ldx, ldw, ldy, s);
+        const Form form = choose_form(M, N, K);
+        if (form.rows == 16) return launch_tiles<16>(X, W, Y, M, N, K, ldx, ldw, ldy, form.shares, s);
+        if (form.rows == 32) return launch_tiles<32>(X, W, Y, M, N, K, ldx, ldw, ldy, form.shares, s);
+        if (form.rows == 64) return launch_tiles<64>(X, W, Y, M, N, K, ldx, ldw, ldy, form.shares, s);
+        if (form.rows == 128) return launch_tiles<128>(X, W, Y, M, N, K, ldx, ldw, ldy, form.shares, s);
+        const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+        if (grid.y > 65535) return Q3_ERR_TOO_LARGE;
+        return (int)q3_launch(form.shares == 3 ? gemm_tn_kernel<true, 3, float, float> : gemm_tn_kernel<true, 0, float, float>, grid,
+                              dim3(256), 0, s, X, W, Y, M, N, K, ldx, ldw, ldy);
     }
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return Q3_ERR_TOO_LARGE;
-    return (int)q3_launch(gemm_tn_kernel<float, float>, grid, dim3(256), 0, (cudaStream_t)stream, X, W, Y, M, N, K,
+    return (int)q3_launch(gemm_tn_kernel<false, 0, float, float>, grid, dim3(256), 0, (cudaStream_t)stream, X, W, Y, M, N, K,
                           ldx, ldw, ldy);
 }
 
-// bfloat16 operands of any width, 32-bit accumulation in the same fixed order; Y bfloat16 or float.
+// bfloat16 operands of any width, 32-bit accumulation in one ascending chain over K; Y bfloat16 or float.
 Q3_EXPORT int q3_gemm_tn_bf16(const void* X, const void* W, void* Y, int M, int N, int K, int64_t ldx, int64_t ldw,
                               int64_t ldy, int out_is_f32, void* stream) {
     if (M <= 0 || N <= 0) return 0;
@@ -424,8 +531,8 @@ Q3_EXPORT int q3_gemm_tn_bf16(const void* X, const void* W, void* Y, int M, int 
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return Q3_ERR_TOO_LARGE;
     if (out_is_f32)
-        return (int)q3_launch(gemm_tn_kernel<bf16, float>, grid, dim3(256), 0, (cudaStream_t)stream, (const bf16*)X,
+        return (int)q3_launch(gemm_tn_kernel<false, 0, bf16, float>, grid, dim3(256), 0, (cudaStream_t)stream, (const bf16*)X,
                               (const bf16*)W, (float*)Y, M, N, K, ldx, ldw, ldy);
-    return (int)q3_launch(gemm_tn_kernel<bf16, bf16>, grid, dim3(256), 0, (cudaStream_t)stream, (const bf16*)X,
+    return (int)q3_launch(gemm_tn_kernel<false, 0, bf16, bf16>, grid, dim3(256), 0, (cudaStream_t)stream, (const bf16*)X,
                           (const bf16*)W, (bf16*)Y, M, N, K, ldx, ldw, ldy);
 }

@@ -997,6 +997,46 @@ def test_decode_attention_with_pages_shared_out(nq, nkv, d, lengths, window):
         ops.attention_decode_fused(qkv, k1, v1, kept, *args, 3, parts=parts, counters=counters[:-1])
 
 
+@pytest.mark.parametrize("M,N,K", [(64, 64, 64), (107, 96, 96), (33, 50, 4), (70, 333, 100), (300, 2500, 1056), (1000, 2500, 2048), (129, 20000, 96),
+                                   (4000, 130, 64), (300, 130, 4096), (12, 3000, 512), (20, 40000, 32)])
+def test_gemm_f32_same_sums_in_every_form(M, N, K):
+    """Small tiles for short K, tiles of 64 and of 128 rows that sum K by themselves or share it: every row has the bits that the kernel
+    for few rows gives it."""
+    from qwen3_b200.csrc import ops
+    gen = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x, w = torch.randn(M, K, generator=gen, device="cuda"), torch.randn(N, K, generator=gen, device="cuda")
+    out = torch.full((M, N), float("nan"), device="cuda")
+    ops.gemm_f32(x, w, out)
+    few = torch.empty((8, N), device="cuda")
+    for lo in list(range(0, M - 8, max(8, M // 12))) + [M - 8]:
+        ops.gemm_f32(x[lo:lo + 8].contiguous(), w, few)
+        assert torch.equal(out[lo:lo + 8], few), lo
+
+
+def test_gemm_f32_takes_no_more_than_its_share_of_time():
+    """64 short rows against 8 (two kernels, a microsecond of work each), 1,000 long ones against 64."""
+    from qwen3_b200.csrc import ops
+
+    def best(M, N, K, times):
+        x, w, out = torch.randn(M, K, device="cuda"), torch.randn(N, K, device="cuda"), torch.empty(M, N, device="cuda")
+        took = []
+        for _ in range(4):
+            before, after = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                for _ in range(times):
+                    ops.gemm_f32(x, w, out)
+            graph.replay()
+            before.record()
+            graph.replay()
+            after.record()
+            torch.cuda.synchronize()
+            took.append(before.elapsed_time(after))
+        return min(took)
+    assert best(64, 64, 64, 50) < 4 * best(8, 64, 64, 50)
+    assert best(1000, 32768, 2048, 2) < 13 * best(64, 32768, 2048, 2)
+
+
 @pytest.mark.parametrize("rows", [1, 4])
 def test_sampling_short_rows_without_top_k_takes_no_longer_than_long_ones(rows):
     """A quarter of the logits, drawn from without top-k, in less time than all of them (medians over several rows of logits)."""
