@@ -50,10 +50,13 @@ __device__ __forceinline__ float rotated_at(const T* __restrict__ src, int i, in
     return first ? a * c - b * s : a * c + b * s;     // (u, v) -> (u cos - v sin, v cos + u sin)
 }
 
-// Two blocks a token: one for the queries' latent, one for the keys' (8 tokens, query rank 1,536: 6.4 us by one block of 128
-// threads, 3.4 by two of 256).
+// Two blocks a token: one for the queries' latent, one for the keys' (8 tokens, query rank 1,536: 7.5 us by one block for both,
+// 2.9 by two); a layer without a latent of the queries has the second alone (4,100 tokens: 11.5 us with a block that returns at once
+// beside it, 6.2 without).  128 threads whatever the step, so that a row's sums are in one order.
+constexpr int HELD = 12;
+
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128)
 latent_prepare_kernel(const T* __restrict__ proj, int64_t proj_stride, int kv_off, int q_off, const float* __restrict__ w_c,
                       const float* __restrict__ w_q, T* __restrict__ cq, T* __restrict__ k_pages, T* __restrict__ v_pages,
                       const float* __restrict__ cos_tab, const float* __restrict__ sin_tab, const int* __restrict__ token_seq,
@@ -65,18 +68,22 @@ latent_prepare_kernel(const T* __restrict__ proj, int64_t proj_stride, int kv_of
     const int64_t t = blockIdx.x;
     const T* row = proj + t * proj_stride;
     const int tid = threadIdx.x;
-    if (blockIdx.y == 0) {
-        if (q_rank <= 0) return;
+    if (q_rank > 0 && blockIdx.y == 0) {
         const T* qr = row + q_off;
-        float sq = 0.0f;
-#pragma unroll 8
-        for (int i = tid; i < q_rank; i += blockDim.x) {
+        float sq = 0.0f, held[HELD];                     // the first HELD of a thread's values are asked for together
+#pragma unroll
+        for (int n = 0; n < HELD; ++n) held[n] = tid + n * 128 < q_rank ? to_f32<T>(qr[tid + n * 128]) : 0.0f;
+#pragma unroll
+        for (int n = 0; n < HELD; ++n) sq += held[n] * held[n];
+        for (int i = tid + HELD * 128; i < q_rank; i += 128) {
             const float v = to_f32<T>(qr[i]);
             sq += v * v;
         }
         const float inv = rsqrtf(block_sum(sq, scratch) / (float)q_rank + eps);
-#pragma unroll 8
-        for (int i = tid; i < q_rank; i += blockDim.x) cq[t * q_rank + i] = from_f32<T>(to_f32<T>(qr[i]) * inv * w_q[i]);
+#pragma unroll
+        for (int n = 0; n < HELD; ++n)
+            if (tid + n * 128 < q_rank) cq[t * q_rank + tid + n * 128] = from_f32<T>(held[n] * inv * w_q[tid + n * 128]);
+        for (int i = tid + HELD * 128; i < q_rank; i += 128) cq[t * q_rank + i] = from_f32<T>(to_f32<T>(qr[i]) * inv * w_q[i]);
         return;
     }
     if (!write_kv) return;
@@ -302,7 +309,7 @@ bool head_product_tiles<bf16>(const void* x, int64_t x_row, int x_head, int x_of
             (q_rank > 0 && (w_q == nullptr || cq == nullptr)) || (rot_dims > 0 && (cos_tab == nullptr || sin_tab == nullptr)) || \
             n_tokens > 0x7fffffffLL)                                                                                        \
             return Q3_ERR_BAD_SIZE;                                                                                         \
-        return (int)q3_launch(latent_prepare_kernel<T>, dim3((unsigned)n_tokens, 2), dim3(256), 0, (cudaStream_t)stream,       \
+        return (int)q3_launch(latent_prepare_kernel<T>, dim3((unsigned)n_tokens, q_rank > 0 && write_kv ? 2 : 1), dim3(128), 0, (cudaStream_t)stream, \
                               (const T*)proj, proj_stride, kv_off, q_off, w_c, w_q, (T*)cq, (T*)k_pages, (T*)v_pages, cos_tab, \
                               sin_tab, token_seq, token_pos, page_table, pages_per_seq, rank, rot, rot_dims, interleaved,    \
                               q_rank, eps, write_kv);                                                                       \

@@ -261,6 +261,63 @@ def test_single_tokens_over_a_state_off_its_16_byte_boundary(dtype):
     assert torch.equal(out[0], out[1]) and torch.equal(aligned, shifted)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("q_rank", [1, 127, 128, 1535, 1536, 1537, 1700])
+def test_latent_of_the_queries_has_the_same_bits_in_every_step(dtype, q_rank):
+    """Ranks around what a thread holds at once, against 64 bits, and a token alone against the same among others."""
+    import torch
+    from qwen3_b200.csrc import ops
+    n, rank, T = 9, 8, torch_dtype(dtype)
+    gen = torch.Generator(device="cuda").manual_seed(q_rank)
+    proj = torch.randn(n, rank + q_rank, generator=gen, device="cuda").to(T)
+    w = 1.0 + 0.1 * torch.randn(q_rank, generator=gen, device="cuda")
+    k, v = torch.zeros(1, 1, 64, rank, dtype=T, device="cuda"), torch.zeros(1, 1, 64, rank, dtype=T, device="cuda")
+    table, zeros = torch.zeros(1, 1, dtype=torch.int32, device="cuda"), torch.zeros(n, dtype=torch.int32, device="cuda")
+    pos, ones = torch.arange(n, dtype=torch.int32, device="cuda"), torch.ones(rank, device="cuda")
+    cq = torch.full((n, q_rank), 9.0, dtype=T, device="cuda")
+    ops.latent_prepare(proj, 0, rank, ones, w, cq, k, v, None, None, zeros, pos, table, n, rank, 0, 0, False, 1e-6)
+    x = proj[:, rank:].double()
+    want = x * torch.rsqrt(x.square().mean(1, keepdim=True) + 1e-6) * w.double()
+    # a chain of 14 terms, ten additions, the mean, a root and two products; bfloat16 rounds once more
+    bound = want.abs() * (32 * 2.0 ** -24 + (0.0 if dtype == "float32" else 2.0 ** -8)) + 1e-30
+    assert bool(((cq.double() - want).abs() <= bound).all())
+    one = torch.empty(1, q_rank, dtype=T, device="cuda")
+    ops.latent_prepare(proj[4:5].contiguous(), 0, rank, ones, w, one, k, v, None, None, zeros[:1], pos[:1], table, 1, rank, 0, 0, False, 1e-6)
+    assert torch.equal(one[0], cq[4])
+
+
+def test_latents_without_a_latent_of_the_queries_take_less_time():
+    """4,100 tokens: the keys' latents alone against those of the keys and, beside them, short ones of the queries."""
+    import torch
+    from qwen3_b200.csrc import ops
+    n, rank, rot, q_rank = 4100, 192, 64, 64
+    k, v = torch.zeros(65, 1, 64, rank + rot, device="cuda"), torch.zeros(65, 1, 64, rank, device="cuda")
+    table = torch.arange(65, dtype=torch.int32, device="cuda").view(65, 1)
+    at = torch.arange(n, dtype=torch.int32, device="cuda")
+    seq, pos = at // 64, at % 64
+    proj, cq = torch.randn(n, rank + rot + q_rank, device="cuda"), torch.empty(n, q_rank, device="cuda")
+    cos = sin = torch.rand(64, rot // 2, device="cuda")
+    ones = torch.ones(rank, device="cuda")
+
+    def best(queries):
+        took = []
+        for _ in range(5):
+            before, after = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                for _ in range(50):
+                    ops.latent_prepare(proj, 0, rank + rot, ones, ones[:q_rank] if queries else None, cq if queries else None, k, v, cos, sin,
+                                       seq, pos, table, n, rank, rot, rot, False, 1e-6)
+            graph.replay()
+            before.record()
+            graph.replay()
+            after.record()
+            torch.cuda.synchronize()
+            took.append(before.elapsed_time(after))
+        return min(took)
+    assert best(False) < 0.85 * best(True)
+
+
 def test_prompts_of_many_sequences_take_time_in_proportion():
     """The scan of 1,536 short sequences against that of 96: sixteen times the work is not a hundred times as slow."""
     import torch
