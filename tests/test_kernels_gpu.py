@@ -1037,6 +1037,44 @@ def test_gemm_f32_takes_no_more_than_its_share_of_time():
     assert best(1000, 32768, 2048, 2) < 13 * best(64, 32768, 2048, 2)
 
 
+def test_scaled_embedding_of_half_as_many_bytes_takes_no_longer():
+    """1,184 rows of width 7,168 from a bfloat16 table against a float32 one (the rows that are written are the same)."""
+    from qwen3_b200.csrc import ops
+    ids = torch.randint(0, 5000, (1184,), device="cuda", dtype=torch.int32)
+    out = torch.empty(1184, 7168, device="cuda")
+
+    def best(dtype):
+        table, took = torch.randn(5000, 7168, device="cuda").to(dtype), []
+        for _ in range(5):
+            before, after = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                for _ in range(40):
+                    ops.embedding_scaled(ids, table, out, 2.0)
+            graph.replay()
+            before.record()
+            graph.replay()
+            after.record()
+            torch.cuda.synchronize()
+            took.append(before.elapsed_time(after))
+        return min(took)
+    assert best(torch.bfloat16) < 1.25 * best(torch.float32)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("hidden", [4, 508, 510, 512, 516, 1028, 2052])
+def test_scaled_embedding_in_fours_and_value_by_value(hidden, dtype):
+    """Widths on both sides of the rule and ones that leave threads without a packet; ids outside the table give zero rows."""
+    from qwen3_b200.csrc import ops
+    table = torch.randn(7, hidden, device="cuda").to(DT[dtype])
+    ids = torch.tensor([6, 0, -1, 3, 7, 3], dtype=torch.int32, device="cuda")
+    out = torch.full((6, hidden), 9.0, device="cuda")
+    ops.embedding_scaled(ids, table, out, 1.5)
+    inside = (ids >= 0) & (ids < 7)
+    want = torch.where(inside[:, None], table[ids.clamp(0, 6).long()].float() * 1.5, 0.0)
+    assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("rows", [1, 4])
 def test_sampling_short_rows_without_top_k_takes_no_longer_than_long_ones(rows):
     """A quarter of the logits, drawn from without top-k, in less time than all of them (medians over several rows of logits)."""
