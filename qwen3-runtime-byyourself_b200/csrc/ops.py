@@ -1003,12 +1003,11 @@ def moe_experts(h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, 
     if w_gate_up.numel() != n_real * (2 if gated else 1) * ff * hidden or w_down.numel() != n_real * hidden * ff or act.numel() < n_pairs * ff \
             or y.numel() < n_pairs * hidden or y.dtype != torch.float32 or act.dtype != h.dtype or w_gate_up.dtype != h.dtype:
         raise KernelError("moe_experts: shapes do not fit")
-    tensor_cores = h.dtype == torch.bfloat16 and hidden % 32 == 0 and ff % 32 == 0 and moe_tensor_cores
     ptrs = [_dev(h, "h"), _dev(w_gate_up, "w_gate_up"), _dev(w_down, "w_down"), _dev(offsets, "offsets", torch.int32),
             _dev(pair_of_slot, "pair_of_slot", torch.int32)]
     numbers = [int(n_pairs), int(n_real), int(top), hidden, int(ff), float(limit), float(alpha), float(up_offset), int(bool(gated))]
     kinds = [c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int]
-    if tensor_cores and moe_wide(n_pairs, n_real):
+    if moe_wide(h.dtype, hidden, ff, n_pairs, n_real):
         if rows is None:
             rows = torch.empty(n_pairs, hidden, dtype=h.dtype, device=h.device)
         if rows.numel() < n_pairs * hidden or rows.dtype != h.dtype:
@@ -1017,16 +1016,20 @@ def moe_experts(h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, 
         _check(fn(*ptrs, _dev(rows, "rows"), _dev(act, "act"), _dev(y, "y"), *numbers, _status_word(h.device).data_ptr(), _stream()), "moe_experts")
         _count_extra(2)
         return
-    name = "q3_moe_experts_tc_bf16" if tensor_cores else f"q3_moe_experts_{_suffix(h)}"
+    name = "q3_moe_experts_tc_bf16" if _moe_on_tensor_cores(h.dtype, hidden, ff) else f"q3_moe_experts_{_suffix(h)}"
     fn = _fn("moe.cu", name, [c_void_p] * 7 + kinds + [c_void_p])
     _check(fn(*ptrs, _dev(act, "act"), _dev(y, "y"), *numbers, _stream()), "moe_experts")
     _count_extra(1)
 
 
-def moe_wide(n_pairs: int, n_real: int) -> bool:
-    """Whether the experts' bfloat16 products run on tcgen05 tiles of many tokens (moe_tcgen05.cu) and not on the kernel for a
-    few tokens per expert: from MOE_WIDE_PAIRS pairs per expert on average."""
-    return n_pairs >= MOE_WIDE_PAIRS * n_real
+def _moe_on_tensor_cores(dtype, hidden: int, ff: int) -> bool:
+    return dtype == torch.bfloat16 and hidden % 32 == 0 and ff % 32 == 0 and moe_tensor_cores
+
+
+def moe_wide(dtype, hidden: int, ff: int, n_pairs: int, n_real: int) -> bool:
+    """Whether the experts' products run on tcgen05 tiles of many tokens (moe_tcgen05.cu; `moe_experts` then wants `rows`) and not on a
+    kernel for a few tokens per expert or without tensor cores: from MOE_WIDE_PAIRS pairs per expert on average."""
+    return _moe_on_tensor_cores(dtype, hidden, ff) and n_pairs >= MOE_WIDE_PAIRS * n_real
 
 
 # Both forms, 16 experts, microseconds from cold caches (few / wide): 2 pairs per expert 77 / 103 at width 2,048 and 194 / 220 at

@@ -286,6 +286,24 @@ def test_latent_of_the_queries_has_the_same_bits_in_every_step(dtype, q_rank):
     assert torch.equal(one[0], cq[4])
 
 
+@pytest.mark.parametrize("dtype,ff,held", [("bfloat16", 32, True), ("bfloat16", 40, False), ("float32", 32, False)])
+def test_room_for_the_pairs_rows_is_asked_for_where_it_is_used(tmp_path, dtype, ff, held):
+    """Only the experts' products on tcgen05 tiles gather the pairs' rows first."""
+    import torch
+    import qwen3_b200 as q
+    from qwen3_b200.engine.engine import Engine
+    spec = {"architecture": "Fagunex", "vocab": 64, "width": 64, "norm": {"eps": 1e-5},
+            "layers": [layer(hgrn2(1, 16, 16), moe_spec(ff, 2, 2, shared=16))]}
+    config = q.config_from_dict(spec)
+    model = q.build_model(config.plan())
+    model.bind(q.random_weights(model.weight_specs(), seed=3, dtype=torch_dtype(dtype), device="cuda"), torch_dtype(dtype), "cuda")
+    engine = Engine(model, config, max_tokens=128)
+    slot = engine.new_sequence()
+    logits = engine.step([q.StepEntry(slot, list(range(40)), [39])])
+    assert bool(torch.isfinite(logits).all())
+    assert any(key[0] == "moe.rows" for key in engine.scratch._flat) == held
+
+
 def test_latents_without_a_latent_of_the_queries_take_less_time():
     """4,100 tokens: the keys' latents alone against those of the keys and, beside them, short ones of the queries."""
     import torch
