@@ -8,6 +8,7 @@ to a library: a CPU tensor or a missing compiler is an error.
 from __future__ import annotations
 
 import ctypes
+import math
 import os
 from dataclasses import dataclass
 from ctypes import c_float, c_int, c_int64, c_uint64, c_void_p
@@ -1007,7 +1008,7 @@ def moe_experts(h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, 
             _dev(pair_of_slot, "pair_of_slot", torch.int32)]
     numbers = [int(n_pairs), int(n_real), int(top), hidden, int(ff), float(limit), float(alpha), float(up_offset), int(bool(gated))]
     kinds = [c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int]
-    if moe_wide(h.dtype, hidden, ff, n_pairs, n_real):
+    if moe_wide(h.dtype, hidden, ff, n_pairs, n_real, gated):
         if rows is None:
             rows = torch.empty(n_pairs, hidden, dtype=h.dtype, device=h.device)
         if rows.numel() < n_pairs * hidden or rows.dtype != h.dtype:
@@ -1026,14 +1027,26 @@ def _moe_on_tensor_cores(dtype, hidden: int, ff: int) -> bool:
     return dtype == torch.bfloat16 and hidden % 32 == 0 and ff % 32 == 0 and moe_tensor_cores
 
 
-def moe_wide(dtype, hidden: int, ff: int, n_pairs: int, n_real: int) -> bool:
+def moe_wide(dtype, hidden: int, ff: int, n_pairs: int, n_real: int, gated: bool = True) -> bool:
     """Whether the experts' products run on tcgen05 tiles of many tokens (moe_tcgen05.cu; `moe_experts` then wants `rows`) and not on a
-    kernel for a few tokens per expert or without tensor cores: from MOE_WIDE_PAIRS pairs per expert on average."""
-    return _moe_on_tensor_cores(dtype, hidden, ff) and n_pairs >= MOE_WIDE_PAIRS * n_real
+    kernel for a few tokens per expert or without tensor cores.
+
+    The tiles read all experts' weights at the memory's rate, after a start of about 40 us; the kernel for few tokens reads those of the
+    experts that tokens chose, at a lower rate, and again for every 8 pairs of an expert.  So the tiles are ahead from MOE_WIDE_PAIRS
+    pairs per expert on average, and with large weights as soon as most experts are chosen."""
+    if not _moe_on_tensor_cores(dtype, hidden, ff):
+        return False
+    if n_pairs >= MOE_WIDE_PAIRS * n_real:
+        return True
+    weights = (6.0 if gated else 4.0) * n_real * hidden * ff            # bytes
+    chosen = 1.0 - math.exp(-n_pairs / n_real)                          # of the experts, about
+    return weights * chosen / 4.6e6 > weights / 6.2e6 + 40.0
 
 
-# Both forms, 16 experts, microseconds from cold caches (few / wide): 2 pairs per expert 77 / 103 at width 2,048 and 194 / 220 at
-# 4,096; 4 pairs 91 / 103 and 200 / 220; 6 pairs 108 / 103 and 265 / 241; 16 pairs 146 / 106 and 388 / 247.
+# Both forms, microseconds from cold caches (few / wide), experts x ff at width: 16 x 2,048 at 2,048, 2 pairs per expert 77 / 103, 4 pairs
+# 95 / 103, 6 pairs 108 / 103, 16 pairs 146 / 106; 8 x 3,072 at 4,096, 4 pairs 120 / 138; 64 x 1,408 at 2,048, 3 pairs 226 / 211;
+# 128 x 768 at 2,048, 4 pairs 320 / 238; 256 x 1,024 at 4,096, 1 pair 970 / 1,030, 2 pairs 1,254 / 1,033, 4 pairs 1,504 / 1,033.  With
+# every token on the same experts, 64 x 1,408 at 3 pairs 116 / 66, 128 x 768 at 4 pairs 199 / 89.
 MOE_WIDE_PAIRS = 5
 
 

@@ -132,7 +132,7 @@ class RoutedExperts(Part):
         y = s.get("moe.y", (P, H), torch.float32)
         if self.experts:
             act = s.get("moe.act", (P, I), ctx.dtype)
-            rows = s.get("moe.rows", (P, H), ctx.dtype) if ops.moe_wide(ctx.dtype, H, I, P, self.experts) else None
+            rows = s.get("moe.rows", (P, H), ctx.dtype) if ops.moe_wide(ctx.dtype, H, I, P, self.experts, self.gated) else None
             ops.moe_experts(x, self.w_gate_up, self.w_down, offsets, pair_of_slot, act, y, P, self.experts, top, I, self.limit,
                             self.alpha, self.up_offset, gated=self.gated, rows=rows)
         shared = None

@@ -364,6 +364,70 @@ def test_router_by_lanes_and_with_four_tokens_a_block(outputs, real, top, correc
         assert torch.equal(x[picked][finite], y[finite])
 
 
+def test_experts_that_every_token_chooses_take_less_time():
+    """64 tokens on the same 8 of 128 experts (75 MB of weights) against 64 tokens on all of them (1.2 GB)."""
+    import torch
+    from qwen3_b200.csrc import ops
+    experts, top, hidden, ff, n = 128, 8, 2048, 768, 64
+    pairs = n * top
+    w_up = torch.randn(experts, 2 * ff, hidden, device="cuda", dtype=torch.bfloat16)
+    w_down = torch.randn(experts, hidden, ff, device="cuda", dtype=torch.bfloat16)
+    h, away = torch.randn(n, hidden, device="cuda", dtype=torch.bfloat16), torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
+    act, y = torch.empty(pairs, ff, device="cuda", dtype=torch.bfloat16), torch.empty(pairs, hidden, device="cuda")
+    rows = torch.empty(pairs, hidden, device="cuda", dtype=torch.bfloat16)
+
+    def best(ids):
+        offsets = torch.empty(experts + 1, dtype=torch.int32, device="cuda")
+        slot, pair = (torch.empty(pairs, dtype=torch.int32, device="cuda") for _ in range(2))
+        ops.moe_sort(ids.to("cuda", torch.int32).reshape(-1).contiguous(), pairs, experts, offsets, slot, pair)
+        took = []
+        for _ in range(6):
+            before, after = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            away.zero_()
+            before.record()
+            ops.moe_experts(h, w_up, w_down, offsets, pair, act, y, pairs, experts, top, ff, float("inf"), 1.0, 0.0, rows=rows)
+            after.record()
+            torch.cuda.synchronize()
+            took.append(before.elapsed_time(after))
+        return min(took)
+    assert best(torch.arange(top).expand(n, top)) < 0.5 * best(torch.stack([torch.randperm(experts)[:top] for _ in range(n)]))
+
+
+@pytest.mark.parametrize("hidden,ff,experts,top", [(128, 96, 4, 2), (256, 160, 8, 3)])
+def test_a_token_on_either_side_of_the_experts_rule(hidden, ff, experts, top, monkeypatch):
+    """The bits of a token's experts hang on the form that the number of pairs selects; the two forms are sums of the same products in
+    two orders, in 32-bit: bfloat16 activations may round apart, by 2^-8 of themselves, and the results by what those weigh."""
+    import torch
+    from qwen3_b200.csrc import ops
+    gen = torch.Generator(device="cuda").manual_seed(hidden)
+    n = 2 * experts
+    h = torch.randn(n, hidden, generator=gen, device="cuda").to(torch.bfloat16)
+    w_up = (torch.randn(experts, 2 * ff, hidden, generator=gen, device="cuda") / hidden ** 0.5).to(torch.bfloat16)
+    w_down = (torch.randn(experts, hidden, ff, generator=gen, device="cuda") / ff ** 0.5).to(torch.bfloat16)
+    ids = torch.rand(n, experts, generator=gen, device="cuda").argsort(1)[:, :top].to(torch.int32)
+    assert not ops.moe_wide(torch.bfloat16, hidden, ff, top, experts) and ops.moe_wide(torch.bfloat16, hidden, ff, n * top * 5, experts)
+
+    def run(tokens, wide):
+        monkeypatch.setattr(ops, "MOE_WIDE_PAIRS", 0 if wide else 10 ** 9)
+        pairs = len(tokens) * top
+        offsets = torch.empty(experts + 1, dtype=torch.int32, device="cuda")
+        slot, pair = (torch.empty(pairs, dtype=torch.int32, device="cuda") for _ in range(2))
+        ops.moe_sort(ids[tokens].reshape(-1).contiguous(), pairs, experts, offsets, slot, pair)
+        act, y = torch.empty(pairs, ff, device="cuda", dtype=torch.bfloat16), torch.empty(pairs, hidden, device="cuda")
+        ops.moe_experts(h[tokens].contiguous(), w_up, w_down, offsets, pair, act, y, pairs, experts, top, ff, float("inf"), 1.0, 0.0)
+        return y[slot.long()].view(len(tokens), top, hidden), act[slot.long()].view(len(tokens), top, ff)
+    alone = run([3], False)
+    for wide in (False, True):
+        y, act = run(list(range(n)), wide)
+        if not wide:
+            assert torch.equal(y[3], alone[0][0]) and torch.equal(act[3], alone[1][0])
+        apart = (act[3].double() - alone[1][0].double()).abs()
+        assert bool((apart <= 2.0 ** -8 * act[3].double().abs() + 2.0 ** -20).all())
+        w = w_down[ids[3].long()].double().abs()                                            # [top, hidden, ff]
+        weighed = torch.einsum("tf,thf->th", apart, w) + ff * 2.0 ** -24 * 2 * torch.einsum("tf,thf->th", act[3].double().abs(), w)
+        assert bool(((y[3] - alone[0][0]).double().abs() <= weighed + 1e-30).all())
+
+
 def test_router_of_a_long_prompt_takes_its_share_of_time():
     """4,100 tokens and 300 outputs against 64 tokens, whose blocks are all resident at once."""
     import torch
