@@ -440,7 +440,8 @@ moe_down_kernel(const T* __restrict__ act, const T* __restrict__ w_down, const i
 
 // Bound by the bytes of y, the shared expert's rows and the output; rows of whole 16-byte packets in packets (VEC), the slots
 // and weights of the token read once.  4,162 tokens of width 4,096, two experts and a shared one: 85.7 us value by value,
-// 35.9 in packets; a decode step of 8 tokens of width 2,048: 7.6 and 2.9.
+// 35.9 in packets; a decode step of 8 tokens of width 2,048: 7.6 and 2.9.  Below 512 the threads of value by value are ahead
+// (1,184 tokens of width 96: 2.3 us, 2.5 in packets).
 template <typename T, int VEC>
 __global__ void moe_combine_kernel(const float* __restrict__ y, const T* __restrict__ h, const int* __restrict__ slot_of_pair,
                                    const float* __restrict__ top_w, const float* __restrict__ id_weight, T* __restrict__ out,
@@ -705,7 +706,7 @@ int moe_experts_launch(const T* h, const T* w_gate_up, const T* w_down, const in
         if (n_tokens <= 0) return 0;                                                                                      \
         if (n_tokens > 0x7fffffffLL) return Q3_ERR_BAD_SIZE;                                                              \
         constexpr int V = Pack<T>::N;                                                                                     \
-        if (hidden % V == 0 && aligned16(y) && aligned16(h) && aligned16(out) && (shared == nullptr || aligned16(shared))) { \
+        if (hidden % V == 0 && hidden >= 512 && aligned16(y) && aligned16(h) && aligned16(out) && (shared == nullptr || aligned16(shared))) { \
             const int threads = hidden / V >= 256 ? 256 : (hidden / V + 31) / 32 * 32;                                    \
             return (int)q3_launch(moe_combine_kernel<T, V>, dim3((unsigned)n_tokens), dim3(threads), 0, (cudaStream_t)stream, y, \
                                   (const T*)h, slot_of_pair, top_w, id_weight, (T*)out, top, hidden, (const T*)shared, shared_w); \

@@ -428,6 +428,23 @@ def test_a_token_on_either_side_of_the_experts_rule(hidden, ff, experts, top, mo
         assert bool(((y[3] - alone[0][0]).double().abs() <= weighed + 1e-30).all())
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("hidden", [96, 504, 512, 520])
+def test_combining_on_both_sides_of_the_width_for_packets(dtype, hidden):
+    import torch
+    from qwen3_b200.csrc import ops
+    N, top, T = 6, 2, torch.float32 if dtype == "float32" else torch.bfloat16
+    gen = torch.Generator(device="cuda").manual_seed(hidden)
+    y, w = torch.randn(N * top, hidden, generator=gen, device="cuda"), torch.rand(N * top, generator=gen, device="cuda")
+    h, idw = torch.randn(N, hidden, generator=gen, device="cuda").to(T), torch.rand(N, generator=gen, device="cuda")
+    slots = torch.randperm(N * top, generator=gen, device="cuda").to(torch.int32)
+    out = torch.empty_like(h)
+    ops.moe_combine(y, h, slots, w, idw, out, top)
+    want = (y[slots.long()].double() * w.double()[:, None]).view(N, top, hidden).sum(1) + idw.double()[:, None] * h.double()
+    size = (y[slots.long()].double() * w.double()[:, None]).abs().view(N, top, hidden).sum(1) + (idw.double()[:, None] * h.double()).abs()
+    assert bool(((out.double() - want).abs() <= 4 * 2.0 ** -24 * size + (0.0 if dtype == "float32" else 2.0 ** -8 * want.abs())).all())
+
+
 def test_router_of_a_long_prompt_takes_its_share_of_time():
     """4,100 tokens and 300 outputs against 64 tokens, whose blocks are all resident at once."""
     import torch
