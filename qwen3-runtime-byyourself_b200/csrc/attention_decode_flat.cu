@@ -95,6 +95,11 @@ __device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
     return r;
 }
 
+// A mask for a register of two bfloat16 values, of keys `key` and `key` + 1: all ones where the key lies in [lo, pos].
+__device__ __forceinline__ uint32_t keys_seen(int key, int lo, int pos) {
+    return (key >= lo && key <= pos ? 0x0000ffffu : 0u) | (key + 1 >= lo && key + 1 <= pos ? 0xffff0000u : 0u);
+}
+
 // Pages that the query of token t reads, from page `first` on.
 struct Row {
     int pos, lo, first, n;
@@ -295,7 +300,8 @@ decode_flat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                 for (int e = 0; e < 4; ++e) sc[e] = (sc[e] + sd[e]) * a.scale_log2;
                 // keys outside [lo, pos]; sc[0], sc[1] are of key page*64 + warp*16 + quad, sc[2], sc[3] of the eighth after it
                 const int key0 = (row.first + p) * PAGE;
-                if (key0 < row.lo || key0 + PAGE - 1 > pos) {
+                const bool edge = key0 < row.lo || key0 + PAGE - 1 > pos;
+                if (edge) {
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const int key = key0 + warp * KEYS + quad + h * 8;
@@ -328,11 +334,25 @@ decode_flat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                     }
                 }
                 const int vrow = warp * KEYS + (lane & 7) + ((lane >> 4) << 3);
+                if (edge) {
+                    // what the page holds outside [lo, pos] was left by whoever had it before: its weight is zero, and zero times an
+                    // infinity or a NaN would not be zero
+                    const int key = key0 + warp * KEYS + tq * 2;
+                    const uint32_t near = keys_seen(key, row.lo, pos), far = keys_seen(key + 8, row.lo, pos);
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt) {
-                    uint32_t va[4];
-                    ldmatrix_x4_trans(va, vbuf + packet(vrow, 2 * mt + ((lane >> 3) & 1)));
-                    mma_bf16(o[mt], va, pb0, pb1);
+                    for (int mt = 0; mt < MT; ++mt) {
+                        uint32_t va[4];
+                        ldmatrix_x4_trans(va, vbuf + packet(vrow, 2 * mt + ((lane >> 3) & 1)));
+                        va[0] &= near; va[1] &= near; va[2] &= far; va[3] &= far;
+                        mma_bf16(o[mt], va, pb0, pb1);
+                    }
+                } else {
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt) {
+                        uint32_t va[4];
+                        ldmatrix_x4_trans(va, vbuf + packet(vrow, 2 * mt + ((lane >> 3) & 1)));
+                        mma_bf16(o[mt], va, pb0, pb1);
+                    }
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(empty + bar);

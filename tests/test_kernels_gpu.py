@@ -1099,6 +1099,38 @@ def test_sampling_short_rows_without_top_k_takes_no_longer_than_long_ones(rows):
     assert sorted(times[4096])[4] < 0.95 * sorted(times[16384])[4], times
 
 
+@pytest.mark.parametrize("d,window", [(64, None), (128, None), (128, 50)])
+def test_decode_attention_with_pages_shared_out_takes_nothing_from_rows_that_are_not_its_keys(d, window):
+    """Infinities and NaN in every row of the pages beyond the newest key and before the window, as a sequence that had the pages
+    before may leave them: the results are those over clean pages."""
+    from qwen3_b200.csrc import ops
+    rng = np.random.default_rng(d)
+    nq, nkv, lengths = 8, 2, [70, 130, 64, 1, 449]
+    table, kp, vp = paged_case(rng, lengths, nkv, d, "bfloat16")
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    kp.normal_(generator=gen)
+    vp.normal_(generator=gen)
+    B, table_d = len(lengths), torch.as_tensor(table).cuda()
+    seq = torch.arange(B, dtype=torch.int32, device="cuda")
+    pos = torch.as_tensor([n - 1 for n in lengths], dtype=torch.int32).cuda()
+    qkv = torch.randn(B, (nq + 2 * nkv) * d, generator=gen, device="cuda").to(torch.bfloat16)
+    parts = torch.empty(ops.attention_decode_flat_parts(d, nq // nkv), dtype=torch.float32, device="cuda")
+    counters = torch.zeros(B * nkv, dtype=torch.int32, device="cuda")
+    foul_k, foul_v = torch.full_like(kp, float("inf")), torch.full_like(vp, float("nan"))
+    foul_v[..., ::2] = -float("inf")
+    for s, n in enumerate(lengths):
+        for at in range(max(0, n - window) if window else 0, n - 1):                    # the newest row is the kernel's to write
+            page = int(table[s, at // 64])
+            foul_k[page, :, at % 64], foul_v[page, :, at % 64] = kp[page, :, at % 64], vp[page, :, at % 64]
+    got = []
+    for k, v in ((kp, vp), (foul_k, foul_v)):
+        out = torch.empty(B, nq * d, dtype=torch.bfloat16, device="cuda")
+        ops.attention_decode_fused(qkv, k, v, out, None, None, None, None, 0.0, seq, pos, table_d, B, nq, nkv, d, d ** -0.5, window, 3,
+                                   parts=parts, counters=counters)
+        got.append(out)
+    assert bool(torch.isfinite(got[0]).all()) and torch.equal(got[0], got[1])
+
+
 @pytest.mark.parametrize("form", ["cluster", "shared out", "split"])
 def test_decode_attention_reads_a_cache_that_another_kernel_writes_after_that_kernel(form):
     """With dependent launch on, behind a slow kernel and the one that writes the new token's key and value into the pages: the
