@@ -5,7 +5,10 @@
 // A row is one (sequence, kv head): the pages of 64 keys that its query reads, with the query heads of the group as the
 // eight columns of mma.m16n8k16 (keys and values are its 16-row operands).  Rows are cut into parts of at most `c` pages,
 // c being the smallest number that gives no more parts than blocks are resident at once: contexts of unequal length take
-// about as long as equal ones of the same total.  Every block finds c and its part from the positions by itself.
+// about as long as equal ones of the same total.  Where there are more rows than blocks, or long ones that leave many blocks
+// without, c is smaller and a block takes several parts, if that should be ahead (`time_of`); short rows beyond the grid are taken
+// whole.  Every block finds c and its parts from the positions by itself; c, and with it the order of a row's sums, hangs on the
+// lengths of all sequences of the step.
 //   warp 4     copies the pages' K and V panels (16 KB each at head size 128, contiguous) by TMA into a ring.  (With
 //              cp.async, as in attention_decode.cu, an SM does not move more than about 45 GB/s whatever is in flight.)
 //   warps 0-3  take 16 of a page's 64 keys each, with an online softmax of their own, and meet at the end of the part.
@@ -15,10 +18,10 @@
 // `parts` and counts itself at the row's counter; the one that comes last adds them up, in the order of the parts - a
 // fixed order whichever comes last - and sets the counter back to zero.  Nobody waits for another block.
 //
-// Bound by its chain of steps, not by memory: 64 sequences of 130 tokens, 32 heads over 8 of 128, 19.4 us for 34 MB where the
-// form of attention_decode.cu, which does not split so many rows and runs them in two waves, takes 28.9; 16 of 250 to 1,500
-// tokens 20.7 and 21.7.  Where that form has blocks to split the rows with it is ahead: 8 sequences of 3,500 tokens 27.1 there,
-// 30.0 here; one of 24,571 tokens 32.6 and 43.8.
+// Bound by its chain of steps with short contexts, by memory with long ones: 64 sequences of 130 tokens, 32 heads over 8 of 128, 17 us
+// for 34 MB where the form of attention_decode.cu, which does not split so many rows and runs them in two waves, takes 29; 64 of 60 to
+// 8,000 tokens 170 and 218; one of 24,000 among 63 of 100 43 and 257 (250 here with whole rows); 96 of 4,000 230 and 252 (6.9 TB/s);
+// 64 of 16,000 620 and 630.  Equal rows that are a little more than the grid are its worst: 64 of 6,000 257 and 246.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -43,6 +46,8 @@ constexpr int MAX_STAGES = 4;
 constexpr int MT = D / 16, KT = D / 16;             // tiles of 16 values of the output, of a score's dot
 constexpr int LDO = D + 4;                          // a result row in shared memory: the lanes' stores fall into different banks
 constexpr int MIN_PART = 4;                         // pages below which a row is not cut
+constexpr int MAX_WAVES = 8;                        // parts of a block, where rows are cut
+constexpr int LONG_ROW = 48;                        // pages of the longest row from which more rows than blocks are cut
 constexpr int BLOCKS_PER_SM = 3;
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
@@ -75,7 +80,7 @@ struct Args {
     bf16* k_pages;
     bf16* v_pages;
     bf16* out;                     // [tokens, nq * D]
-    float* parts;                  // [blocks][G][D + 2]: sums, then (max, sum)
+    float* parts;                  // [MAX_WAVES blocks][G][D + 2]: sums, then (max, sum)
     int* counters;                 // [tokens * nkv], zero between launches
     const float* q_norm_w;         // [D] or null
     const float* k_norm_w;
@@ -123,8 +128,41 @@ __device__ __forceinline__ int count_parts(const Args& a, int c, int lane, int m
     return count * a.nkv;
 }
 
+// Pages of the busiest block when every block takes whole rows, every gridDim.x-th (by one warp).
+__device__ __forceinline__ int busiest_block(const Args& a, int lane) {
+    int most = 0;
+    for (int block = lane; block < (int)gridDim.x; block += 32) {
+        int pages = 0;
+        for (int row = block; row < a.n_tokens * a.nkv; row += (int)gridDim.x) pages += Row(a, row / a.nkv).n;
+        most = max(most, pages);
+    }
+    return __reduce_max_sync(0xffffffffu, most);
+}
+
+// What a step takes, in microseconds, from the pages of its busiest block and of all blocks on average.  (Fitted to measured steps of 56 to
+// 128 sequences of 8 kv heads, 60 to 24,000 tokens, with whole rows and cut ones: within a tenth for most.)
+__device__ __forceinline__ float time_of(float busiest, float share) { return 0.65f * busiest + 1.25f * share; }
+
+// Long rows that fill the grid badly - more of them than blocks, so that some blocks have a row when the others are done, or a little
+// more than half as many: several parts a block where that should be ahead.  A part more is 6 us of starts and ends, a part of a row
+// 0.5 where they are added up.  Returns the pages of a part.  (Not inlined: steps of short rows, which do not come here, took 1 us longer.)
+__device__ __noinline__ int cut_long_rows(const Args& a, int c, int most, int share, int first_pages) {
+    const int grid = gridDim.x, lane = threadIdx.x & 31;
+    const float as_is = a.n_tokens * a.nkv > grid ? time_of(busiest_block(a, lane), share) : time_of(c, share) + 6.0f + 0.5f * parts_of(most, c);
+    float least = 0.93f * as_is;
+    for (int m = 1; m <= MAX_WAVES - 2; ++m) {
+        const int smaller = max(MIN_PART, (share + m - 1) / m), parts = count_parts(a, smaller, lane, first_pages);
+        const float time = time_of(share + 0.5f * smaller, share) + 6.0f * ((parts + grid - 1) / grid) + 0.5f * parts_of(most, smaller);
+        if (parts <= MAX_WAVES * grid && time < least) {
+            least = time;
+            c = smaller;
+        }
+    }
+    return c;
+}
+
 __global__ void __launch_bounds__(THREADS, BLOCKS_PER_SM)
-decode_flat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const Args a) {
+decode_flat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const __grid_constant__ Args a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int G = a.nq / a.nkv, stages = a.stages;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -159,14 +197,16 @@ decode_flat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
             total += __reduce_add_sync(0xffffffffu, n);
             most = max(most, __reduce_max_sync(0xffffffffu, n));
         }
-        int lo = max(MIN_PART, (int)((total * a.nkv + gridDim.x - 1) / gridDim.x));
+        const int grid = gridDim.x, share = (int)((total * a.nkv + grid - 1) / grid);
+        int lo = max(MIN_PART, share);
         int hi = max(lo, most);                  // whole rows: as many parts as there are rows, whether they fit or not
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
-            if (count_parts(a, mid, lane, first_pages) <= (int)gridDim.x) hi = mid;
+            if (count_parts(a, mid, lane, first_pages) <= grid) hi = mid;
             else lo = mid + 1;
         }
         c = lo;
+        if (most >= LONG_ROW) c = cut_long_rows(a, c, most, share, first_pages);
     }
     __syncthreads();                             // the barriers are set up
 
@@ -178,7 +218,7 @@ decode_flat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     int s = 0;                                   // place in the ring
     uint32_t phase = 0;
     bool ok = true, waited = false;
-    // this block's parts: of a list that is longer than the grid (rows that are not cut) every gridDim.x-th
+    // this block's parts: of a list that is longer than the grid every gridDim.x-th
     int before = 0, chunk = blockIdx.x;      // parts of the tokens before `base`
     for (int base = 0; base < a.n_tokens; base += 32) {
         const int n = base == 0 ? first_pages : pages_of(a, base + lane);
@@ -474,7 +514,7 @@ Q3_EXPORT int q3_attention_decode_flat_blocks(int group) { return blocks_per_sm(
 
 // Float32 elements of `parts`; `counters` holds n_tokens * nkv ints, zero before the first launch and left zero by each.
 Q3_EXPORT int64_t q3_attention_decode_flat_parts(int group) {
-    return (int64_t)q3_attention_decode_flat_blocks(group) * group * (D + 2);
+    return (int64_t)MAX_WAVES * q3_attention_decode_flat_blocks(group) * group * (D + 2);
 }
 
 Q3_EXPORT int q3_attention_decode_flat_bf16(const void* qkv, void* k_pages, void* v_pages, void* out, float* parts, int* counters,

@@ -1131,6 +1131,72 @@ def test_decode_attention_with_pages_shared_out_takes_nothing_from_rows_that_are
     assert bool(torch.isfinite(got[0]).all()) and torch.equal(got[0], got[1])
 
 
+def _decode_case(lengths, nq, nkv, d, seed):
+    """Pages, tables and projections of a decode step; pages of a sequence that is longer than 64 tokens are its own."""
+    rng = np.random.default_rng(seed)
+    table, kp, vp = paged_case(rng, lengths, nkv, d, "bfloat16")
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    kp.normal_(generator=gen)
+    vp.normal_(generator=gen)
+    B = len(lengths)
+    qkv = torch.randn(B, (nq + 2 * nkv) * d, generator=gen, device="cuda").to(torch.bfloat16)
+    seq, pos = torch.arange(B, dtype=torch.int32, device="cuda"), torch.as_tensor([n - 1 for n in lengths], dtype=torch.int32).cuda()
+    return torch.as_tensor(table).cuda(), kp, vp, qkv, seq, pos
+
+
+@pytest.mark.parametrize("nq,nkv,d,lengths,window", [
+    (16, 8, 64, [3000 - 31 * i for i in range(63)] + [9000], None),       # more rows than blocks, cut into several parts a block
+    (16, 8, 64, [100] * 63 + [24000], None),                              # one long among many short
+    (16, 8, 64, [100] * 63 + [24000], 5000),
+    (16, 8, 64, [20 + i % 180 for i in range(449)] + [5000], None),       # more rows than parts that there is room for
+    (8, 4, 128, [4000] * 64, None),                                       # rows that fill a little more than half of the blocks
+])
+def test_decode_attention_shared_out_over_more_rows_than_blocks(nq, nkv, d, lengths, window):
+    """The same bits when run again, the counters at zero, and every row within what the rounding of its weights allows (2^-7 of
+    the sum of its weighted values' sizes)."""
+    from qwen3_b200.csrc import ops
+    table, kp, vp, qkv, seq, pos = _decode_case(lengths, nq, nkv, d, len(lengths) + nq)
+    B, G = len(lengths), nq // nkv
+    parts = torch.full((ops.attention_decode_flat_parts(d, G),), float("nan"), device="cuda")
+    counters = torch.zeros(B * nkv, dtype=torch.int32, device="cuda")
+    out = [torch.empty(B, nq * d, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    for o in out:
+        ops.attention_decode_fused(qkv, kp, vp, o, None, None, None, None, 0.0, seq, pos, table, B, nq, nkv, d, d ** -0.5, window, 1,
+                                   parts=parts, counters=counters)
+    assert ops.tcgen05_status("cuda:0") == 0 and not counters.any() and torch.equal(out[0], out[1])
+    for s in list(range(0, B, max(1, B // 24))) + [B - 1]:
+        n = lengths[s]
+        lo = max(0, n - window) if window else 0
+        pages = table[s, :-(-n // 64)].long()
+        ks, vs = (x[pages].double().transpose(1, 2).reshape(-1, nkv, d)[lo:n].transpose(0, 1) for x in (kp, vp))
+        p = torch.softmax(qkv[s, :nq * d].double().view(nkv, G, d) @ ks.transpose(1, 2) * d ** -0.5, dim=-1)
+        bound = 2.0 ** -7 * (1 + 2.0 ** -8) * (p @ vs.abs()) + 1e-6
+        assert bool(((out[0][s].double().view(nkv, G, d) - p @ vs).abs() <= bound).all()), s
+
+
+def test_decode_attention_shares_out_a_long_sequence_among_many_short_ones():
+    """One of 24,000 tokens among 63 of 100 (more rows than blocks) against the same among 31."""
+    from qwen3_b200.csrc import ops
+
+    def best(lengths):
+        nq, nkv, d = 32, 8, 128
+        table, kp, vp, qkv, seq, pos = _decode_case(lengths, nq, nkv, d, 5)
+        parts = torch.empty(ops.attention_decode_flat_parts(d, nq // nkv), device="cuda")
+        counters, out = torch.zeros(len(lengths) * nkv, dtype=torch.int32, device="cuda"), torch.empty(len(lengths), nq * d, dtype=torch.bfloat16, device="cuda")
+        took = []
+        for _ in range(6):
+            before, after = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            before.record()
+            for _ in range(8):
+                ops.attention_decode_fused(qkv, kp, vp, out, None, None, None, None, 0.0, seq, pos, table, len(lengths), nq, nkv, d,
+                                           d ** -0.5, None, 1, parts=parts, counters=counters)
+            after.record()
+            torch.cuda.synchronize()
+            took.append(before.elapsed_time(after))
+        return min(took)
+    assert best([100] * 63 + [24000]) < 3 * best([100] * 31 + [24000])
+
+
 @pytest.mark.parametrize("form", ["cluster", "shared out", "split"])
 def test_decode_attention_reads_a_cache_that_another_kernel_writes_after_that_kernel(form):
     """With dependent launch on, behind a slow kernel and the one that writes the new token's key and value into the pages: the
