@@ -465,7 +465,7 @@ def _decode_fused_kernel(part, qkv, cache, out, ctx, table, q_norm_w, k_norm_w, 
         splits = wide if ctx.max_context > long_context_keys else 8
     parts = counters = None
     # rows (sequences x kv heads) that the form below cannot split any more: parts of equal length instead
-    if ctx.n_tokens * nkv > shared_out_rows and ops.attention_decode_flat_fits(d, nq // nkv):
+    if ctx.n_tokens * nkv > shared_out_rows_per_sm * _sm_count(ctx.device) and ops.attention_decode_flat_fits(d, nq // nkv):
         parts = ctx.scratch.get("attn.decode_parts", (ops.attention_decode_flat_parts(d, nq // nkv),), torch.float32)
         counters = ctx.scratch.counters("attn.decode_counters", ctx.n_tokens * nkv)
     ops.attention_decode_fused(qkv, cache.keys, cache.values, out, q_norm_w, k_norm_w, cos, sin, eps, ctx.token_seq,
@@ -573,11 +573,12 @@ def _decode_capped_fused_kernel(part, qkv, cache, out, ctx, table, q_norm_w, k_n
 
 
 long_context_keys = 4096  # a decode step whose sequences may be longer takes wider clusters (if they are few)
-# Rows (sequences x kv heads) of a decode step beyond which its pages are shared out evenly: the other form has two blocks an SM, so
-# beyond 148 rows it takes every row in one block.  Steps of 12 layers of the 8B shape there / here, us: 20 sequences of 120 tokens
-# 1337 / 1280, of 60 to 3,000 1688 / 1513, 32 of 120 1376 / 1314, 64 of 120 1643 / 1503, 64 of 60 to 960 1790 / 1643, 128 of
-# 150 2293 / 1948.  At 128 rows and below the two are level or that form is ahead.
-shared_out_rows = 148
+# Rows (sequences x kv heads) an SM of a decode step beyond which its pages are shared out evenly: the other form has two blocks an SM,
+# so beyond as many rows as SMs it takes every row in one block.  The attention of 8 kv heads of 128 there / here, us: 19 sequences of 130
+# tokens 12.8 / 7.0, of 4,000 68 / 53, of 16,000 230 / 190; 32 of 130 14.3 / 8.1, of 16,000 338 / 321; 64 of 130 29 / 17, of 4,000 172 / 176,
+# of 16,000 627 / 621; 64 of 60 to 8,000 218 / 170; 128 of 60 to 12,000 520 / 498.  Equal contexts of 4,000 to 6,000 tokens in a few rows more
+# than there are blocks are up to 5 % behind.  With fewer rows steps of the 8B shape were level or that form ahead.
+shared_out_rows_per_sm = 1
 wide_cluster_blocks = 200 # blocks of a decode step with clusters beyond the portable size
 tc_prefill_rows = 128     # from this many new tokens of the longest sequence on, the tcgen05 kernel runs
 # From this many tokens in a step on, the q/k/v product does norm, rotation and cache write in its epilogue: with

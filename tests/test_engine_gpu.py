@@ -296,3 +296,80 @@ def test_8b_layer_shapes_in_32_bit_match_the_plain_model():
         if ("r", p) in one:
             assert np.max(np.abs(one[("r", p)] - exact[p])) <= FP32_TOL, p
     assert float(np.abs(exact).max()) > 0.5      # the bound is meaningful: logits are of order one
+
+
+def _counters(engine):
+    """Every buffer of counters that the engine's launched and captured steps hold."""
+    scratches = [engine.scratch] + [g.scratch for g in list(engine._graphs.values()) + list(engine._long_graphs.values())]
+    return [flat for s in scratches for key, flat in s._flat.items() if key[1] == "counters"]
+
+
+@pytest.mark.parametrize("use_graphs", [True, False])
+def test_engine_with_the_decode_pages_shared_out(folders, use_graphs, monkeypatch):
+    """The decode attention for many sequences in an engine: batches that grow (1, 9, 12 sequences, the larger ones padded when captured)
+    and shrink as requests end, activation buffers between guard zones, counters that are zero again."""
+    import torch
+    from qwen3_b200 import Engine
+    from qwen3_b200.csrc import ops
+    from qwen3_b200.parts import attention as attention_part
+    monkeypatch.setattr(attention_part, "shared_out_rows_per_sm", 0)
+    forms, real = set(), ops.attention_decode_fused
+
+    def fused(*a, **k):
+        forms.add(k.get("parts") is not None)
+        return real(*a, **k)
+    monkeypatch.setattr(ops, "attention_decode_fused", fused)
+    folder, weights = folders["D"]
+    cfg = tiny("D")
+    lengths = [70] + [13, 90, 66, 30, 140, 65, 64, 9, 17] + [20, 33, 131, 7, 64, 72, 11, 100, 129, 40, 5, 128]
+    requests = make_requests(cfg, lengths, seed=12)
+    prompts = {rid: max(1, n - 3 - 2 * (i % 4)) for i, (rid, n) in enumerate(zip(requests, lengths))}
+    ids = list(requests)
+    engine = Engine.from_folder(folder, dtype="bfloat16", max_tokens=64 * 40, use_graphs=use_graphs, guard_scratch=True)
+    for group in (ids[:1], ids[1:10], ids[10:]):
+        steps, rows = schedules.batched({rid: requests[rid] for rid in group}, prompts, len(group))
+        got = run_steps(engine, steps, rows)
+        check(got, {rid: requests[rid] for rid in group}, cfg, weights, "bfloat16", f"{len(group)} sequences, pages shared out")
+    engine.check_kernels()
+    torch.cuda.synchronize()
+    assert forms == {True} and (len(engine._graphs) > 0) == use_graphs
+    assert engine.scratch_violations() == []
+    counters = _counters(engine)
+    assert counters and not any(bool(c.any()) for c in counters)
+
+
+def test_a_layer_that_reads_another_layers_cache_with_the_pages_shared_out(monkeypatch):
+    """Layer 2 attends over layer 0's keys and values, in steps of 5 sequences, with dependent launch as it is by default and for every
+    kernel: the same bits, and those of the other form within what a bfloat16 rounding here and there moves."""
+    import dataclasses
+    import torch
+    import qwen3_b200 as q
+    from qwen3_b200.csrc import ops
+    from qwen3_b200.engine.engine import Engine
+    from qwen3_b200.parts import attention as attention_part
+    cfg = tiny("D", num_hidden_layers=3)
+    config = q.config_from_dict(cfg)
+    plan = config.plan()
+    shared = dataclasses.replace(plan, layers=[plan.layers[0], plan.layers[1], dataclasses.replace(plan.layers[2], cache_from=0)])
+    model = q.build_model(shared)
+    model.bind(q.random_weights(model.weight_specs(), seed=8, dtype=torch.bfloat16, device="cuda"), torch.bfloat16, "cuda")
+    rng = np.random.default_rng(3)
+    prompts = [random_tokens(rng, n, cfg["vocab_size"]) for n in (70, 5, 64, 129, 33)]
+    later = [random_tokens(rng, 5, cfg["vocab_size"]) for _ in range(6)]
+
+    def run(rows_per_sm, pdl):
+        monkeypatch.setattr(attention_part, "shared_out_rows_per_sm", rows_per_sm)
+        ops.set_pdl(pdl)
+        try:
+            engine = Engine(model, config, max_tokens=64 * 20)
+            slots = [engine.new_sequence() for _ in prompts]
+            engine.step([q.StepEntry(s, t, []) for s, t in zip(slots, prompts)])
+            out = [engine.step([q.StepEntry(s, [t], [0]) for s, t in zip(slots, row)]).clone() for row in later]
+            engine.check_kernels()
+            assert not any(bool(c.any()) for c in _counters(engine)) and bool(_counters(engine)) == (rows_per_sm == 0)
+            return torch.stack(out)
+        finally:
+            ops.set_pdl(None)
+    other, got, early = run(10 ** 6, None), run(0, None), run(0, True)
+    assert torch.equal(got, early)
+    assert float((got - other).norm()) <= 0.02 * float(other.norm())
