@@ -11,6 +11,8 @@ def all_variants():
         ("sampling.cu", ()),
         ("attention_decode.cu", ("Q3_HEAD_DIM=128",)),
         ("attention_decode_flat.cu", ("Q3_HEAD_DIM=128",)),
+        # of heads of 64 it is first asked for when a running server has many sequences: not the time to compile
+        ("attention_decode_flat.cu", ("Q3_HEAD_DIM=64",)),
         ("gemm_skinny_bf16.cu", ()),
         ("attention_prefill.cu", ("Q3_HEAD_DIM=128",)),
         ("attention_decode_static.cu", ("Q3_HEAD_DIM=128",)),
