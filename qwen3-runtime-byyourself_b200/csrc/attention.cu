@@ -434,8 +434,11 @@ attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_pages,
 // up to 76 tokens, 8 heads of 32: 17.9 and 3.0; prompts of 183 tokens in all, 32 heads of 128: 96 and 57.  The order of the sums depends on the position alone, not on the step.
 constexpr int PLAIN_WARPS = 8, PLAIN_KEYS = PAGE / PLAIN_WARPS;      // keys of a page that a warp takes
 
+// Heads beyond 128 (CH 2) ask for the values after the scores: with both in registers an SM had one block, and prompts behind a short
+// window, whose blocks do little but start and end, took half as long again as the general form (2,000 tokens, window 20, 8 heads of
+// 256: 186 us there, 283 with one block an SM, 163 with two; a decode step of one sequence of 2,000 tokens 448, 54 and 46).
 template <int LPK, int CH>
-__global__ void __launch_bounds__(PLAIN_WARPS * 32)
+__global__ void __launch_bounds__(PLAIN_WARPS * 32, CH == 1 ? 1 : 2)
 attention_plain_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages,
                        float* __restrict__ out, const int* __restrict__ token_seq, const int* __restrict__ token_pos,
                        const int* __restrict__ page_table, int pages_per_seq, int nq, int nkv, int d, float scale, int window) {
@@ -471,7 +474,7 @@ attention_plain_kernel(const float* __restrict__ q, const float* __restrict__ k_
             for (int n = 0; n < CH; ++n) {
                 const int64_t at = base + (int64_t)j * d + (c + n * LPK) * 4;
                 k4[u][n] = seen[u] && in[n] ? *reinterpret_cast<const float4*>(k_pages + at) : make_float4(0.f, 0.f, 0.f, 0.f);
-                v4[u][n] = seen[u] && in[n] ? *reinterpret_cast<const float4*>(v_pages + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+                if (CH == 1) v4[u][n] = seen[u] && in[n] ? *reinterpret_cast<const float4*>(v_pages + at) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
         float dot[U], m_new = m_run;
@@ -487,6 +490,14 @@ attention_plain_kernel(const float* __restrict__ q, const float* __restrict__ k_
             m_new = fmaxf(m_new, dot[u]);
         }
         if (m_new == -INFINITY) continue;                                // these lanes have seen no key yet
+        if (CH > 1) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int n = 0; n < CH; ++n)
+                    v4[u][n] = seen[u] && in[n] ? *reinterpret_cast<const float4*>(v_pages + base + (int64_t)(j0 + u * SUBS) * d + (c + n * LPK) * 4)
+                                                : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
         const float alpha = expf(m_run - m_new);
         l_run *= alpha;
 #pragma unroll
