@@ -9,11 +9,11 @@
 // without, c is smaller and a block takes several parts, if that should be ahead (`time_of`); short rows beyond the grid are taken
 // whole.  Every block finds c and its parts from the positions by itself; c, and with it the order of a row's sums, hangs on the
 // lengths of all sequences of the step.
-//   warp 4     copies the pages' K and V panels (16 KB each at head size 128, contiguous) by TMA into a ring.  (With
-//              cp.async, as in attention_decode.cu, an SM does not move more than about 45 GB/s whatever is in flight.)
+//   warp 4     copies the pages' K and V panels (16 KB each at head size 128, contiguous) by TMA into a ring.
 //   warps 0-3  take 16 of a page's 64 keys each, with an online softmax of their own, and meet at the end of the part.
-//              A page is a chain of dependent steps - score products, maximum, exponentials, value products - of about a
-//              microsecond, so what counts is how many blocks are on an SM: three with a ring of two pages.
+//              A page is a chain of dependent steps - score products, maximum, exponentials, value products - of 0.65 us for a
+//              block by itself and about 1.25 for one of three on an SM (from steps whose busiest block had 60 to 500 pages), so what
+//              counts is how many blocks are on an SM: three with a ring of two pages.
 // A row that one block holds whole is finished there.  Of a row that is cut, every block leaves its sums in
 // `parts` and counts itself at the row's counter; the one that comes last adds them up, in the order of the parts - a
 // fixed order whichever comes last - and sets the counter back to zero.  Nobody waits for another block.

@@ -1,7 +1,8 @@
 // A routed feed-forward (mixture of experts) in five kernels, none of which needs the host to know how many
 // tokens an expert received, so a step can be captured:
 //
-//   moe_route   : one block per token.  Router logits z = W_r h in 32-bit (ascending order of the sum),
+//   moe_route   : a block per token, or per four tokens of a long prompt.  Router logits z = W_r h in 32-bit (a warp per
+//                 output, a lane's terms in ascending order, then the lanes': one order whatever the step),
 //                 scores s = softmax(z) over all outputs, choice scores s + correction, restricted to the
 //                 `keep` groups (of `count` equal groups of neighbours) whose best choice score is largest;
 //                 the `top` largest choice scores win (ties: the lower index); the weights are their plain
@@ -24,7 +25,9 @@
 //
 // The products accumulate in 32-bit.  Float tiles run on fmaf in ascending order of k whatever the tile a pair falls into, so
 // a token's result does not depend on what else is in the step; bfloat16 tiles run on the tensor cores when the widths are
-// multiples of 32 (few tokens per expert: `few` below; more: moe_tcgen05.cu), else on fmaf too.
+// multiples of 32, else on fmaf too.  Of the two tensor-core forms (few tokens per expert: `few` below, eight warps' shares of K added;
+// more: moe_tcgen05.cu) the step's number of pairs selects one, so there a token's result does hang on the rest of the step, by the
+// rounding of sums in another order.
 #include "common.cuh"
 
 namespace {

@@ -221,7 +221,8 @@ int q3_attention_prefill_tc_bf16(const void* q, const void* k_pages, const void*
                                  int64_t n_tokens, int64_t n_cache_pages, int nq, int nkv, float scale, int* status, void* stream);
 
 /* ---- matrix products Y[M, N] = X[M, K] . W[N, K]^T -------------------------------------------------------- */
-/* gemm_f32.cu: true 32-bit (fmaf, ascending k); and bfloat16 operands of any width on the CUDA cores */
+/* gemm_f32.cu: true 32-bit (fmaf; the order of a sum hangs on K alone: up to 8 ranges, even and odd k apart, where rows are whole
+   16-byte packets, else one ascending chain); and bfloat16 operands of any width on the CUDA cores (one ascending chain) */
 int q3_gemm_tn_f32(const float* X, const float* W, float* Y, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldy, void* stream);
 int q3_gemm_tn_bf16(const void* X, const void* W, void* Y, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldy, int out_is_f32,
                     void* stream);
