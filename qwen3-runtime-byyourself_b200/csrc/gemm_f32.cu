@@ -358,8 +358,10 @@ template <bool RANGES, int RESIDENT, typename InT, typename OutT>
 __global__ void __launch_bounds__(256, RESIDENT)
 gemm_tn_kernel(const InT* __restrict__ X, const InT* __restrict__ W, OutT* __restrict__ Y, int M, int N, int K,
                int64_t ldx, int64_t ldw, int64_t ldy) {
-    __shared__ float Xs[2][BK][BM + 4];                  // two tiles: one barrier a tile, the next is fetched under the products of this
-    __shared__ float Ws[2][BK][BN + 4];
+    // RANGES: two tiles, one barrier a tile, the next is fetched under the products of this.  (Rows that are not packets come value by value,
+    // and then that costs more than it hides: 64 rows, K 1,001, 1,000 wide 57.7 us, 68.8 with it.)
+    __shared__ float Xs[RANGES ? 2 : 1][BK][BM + 4];
+    __shared__ float Ws[RANGES ? 2 : 1][BK][BN + 4];
     pdl_launch_dependents();
     pdl_wait();
     const int tid = threadIdx.x;
@@ -380,28 +382,37 @@ gemm_tn_kernel(const InT* __restrict__ X, const InT* __restrict__ W, OutT* __res
         const int gm = m0 + lr, gn = n0 + lr, gk = k0 + lk;
 #pragma unroll
         for (int i = 0; i < 4; ++i) xv[i] = wv[i] = 0.0f;
-        const InT *px = X + (int64_t)gm * ldx + gk, *pw = W + (int64_t)gn * ldw + gk;
         if constexpr (RANGES) {
+            const InT *px = X + (int64_t)gm * ldx + gk, *pw = W + (int64_t)gn * ldw + gk;
             if (gm < M && gk < K) *reinterpret_cast<float4*>(xv) = *reinterpret_cast<const float4*>(px);
             if (gn < N && gk < K) *reinterpret_cast<float4*>(wv) = *reinterpret_cast<const float4*>(pw);
         } else {
+            if (gm < M) {
+                const InT* p = X + (int64_t)gm * ldx + gk;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if (gm < M && gk + i < K) xv[i] = to_f32<InT>(px[i]);
-                if (gn < N && gk + i < K) wv[i] = to_f32<InT>(pw[i]);
+                for (int i = 0; i < 4; ++i) if (gk + i < K) xv[i] = to_f32<InT>(p[i]);
+            }
+            if (gn < N) {
+                const InT* p = W + (int64_t)gn * ldw + gk;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) if (gk + i < K) wv[i] = to_f32<InT>(p[i]);
             }
         }
     };
-    fetch(0);
+    if (RANGES) fetch(0);
     for (int k0 = 0; k0 < K; k0 += BK) {
-        const int at = k0 / BK & 1;
+        const int at = RANGES ? k0 / BK & 1 : 0;
+        if (!RANGES) {
+            fetch(k0);
+            __syncthreads();                             // the previous tile has been consumed
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             Xs[at][lk + i][lr] = xv[i];
             Ws[at][lk + i][lr] = wv[i];
         }
         __syncthreads();
-        if (k0 + BK < K) fetch(k0 + BK);
+        if (RANGES && k0 + BK < K) fetch(k0 + BK);
 #pragma unroll
         for (int kk = 0; kk < BK; ++kk) {
             float a[TM], b[TN];
