@@ -235,51 +235,60 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = idesc(BM, PAGE, false), idesc_pv = idesc(BM, D, true);
-            auto issue_s = [&](int j) {
-                const uint32_t k_src = k_smem + (j % K_STAGES) * PANEL_BYTES;
+        // ------------------------------------------------ MMA issuer: the whole warp walks and one elected thread issues, so the
+        // compiler keeps descriptors in uniform registers, which is what the instruction takes
+        constexpr uint32_t idesc_s = idesc(BM, PAGE, false), idesc_pv = idesc(BM, D, true);
+        const uint32_t acc = __shfl_sync(0xffffffffu, tmem, 0);
+        const uint64_t q_desc = desc_k_major(q_smem), k_desc = desc_k_major(k_smem), v_desc = desc_mn_major(v_smem, PAGE * 128);
+        auto issue_s = [&](int j) {
+            const uint32_t s = (uint32_t)j % K_STAGES;
+            const uint64_t k_src = k_desc + (uint64_t)(s * (PANEL_BYTES >> 4));
+            if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk) {
                     const uint32_t off = (kk >> 2) * (BM * 128) + (kk & 3) * 32, koff = (kk >> 2) * (PAGE * 128) + (kk & 3) * 32;
-                    tc_mma_ss(tmem + COL_S, desc_k_major(q_smem + off), desc_k_major(k_src + koff), idesc_s, kk > 0 ? 1u : 0u);
+                    tc_mma_ss(acc + COL_S, q_desc + (uint64_t)(off >> 4), k_src + (uint64_t)(koff >> 4), idesc_s, kk > 0 ? 1u : 0u);
                 }
                 tc_commit(bar_s_full);
-                tc_commit(bar_k_empty + 8 * (j % K_STAGES));                 // the page's K is consumed
-            };
-            bool ok = mbar_wait(bar_q, 0) && mbar_wait(bar_k_full, 0);
-            if (!ok) atomicExch(status, 12);
-            if (ok) {
-                tc_fence_after();
-                issue_s(0);
+                tc_commit(bar_k_empty + 8 * s);                              // the page's K is consumed
             }
-            for (int j = 0; j < n_pages && ok; ++j) {
-                // S(j+1) may overwrite the score columns once the softmax warps hold S(j) in registers
-                if (j + 1 < n_pages) {
-                    ok = mbar_wait(bar_s_read, (uint32_t)j & 1u) &&
-                         mbar_wait(bar_k_full + 8 * ((j + 1) % K_STAGES), (uint32_t)((j + 1) / K_STAGES) & 1u);
-                    if (!ok) { atomicExch(status, 13); break; }
-                    tc_fence_after();
-                    issue_s(j + 1);
-                }
-                ok = mbar_wait(bar_p_full, (uint32_t)j & 1u) &&              // P(j) is in TMEM, O is rescaled
-                     mbar_wait(bar_v_full + 8 * (j % V_STAGES), (uint32_t)(j / V_STAGES) & 1u);
-                if (!ok) { atomicExch(status, 14); break; }
+            __syncwarp();
+        };
+        auto failed = [&](int where) { if (lane == 0) atomicExch(status, where); };
+        bool ok = mbar_wait_warp(bar_q, 0) && mbar_wait_warp(bar_k_full, 0);
+        if (!ok) failed(12);
+        if (ok) {
+            tc_fence_after();
+            issue_s(0);
+        }
+        for (int j = 0; j < n_pages && ok; ++j) {
+            // S(j+1) may overwrite the score columns once the softmax warps hold S(j) in registers
+            if (j + 1 < n_pages) {
+                ok = mbar_wait_warp(bar_s_read, (uint32_t)j & 1u) &&
+                     mbar_wait_warp(bar_k_full + 8 * ((j + 1) % K_STAGES), (uint32_t)((j + 1) / K_STAGES) & 1u);
+                if (!ok) { failed(13); break; }
                 tc_fence_after();
-                const uint32_t v_src = v_smem + (j % V_STAGES) * PANEL_BYTES;
+                issue_s(j + 1);
+            }
+            ok = mbar_wait_warp(bar_p_full, (uint32_t)j & 1u) &&             // P(j) is in TMEM, O is rescaled
+                 mbar_wait_warp(bar_v_full + 8 * (j % V_STAGES), (uint32_t)(j / V_STAGES) & 1u);
+            if (!ok) { failed(14); break; }
+            tc_fence_after();
+            const uint32_t s = (uint32_t)j % V_STAGES;
+            const uint64_t v_src = v_desc + (uint64_t)(s * (PANEL_BYTES >> 4));
+            if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < PAGE / 16; ++kk)
-                    tc_mma_ts(tmem + COL_O, tmem + COL_P + kk * 8, desc_mn_major(v_src + kk * 16 * 128, PAGE * 128), idesc_pv,
-                              (j > 0 || kk > 0) ? 1u : 0u);
+                    tc_mma_ts(acc + COL_O, acc + COL_P + kk * 8, v_src + (uint64_t)(kk * 16 * 128 >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
                 if constexpr (CAPPED) {                                      // the low term of the weights on the same V
 #pragma unroll
                     for (int kk = 0; kk < PAGE / 16; ++kk)
-                        tc_mma_ts(tmem + COL_O, tmem + COL_P_LO + kk * 8, desc_mn_major(v_src + kk * 16 * 128, PAGE * 128), idesc_pv, 1u);
+                        tc_mma_ts(acc + COL_O, acc + COL_P_LO + kk * 8, v_src + (uint64_t)(kk * 16 * 128 >> 4), idesc_pv, 1u);
                 }
-                tc_commit(bar_v_empty + 8 * (j % V_STAGES));                 // the page's V is consumed
+                tc_commit(bar_v_empty + 8 * s);                              // the page's V is consumed
                 tc_commit(bar_pv_done);
             }
+            __syncwarp();
         }
     } else {
         // ------------------------------------------------ softmax and epilogue: thread = query row

@@ -151,26 +151,31 @@ gemm_tcgen05_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc(MT);
-            for (int i = 0; i < nkb; ++i) {
-                const int s = i % STAGES;
-                const uint32_t phase = (uint32_t)(i / STAGES) & 1u;
-                if (!mbar_wait(bars + s * 8, phase)) {                       // the tiles have landed
-                    atomicExch(status, 2);
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t a = base + s * STAGE_BYTES, b = a + A_BYTES;
-                const uint64_t da = make_desc(a), db = make_desc(b);
+        // ---------------- MMA issuer.  The whole warp walks the K steps and one elected thread issues: with the addresses the same for
+        // all lanes the compiler keeps descriptors in uniform registers, which is what the instruction takes.  With the loop inside
+        // `if (lane == 0)` the issue itself was the longest chain of a K step of the pairs kernel (2,048 tokens, gate/up 325 us against
+        // 307; 527 tokens, q/k/v 33 against 30).
+        constexpr uint32_t idesc = make_idesc(MT);
+        const uint64_t desc0 = make_desc(base);
+        const uint32_t acc = __shfl_sync(0xffffffffu, tmem_base, 0);
+        for (int i = 0; i < nkb; ++i) {
+            const uint32_t s = (uint32_t)i % STAGES;
+            if (!mbar_wait_warp(bars + s * 8, ((uint32_t)i / STAGES) & 1u)) {    // the tiles have landed
+                if (lane == 0) atomicExch(status, 2);
+                break;
+            }
+            tc_fence_after();
+            const uint64_t da = desc0 + (uint64_t)(s * (STAGE_BYTES >> 4)), db = da + (A_BYTES >> 4);
+            if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < BK / UMMA_K; ++k)                        // 32 bytes further along K per step
-                    tc_mma(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+                    tc_mma(acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
                 tc_commit(bars + (STAGES + s) * 8);                          // frees the stage when the MMAs are done
             }
-            tc_commit(bar_done);                                             // accumulator complete (or abandoned)
+            __syncwarp();
         }
+        if (elect_one()) tc_commit(bar_done);                                // accumulator complete (or abandoned)
+        __syncwarp();
     } else {
         // ---------------- warps 2..5 own TMEM lanes 32*(warp % 4) ..: accumulator -> part[token][row of W]
         const bool ok = mbar_wait(bar_done, 0);                              // every load has landed and been consumed,
@@ -376,30 +381,39 @@ gemm_tcgen05_prompt_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc_mn(BM, BN);
-            uint32_t it = 0, local = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++local) {
-                const uint32_t buf = local & 1u;
-                ok = mbar_wait(bar_acc_empty + buf * 8, ((local >> 1) & 1u) ^ 1u);      // the epilogue has drained it
-                if (!ok) { atomicExch(status, 4); break; }
+        constexpr uint32_t idesc = make_idesc_mn(BM, BN);
+        const uint64_t desc0 = make_desc(base);
+        tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);
+        uint32_t it = 0, local = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++local) {
+            const uint32_t buf = local & 1u;
+            ok = mbar_wait_warp(bar_acc_empty + buf * 8, ((local >> 1) & 1u) ^ 1u);     // the epilogue has drained it
+            if (!ok) {
+                if (lane == 0) atomicExch(status, 4);
+                break;
+            }
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_base + buf * BN;
+            for (int kb = 0; kb < nkb; ++kb, ++it) {
+                const uint32_t s = it % STAGES;
+                ok = mbar_wait_warp(bars + s * 8, (it / STAGES) & 1u);
+                if (!ok) {
+                    if (lane == 0) atomicExch(status, 2);
+                    break;
+                }
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + buf * BN;
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    ok = mbar_wait(bars + s * 8, (it / STAGES) & 1u);
-                    if (!ok) { atomicExch(status, 2); break; }
-                    tc_fence_after();
-                    const uint32_t a = base + s * STAGE_BYTES, b = a + A_BYTES;
-                    const uint64_t da = make_desc(a), db = make_desc(b);
+                const uint64_t da = desc0 + (uint64_t)(s * (STAGE_BYTES >> 4)), db = da + (A_BYTES >> 4);
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k)
                         tc_mma(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     tc_commit(bars + (STAGES + s) * 8);
                 }
-                tc_commit(bar_acc_full + buf * 8);
+                __syncwarp();
             }
+            if (elect_one()) tc_commit(bar_acc_full + buf * 8);
+            __syncwarp();
         }
     } else {
         pdl_wait();
@@ -722,29 +736,40 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             constexpr uint32_t idesc = make_idesc_mn(PAIR_M, BN);
+            const uint64_t desc0 = make_desc(base);
             uint32_t it = 0, local = 0;
             bool ok = true;
+            tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);
             for (int tile = first; tile < tiles && ok; tile += stride, ++local) {
                 const uint32_t buf = local & 1u;
-                ok = mbar_wait(bar_acc_empty + buf * 8, ((local >> 1) & 1u) ^ 1u);      // both blocks have drained it
-                if (!ok) { atomicExch(status, 4); break; }
+                ok = mbar_wait_warp(bar_acc_empty + buf * 8, ((local >> 1) & 1u) ^ 1u);      // both blocks have drained it
+                if (!ok) {
+                    if (lane == 0) atomicExch(status, 4);
+                    break;
+                }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * BN;
                 for (int kb = 0; kb < nkb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    ok = mbar_wait(bars + s * 8, (it / STAGES) & 1u);
-                    if (!ok) { atomicExch(status, 2); break; }
+                    const uint32_t s = it % STAGES;
+                    ok = mbar_wait_warp(bars + s * 8, (it / STAGES) & 1u);
+                    if (!ok) {
+                        if (lane == 0) atomicExch(status, 2);
+                        break;
+                    }
                     tc_fence_after();
-                    const uint32_t a = base + s * STAGE_BYTES, b = a + A_BYTES;
-                    const uint64_t da = make_desc(a), db = make_desc(b);
+                    const uint64_t da = desc0 + (uint64_t)(s * (STAGE_BYTES >> 4)), db = da + (A_BYTES >> 4);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; ++k)
-                        tc_mma_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    tc_commit_pair(bars + (STAGES + s) * 8);
+                        for (int k = 0; k < BK / UMMA_K; ++k)
+                            tc_mma_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        tc_commit_pair(bars + (STAGES + s) * 8);
+                    }
+                    __syncwarp();
                 }
-                tc_commit_pair(bar_acc_full + buf * 8);
+                if (elect_one()) tc_commit_pair(bar_acc_full + buf * 8);
+                __syncwarp();
             }
         }
     } else {
@@ -866,21 +891,29 @@ gemm_tcgen05_pair_splitk_kernel(const __grid_constant__ CUtensorMap map_x, const
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && parity == 0) {
+        if (parity == 0) {
             constexpr uint32_t idesc = make_idesc_mn(PAIR_M, BN);
+            const uint64_t desc0 = make_desc(base);
             const uint16_t mask = (uint16_t)(3u << leader);
+            const uint32_t acc = __shfl_sync(0xffffffffu, tmem_base, 0);
             for (int i = 0; i < nkb; ++i) {
-                const int s = i % STAGES;
-                if (!mbar_wait(bars + s * 8, (uint32_t)(i / STAGES) & 1u)) { atomicExch(status, 2); break; }
+                const uint32_t s = (uint32_t)i % STAGES;
+                if (!mbar_wait_warp(bars + s * 8, ((uint32_t)i / STAGES) & 1u)) {
+                    if (lane == 0) atomicExch(status, 2);
+                    break;
+                }
                 tc_fence_after();
-                const uint32_t a = base + s * STAGE_BYTES, b = a + A_BYTES;
-                const uint64_t da = make_desc(a), db = make_desc(b);
+                const uint64_t da = desc0 + (uint64_t)(s * (STAGE_BYTES >> 4)), db = da + (A_BYTES >> 4);
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < BK / UMMA_K; ++k)
-                    tc_mma_pair(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
-                tc_commit_pair(bars + (STAGES + s) * 8, mask);
+                    for (int k = 0; k < BK / UMMA_K; ++k)
+                        tc_mma_pair(acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+                    tc_commit_pair(bars + (STAGES + s) * 8, mask);
+                }
+                __syncwarp();
             }
-            tc_commit_pair(bar_acc_full, mask);               // accumulator complete (or abandoned)
+            if (elect_one()) tc_commit_pair(bar_acc_full, mask);     // accumulator complete (or abandoned)
+            __syncwarp();
         }
     } else {
         acc_ok = mbar_wait(bar_acc_full, 0);

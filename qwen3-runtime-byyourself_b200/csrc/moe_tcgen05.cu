@@ -130,28 +130,40 @@ expert_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        // the whole warp walks and one elected thread issues: descriptors in uniform registers, which the instruction takes
+        if (rank == 0) {
+            const uint64_t desc0 = desc_k_major(base);
             uint32_t it = 0, local = 0;
             bool ok = true;
+            tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);
             for (int tile = first; ok && walk.at(tile, row_tile, slot, tokens, n); tile += stride, ++local) {
-                const uint32_t buf = local & 1u, idesc = make_idesc_mn(2 * ROWS, n);
-                ok = mbar_wait(bar_acc_empty + buf * 8, ((local >> 1) & 1u) ^ 1u);      // both blocks have drained it
-                if (!ok) { atomicExch(status, 4); break; }
+                const uint32_t buf = local & 1u, idesc = make_idesc_mn(2 * ROWS, __shfl_sync(0xffffffffu, n, 0));
+                ok = mbar_wait_warp(bar_acc_empty + buf * 8, ((local >> 1) & 1u) ^ 1u);      // both blocks have drained it
+                if (!ok) {
+                    if (lane == 0) atomicExch(status, 4);
+                    break;
+                }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * MAX_TOKENS;
                 for (int kb = 0; kb < nkb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    ok = mbar_wait(bars + s * 8, (it / STAGES) & 1u);
-                    if (!ok) { atomicExch(status, 2); break; }
+                    const uint32_t s = it % STAGES;
+                    ok = mbar_wait_warp(bars + s * 8, (it / STAGES) & 1u);
+                    if (!ok) {
+                        if (lane == 0) atomicExch(status, 2);
+                        break;
+                    }
                     tc_fence_after();
-                    const uint32_t a = base + s * STAGE_BYTES, b = a + A_BYTES;
-                    const uint64_t da = desc_k_major(a), db = desc_k_major(b);
+                    const uint64_t da = desc0 + (uint64_t)(s * (STAGE_BYTES >> 4)), db = da + (A_BYTES >> 4);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; ++k)
-                        tc_mma_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    tc_commit_pair(bars + (STAGES + s) * 8);
+                        for (int k = 0; k < BK / UMMA_K; ++k)
+                            tc_mma_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        tc_commit_pair(bars + (STAGES + s) * 8);
+                    }
+                    __syncwarp();
                 }
-                tc_commit_pair(bar_acc_full + buf * 8);
+                if (elect_one()) tc_commit_pair(bar_acc_full + buf * 8);
+                __syncwarp();
             }
         }
     } else {

@@ -37,6 +37,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     }
     return false;
 }
+// The same for a whole converged warp, which goes on or gives up together.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
 // Orders this thread's earlier reads and writes of shared memory before later writes of the
 // asynchronous proxy to it (a stage that was read is handed back to the TMA unit).
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
