@@ -26,6 +26,8 @@
 // cluster barriers are reached by every thread on every path).
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "tcgen05.cuh"
 #include "tcgen05_pair.cuh"
@@ -37,6 +39,7 @@ constexpr int BM = 128;                 // rows of W per tile (the UMMA M)
 constexpr int BK = 64;                  // K per stage: 64 bf16 = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
 constexpr int THREADS = 192;
+constexpr int PAIR_THREADS = 320;        // the prompt form on pairs of SMs: eight drain warps
 __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     tc_mma_ss(d_tmem, a_desc, b_desc, idesc, accumulate);
 }
@@ -262,19 +265,40 @@ gemm_tcgen05_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
 // (tile = blockIdx.x, += gridDim.x; the token tile varies fastest so that blocks running at the
 // same time share W tiles in the L2); the accumulator is double-buffered in tensor memory
 // (2 x BN columns), so the epilogue of one tile runs under the products of the next.
+__device__ __forceinline__ uint32_t pack_bf16(uint32_t lo, uint32_t hi) {
+    const __nv_bfloat162 t = __floats2bfloat162_rn(__uint_as_float(lo), __uint_as_float(hi));
+    return *reinterpret_cast<const uint32_t*>(&t);
+}
 template <typename OutT> __device__ __forceinline__ void store_run8(OutT* p, const uint32_t* r);
 template <> __device__ __forceinline__ void store_run8<float>(float* p, const uint32_t* r) {
     reinterpret_cast<uint4*>(p)[0] = make_uint4(r[0], r[1], r[2], r[3]);
     reinterpret_cast<uint4*>(p)[1] = make_uint4(r[4], r[5], r[6], r[7]);
 }
 template <> __device__ __forceinline__ void store_run8<bf16>(bf16* p, const uint32_t* r) {
-    uint4 v;
-    __nv_bfloat162 t;
-    t = __floats2bfloat162_rn(__uint_as_float(r[0]), __uint_as_float(r[1])); v.x = *reinterpret_cast<uint32_t*>(&t);
-    t = __floats2bfloat162_rn(__uint_as_float(r[2]), __uint_as_float(r[3])); v.y = *reinterpret_cast<uint32_t*>(&t);
-    t = __floats2bfloat162_rn(__uint_as_float(r[4]), __uint_as_float(r[5])); v.z = *reinterpret_cast<uint32_t*>(&t);
-    t = __floats2bfloat162_rn(__uint_as_float(r[6]), __uint_as_float(r[7])); v.w = *reinterpret_cast<uint32_t*>(&t);
-    *reinterpret_cast<uint4*>(p) = v;
+    *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]), pack_bf16(r[4], r[5]), pack_bf16(r[6], r[7]));
+}
+// 16 values as whole sectors of 32 bytes: a thread writes a row of its own, so a store of 16 bytes is half a sector of 32
+// different lines and the L2 takes two writes where one would do (2,048 tokens, q/k/v of an 8B-sized layer 89 us against 86).
+__device__ __forceinline__ void store_sector(void* p, const uint32_t (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+                 "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+template <typename OutT> __device__ __forceinline__ void store_run16(OutT* p, const uint32_t* r);
+template <> __device__ __forceinline__ void store_run16<float>(float* p, const uint32_t* r) {
+    const uint32_t a[8] = {r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7]}, b[8] = {r[8], r[9], r[10], r[11], r[12], r[13], r[14], r[15]};
+    store_sector(p, a);
+    store_sector(p + 8, b);
+}
+template <> __device__ __forceinline__ void store_run16<bf16>(bf16* p, const uint32_t* r) {
+    const uint32_t v[8] = {pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]), pack_bf16(r[4], r[5]), pack_bf16(r[6], r[7]),
+                           pack_bf16(r[8], r[9]), pack_bf16(r[10], r[11]), pack_bf16(r[12], r[13]), pack_bf16(r[14], r[15])};
+    store_sector(p, v);
+}
+// Bytes that a thread may write at once into rows of `cols` values at Y: 32, 16 or one value at a time (0).
+template <typename OutT> __device__ __forceinline__ int store_bytes(const OutT* Y, int cols) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(Y);
+    if (cols % 16 == 0 && (at & 31u) == 0) return 32;
+    return cols % 8 == 0 && (at & 15u) == 0 ? 16 : 0;
 }
 
 // GATED: W holds gate and up rows interleaved in blocks of eight (as the decode kernel's gated form);
@@ -285,41 +309,52 @@ template <> __device__ __forceinline__ void store_run8<bf16>(bf16* p, const uint
 // relu of every value.
 template <int GATED, typename OutT>
 __device__ __forceinline__ void store_chunk32(const uint32_t (&r)[32], OutT* row, int c, int n0, bool token_valid, int N,
-                                              bool vec_ok) {
+                                              int vec_bytes) {
     if (!token_valid) return;
     if constexpr (q3_paired<GATED>) {
+        uint32_t packed[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+            const float g = round_to<bf16>(__uint_as_float(r[(e >> 3) * 16 + (e & 7)]));
+            const float u = round_to<bf16>(__uint_as_float(r[(e >> 3) * 16 + 8 + (e & 7)]));
+            packed[e] = __float_as_uint(round_to<bf16>(gate_activation<GATED>(g)) * u);
+        }
+        OutT* dst = row + (c >> 1);
+        if (vec_bytes == 32 && n0 + c + 32 <= N) {
+            store_run16<OutT>(dst, packed);
+            return;
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int n = n0 + c + h * 16;           // first gate column of this block
-            uint32_t packed[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const float g = round_to<bf16>(__uint_as_float(r[h * 16 + e]));
-                const float u = round_to<bf16>(__uint_as_float(r[h * 16 + 8 + e]));
-                packed[e] = __float_as_uint(round_to<bf16>(gate_activation<GATED>(g)) * u);
-            }
-            OutT* dst = row + ((c + h * 16) >> 1);
-            if (n + 16 <= N && vec_ok) {
-                store_run8<OutT>(dst, packed);
+            if (vec_bytes != 0 && n + 16 <= N) {
+                store_run8<OutT>(dst + h * 8, packed + h * 8);
             } else {
 #pragma unroll
                 for (int e = 0; e < 8; ++e)
-                    if (n + 8 + e < N) dst[e] = to_out<OutT>(__uint_as_float(packed[e]));
+                    if (n + 8 + e < N) dst[h * 8 + e] = to_out<OutT>(__uint_as_float(packed[h * 8 + e]));
             }
         }
     } else {
 #pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-            const int n = n0 + c + j;
-            uint32_t v[8];
+        for (int j = 0; j < 32; j += 16) {
+            uint32_t v[16];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] = __float_as_uint(q3_plain_epilogue<GATED>(__uint_as_float(r[j + e])));
-            if (vec_ok && n + 8 <= N) {
-                store_run8<OutT>(row + c + j, v);
-            } else {
+            for (int e = 0; e < 16; ++e) v[e] = __float_as_uint(q3_plain_epilogue<GATED>(__uint_as_float(r[j + e])));
+            if (vec_bytes == 32 && n0 + c + j + 16 <= N) {
+                store_run16<OutT>(row + c + j, v);
+                continue;
+            }
 #pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    if (n + e < N) row[c + j + e] = to_out<OutT>(__uint_as_float(v[e]));
+            for (int h = 0; h < 16; h += 8) {
+                const int n = n0 + c + j + h;
+                if (vec_bytes != 0 && n + 8 <= N) {
+                    store_run8<OutT>(row + c + j + h, v + h);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        if (n + e < N) row[c + j + h + e] = to_out<OutT>(__uint_as_float(v[h + e]));
+                }
             }
         }
     }
@@ -418,7 +453,7 @@ gemm_tcgen05_prompt_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
     } else {
         pdl_wait();
         const int lane_base = (warp & 3) * 32;
-        const bool vec_ok = ((q3_paired<GATED> ? (N >> 1) : N) % 8 == 0) && ((reinterpret_cast<uintptr_t>(Y) & 15u) == 0);
+        const int vec_bytes = store_bytes(Y, q3_paired<GATED> ? (N >> 1) : N);
         uint32_t local = 0;
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
             const uint32_t buf = local & 1u;
@@ -435,7 +470,7 @@ gemm_tcgen05_prompt_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
                 uint32_t r[32];
                 tc_ld32(tmem_base + ((uint32_t)lane_base << 16) + buf * BN + (uint32_t)c, r);
                 tc_wait_ld();
-                store_chunk32<GATED, OutT>(r, row, c, n0, m < M, N, vec_ok);
+                store_chunk32<GATED, OutT>(r, row, c, n0, m < M, N, vec_bytes);
             }
             tc_fence_before();
             __syncwarp();
@@ -463,7 +498,7 @@ gemm_tcgen05_prompt_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
 //   full[s]       in the leader: both blocks' TMA loads report their bytes there
 //   empty[s]      in each block: the leader's tcgen05.commit arrives at both (multicast)
 //   acc_full[b]   in each block: likewise, when a tile's accumulator is complete
-//   acc_empty[b]  in the leader: the eight drain warps of both blocks arrive there
+//   acc_empty[b]  in the leader: the sixteen drain warps of both blocks arrive there
 // Only the leader issues tcgen05.mma.  Every wait is bounded as above, and both blocks meet at a
 // cluster barrier before either leaves (the peer's shared memory and barriers are in use until then).
 // The epilogue of the q/k/v product for prompts: what qkv_prepare (attention.cu) does to the product's output, done
@@ -509,28 +544,42 @@ __device__ __forceinline__ void load_f32x8(const float* p, float (&v)[8]) {
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
-// One head of one token: D accumulator columns from `acc` on.  D = 64 or 128: the whole head is taken into
-// registers with one wait, so the sum of squares, the normalisation and the rotation need no second pass over
-// tensor memory.
-template <int D>
-__device__ __forceinline__ void qkv_head_in_registers(uint32_t acc, bool live, bf16* dst, const float* nw, float eps,
-                                                      const float* cs_row, const float* sn_row) {
-    constexpr int HALF = D / 2, CHUNKS = D / 32;
-    uint32_t r[CHUNKS][32];
-#pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) tc_ld32(acc + (uint32_t)(c * 32), r[c]);
-    tc_wait_ld();
-    if (!live) return;
+// Where head `head` of token `m` goes and what is done to it on the way.
+struct QkvHead {
+    bf16* dst;
+    const float *nw, *cs_row, *sn_row;
+    bool live;
+};
+__device__ __forceinline__ QkvHead qkv_head_place(int head, int m, bool token_valid, int pos, int64_t page, const QkvEpilogue& e) {
+    const bool is_q = head < e.nq, is_v = head >= e.nq + e.nkv, rotate = e.cos_tab != nullptr && !is_v;
+    QkvHead h;
+    h.nw = is_q ? e.q_norm_w : (is_v ? nullptr : e.k_norm_w);
+    h.live = token_valid && head < e.nq + 2 * e.nkv && (is_q || e.write_kv);
+    h.dst = nullptr;
+    if (h.live)
+        h.dst = is_q ? e.q_out + ((int64_t)m * e.nq + head) * e.d
+                     : (is_v ? e.v_pages : e.k_pages) +
+                           ((page * e.nkv + (head - e.nq) % e.nkv) * Q3_PAGE_TOKENS + pos % Q3_PAGE_TOKENS) * e.d;
+    h.cs_row = rotate ? e.cos_tab + (int64_t)pos * (e.d >> 1) : nullptr;
+    h.sn_row = rotate ? e.sin_tab + (int64_t)pos * (e.d >> 1) : nullptr;
+    return h;
+}
+
+// One head of one token: the D = 64 or 128 values, two a register and rounded to bfloat16, from register FIRST on, so the sum of
+// squares, the normalisation and the rotation need no second pass over tensor memory.
+template <int D, int FIRST>
+__device__ __forceinline__ void qkv_head_in_registers(const uint32_t (&all)[64], const QkvHead& head, float eps) {
+    constexpr int HALF = D / 2;
+    auto value = [&](int i) {
+        const uint32_t v = all[FIRST + i / 2];
+        return __uint_as_float(i & 1 ? v & 0xFFFF0000u : v << 16);
+    };
+    if (!head.live) return;
     float inv = 1.0f;
-    if (nw != nullptr) {
+    if (head.nw != nullptr) {
         float sq = 0.0f;
 #pragma unroll
-        for (int c = 0; c < CHUNKS; ++c)
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const float v = round_to<bf16>(__uint_as_float(r[c][j]));
-                sq += v * v;
-            }
+        for (int i = 0; i < D; ++i) sq += value(i) * value(i);
         inv = rsqrtf(sq / (float)D + eps);
     }
 #pragma unroll
@@ -538,23 +587,23 @@ __device__ __forceinline__ void qkv_head_in_registers(uint32_t acc, bool live, b
         float x[8], y[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            x[i] = round_to<bf16>(__uint_as_float(r[(i0 + i) / 32][(i0 + i) % 32]));
-            y[i] = round_to<bf16>(__uint_as_float(r[(HALF + i0 + i) / 32][(HALF + i0 + i) % 32]));
+            x[i] = value(i0 + i);
+            y[i] = value(HALF + i0 + i);
         }
-        if (nw != nullptr) {
+        if (head.nw != nullptr) {
             float wx[8], wy[8];
-            load_f32x8(nw + i0, wx);
-            load_f32x8(nw + HALF + i0, wy);
+            load_f32x8(head.nw + i0, wx);
+            load_f32x8(head.nw + HALF + i0, wy);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 x[i] = round_to<bf16>(round_to<bf16>(x[i] * inv) * wx[i]);
                 y[i] = round_to<bf16>(round_to<bf16>(y[i] * inv) * wy[i]);
             }
         }
-        if (cs_row != nullptr) {
+        if (head.cs_row != nullptr) {
             float cs[8], sn[8];
-            load_f32x8(cs_row + i0, cs);
-            load_f32x8(sn_row + i0, sn);
+            load_f32x8(head.cs_row + i0, cs);
+            load_f32x8(head.sn_row + i0, sn);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const float xr = x[i] * cs[i] - y[i] * sn[i], yr = y[i] * cs[i] + x[i] * sn[i];
@@ -562,8 +611,8 @@ __device__ __forceinline__ void qkv_head_in_registers(uint32_t acc, bool live, b
                 y[i] = yr;
             }
         }
-        store_bf16x8(dst + i0, x);
-        store_bf16x8(dst + HALF + i0, y);
+        store_bf16x8(head.dst + i0, x);
+        store_bf16x8(head.dst + HALF + i0, y);
     }
 }
 
@@ -629,34 +678,6 @@ __device__ __forceinline__ void qkv_head_two_passes(uint32_t acc, int d, bool li
     }
 }
 
-// `acc`: the thread's row of the tile's accumulator in tensor memory; token `m`, tile columns n0 .. n0 + 255.
-__device__ __forceinline__ void qkv_tile_epilogue(uint32_t acc, int m, bool token_valid, int n0, int N, const QkvEpilogue& e) {
-    const int d = e.d, half = d >> 1;
-    int pos = 0;
-    int64_t page = 0;
-    if (token_valid) {
-        pos = e.token_pos[m];
-        if (e.write_kv) page = e.page_table[(int64_t)e.token_seq[m] * e.pages_per_seq + pos / Q3_PAGE_TOKENS];
-    }
-    for (int h0 = 0; h0 < 256 && n0 + h0 < N; h0 += d) {       // the same heads for every thread of the warp
-        const int head = (n0 + h0) / d;
-        const bool is_q = head < e.nq, is_v = head >= e.nq + e.nkv;
-        const float* nw = is_q ? e.q_norm_w : (is_v ? nullptr : e.k_norm_w);
-        const bool live = token_valid && (is_q || e.write_kv);
-        const bool rotate = e.cos_tab != nullptr && !is_v;
-        bf16* dst = nullptr;
-        if (live)
-            dst = is_q ? e.q_out + ((int64_t)m * e.nq + head) * d
-                       : (is_v ? e.v_pages : e.k_pages) +
-                             ((page * e.nkv + (head - e.nq) % e.nkv) * Q3_PAGE_TOKENS + pos % Q3_PAGE_TOKENS) * d;
-        const float* cs_row = rotate ? e.cos_tab + (int64_t)pos * half : nullptr;
-        const float* sn_row = rotate ? e.sin_tab + (int64_t)pos * half : nullptr;
-        if (d == 128) qkv_head_in_registers<128>(acc + (uint32_t)h0, live, dst, nw, e.eps, cs_row, sn_row);
-        else if (d == 64) qkv_head_in_registers<64>(acc + (uint32_t)h0, live, dst, nw, e.eps, cs_row, sn_row);
-        else qkv_head_two_passes(acc + (uint32_t)h0, d, live, dst, nw, e.eps, cs_row, sn_row);
-    }
-}
-
 // The order of the tiles: bands of at most 16 tiles of tokens, all tiles of W inside a band, the tokens fastest.  The
 // 74 pairs that run together then hold about 16 tiles of tokens and five of W (42 MB at K = 4,096) and the band's
 // tokens stay in the L2 while W passes.  With all tokens first a wave read 74 tiles of tokens and one of W, 157 MB for 21 us of
@@ -672,20 +693,72 @@ __device__ __forceinline__ void tile_place(int tile, int tiles_m, int tiles_n, i
     tm = band * high + inside - tn * own;
 }
 
-template <int STAGES, int GATED, typename OutT, bool QKV = false>
-__global__ void __launch_bounds__(THREADS, 1)
+// What a warp of the drain holds of 32 rows of W from `row0` on - lane = row, v[i] = the values of tokens 2 i and 2 i + 1, rounded to
+// bfloat16 - written for `tokens` tokens from m0 on.  Lanes next to each other exchange values, so that one takes both rows of the even
+// token and the other those of the odd one: 64 consecutive bytes a token and instruction.  GATED: the rows are gate[8] up[8] gate[8]
+// up[8] of 16 features; a gate's lane and its up's (eight further) exchange first and take a token each.  Rows of Y are whole 16-byte
+// packets.
+template <int GATED>
+__device__ __forceinline__ void store_rows(const uint32_t (&v)[64], bf16* Y, int m0, int tokens, int row0, int lane, int N) {
+    if constexpr (q3_paired<GATED>) {
+        const int out_n = N >> 1, feature = (row0 >> 1) + ((lane >> 4) << 3) + (lane & 7), token = (lane >> 3) & 1;
+        const bool odd = lane & 1, valid = row0 + (lane & 16) + 16 <= N;
+        bf16* to = Y + (int64_t)(m0 + token) * out_n + (feature & ~1);
+#pragma unroll
+        for (int i = 0; i < 64; i += 2) {
+            if (2 * i >= tokens) return;
+            uint32_t x[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const uint32_t own = v[i + j], other = __shfl_xor_sync(0xffffffffu, own, 8);
+                const float g = __uint_as_float(token ? other & 0xFFFF0000u : own << 16);
+                const float u = __uint_as_float(token ? own & 0xFFFF0000u : other << 16);
+                x[j] = __float_as_uint(round_to<bf16>(round_to<bf16>(gate_activation<GATED>(g)) * u)) >> 16;
+            }
+            // even lanes write the two features for v[i]'s token, odd lanes for v[i + 1]'s
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? x[0] : x[1], 1);
+            const uint32_t both = odd ? got | x[1] << 16 : x[0] | got << 16;
+            const int at = 2 * (i + (odd ? 1 : 0));
+            if (valid && at + token < tokens) *reinterpret_cast<uint32_t*>(to + (int64_t)at * out_n) = both;
+        }
+    } else {
+        const int row = row0 + lane, odd = lane & 1;
+        bf16* to = Y + (int64_t)(m0 + odd) * N + (row & ~1);
+#pragma unroll
+        for (int i = 0; i < 64; ++i) {
+            if (2 * i >= tokens) return;
+            const uint32_t own = v[i], other = __shfl_xor_sync(0xffffffffu, own, 1);
+            const uint32_t both = odd ? __byte_perm(other, own, 0x7632) : __byte_perm(own, other, 0x5410);
+            if (row < N && 2 * i + odd < tokens) *reinterpret_cast<uint32_t*>(to + (int64_t)(2 * i) * N) = both;
+        }
+    }
+}
+
+// ROWS: W is the 256-row operand instead and the tokens are the other one, of which a tile may have any multiple of 32 (`tile`; 256
+// without ROWS): a few hundred tokens are cut into equal tiles instead of whole 256s.  A thread of the drain then owns a row of W.
+// The eight drain warps take their share of an accumulator (32 lanes by half of its columns) into registers at once, rounded and two a
+// register, and give it back before they finish and store.  Measured for an 8B-sized layer, launches back to back (before, with
+// whole 256s and four drain warps / now / cuBLAS, us): 527 tokens gate/up 117 / 90 / 78, down 73 / 56 / 49, q/k/v 31 / 25 / 22, output
+// 27 / 21 / 18; 1,300 tokens 255 / 200 / 203, 149 / 111 / 94, 62 / 53 / 52, 52 / 43 / 35; 2,048 tokens (whole 256s now, too) 333 / 303 / 341,
+// 158 / 149 / 151, 85 / 79 / 82, 56 / 54 / 54; 7,000 tokens 1,094 / 970 / 1,204, 553 / 533 / 545, 280 / 261 / 277, 188 / 179 / 195.
+template <int GATED, typename OutT, bool QKV = false, bool ROWS = false>
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
-                         OutT* __restrict__ Y, int M, int N, int K, int* __restrict__ status, const QkvEpilogue qkv) {
+                         OutT* __restrict__ Y, int M, int N, int K, int tile, int* __restrict__ status, const QkvEpilogue qkv) {
     extern __shared__ unsigned char smem_raw[];
-    constexpr int BN = 256, PAIR_M = 2 * BM;
+    constexpr int BN = 256, STAGES = 6;
     constexpr int A_BYTES = BM * BK * 2, B_BYTES = (BN / 2) * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
-    constexpr uint32_t TMEM_COLS = 2 * BN;                    // two accumulators of 128 tokens x 256 rows of W
+    constexpr uint32_t TMEM_COLS = 2 * BN;                    // two accumulators
+    constexpr bool PACKED = std::is_same<OutT, bf16>::value && GATED != 3;       // a value is rounded before anything else is done to it
+    static_assert(PACKED || !ROWS, "a row's values are exchanged two by two");
+    static_assert(!(QKV && ROWS), "a head's values are one thread's");
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t bars = base + STAGES * STAGE_BYTES;       // full[S], empty[S], acc_full[2], acc_empty[2], slot
     const uint32_t bar_acc_full = bars + 2 * STAGES * 8, bar_acc_empty = bar_acc_full + 16, tmem_slot = bar_acc_empty + 16;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
-    const int pairs_m = (M + PAIR_M - 1) / PAIR_M, n_tiles = (N + BN - 1) / BN, tiles = pairs_m * n_tiles;
+    if (!ROWS) tile = 2 * BM;
+    const int tiles_m = (M + tile - 1) / tile, tiles_n = (N + BN - 1) / BN, tiles = tiles_m * tiles_n;
     const int first = blockIdx.x >> 1, stride = gridDim.x >> 1;
     const int nkb = (K + BK - 1) / BK;
 
@@ -699,7 +772,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(bar_acc_full + b * 8, 1);
-            mbar_init(bar_acc_empty + b * 8, 8);             // one arrival per drain warp of the pair
+            mbar_init(bar_acc_empty + b * 8, 16);            // one arrival per drain warp of the pair
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -719,17 +792,17 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
             pdl_wait();                                       // X is the output of the kernel before
             uint32_t it = 0;
             bool ok = true;
-            for (int tile = first; tile < tiles && ok; tile += stride) {
+            for (int i = first; i < tiles && ok; i += stride) {
                 int tm, tn;
-                tile_place(tile, pairs_m, n_tiles, tm, tn);
-                const int m0 = tm * PAIR_M + (int)rank * BM, n0 = tn * BN + (int)rank * (BN / 2);
+                tile_place(i, tiles_m, tiles_n, tm, tn);
+                const int m0 = tm * tile + (int)rank * (tile / 2), n0 = tn * BN + (int)rank * (BN / 2);
                 for (int kb = 0; kb < nkb; ++kb, ++it) {
                     const int s = it % STAGES;
                     ok = mbar_wait(bars + (STAGES + s) * 8, ((it / STAGES) & 1u) ^ 1u);
                     if (!ok) { atomicExch(status, 1); break; }
                     const uint32_t a = base + s * STAGE_BYTES, b = a + A_BYTES;
                     const uint32_t full_in_leader = map_to_rank(bars + s * 8, 0);
-                    if (rank == 0) mbar_expect_tx(bars + s * 8, 2 * STAGE_BYTES);       // both blocks' bytes
+                    if (rank == 0) mbar_expect_tx(bars + s * 8, 2 * (tile / 2 * BK * 2 + B_BYTES));   // both blocks' bytes
                     tma_load_2d_pair(a, &map_x, full_in_leader, kb * BK, m0);
                     tma_load_2d_pair(b, &map_w, full_in_leader, kb * BK, n0);
                 }
@@ -737,12 +810,12 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
         }
     } else if (warp == 1) {
         if (rank == 0) {
-            constexpr uint32_t idesc = make_idesc_mn(PAIR_M, BN);
+            const uint32_t idesc = make_idesc_mn(2 * BM, ROWS ? tile : BN);
             const uint64_t desc0 = make_desc(base);
             uint32_t it = 0, local = 0;
             bool ok = true;
             tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);
-            for (int tile = first; tile < tiles && ok; tile += stride, ++local) {
+            for (int i = first; i < tiles && ok; i += stride, ++local) {
                 const uint32_t buf = local & 1u;
                 ok = mbar_wait_warp(bar_acc_empty + buf * 8, ((local >> 1) & 1u) ^ 1u);      // both blocks have drained it
                 if (!ok) {
@@ -759,11 +832,12 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                         break;
                     }
                     tc_fence_after();
-                    const uint64_t da = desc0 + (uint64_t)(s * (STAGE_BYTES >> 4)), db = da + (A_BYTES >> 4);
+                    const uint64_t dx = desc0 + (uint64_t)(s * (STAGE_BYTES >> 4)), dw = dx + (A_BYTES >> 4);
                     if (elect_one()) {
 #pragma unroll
                         for (int k = 0; k < BK / UMMA_K; ++k)
-                            tc_mma_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                            tc_mma_pair(d_tmem, (ROWS ? dw : dx) + (uint64_t)(k * 2), (ROWS ? dx : dw) + (uint64_t)(k * 2), idesc,
+                                        (kb > 0 || k > 0) ? 1u : 0u);
                         tc_commit_pair(bars + (STAGES + s) * 8);
                     }
                     __syncwarp();
@@ -774,35 +848,84 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
         }
     } else {
         pdl_wait();
-        const int lane_base = (warp & 3) * 32;
-        const bool vec_ok = ((q3_paired<GATED> ? (N >> 1) : N) % 8 == 0) && ((reinterpret_cast<uintptr_t>(Y) & 15u) == 0);
+        const int lane_base = (warp & 3) * 32, set = (warp - 2) >> 2;
+        // 32 tokens by columns c0 .. c0 + 127; ROWS: 32 rows of W by the tokens of the tile's first or second half
+        const int half = ROWS ? (tile / 2 + 7) / 8 * 8 : 128, c0 = set * half;
+        const int vec_bytes = store_bytes(Y, q3_paired<GATED> ? (N >> 1) : N);
         uint32_t local = 0;
-        for (int tile = first; tile < tiles; tile += stride, ++local) {
+        for (int i = first; i < tiles; i += stride, ++local) {
             const uint32_t buf = local & 1u;
             int tm, tn;
-            tile_place(tile, pairs_m, n_tiles, tm, tn);
-            const int m0 = tm * PAIR_M + (int)rank * BM, n0 = tn * BN;
+            tile_place(i, tiles_m, tiles_n, tm, tn);
+            const int m = tm * tile + (ROWS ? 0 : (int)rank * BM + lane_base + lane), n0 = tn * BN;
+            const uint32_t acc = tmem_base + ((uint32_t)lane_base << 16) + buf * BN;
             if (!mbar_wait(bar_acc_full + buf * 8, (local >> 1) & 1u)) {
                 if (lane == 0) atomicExch(status, 3);
                 break;
             }
             tc_fence_after();
-            const int m = m0 + lane_base + lane;
-            if constexpr (QKV) {
-                qkv_tile_epilogue(tmem_base + ((uint32_t)lane_base << 16) + buf * BN, m, m < M, n0, N, qkv);
-            } else {
-                OutT* row = Y + (int64_t)m * (q3_paired<GATED> ? (N >> 1) : N) + (q3_paired<GATED> ? (n0 >> 1) : n0);
-#pragma unroll 1
-                for (int c = 0; c < BN; c += 32) {
-                    uint32_t r[32];
-                    tc_ld32(tmem_base + ((uint32_t)lane_base << 16) + buf * BN + (uint32_t)c, r);
-                    tc_wait_ld();
-                    store_chunk32<GATED, OutT>(r, row, c, n0, m < M, N, vec_ok);
-                }
+            auto release = [&]() {                           // this warp's share of the accumulator may be overwritten
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(map_to_rank(bar_acc_empty + buf * 8, 0));
+            };
+            int pos = 0;
+            int64_t page = 0;
+            if (QKV && m < M) {
+                pos = qkv.token_pos[m];
+                if (qkv.write_kv) page = qkv.page_table[(int64_t)qkv.token_seq[m] * qkv.pages_per_seq + pos / Q3_PAGE_TOKENS];
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_rank(bar_acc_empty + buf * 8, 0));   // this warp's share is drained
+            if (QKV && qkv.d == 256) {
+                if (set == (int)buf) {                       // a head of 256 is one thread's: the two sets of warps take turns
+                    const QkvHead e = qkv_head_place(n0 / 256, m, m < M, pos, page, qkv);
+                    qkv_head_two_passes(acc, 256, e.live, e.dst, e.nw, qkv.eps, e.cs_row, e.sn_row);
+                }
+                release();
+            } else if constexpr (PACKED) {
+                uint32_t v[64];                              // as the output is rounded, and gate and up before it
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t r[32];
+                    tc_ld32(acc + (uint32_t)(c0 + c * 32), r);
+                    tc_wait_ld();
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) v[c * 16 + e] = pack_bf16(r[2 * e], r[2 * e + 1]);
+                }
+                release();
+                if constexpr (ROWS) {
+                    store_rows<GATED>(v, Y, m + c0, min(half, min(tile - c0, M - m - c0)), n0 + (int)rank * BM + lane_base, lane, N);
+                } else if constexpr (QKV) {                  // the heads are the same for every thread of the warp
+                    const int head = (n0 + c0) / qkv.d;
+                    const QkvHead e = qkv_head_place(head, m, m < M, pos, page, qkv);
+                    if (qkv.d == 128) {
+                        qkv_head_in_registers<128, 0>(v, e, qkv.eps);
+                    } else {
+                        qkv_head_in_registers<64, 0>(v, e, qkv.eps);
+                        qkv_head_in_registers<64, 32>(v, qkv_head_place(head + 1, m, m < M, pos, page, qkv), qkv.eps);
+                    }
+                } else {
+                    OutT* row = Y + (int64_t)m * (q3_paired<GATED> ? (N >> 1) : N) + (q3_paired<GATED> ? (n0 >> 1) : n0);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t r[32];
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) {
+                            r[2 * e] = v[c * 16 + e] << 16;
+                            r[2 * e + 1] = v[c * 16 + e] & 0xFFFF0000u;
+                        }
+                        store_chunk32<GATED, OutT>(r, row, c0 + c * 32, n0, m < M, N, vec_bytes);
+                    }
+                }
+            } else {
+                uint32_t r[4][32];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) tc_ld32(acc + (uint32_t)(c0 + c * 32), r[c]);
+                tc_wait_ld();
+                release();
+                OutT* row = Y + (int64_t)m * N + n0;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) store_chunk32<GATED, OutT>(r[c], row, c0 + c * 32, n0, m < M, N, vec_bytes);
+            }
         }
     }
     tc_fence_before();
@@ -948,7 +1071,7 @@ gemm_tcgen05_pair_splitk_kernel(const __grid_constant__ CUtensorMap map_x, const
 
     if (warp >= 2 && acc_ok) {
         pdl_wait();                                           // no global write before this
-        const bool vec_ok = ((q3_paired<GATED> ? (N >> 1) : N) % 8 == 0) && ((reinterpret_cast<uintptr_t>(Y) & 15u) == 0);
+        const int vec_bytes = store_bytes(Y, q3_paired<GATED> ? (N >> 1) : N);
         const int m = m0 + row;
         OutT* out_row = Y + (int64_t)m * (q3_paired<GATED> ? (N >> 1) : N) + (q3_paired<GATED> ? (n0 >> 1) : n0);
 #pragma unroll 1
@@ -976,7 +1099,7 @@ gemm_tcgen05_pair_splitk_kernel(const __grid_constant__ CUtensorMap map_x, const
                     }
                 }
             }
-            store_chunk32<GATED, OutT>(r, out_row, c * 32, n0, m < M, N, vec_ok);
+            store_chunk32<GATED, OutT>(r, out_row, c * 32, n0, m < M, N, vec_bytes);
         }
     }
     tc_fence_before();
@@ -1057,21 +1180,68 @@ int launch_prompt(const bf16* X, const bf16* W, OutT* Y, int M, int N, int K, in
                           map_x, map_w, Y, M, N, K, status);
 }
 
-template <int STAGES, int GATED, typename OutT, bool QKV = false>
-int launch_pair(const bf16* X, const bf16* W, OutT* Y, int M, int N, int K, int* status, cudaStream_t stream,
-                const QkvEpilogue& qkv = QkvEpilogue{}) {
-    constexpr int SMEM = STAGES * (BM * BK * 2 + 128 * BK * 2) + 1024 + 256;
+// Which tiles a product gets: `rows` (W the 256-row operand, tiles of `tile` tokens) or tokens first in tiles of 256; `us`, what it
+// should take.
+struct PairForm {
+    bool rows;
+    int tile;
+    float us;
+};
+
+// Microseconds of a K step of a tile - of a 256 x 256 one, and at least what an SM's share of the copies takes when the tile has few
+// tokens - and of a launch aside from its K steps.  (One tile a pair, K 4,096 and 12,288: 27 and 71 us tokens first, 19 and 48 with up to
+// 128 tokens a tile, 21 and 51 with 160, 23 and 56 with 192, 26 and 62 with 224, 29 and 73 with 256.)
+constexpr float TOKENS_STEP_US = 0.343f, ROWS_STEP_US = 0.224f, TOKENS_LAUNCH_US = 5.0f, ROWS_LAUNCH_US = 6.0f;
+
+PairForm pair_tiles(bool rows, int tile, int64_t M, int64_t N, int K, int pairs) {
+    const int64_t tiles = (M + tile - 1) / tile * ((N + 255) / 256);
+    const float steps = (float)((K + BK - 1) / BK) * (float)((tiles + pairs - 1) / pairs);
+    const float step = rows ? fmaxf(ROWS_STEP_US, TOKENS_STEP_US * tile / 256.0f) : TOKENS_STEP_US;
+    return PairForm{rows, tile, (rows ? ROWS_LAUNCH_US : TOKENS_LAUNCH_US) + steps * step};
+}
+
+// `may_row`: the output is bfloat16 in rows of whole 16-byte packets, which is what the drain of the rows form writes.  Equal tiles of as
+// many tokens as one to four cuts more than whole 256s would make; taken where they save 3 %.
+PairForm pair_form(int M, int N, int K, bool may_row) {
+    const int pairs = sm_count() / 2;
+    PairForm best = pair_tiles(false, 2 * BM, M, N, K, pairs);
+    if (may_row) {
+        const float most = 0.97f * best.us;
+        const int whole = (M + 255) / 256;
+        for (int cuts = whole; cuts <= whole + 3 && cuts <= (M + 63) / 64; ++cuts) {
+            const PairForm f = pair_tiles(true, ((M + cuts - 1) / cuts + 31) / 32 * 32, M, N, K, pairs);
+            if (f.us < most && f.us < best.us) best = f;
+        }
+    }
+    return best;
+}
+
+template <int GATED, typename OutT, bool QKV, bool ROWS>
+int launch_pair_form(const bf16* X, const bf16* W, OutT* Y, int M, int N, int K, int tile, int* status, cudaStream_t stream,
+                     const QkvEpilogue& qkv) {
+    constexpr int SMEM = 6 * (BM * BK * 2 + 128 * BK * 2) + 1024 + 256;
+    const auto kernel = gemm_tcgen05_pair_kernel<GATED, OutT, QKV, ROWS>;
     static Q3PerDevice configured;
     {
-        cudaError_t e = q3_allow_shared_memory(gemm_tcgen05_pair_kernel<STAGES, GATED, OutT, QKV>, SMEM, configured);
+        cudaError_t e = q3_allow_shared_memory(kernel, SMEM, configured);
         if (e != cudaSuccess) return (int)e;
     }
     CUtensorMap map_x, map_w;
-    if (!make_map(&map_x, X, M, K, BM) || !make_map(&map_w, W, N, K, 128)) return Q3_ERR_BAD_SIZE;
-    const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
+    if (!make_map(&map_x, X, M, K, tile / 2) || !make_map(&map_w, W, N, K, 128)) return Q3_ERR_BAD_SIZE;
+    const int tiles = ((M + tile - 1) / tile) * ((N + 255) / 256);
     const int pairs = tiles < sm_count() / 2 ? tiles : sm_count() / 2;
-    return (int)q3_launch_cluster(gemm_tcgen05_pair_kernel<STAGES, GATED, OutT, QKV>, dim3(2 * pairs), dim3(THREADS), (size_t)SMEM,
-                                  stream, dim3(2, 1, 1), map_x, map_w, Y, M, N, K, status, qkv);
+    return (int)q3_launch_cluster(kernel, dim3(2 * pairs), dim3(PAIR_THREADS), (size_t)SMEM, stream, dim3(2, 1, 1), map_x, map_w, Y, M, N, K,
+                                  tile, status, qkv);
+}
+
+template <int GATED, typename OutT, bool QKV = false>
+int launch_pair(const bf16* X, const bf16* W, OutT* Y, int M, int N, int K, int* status, cudaStream_t stream,
+                const QkvEpilogue& qkv = QkvEpilogue{}) {
+    if constexpr (std::is_same<OutT, bf16>::value && GATED != 3 && !QKV) {
+        const PairForm f = pair_form(M, N, K, (q3_paired<GATED> ? N / 2 : N) % 8 == 0 && aligned16(Y));
+        if (f.rows) return launch_pair_form<GATED, OutT, false, true>(X, W, Y, M, N, K, f.tile, status, stream, qkv);
+    }
+    return launch_pair_form<GATED, OutT, QKV, false>(X, W, Y, M, N, K, 2 * BM, status, stream, qkv);
 }
 
 template <int STAGES, int GATED, typename OutT>
@@ -1158,11 +1328,16 @@ Q3_EXPORT int q3_gemm_tcgen05_pair_bf16(const void* X, const void* W, void* Y, i
         return out_is_f32 ? launch_pair_splitk<6, 0, float>(x, w, (float*)Y, M, N, K, splits, status, stream)
                           : launch_pair_splitk<6, 0, bf16>(x, w, (bf16*)Y, M, N, K, splits, status, stream);
     }
-    if (gated == 3) return launch_pair<6, 3, bf16>(x, w, (bf16*)Y, M, N, K, status, stream);
-    if (gated == 2) return launch_pair<6, 2, bf16>(x, w, (bf16*)Y, M, N, K, status, stream);
-    if (gated) return launch_pair<6, 1, bf16>(x, w, (bf16*)Y, M, N, K, status, stream);
-    return out_is_f32 ? launch_pair<6, 0, float>(x, w, (float*)Y, M, N, K, status, stream)
-                      : launch_pair<6, 0, bf16>(x, w, (bf16*)Y, M, N, K, status, stream);
+    if (gated == 3) return launch_pair<3, bf16>(x, w, (bf16*)Y, M, N, K, status, stream);
+    if (gated == 2) return launch_pair<2, bf16>(x, w, (bf16*)Y, M, N, K, status, stream);
+    if (gated) return launch_pair<1, bf16>(x, w, (bf16*)Y, M, N, K, status, stream);
+    return out_is_f32 ? launch_pair<0, float>(x, w, (float*)Y, M, N, K, status, stream)
+                      : launch_pair<0, bf16>(x, w, (bf16*)Y, M, N, K, status, stream);
+}
+
+// Microseconds that q3_gemm_tcgen05_pair_bf16 without a split of K should take (`may_row`: bfloat16 output, aligned).
+Q3_EXPORT float q3_gemm_tcgen05_pair_us(int M, int N, int K, int may_row) {
+    return M > 0 && N > 0 && K > 0 ? pair_form(M, N, K, may_row && N % 8 == 0).us : 0.0f;
 }
 
 // Pairs of SMs that run at once when K is split over `splits` pairs of a cluster (0: the device cannot place it).
@@ -1189,7 +1364,7 @@ Q3_EXPORT int q3_gemm_tcgen05_pair_qkv_bf16(const void* X, const void* W, int M,
     e.q_norm_w = q_norm_w; e.k_norm_w = k_norm_w; e.cos_tab = cos_tab; e.sin_tab = sin_tab;
     e.token_seq = token_seq; e.token_pos = token_pos; e.page_table = page_table;
     e.pages_per_seq = pages_per_seq; e.nq = nq; e.nkv = nkv; e.d = d; e.write_kv = write_kv; e.eps = eps;
-    return launch_pair<6, 0, bf16, true>((const bf16*)X, (const bf16*)W, (bf16*)nullptr, M, (int)N, K, status,
+    return launch_pair<0, bf16, true>((const bf16*)X, (const bf16*)W, (bf16*)nullptr, M, (int)N, K, status,
                                              (cudaStream_t)stream_, e);
 }
 

@@ -1522,6 +1522,13 @@ def gemm_tcgen05_pair_capacity(splits: int) -> int:
     return int(fn(int(splits)))
 
 
+def gemm_tcgen05_pair_us(M: int, N: int, K: int, out_bf16: bool = True) -> float:
+    """Microseconds that `gemm_tcgen05_pair` without a split of K should take, in the tiles it would choose."""
+    fn = _fn_untimed("gemm_tcgen05.cu", "q3_gemm_tcgen05_pair_us", [c_int, c_int, c_int, c_int])
+    fn.restype = c_float
+    return float(fn(int(M), int(N), int(K), int(bool(out_bf16))))
+
+
 PAIR_QKV_HEAD_DIMS = (64, 128, 256)
 
 

@@ -253,6 +253,8 @@ int q3_gemm_tcgen05_pair_qkv_bf16(const void* X, const void* W, int M, int K, vo
 int q3_gemm_tcgen05_pair_bf16(const void* X, const void* W, void* Y, int M, int N, int K, int out_is_f32, int gated, int splits,
                               int* status, void* stream);
 int q3_gemm_tcgen05_pair_capacity(int splits);
+/* microseconds that q3_gemm_tcgen05_pair_bf16 with splits 1 should take; may_row: bfloat16 output, aligned to 16 bytes */
+float q3_gemm_tcgen05_pair_us(int M, int N, int K, int may_row);
 
 /* ---- hyper.cu: a hidden state of several streams per token, float32 [token, streams, hidden] ------------------ */
 /* out[t] = `copies` times table[ids[t]] * scale side by side */

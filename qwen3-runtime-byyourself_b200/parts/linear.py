@@ -33,21 +33,23 @@ def set_bf16_kernel_active() -> bool:
     return _bf16_kernel is not None
 
 
-# Microseconds per 64-wide K step of a tile and per block for its start and end, measured on B200.
+# Microseconds per 64-wide K step of a tile and per block for its start and end, measured on B200 (the unsplit pairs form
+# gives its own estimate, of the tiles it would take).
 _STEP_US = {"pair": 0.33, "prompt128": 0.29, "weights_first": 0.40}
-_BLOCK_US = {"pair": 8.0, "prompt128": 5.0}
+_BLOCK_US = {"prompt128": 5.0}
 # A tile with K split over the pairs of a cluster is not persistent: every wave pays the start of the stream and the
-# meeting of the partial tiles over distributed shared memory, and the launch a little more.
-_PAIR_SPLIT_WAVE_US, _PAIR_SPLIT_LAUNCH_US = 8.5, 2.5
+# meeting of the partial tiles over distributed shared memory, and the launch a little more.  (K 4,096 and 12,288: two ranges
+# 18.3 and 39.7 us, three 16.2 and 29.5; the weights-first form with a range per block of a cluster 13.4 and 26.4 with four, 19.7 with two.)
+_PAIR_SPLIT_WAVE_US, _PAIR_SPLIT_LAUNCH_US = 6.0, 2.5
+_WEIGHTS_FIRST_SPLIT_US = 7.0
 
 
 @functools.lru_cache(maxsize=4096)
-def pair_plan(M: int, N: int, K: int) -> tuple:
+def pair_plan(M: int, N: int, K: int, out_bf16: bool = True) -> tuple:
     """(estimated microseconds, K ranges) of the pairs-of-SMs form: the number of K ranges per tile (1 = persistent
-    pairs, no split) whose waves of tiles x K steps cost least."""
-    sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    pairs, no split, in the tiles that the kernel chooses) whose waves of tiles x K steps cost least."""
     nkb, tiles = -(-K // 64), -(-M // 256) * -(-N // 256)
-    best = (-(-tiles // (sms // 2)) * nkb * _STEP_US["pair"] + _BLOCK_US["pair"], 1)
+    best = (ops.gemm_tcgen05_pair_us(M, N, K, out_bf16), 1)
     for splits in range(2, ops.PAIR_MAX_SPLITS + 1):
         capacity = ops.gemm_tcgen05_pair_capacity(splits)
         if capacity <= 0 or splits > nkb or tiles > 65535:
@@ -60,7 +62,7 @@ def pair_plan(M: int, N: int, K: int) -> tuple:
 
 
 @functools.lru_cache(maxsize=4096)
-def tcgen05_form(M: int, N: int, K: int, gated: bool = False) -> str:
+def tcgen05_form(M: int, N: int, K: int, gated: bool = False, out_bf16: bool = True) -> str:
     """Which form of the tcgen05 product takes M rows (M > skinny_rows, K a multiple of 8): weights first
     (K split over a cluster; the only form that fills the GPU when M and N give few tiles), or tokens first
     and persistent, on single SMs with 128 x 128 tiles or on pairs of SMs with 256 x 256 tiles.  A small
@@ -73,13 +75,13 @@ def tcgen05_form(M: int, N: int, K: int, gated: bool = False) -> str:
     def waves(blocks, slots):
         return -(-blocks // slots)
 
-    cost = {"pair": pair_plan(M, N, K)[0]}
+    cost = {"pair": pair_plan(M, N, K, out_bf16)[0]}
     if not gated:                                        # the gated epilogue exists for the 256-row tiles
         cost["prompt128"] = waves(-(-M // 128) * -(-N // 128), sms) * nkb * _STEP_US["prompt128"] + _BLOCK_US["prompt128"]
     if M <= 1024:
         splits = ops.gemm_tcgen05_mid_splits(M, N, K)
         blocks = -(-N // 128) * -(-M // 256) * splits
-        cost["weights_first"] = waves(blocks, sms) * (-(-nkb // splits) * _STEP_US["weights_first"] + (10.0 if splits > 1 else 5.0))
+        cost["weights_first"] = waves(blocks, sms) * (-(-nkb // splits) * _STEP_US["weights_first"] + (_WEIGHTS_FIRST_SPLIT_US if splits > 1 else 5.0))
     return min(cost, key=cost.get)
 
 
@@ -100,9 +102,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         return ops.gemm_bf16_any_width(x, w, out)
     if M <= skinny_rows:
         return ops.gemm_skinny(x, w, out)
-    form = tcgen05_form(M, w.shape[0], K)
+    out_bf16 = out.dtype == torch.bfloat16
+    form = tcgen05_form(M, w.shape[0], K, out_bf16=out_bf16)
     if form == "weights_first":
         return ops.gemm_tcgen05_mid(x, w, out)
     if form == "pair":
-        return ops.gemm_tcgen05_pair(x, w, out, splits=pair_plan(M, w.shape[0], K)[1])
+        return ops.gemm_tcgen05_pair(x, w, out, splits=pair_plan(M, w.shape[0], K, out_bf16)[1])
     return ops.gemm_tcgen05_prompt(x, w, out, tile_n=128)

@@ -34,3 +34,46 @@ def test_bands_of_token_tiles(M, N):
     out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
     ops.gemm_tcgen05_pair(x, w, out)
     check(out, x, w)
+
+
+# tiles of 32 to 256 tokens (equal, with a short last one, one token in it), rows of W that end inside a warp's 32, a pair's second
+# block without rows, more tiles than pairs; outputs whose rows are no whole packets, which stay with whole 256s
+@pytest.mark.parametrize("M,N,K", [(129, 4096, 200), (160, 264, 64), (289, 4096, 72), (300, 1288, 136), (527, 24576, 72), (385, 6144, 512),
+                                   (1300, 4096, 264), (2500, 4096, 72), (527, 4100, 72), (200, 8, 64)])
+def test_tiles_of_equal_tokens(M, N, K):
+    from qwen3_b200.csrc import ops
+    x, w = operands(M, N, K)
+    out = torch.full((M + 1, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.gemm_tcgen05_pair(x, w, out[:M])
+    check(out[:M], x, w)
+    assert bool(out[M].isnan().all()), "written beyond the last token"
+    wide = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")     # tokens first: 32-bit output
+    ops.gemm_tcgen05_pair(x, w, wide)
+    assert torch.equal(wide.to(torch.bfloat16), out[:M])
+
+
+@pytest.mark.parametrize("M,inter,K", [(129, 4096, 136), (300, 1160, 72), (527, 12288, 64), (385, 104, 200), (1300, 2048, 72)])
+@pytest.mark.parametrize("activation", ["silu", "gelu_tanh"])
+def test_tiles_of_equal_tokens_gated(M, inter, K, activation):
+    """The gate in the drain of the rows form gives the bits of the product followed by the gating kernel."""
+    from qwen3_b200.csrc import ops
+    x, gate = operands(M, inter, K)
+    up = operands(M + 1, inter, K)[1]
+    w = ops.interleave_gate_up(gate * 0.2, up * 0.2)
+    fused = torch.full((M + 1, inter), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.gemm_tcgen05_pair(x, w, fused[:M], gated=True, activation=activation)
+    assert ops.tcgen05_status("cuda") == 0
+    gate_up = torch.empty(M, 2 * inter, dtype=torch.bfloat16, device="cuda")
+    ops.gemm_tcgen05_pair(x, w, gate_up)
+    check(gate_up, x, w)
+    blocks = gate_up.float().view(M, inter // 8, 2, 8)
+    g, u = blocks[:, :, 0].reshape(M, inter), blocks[:, :, 1].reshape(M, inter)
+    act = torch.nn.functional.silu(g) if activation == "silu" else torch.nn.functional.gelu(g, approximate="tanh")
+    want = act.to(torch.bfloat16).float() * u
+    # the activation's last bit may round to the other neighbour: one rounding of it and one of the product
+    assert bool(((fused[:M].float() - want).abs() <= 2.0 ** -7 * want.abs() + 1e-30).all())
+    assert bool(fused[M].isnan().all()), "written beyond the last token"
+    if activation == "silu":
+        two = torch.empty(M, inter, dtype=torch.bfloat16, device="cuda")
+        ops.silu_mul(gate_up, two, interleaved=True)
+        assert torch.equal(fused[:M], two)
