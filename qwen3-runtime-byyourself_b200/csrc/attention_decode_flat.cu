@@ -49,6 +49,7 @@ constexpr int MIN_PART = 4;                         // pages below which a row i
 constexpr int MAX_WAVES = 8;                        // parts of a block, where rows are cut
 constexpr int LONG_ROW = 48;                        // pages of the longest row from which more rows than blocks are cut
 constexpr int BLOCKS_PER_SM = 3;
+constexpr int MERGE = 12;                           // parts of a row added up in one round
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
@@ -75,12 +76,15 @@ __device__ __forceinline__ uint32_t packet(int r, int c) {
     return (uint32_t)((c >> 3) * HALF_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4));
 }
 
+// Floats between the parts' sums: [G][D], then (max, sum) [G][2], whole 16-byte packets.
+__host__ __device__ constexpr int part_floats(int G) { return (G * (D + 2) + 3) / 4 * 4; }
+
 struct Args {
     const bf16* qkv;               // [tokens, (nq + 2 nkv) * D]: the projection output as it is
     bf16* k_pages;
     bf16* v_pages;
     bf16* out;                     // [tokens, nq * D]
-    float* parts;                  // [MAX_WAVES blocks][G][D + 2]: sums, then (max, sum)
+    float* parts;                  // [MAX_WAVES blocks][part_floats(G)], 16-byte aligned
     int* counters;                 // [tokens * nkv], zero between launches
     const float* q_norm_w;         // [D] or null
     const float* k_norm_w;
@@ -422,7 +426,7 @@ decode_flat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                 }
             }
             meet();
-            float* mine = a.parts + (int64_t)chunk * G * (D + 2);
+            float* mine = a.parts + (int64_t)chunk * part_floats(G);
             bf16* out = a.out + ((int64_t)t * a.nq + kvh * G) * D;
             for (int idx = threadIdx.x; idx < G * D; idx += WARPS * 32) {
                 const int g = idx / D, col = idx % D;
@@ -459,37 +463,45 @@ decode_flat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                 meet();
                 if (*last_one) {
                     __threadfence();
-                    const float* parts = a.parts + (int64_t)(chunk - part) * G * (D + 2);
-                    for (int idx = threadIdx.x; idx < G * D; idx += WARPS * 32) {
+                    // Four values a thread and MERGE parts' packets asked for together: a row of one long sequence has some fifty
+                    // parts, and a round of loads takes about a microsecond whatever it brings.
+                    const float* parts = a.parts + (int64_t)(chunk - part) * part_floats(G);
+                    for (int idx = threadIdx.x * 4; idx < G * D; idx += WARPS * 32 * 4) {
                         const int g = idx / D;
-                        float m = -INFINITY, l = 0.0f, acc = 0.0f;
-                        for (int b = 0; b < k; b += 8) {                 // eight parts' values asked for together
-                            float ms[8], ls[8], os[8], top = m;
+                        float m = -INFINITY, l = 0.0f;
+                        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                        for (int b = 0; b < k; b += MERGE) {
+                            float ms[MERGE], ls[MERGE], top = m;
+                            float4 os[MERGE];
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) {
+                            for (int i = 0; i < MERGE; ++i) {
                                 ms[i] = -INFINITY;
-                                ls[i] = os[i] = 0.0f;
+                                ls[i] = 0.0f;
+                                os[i] = make_float4(0.f, 0.f, 0.f, 0.f);
                                 if (b + i < k) {
-                                    const float* from = parts + (int64_t)(b + i) * G * (D + 2);
-                                    os[i] = __ldcg(from + idx);
+                                    const float* from = parts + (int64_t)(b + i) * part_floats(G);
+                                    os[i] = __ldcg(reinterpret_cast<const float4*>(from + idx));
                                     ms[i] = __ldcg(from + G * D + 2 * g);
                                     ls[i] = __ldcg(from + G * D + 2 * g + 1);
                                 }
                             }
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) top = fmaxf(top, ms[i]);
+                            for (int i = 0; i < MERGE; ++i) top = fmaxf(top, ms[i]);
                             const float use = top == -INFINITY ? 0.0f : top, f = exp2f(m - use);
                             l *= f;
-                            acc *= f;
+                            acc.x *= f; acc.y *= f; acc.z *= f; acc.w *= f;
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) {
+                            for (int i = 0; i < MERGE; ++i) {
                                 const float w = exp2f(ms[i] - use);      // 0 where the part has seen no key
                                 l += w * ls[i];
-                                acc += w * os[i];
+                                acc.x += w * os[i].x; acc.y += w * os[i].y; acc.z += w * os[i].z; acc.w += w * os[i].w;
                             }
                             m = top;
                         }
-                        out[idx] = __float2bfloat16_rn(acc / l);
+                        out[idx] = __float2bfloat16_rn(acc.x / l);
+                        out[idx + 1] = __float2bfloat16_rn(acc.y / l);
+                        out[idx + 2] = __float2bfloat16_rn(acc.z / l);
+                        out[idx + 3] = __float2bfloat16_rn(acc.w / l);
                     }
                 }
             }
@@ -514,7 +526,7 @@ Q3_EXPORT int q3_attention_decode_flat_blocks(int group) { return blocks_per_sm(
 
 // Float32 elements of `parts`; `counters` holds n_tokens * nkv ints, zero before the first launch and left zero by each.
 Q3_EXPORT int64_t q3_attention_decode_flat_parts(int group) {
-    return (int64_t)MAX_WAVES * q3_attention_decode_flat_blocks(group) * group * (D + 2);
+    return (int64_t)MAX_WAVES * q3_attention_decode_flat_blocks(group) * part_floats(group) + 4;      // 4: to a 16-byte boundary
 }
 
 Q3_EXPORT int q3_attention_decode_flat_bf16(const void* qkv, void* k_pages, void* v_pages, void* out, float* parts, int* counters,
@@ -538,7 +550,8 @@ Q3_EXPORT int q3_attention_decode_flat_bf16(const void* qkv, void* k_pages, void
         return Q3_ERR_BAD_SIZE;
     Args a;
     a.qkv = (const bf16*)qkv; a.k_pages = (bf16*)k_pages; a.v_pages = (bf16*)v_pages; a.out = (bf16*)out;
-    a.parts = parts; a.counters = counters;
+    a.parts = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(parts) + 15) & ~(uintptr_t)15);
+    a.counters = counters;
     a.q_norm_w = q_norm_w; a.k_norm_w = k_norm_w; a.cos_tab = cos_tab; a.sin_tab = sin_tab;
     a.token_seq = token_seq; a.token_pos = token_pos; a.page_table = page_table;
     a.pages_per_seq = pages_per_seq; a.n_tokens = (int)n_tokens; a.nq = nq; a.nkv = nkv; a.window = window;

@@ -463,9 +463,15 @@ def _decode_fused_kernel(part, qkv, cache, out, ctx, table, q_norm_w, k_norm_w, 
         # two: 54.7 with 12 against 64.8; at 2,048 keys 11.8 against 11.1)
         wide = min(splits, max(8, wide_cluster_blocks // (ctx.n_tokens * nkv)), ops.attention_decode_fused_max_splits(d, ctx.device))
         splits = wide if ctx.max_context > long_context_keys else 8
+    elif splits in (6, 7):
+        # a cluster of six or seven blocks leaves SMs empty where four fit (8 kv heads, contexts of 300 to 3,000 tokens: five sequences
+        # 14.6 us in fours against 22.6 in sevens, six 13.8 against 20.2; of 4,000 tokens 23.8 / 34.1 and 24.7 / 36.7)
+        splits = 4
     parts = counters = None
-    # rows (sequences x kv heads) that the form below cannot split any more: parts of equal length instead
-    if ctx.n_tokens * nkv > shared_out_rows_per_sm * _sm_count(ctx.device) and ops.attention_decode_flat_fits(d, nq // nkv):
+    # rows (sequences x kv heads) that the form below cannot split any more, or in three: parts of equal length instead (twelve sequences of
+    # 100 to 3,000 tokens 19.7 us against 23.2 in threes, of 100 to 300 10.6 against 17.0)
+    shared_out = splits == 3 or ctx.n_tokens * nkv > shared_out_rows_per_sm * _sm_count(ctx.device)
+    if shared_out and ops.attention_decode_flat_fits(d, nq // nkv):
         parts = ctx.scratch.get("attn.decode_parts", (ops.attention_decode_flat_parts(d, nq // nkv),), torch.float32)
         counters = ctx.scratch.counters("attn.decode_counters", ctx.n_tokens * nkv)
     ops.attention_decode_fused(qkv, cache.keys, cache.values, out, q_norm_w, k_norm_w, cos, sin, eps, ctx.token_seq,
