@@ -15,7 +15,7 @@ def test_blocks_of_a_row(n_tokens, nkv, expected, monkeypatch):
     monkeypatch.setattr(attention, "_sm_count", lambda device: 148)
     monkeypatch.setattr(ops, "attention_decode_flat_parts", lambda d, group: 64)
     monkeypatch.setattr(ops, "attention_decode_fused_max_splits", lambda d, device: 16)
-    monkeypatch.setattr(ops, "attention_decode_fused", lambda *a, **k: seen.update(splits=a[17], parts=k["parts"]))
+    monkeypatch.setattr(ops, "attention_decode_fused", lambda *a, **k: seen.update(splits=a[18], parts=k["parts"]))
     part = types.SimpleNamespace(plain=True, num_heads=4 * nkv, num_kv_heads=nkv, head_dim=128, scale=1.0, window=None)
     scratch = types.SimpleNamespace(get=lambda name, shape, dtype: torch.empty(shape, dtype=dtype),
                                     counters=lambda name, n: torch.zeros(n, dtype=torch.int32))
