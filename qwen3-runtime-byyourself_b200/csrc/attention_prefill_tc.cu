@@ -28,6 +28,10 @@
 //   starts at 0 and the running sum at the sink's weight.  The softmax and its weights are computed in 32-bit and
 //   enter the second product as two bfloat16 terms, p = hi + lo with hi = bf16(p) and lo = bf16(p - hi) (TMEM
 //   columns [64,96) and [96,128), two sets of tcgen05.mma per page), so the product sees them to 16 bits of mantissa.
+//   -DQ3_VALUE_DIM=<size> beside -DQ3_CAPPED=1: heads of 192 or 256 with values of their own size (multiples of 64), and a window
+//   instead of a cap or chunks (latent attention: one key head of 192 + 64, values of 192).  One block an SM then, as Q and the
+//   rings take 209 KB; three prompts of 2,048, 911 and 1,203 tokens with 16 heads 97 us (438 on
+//   mma.sync tiles), behind a window of 1,024 91 (379), one of 128 16 (16), of 512 22 (40), of 8,000 586 (3,691).  Bound by the softmax of one tile an SM.
 //   -DQ3_CAPPED=2: with a sink and biases by distance instead of a cap or chunks; the biases are added to the scaled scores: one number a page for pages far enough back, else one a score.
 #include <cuda.h>
 
@@ -55,20 +59,26 @@ struct CapArgs {
     const float* sink_values;   // one score per query head instead of that 0 (may be null)
     const float* bias;          // biases by distance, [query heads][bias_count], the last one for all that is further (may be null;
     int bias_count;             // not together with a cap)
+    int window;                 // the wide form: keys seen before a token, itself included (0: all)
 };
 
-constexpr int D = Q3_HEAD_DIM;
-static_assert(D == 64 || D == 128, "the tcgen05 attention takes head sizes 64 and 128");
-constexpr int PAGE = Q3_PAGE_TOKENS, BM = 128, HALVES = D / 64;
+#ifndef Q3_VALUE_DIM
+#define Q3_VALUE_DIM Q3_HEAD_DIM
+#endif
+constexpr int D = Q3_HEAD_DIM, VD = Q3_VALUE_DIM;
+constexpr bool WIDE = D > 128;                           // one block an SM, a window
+static_assert(WIDE ? Q3_CAPPED == 1 && D % 64 == 0 && D <= 256 && VD % 64 == 0 && VD >= 64 && VD <= 256 : VD == D && (D == 64 || D == 128),
+              "the tcgen05 attention takes head sizes 64 and 128, with options also 192 and 256");
+constexpr int PAGE = Q3_PAGE_TOKENS, BM = 128, HALVES = D / 64, V_HALVES = VD / 64;
 static_assert(PAGE == 64, "the tcgen05 prompt attention takes one page of 64 keys per product");
 constexpr int THREADS = 224;
 constexpr int K_STAGES = 3, V_STAGES = 2;                // pages of K and of V in flight or in use
 constexpr int Q_BYTES = HALVES * BM * 128;               // 128 rows x 128 bytes per half
-constexpr int PANEL_BYTES = HALVES * PAGE * 128;         // one page of K (or V): 64 keys x 128 bytes per half
+constexpr int K_PANEL_BYTES = HALVES * PAGE * 128, V_PANEL_BYTES = V_HALVES * PAGE * 128;   // one page: 64 keys x 128 bytes per half
 // no slack for alignment: two blocks of head size 128 have to fit one SM, and the dynamic shared memory of
 // a kernel without static shared memory starts at a 1024-byte boundary (checked when the kernel starts)
-constexpr int SMEM_BYTES = Q_BYTES + (K_STAGES + V_STAGES) * PANEL_BYTES + 256;
-constexpr uint32_t TMEM_COLS = 256;
+constexpr int SMEM_BYTES = Q_BYTES + K_STAGES * K_PANEL_BYTES + V_STAGES * V_PANEL_BYTES + 256;
+constexpr uint32_t TMEM_COLS = VD > 128 ? 512 : 256;
 constexpr uint32_t COL_S = 0, COL_P = 64, COL_P_LO = 96, COL_O = 128;   // COL_P_LO: the capped form's second term of the weights
 constexpr float RESCALE_THRESHOLD = 8.0f;                // in log2 units: probabilities stay below 2^8
 
@@ -163,8 +173,13 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const int* pages = page_table + (int64_t)seq * pages_per_seq;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rows = min(BM, n_new - tile * BM);
-    // pages first_page .. the one of the last row (first_page: where the chunk of the tile's first row starts)
-    const int first_page = (CAPPED && !BIAS && capped.chunk > 0) ? ((pos0 + tile * BM) / capped.chunk * capped.chunk) / PAGE : 0;
+    // the first key that the row at position p sees
+    auto first_key = [&](int p) {
+        if (WIDE) return capped.window > 0 ? max(0, p - capped.window + 1) : 0;
+        return (CAPPED && !BIAS && capped.chunk > 0) ? p / capped.chunk * capped.chunk : 0;
+    };
+    // pages first_page .. the one of the last row (first_page: the one of the first key of the tile's first row)
+    const int first_page = first_key(pos0 + tile * BM) / PAGE;
     const int n_pages = (pos0 + tile * BM + rows - 1) / PAGE + 1 - first_page;
 
     const uint32_t base = smem_u32(smem_raw);
@@ -172,8 +187,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         if (threadIdx.x == 0) atomicExch(status, 18);
         return;
     }
-    const uint32_t q_smem = base, k_smem = base + Q_BYTES, v_smem = k_smem + K_STAGES * PANEL_BYTES;
-    const uint32_t bars = v_smem + V_STAGES * PANEL_BYTES;
+    const uint32_t q_smem = base, k_smem = base + Q_BYTES, v_smem = k_smem + K_STAGES * K_PANEL_BYTES;
+    const uint32_t bars = v_smem + V_STAGES * V_PANEL_BYTES;
     const uint32_t bar_q = bars, bar_k_full = bars + 8, bar_k_empty = bar_k_full + 8 * K_STAGES;
     const uint32_t bar_v_full = bar_k_empty + 8 * K_STAGES, bar_v_empty = bar_v_full + 8 * V_STAGES;
     const uint32_t bar_s_full = bar_v_empty + 8 * V_STAGES, bar_s_read = bar_s_full + 8, bar_p_full = bar_s_read + 8;
@@ -214,9 +229,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             for (int j = 0; j < n_pages; ++j) {
                 const int s = j % K_STAGES;
                 if (!mbar_wait(bar_k_empty + 8 * s, ((uint32_t)(j / K_STAGES) & 1u) ^ 1u)) { atomicExch(status, 11); break; }
-                const uint32_t dst = k_smem + s * PANEL_BYTES;
+                const uint32_t dst = k_smem + s * K_PANEL_BYTES;
                 const int row = (pages[first_page + j] * nkv + kvh) * PAGE;
-                mbar_expect_tx(bar_k_full + 8 * s, PANEL_BYTES);
+                mbar_expect_tx(bar_k_full + 8 * s, K_PANEL_BYTES);
 #pragma unroll
                 for (int h = 0; h < HALVES; ++h) tma_load_2d(dst + h * PAGE * 128, &map_k, bar_k_full + 8 * s, h * 64, row);
             }
@@ -227,22 +242,22 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             for (int j = 0; j < n_pages; ++j) {
                 const int s = j % V_STAGES;
                 if (!mbar_wait(bar_v_empty + 8 * s, ((uint32_t)(j / V_STAGES) & 1u) ^ 1u)) { atomicExch(status, 19); break; }
-                const uint32_t dst = v_smem + s * PANEL_BYTES;
+                const uint32_t dst = v_smem + s * V_PANEL_BYTES;
                 const int row = (pages[first_page + j] * nkv + kvh) * PAGE;
-                mbar_expect_tx(bar_v_full + 8 * s, PANEL_BYTES);
+                mbar_expect_tx(bar_v_full + 8 * s, V_PANEL_BYTES);
 #pragma unroll
-                for (int h = 0; h < HALVES; ++h) tma_load_2d(dst + h * PAGE * 128, &map_v, bar_v_full + 8 * s, h * 64, row);
+                for (int h = 0; h < V_HALVES; ++h) tma_load_2d(dst + h * PAGE * 128, &map_v, bar_v_full + 8 * s, h * 64, row);
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer: the whole warp walks and one elected thread issues, so the
         // compiler keeps descriptors in uniform registers, which is what the instruction takes
-        constexpr uint32_t idesc_s = idesc(BM, PAGE, false), idesc_pv = idesc(BM, D, true);
+        constexpr uint32_t idesc_s = idesc(BM, PAGE, false), idesc_pv = idesc(BM, VD, true);
         const uint32_t acc = __shfl_sync(0xffffffffu, tmem, 0);
         const uint64_t q_desc = desc_k_major(q_smem), k_desc = desc_k_major(k_smem), v_desc = desc_mn_major(v_smem, PAGE * 128);
         auto issue_s = [&](int j) {
             const uint32_t s = (uint32_t)j % K_STAGES;
-            const uint64_t k_src = k_desc + (uint64_t)(s * (PANEL_BYTES >> 4));
+            const uint64_t k_src = k_desc + (uint64_t)(s * (K_PANEL_BYTES >> 4));
             if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk) {
@@ -275,7 +290,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             if (!ok) { failed(14); break; }
             tc_fence_after();
             const uint32_t s = (uint32_t)j % V_STAGES;
-            const uint64_t v_src = v_desc + (uint64_t)(s * (PANEL_BYTES >> 4));
+            const uint64_t v_src = v_desc + (uint64_t)(s * (V_PANEL_BYTES >> 4));
             if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < PAGE / 16; ++kk)
@@ -299,8 +314,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         float m_run = -INFINITY, l_run = 0.0f;
         bool ok = true;
         // the capped form: the first key this row sees, and the constants of s -> cap * tanh(s * scale / cap) in log2 units
-        const int c_row = (CAPPED && !BIAS && capped.chunk > 0) ? p_row / capped.chunk * capped.chunk : 0;
-        const int c_last = (CAPPED && !BIAS && capped.chunk > 0) ? (pos0 + tile * BM + BM - 1) / capped.chunk * capped.chunk : 0;
+        const int c_row = first_key(p_row), c_last = first_key(pos0 + tile * BM + BM - 1);
         const float cap_l2 = capped.cap * 1.4426950408889634f;                       // the cap in log2 units
         const float tanh_k = capped.cap > 0.0f ? 2.0f * capped.scale * 1.4426950408889634f / capped.cap : 0.0f;
         const float sink_score = CAPPED && capped.sink_values != nullptr ? capped.sink_values[head] * 1.4426950408889634f : 0.0f;
@@ -319,7 +333,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_s_read);
             const int key0 = (first_page + j) * PAGE;
-            // some key of the page lies after some row (or, with chunks, before the chunk of some row)
+            // some key of the page lies after some row (or, with chunks or a window, before the first key of some row)
             const bool edge = key0 + PAGE - 1 > pos0 + tile * BM || (CAPPED && key0 < c_last);
             if (edge) {
 #pragma unroll
@@ -427,7 +441,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 tc_fence_after();
                 if (__any_sync(0xffffffffu, raise)) {                        // the loads and stores are warp-wide
 #pragma unroll 1
-                    for (int c = 0; c < D; c += 32) {
+                    for (int c = 0; c < VD; c += 32) {
                         uint32_t o[32];
                         tc_ld32(t_row + COL_O + c, o);
                         tc_wait_ld();
@@ -457,9 +471,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         if (ok) {
             tc_fence_after();
             const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
-            bf16* dst = out + ((int64_t)(t0 + tile * BM + r) * nq + head) * D;
+            bf16* dst = out + ((int64_t)(t0 + tile * BM + r) * nq + head) * VD;
 #pragma unroll 1
-            for (int c = 0; c < D; c += 32) {
+            for (int c = 0; c < VD; c += 32) {
                 uint32_t o[32];
                 tc_ld32(t_row + COL_O + c, o);
                 tc_wait_ld();
@@ -504,7 +518,7 @@ static int launch_prefill_tc(const void* q, const void* k_pages, const void* v_p
     }
     CUtensorMap map_q, map_k, map_v;
     if (!q3_make_map_bf16(&map_q, q, n_tokens, (int64_t)nq * D, BM, 64, true) || !q3_make_map_bf16(&map_k, k_pages, n_cache_pages * nkv * PAGE, D, PAGE, 64, true) ||
-        !q3_make_map_bf16(&map_v, v_pages, n_cache_pages * nkv * PAGE, D, PAGE, 64, true))
+        !q3_make_map_bf16(&map_v, v_pages, n_cache_pages * nkv * PAGE, VD, PAGE, 64, true))
         return Q3_ERR_BAD_SIZE;
     const int n_tiles = (max_new + BM - 1) / BM;
     const int64_t blocks = (int64_t)n_tiles * n_seqs * nq;
@@ -526,6 +540,20 @@ Q3_EXPORT int q3_attention_capped_prefill_tc_bf16(const void* q, const void* k_p
     CapArgs capped;
     capped.bias = bias; capped.bias_count = bias_count;
     capped.scale = scale; capped.cap = softcap; capped.chunk = chunk; capped.sink = sink ? 1 : 0; capped.sink_values = sink_values;
+    capped.window = 0;
+    if (WIDE && chunk > 0) return Q3_ERR_BAD_SIZE;
+    return launch_prefill_tc(q, k_pages, v_pages, out, seq_start, seq_pos0, page_table, pages_per_seq, n_seqs, max_new, n_tokens,
+                             n_cache_pages, nq, nkv, scale, status, stream, capped);
+}
+
+// The wide form: k_pages [n_cache_pages, nkv, 64, D], v_pages [n_cache_pages, nkv, 64, VD], out [n_tokens, nq * VD]; window 0: none.
+Q3_EXPORT int q3_attention_wide_prefill_tc_bf16(const void* q, const void* k_pages, const void* v_pages, void* out, const int* seq_start,
+                                                const int* seq_pos0, const int* page_table, int pages_per_seq, int n_seqs, int max_new,
+                                                int64_t n_tokens, int64_t n_cache_pages, int nq, int nkv, float scale, int window, int sink,
+                                                const float* sink_values, int* status, void* stream) {
+    if (!WIDE || window < 0) return Q3_ERR_BAD_SIZE;
+    CapArgs capped = {};
+    capped.scale = scale; capped.sink = sink ? 1 : 0; capped.sink_values = sink_values; capped.window = window;
     return launch_prefill_tc(q, k_pages, v_pages, out, seq_start, seq_pos0, page_table, pages_per_seq, n_seqs, max_new, n_tokens,
                              n_cache_pages, nq, nkv, scale, status, stream, capped);
 }

@@ -1193,6 +1193,30 @@ def attention_capped_prefill_tc(q, k_pages, v_pages, out, seq_start, seq_pos0, p
     return out
 
 
+def attention_wide_prefill_tc_fits(d: int, vd: int) -> bool:
+    """Head sizes of `attention_wide_prefill_tc`: 192 and 256, values of any multiple of 64 up to 256."""
+    return d in (192, 256) and vd % 64 == 0 and 0 < vd <= 256
+
+
+def attention_wide_prefill_tc(q, k_pages, v_pages, out, seq_start, seq_pos0, page_table, n_seqs: int, max_new: int, n_tokens: int, nq: int,
+                              nkv: int, d: int, vd: int, scale: float, window: Optional[int] = None, sink: bool = False,
+                              sink_values: Optional[torch.Tensor] = None):
+    """`attention_capped_prefill` without a cap or chunks, both products on tcgen05: heads of up to 256, values of their own size."""
+    if q.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or not attention_wide_prefill_tc_fits(d, vd) or not scale > 0:
+        raise KernelError("attention_wide_prefill_tc: bfloat16, head size 192 or 256, values in multiples of 64 up to 256, a positive scale")
+    if q.shape != (n_tokens, nq * d) or out.shape[-1] != nq * vd or k_pages.shape[1:] != (nkv, PAGE_TOKENS, d) \
+            or v_pages.shape != (*k_pages.shape[:3], vd):
+        raise KernelError("attention_wide_prefill_tc: shapes do not fit")
+    fn = _fn("attention_prefill_tc.cu", "q3_attention_wide_prefill_tc_bf16",
+             [c_void_p] * 7 + [c_int, c_int, c_int, c_int64, c_int64, c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p],
+             defines=(f"Q3_HEAD_DIM={d}", "Q3_CAPPED=1", f"Q3_VALUE_DIM={vd}"))
+    _check(fn(_dev(q, "q"), _dev(k_pages, "k_pages", torch.bfloat16), _dev(v_pages, "v_pages", torch.bfloat16), _dev(out, "out"),
+              _dev(seq_start, "seq_start", torch.int32), _dev(seq_pos0, "seq_pos0", torch.int32), _dev(page_table, "page_table", torch.int32),
+              page_table.shape[-1], n_seqs, max_new, n_tokens, k_pages.shape[0], nq, nkv, float(scale), int(window or 0), int(bool(sink)),
+              _sink_ptr(sink, sink_values, nq), _status_word(q.device).data_ptr(), _stream()), "attention_wide_prefill_tc")
+    return out
+
+
 # ------------------------------------------------------------------ sampling
 def argmax(logits: torch.Tensor, out: torch.Tensor, valid: Optional[int] = None) -> torch.Tensor:
     """out[r] = index of the highest logit of row r (lowest id among equals, NaN as -inf)."""

@@ -34,5 +34,7 @@ def all_variants():
         ("linear_scan.cu", ()),
         ("short_conv.cu", ()),
         ("attention_prefill_tc.cu", ("Q3_HEAD_DIM=128", "Q3_CAPPED=2")),
+        ("attention_prefill_tc.cu", ("Q3_HEAD_DIM=256", "Q3_CAPPED=1", "Q3_VALUE_DIM=192")),
+        ("attention_capped.cu", ("Q3_HEAD_DIM=256", "Q3_VALUE_DIM=192")),
         ("ssd.cu", ("Q3_STATE=128", "Q3_VALUE_DIM=64")),
     ]

@@ -158,6 +158,11 @@ int q3_attention_capped_prefill_tc_bf16(const void* q, const void* k_pages, cons
                                         const int* seq_pos0, const int* page_table, int pages_per_seq, int n_seqs, int max_new,
                                         int64_t n_tokens, int64_t n_cache_pages, int nq, int nkv, float scale, float softcap, int chunk,
                                         int sink, const float* sink_values, const float* bias, int bias_count, int* status, void* stream);
+/* -DQ3_HEAD_DIM=192 or 256 -DQ3_CAPPED=1 -DQ3_VALUE_DIM=<64, 128, 192 or 256>: values of their own size, a window (0: none) */
+int q3_attention_wide_prefill_tc_bf16(const void* q, const void* k_pages, const void* v_pages, void* out, const int* seq_start,
+                                      const int* seq_pos0, const int* page_table, int pages_per_seq, int n_seqs, int max_new,
+                                      int64_t n_tokens, int64_t n_cache_pages, int nq, int nkv, float scale, int window, int sink,
+                                      const float* sink_values, int* status, void* stream);
 
 /* ---- attention_capped.cu (-DQ3_HEAD_DIM, -DQ3_VALUE_DIM): bfloat16 attention with scores capped by softcap * tanh(s / softcap)
    (0: none), chunked visibility (chunk 0: causal only), a sink term in the softmax's denominator, values of their own size */

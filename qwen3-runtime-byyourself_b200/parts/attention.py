@@ -556,6 +556,18 @@ def _prefill_capped_tcgen05_kernel(part, q, cache, out, ctx, table) -> bool:
     return True
 
 
+def _prefill_wide_tcgen05_kernel(part, q, cache, out, ctx, table) -> bool:
+    """Heads of up to 256 with values of their own size (latent attention), a window and a sink on tcgen05."""
+    if part.plain or part.keep_first or part.shared_values or part.softcap or part.chunk or part.bias_table is not None \
+            or part.pooled(ctx, cache) is not None or part.value_heads != part.num_kv_heads or out.dtype != torch.bfloat16 \
+            or not ops.attention_wide_prefill_tc_fits(part.head_dim, part.value_dim) or ctx.max_new < tc_prefill_rows or part.scale <= 0:
+        return False
+    ops.attention_wide_prefill_tc(q[:ctx.n_tokens], cache.keys, cache.values, out, ctx.seq_start, ctx.seq_pos0, table, ctx.n_seqs, ctx.max_new,
+                                  ctx.n_tokens, part.num_heads, part.num_kv_heads, part.head_dim, part.value_dim, part.scale,
+                                  window=part.window, sink=part.sink, sink_values=part.sink_values)
+    return True
+
+
 def _decode_capped_kernel(part, q, cache, out, ctx, table) -> bool:
     """The same for decode steps: split over the keys of the chunk (or of the whole context), merged with the sink."""
     if not part.decodes_split(ctx):
@@ -599,6 +611,7 @@ FUSED_PROJECTION_KERNELS.append(_projection_pair_kernel)
 PREFILL_KERNELS.append(_prefill_tcgen05_kernel)
 PREFILL_KERNELS.append(_prefill_flash_kernel)
 PREFILL_KERNELS.append(_prefill_capped_tcgen05_kernel)
+PREFILL_KERNELS.append(_prefill_wide_tcgen05_kernel)
 PREFILL_KERNELS.append(_prefill_capped_kernel)
 DECODE_KERNELS.append(_decode_capped_kernel)
 
