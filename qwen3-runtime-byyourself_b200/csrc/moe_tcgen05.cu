@@ -9,8 +9,8 @@
 // tiles of at most 256 and a tile costs its tokens rounded up to 64, where a 256-row token side would cost whole
 // 256s.  The tile list is walked on the device from the sorted offsets; the host never learns how many tokens an
 // expert has.  Bound by the tensor cores with hundreds of tokens per expert, by reading the weights with tens:
-//   16 experts of 3,072 at width 4,096, 8,324 pairs: 693 us for the gather and both products (0.91 PFLOP/s; 2,924 us with
-//   mma.sync tiles of 64 x 64); 256 pairs: 243 us, 0.75 of the time that reading the weights takes.
+//   16 experts of 3,072 at width 4,096, 8,324 pairs: 629 us for the gather and both products at first, 703 launched back to back for
+//   longer (0.89 PFLOP/s; 2,924 us with mma.sync tiles of 64 x 64); 500 pairs: 222 us, 0.84 of the rate that reading the weights could have.
 //
 // Roles in a block: warp 0 the TMA producer, warp 1 tensor memory and (in the pair's first block) the products, warps 2-5
 // drain.  The accumulator is double-buffered, so a tile drains under the products of the next.  A block's 128 rows of W are
@@ -24,7 +24,7 @@
 namespace {
 
 constexpr int THREADS = 192, STAGES = 6, BK = 64, ROWS = 128, UMMA_K = 16;
-constexpr int MAX_TOKENS = 256, TOKEN_STEP = 64, BOX = 32;            // tokens per tile, its granularity, rows of a token box
+constexpr int MAX_TOKENS = 256, TOKEN_STEP = 64;                      // tokens per tile, its granularity
 constexpr int A_BYTES = ROWS * BK * 2, B_BYTES = MAX_TOKENS / 2 * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr uint32_t TMEM_COLS = 2 * MAX_TOKENS;
 constexpr int MEET_BYTES = 2 * 32 * 64 * 4;                            // two buffers of 32 tokens x 64 features
@@ -60,7 +60,8 @@ struct Walk {
 
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
-expert_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const int* __restrict__ offsets,
+expert_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x32, const __grid_constant__ CUtensorMap map_x64,
+              const int* __restrict__ offsets,
               void* __restrict__ out, int n_real, int rows, int K, float limit, float alpha, float up_offset, int* __restrict__ status) {
     // rows: features of an expert's output (ff for up, hidden for down)
     extern __shared__ unsigned char smem_raw[];
@@ -76,7 +77,8 @@ expert_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
 
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x32) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x64) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(bars + s * 8, 1);
@@ -103,30 +105,33 @@ expert_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     Walk walk(offsets, n_real, n_tiles);
     int row_tile, slot, tokens, n;
     if (warp == 0) {
-        if (lane == 0) {
-            uint32_t it = 0;
-            bool ok = true;
-            for (int tile = first; ok && walk.at(tile, row_tile, slot, tokens, n); tile += stride) {
-                const int half = n / 2, x0 = slot + (int)rank * half;
-                int w0, w1;                                   // the two boxes of 64 rows of W that this block loads
-                if (MODE == GATED) {
-                    w0 = walk.e * 2 * rows + row_tile * FEATURES + (int)rank * 64;
-                    w1 = w0 + rows;
-                } else {
-                    w0 = walk.e * rows + row_tile * FEATURES + (int)rank * 128;
-                    w1 = w0 + 64;
+        // The whole warp walks and one elected thread copies, as below: what a copy takes is in uniform registers, too.  A block's 128
+        // rows of W are one box (the gate's and up's halves one dimension apart), its tokens one or two: with boxes of 64 and 32 rows, five
+        // of them a K step from a lane by itself, the copies' issue was what a K step waited for (8,324 pairs of 16
+        // experts 3,072 x 4,096 852 us against 703, 3,000 365 / 319; 6,000 of 2,048 x 2,048 278 / 258, 1,400 132 / 124).
+        uint32_t it = 0;
+        bool ok = true;
+        for (int tile = first; ok && walk.at(tile, row_tile, slot, tokens, n); tile += stride) {
+            const int half = __shfl_sync(0xffffffffu, n, 0) / 2, x0 = __shfl_sync(0xffffffffu, slot, 0) + (int)rank * half;
+            const int w0 = __shfl_sync(0xffffffffu, row_tile, 0) * FEATURES + (int)rank * (FEATURES / 2), e = __shfl_sync(0xffffffffu, walk.e, 0);
+            for (int kb = 0; kb < nkb; ++kb, ++it) {
+                const uint32_t s = it % STAGES;
+                ok = mbar_wait_warp(bars + (STAGES + s) * 8, ((it / STAGES) & 1u) ^ 1u);
+                if (!ok) {
+                    if (lane == 0) atomicExch(status, 1);
+                    break;
                 }
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    ok = mbar_wait(bars + (STAGES + s) * 8, ((it / STAGES) & 1u) ^ 1u);
-                    if (!ok) { atomicExch(status, 1); break; }
-                    const uint32_t a = base + s * STAGE_BYTES, b = a + A_BYTES;
-                    const uint32_t full = map_to_rank(bars + s * 8, 0);
+                const uint32_t a = base + s * STAGE_BYTES, b = a + A_BYTES;
+                const uint32_t full = map_to_rank(bars + s * 8, 0);
+                if (elect_one()) {
                     if (rank == 0) mbar_expect_tx(bars + s * 8, 2 * (A_BYTES + half * BK * 2));       // both blocks' bytes
-                    tma_load_2d_pair(a, &map_w, full, kb * BK, w0);
-                    tma_load_2d_pair(a + A_BYTES / 2, &map_w, full, kb * BK, w1);
-                    for (int r = 0; r < half; r += BOX) tma_load_2d_pair(b + r * BK * 2, &map_x, full, kb * BK, x0 + r);
+                    if (MODE == GATED) tma_load_3d_pair(a, &map_w, full, kb * BK, w0, 2 * e);
+                    else tma_load_3d_pair(a, &map_w, full, kb * BK, w0, e);
+                    int r = 0;
+                    for (; r + 64 <= half; r += 64) tma_load_2d_pair(b + r * BK * 2, &map_x64, full, kb * BK, x0 + r);
+                    if (r < half) tma_load_2d_pair(b + r * BK * 2, &map_x32, full, kb * BK, x0 + r);
                 }
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
@@ -256,6 +261,18 @@ gather_tokens_kernel(const uint4* __restrict__ h, const int* __restrict__ pair_o
     }
 }
 
+// `count` matrices [rows, K] one after the other, fetched in boxes of [box_count, box_rows, BK] with 128-byte swizzle; beyond a
+// matrix's last row a box reads zeros.
+bool make_weight_map(CUtensorMap* map, const bf16* W, int count, int rows, int K, int box_rows, int box_count) {
+    const Q3EncodeTiled fn = q3_encode_fn();
+    if (fn == nullptr) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)count};
+    const cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)rows * K * 2};
+    const cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_rows, (cuuint32_t)box_count}, elem[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(W), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <int MODE>
 int launch(const bf16* W, const bf16* X, const int* offsets, void* out, int n_pairs, int n_real, int rows, int K, float limit,
            float alpha, float up_offset, int* status, cudaStream_t stream) {
@@ -264,14 +281,14 @@ int launch(const bf16* W, const bf16* X, const int* offsets, void* out, int n_pa
     static Q3PerDevice configured;
     const cudaError_t e = q3_allow_shared_memory(expert_kernel<MODE>, SMEM, configured);
     if (e != cudaSuccess) return (int)e;
-    CUtensorMap map_w, map_x;
-    if (!q3_make_map_bf16(&map_w, W, (int64_t)n_real * rows * (MODE == GATED ? 2 : 1), K, 64, BK, true) ||
-        !q3_make_map_bf16(&map_x, X, n_pairs, K, BOX, BK, true))
+    CUtensorMap map_w, map_x32, map_x64;
+    if (!make_weight_map(&map_w, W, n_real * (MODE == GATED ? 2 : 1), rows, K, MODE == GATED ? 64 : 128, MODE == GATED ? 2 : 1) ||
+        !q3_make_map_bf16(&map_x32, X, n_pairs, K, 32, BK, true) || !q3_make_map_bf16(&map_x64, X, n_pairs, K, 64, BK, true))
         return Q3_ERR_BAD_SIZE;
     // an upper bound on the tiles of all experts together
     const int64_t tiles = ((int64_t)n_pairs / MAX_TOKENS + (n_real < n_pairs ? n_real : n_pairs)) * ((rows + FEATURES - 1) / FEATURES);
     const int pairs = tiles < q3_device_sm_count() / 2 ? (int)tiles : q3_device_sm_count() / 2;
-    return (int)q3_launch_cluster(expert_kernel<MODE>, dim3(2 * pairs), dim3(THREADS), (size_t)SMEM, stream, dim3(2, 1, 1), map_w, map_x,
+    return (int)q3_launch_cluster(expert_kernel<MODE>, dim3(2 * pairs), dim3(THREADS), (size_t)SMEM, stream, dim3(2, 1, 1), map_w, map_x32, map_x64,
                                   offsets, out, n_real, rows, K, limit, alpha, up_offset, status);
 }
 
