@@ -85,14 +85,14 @@ def tcgen05_form(M: int, N: int, K: int, gated: bool = False, out_bf16: bool = T
     return min(cost, key=cost.get)
 
 
-def few_rows_weights_first(N: int, K: int) -> bool:
-    """Whether the weights-first kernel reads W [N, K] sooner than the weight-streaming one even for up to `skinny_rows` rows: the
-    largest matrices (gate and up of the 8B shape, 201 MB, 32.7 us against 35.7 at 8 rows and 32.1 against 34.5 at 2; of the 14B shape
-    53.7 against 57.1; its 178 MB down 30.0 against 32.9; the vocabulary's 182 against 184, in 32 bits, stays), and rows of W that make
-    little more than one wave of the other kernel's blocks (7,168 x 5,120 14.1 against 17.6).  Smaller ones are slower (4,096 x 4,096
-    8.7 against 7.5, 4,096 x 12,288 18.3 against 17.9)."""
+def few_rows_weights_first(M: int, N: int, K: int) -> bool:
+    """Whether the weights-first kernel reads W [N, K] sooner than the weight-streaming one even for M <= `skinny_rows` rows: the
+    largest matrices from four rows on (gate and up of the 8B shape, 201 MB, 32.7 us against 35.7 at 8 rows, 32.5 against 34.7 at 4; of
+    the 14B shape 53.7 against 57.1; its 178 MB down 30.0 against 32.9; the vocabulary's 182 against 184, in 32 bits, stays), and rows of W
+    that make little more than one wave of the other kernel's blocks (7,168 x 5,120 14.1 against 17.6).  Smaller ones are slower (4,096 x
+    4,096 8.7 against 7.5, 4,096 x 12,288 18.3 against 17.9); of one row the largest gained 2 us in one place and lost 2 in another."""
     wave = 444                                    # three blocks of 16 rows an SM
-    return 2 * N * K >= 150_000_000 and N <= 65536 or K >= 4096 and wave < -(-N // 16) <= wave * 4 // 3
+    return M >= 4 and 2 * N * K >= 150_000_000 and N <= 65536 or K >= 4096 and wave < -(-N // 16) <= wave * 4 // 3
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
@@ -111,7 +111,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     if K % 8 != 0:
         return ops.gemm_bf16_any_width(x, w, out)
     if M <= skinny_rows:
-        if out.dtype == torch.bfloat16 and few_rows_weights_first(w.shape[0], K):
+        if out.dtype == torch.bfloat16 and few_rows_weights_first(M, w.shape[0], K):
             return ops.gemm_tcgen05_mid(x, w, out)
         return ops.gemm_skinny(x, w, out)
     out_bf16 = out.dtype == torch.bfloat16

@@ -52,7 +52,7 @@ class SwiGLU(Part):
         N, I = ctx.n_tokens, self.intermediate_size
         act = ctx.scratch.get("ff.act", (N, I), ctx.dtype)
         fused = self.interleaved and ctx.dtype == torch.bfloat16 and self.hidden_size % 8 == 0 and self.activation != "clamped"
-        if fused and N <= linear_module.skinny_rows and not linear_module.few_rows_weights_first(2 * I, self.hidden_size):
+        if fused and N <= linear_module.skinny_rows and not linear_module.few_rows_weights_first(N, 2 * I, self.hidden_size):
             ops.gemm_skinny_gated(x, self.w_gate_up, act, self.activation)   # product, activation and gating in one kernel
         elif fused and (N <= linear_module.skinny_rows or
                         linear_module.tcgen05_form(N, 2 * I, self.hidden_size, gated=True) == "weights_first"):

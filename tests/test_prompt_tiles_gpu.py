@@ -79,13 +79,13 @@ def test_tiles_of_equal_tokens_gated(M, inter, K, activation):
         assert torch.equal(fused[:M], two)
 
 
-@pytest.mark.parametrize("M", [1, 2, 8])
+@pytest.mark.parametrize("M", [1, 3, 4, 8])
 @pytest.mark.parametrize("N,K", [(7168, 4096), (9472, 4104), (24576, 4096), (7104, 4096)])
 def test_large_matrices_of_few_rows(M, N, K):
-    """Up to eight rows: the weights-first kernel for the largest matrices and for little more than a wave of the other kernel's blocks,
+    """Up to eight rows: the weights-first kernel for the largest matrices from four rows on and for little more than a wave of the other kernel's blocks,
     the other kernel beside (7,104 rows of W are one wave)."""
     from qwen3_b200.parts import linear as L
-    assert L.few_rows_weights_first(N, K) == (N != 7104)
+    assert L.few_rows_weights_first(M, N, K) == (N != 7104 and (N != 24576 or M >= 4))
     x, w = operands(M, N, K)
     for dtype in (torch.bfloat16, torch.float32):
         out = torch.full((M + 1, N), float("nan"), dtype=dtype, device="cuda")
