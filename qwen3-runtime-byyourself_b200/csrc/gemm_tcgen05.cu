@@ -509,11 +509,10 @@ gemm_tcgen05_prompt_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
 // in the pages - are all the thread's own.  The accumulator is rounded to bfloat16 first, as the product's
 // output would have been.  Head sizes 64, 128 and 256 (whole heads in a tile, halves of whole 32-column chunks).
 // What it costs: a thread's token has its own row of the rotation tables and its own rows of q and of the pages, so
-// every load and store of a warp touches 32 lines, and the four warps of a block share one path to memory: a tile's
-// epilogue takes about 12 us where the plain one takes 3.  Under the next tile's K steps (21 us at K = 4,096) that is
-// hidden, for a pair's last tile it is not: at 8,192 tokens the fused product takes 321-338 us against 381-412 for
-// product + qkv_prepare, at 2,048 tokens 83.5 against 86, at 512 tokens (one tile a pair) 41 against 34 - so it
-// is used from 2,048 tokens on (parts/attention.py).
+// every load and store of a warp touches 32 lines, and the warps of a block share one path to memory: a tile's epilogue takes several
+// times as long as the plain one.  Under the next tile's K steps that is hidden, for a pair's last tile it is not: whole prompt steps of
+// 12 layers of the 8B shape, fused / product + qkv_prepare: 300 tokens 2.54 / 2.46 ms, 700 and 1,024 equal, 4,096 16.9 / 17.5, 24,000
+// 142.3 / 144.0 - so it is used from 2,048 tokens on (parts/attention.py).
 
 struct QkvEpilogue {
     bf16* q_out;                   // [tokens, nq * d]

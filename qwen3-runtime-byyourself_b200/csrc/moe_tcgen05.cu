@@ -9,8 +9,8 @@
 // tiles of at most 256 and a tile costs its tokens rounded up to 64, where a 256-row token side would cost whole
 // 256s.  The tile list is walked on the device from the sorted offsets; the host never learns how many tokens an
 // expert has.  Bound by the tensor cores with hundreds of tokens per expert, by reading the weights with tens:
-//   16 experts of 3,072 at width 4,096, 8,324 pairs: 629 us for the gather and both products at first, 703 launched back to back for
-//   longer (0.89 PFLOP/s; 2,924 us with mma.sync tiles of 64 x 64); 500 pairs: 222 us, 0.84 of the rate that reading the weights could have.
+//   16 experts of 3,072 at width 4,096, 8,324 pairs: 629 us for the gather and both products, 703 on a GPU at the
+//   power cap (1.0 and 0.89 PFLOP/s; 2,924 us with mma.sync tiles of 64 x 64); 500 pairs: 222 us, 0.84 of the rate that reading the weights could have.
 //
 // Roles in a block: warp 0 the TMA producer, warp 1 tensor memory and (in the pair's first block) the products, warps 2-5
 // drain.  The accumulator is double-buffered, so a tile drains under the products of the next.  A block's 128 rows of W are
