@@ -373,7 +373,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 if (CAPPED) {
                     // a row may see nothing of its tile's first page (its chunk starts later): a maximum below every
                     // score then lets the next page raise it; the sink is a key of score 0, or of the head's own, that is always seen
-                    m_run = capped.sink ? fmaxf(m_page, sink_score) : (m_page == -INFINITY ? -1.0e30f : m_page);
+                    // (also a sink of minus infinity, or of a number so low that log2(e) makes it that: it then weighs nothing)
+                    m_run = capped.sink ? fmaxf(m_page, sink_score) : m_page;
+                    if (m_run == -INFINITY) m_run = -3.0e38f;
                     l_run = capped.sink ? ex2_approx(sink_score - m_run) : 0.0f;
                 } else {
                     m_run = m_page == -INFINITY ? 0.0f : m_page;             // the first page overwrites O: nothing to rescale
