@@ -7,7 +7,7 @@
 //   grid (tile of 128 new tokens, query head, sequence); three roles per block
 //   warp 0     TMA: the Q tile once, then the K panels of the cache pages (64 keys of the head's kv
 //              group, two 64-column halves at head size 128) into a ring of three
-//   warp 6     TMA: the V panels into a ring of two.  K(j) is free again as soon as S(j) is done and
+//   warp 6     TMA: the V panels into a ring of two (wide heads: and a look through values that are no numbers).  K(j) is free again as soon as S(j) is done and
 //              V(j) only after O += P(j).V(j), so with rings of their own the K loads run two pages
 //              ahead of the products, which covers their latency at two blocks per SM
 //   warp 1     one thread issues the products: S(j) = Q.K_j^T into TMEM columns [0,64), then
@@ -30,8 +30,8 @@
 //   columns [64,96) and [96,128), two sets of tcgen05.mma per page), so the product sees them to 16 bits of mantissa.
 //   -DQ3_VALUE_DIM=<size> beside -DQ3_CAPPED=1: heads of 192 or 256 with values of their own size (multiples of 64), and a window
 //   instead of a cap or chunks (latent attention: one key head of 192 + 64, values of 192).  One block an SM then, as Q and the
-//   rings take 209 KB; three prompts of 2,048, 911 and 1,203 tokens with 16 heads 97 us (438 on
-//   mma.sync tiles), behind a window of 1,024 91 (379), one of 128 16 (16), of 512 22 (40), of 8,000 586 (3,691).  Bound by the softmax of one tile an SM.
+//   rings take 209 KB; three prompts of 2,048, 911 and 1,203 tokens with 16 heads 98 us (437 on
+//   mma.sync tiles), behind a window of 1,024 94 (378), one of 128 15 (16), of 512 22 (40), of 8,000 603 (3,690).  Bound by the softmax of one tile an SM.
 //   -DQ3_CAPPED=2: with a sink and biases by distance instead of a cap or chunks; the biases are added to the scaled scores: one number a page for pages far enough back, else one a score.
 #include <cuda.h>
 
@@ -152,6 +152,102 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// The halves of two packed bfloat16 that are infinities or NaNs, each marked by its highest bit.
+__device__ __forceinline__ uint32_t no_numbers(uint32_t w) { return ((w & 0x7f807f80u) + 0x00800080u) & 0x80008000u; }
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t at) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_shared_v4(uint32_t at, uint4 v) {
+    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ uint32_t ld_shared(uint32_t at) {
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_shared(uint32_t at, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(v) : "memory"); }
+
+// The wide form takes a page's values with weight 0 for the rows of its tile that do not see them, and 0 times an infinity or a NaN is a NaN:
+// such a value, another row's or one left in a slot that nobody has written, would reach up to 127 rows that do not see it.
+// So the warp that copies the values looks through those of every page that some row does not see in whole.  Where it finds some that are
+// no numbers, each thread of the softmax adds those that its row sees to its row of the output, and zeros take their place before the
+// product.  What the looking costs, 16 heads of 256 over values of 192, with / without: three prompts of 2,048, 911 and 1,203 tokens 98 / 94 us,
+// behind a window of 1,024 94 / 89; one of 8,000 645 / 619, behind a window of 128 114 / 106; one of 512 22 / 21.
+struct ValueCheck {
+    uint32_t bar_looked, found;       // the page is looked through; 1: some of its values are no numbers
+    uint32_t bar_added, started;      // the four softmax warps have added them; 1: the output began with such values
+};
+
+// Adds the values of keys from .. to of a page that are no numbers to a row of the output in tensor memory (`fresh`: it begins here).
+__device__ __forceinline__ void add_no_numbers(uint32_t v_page, uint32_t row_out, int from, int to, bool fresh) {
+#pragma unroll 1
+    for (int c = 0; c < VD; c += 32) {
+        uint32_t o[32];
+        if (fresh) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) o[e] = 0u;
+        } else {
+            tc_ld32(row_out + c, o);
+            tc_wait_ld();
+        }
+#pragma unroll 1
+        for (int key = 0; key < PAGE; ++key) {
+            const bool seen = key >= from && key <= to;
+            const uint32_t row = v_page + (c >> 6) * (PAGE * 128) + key * 128;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint4 w = ld_shared_v4(row + (((((c & 32) >> 3) + q) ^ (key & 7)) << 4));
+                const uint32_t v[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const uint32_t bad = seen ? no_numbers(v[h]) : 0u;
+                    uint32_t &lo = o[q * 8 + h * 2], &hi = o[q * 8 + h * 2 + 1];
+                    if (bad & 0x8000u) lo = __float_as_uint(__uint_as_float(lo) + __uint_as_float(v[h] << 16));
+                    if (bad & 0x80000000u) hi = __float_as_uint(__uint_as_float(hi) + __uint_as_float(v[h] & 0xFFFF0000u));
+                }
+            }
+        }
+        tc_st32(row_out + c, o);
+    }
+    tc_wait_st();
+}
+
+// The softmax's side of it, for a page that some row does not see in whole; thread r's row sees the keys from .. to.  `turns`: the two
+// barriers' parities (bit 0 bar_looked, bit 1 bar_added); returns the next ones, or GAVE_UP.  Not inlined: the loop over the pages was up to
+// 7 % slower with it inside.
+constexpr uint32_t GAVE_UP = 4;
+__device__ __noinline__ uint32_t settle_values(const ValueCheck values, uint32_t v_page, uint32_t row_out, int from, int to, bool fresh, int r,
+                                               uint32_t turns, int* status) {
+    const int lane = r & 31;
+    if (!mbar_wait_warp(values.bar_looked, turns & 1u)) {
+        if (lane == 0) atomicExch(status, 21);
+        return GAVE_UP;
+    }
+    turns ^= 1u;
+    if (ld_shared(values.found) != 0) {
+        __syncwarp();
+        add_no_numbers(v_page, row_out, from, to, fresh);
+        if (fresh && lane == 0) st_shared(values.started, 1);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(values.bar_added);
+        if (!mbar_wait_warp(values.bar_added, turns >> 1)) {                           // every warp has read them
+            if (lane == 0) atomicExch(status, 22);
+            return GAVE_UP;
+        }
+        turns ^= 2u;
+        for (int i = r; i < V_PANEL_BYTES / 16; i += BM) {
+            const uint4 w = ld_shared_v4(v_page + i * 16);
+            auto numbers = [](uint32_t v) { return v & ~((no_numbers(v) >> 15) * 0xFFFFu); };
+            st_shared_v4(v_page + i * 16, make_uint4(numbers(w.x), numbers(w.y), numbers(w.z), numbers(w.w)));
+        }
+        fence_proxy_async();
+        __syncwarp();
+    }
+    return turns;
+}
+
 __global__ void __launch_bounds__(THREADS)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                   const __grid_constant__ CUtensorMap map_v, bf16* __restrict__ out, const int* __restrict__ seq_start,
@@ -181,6 +277,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     // pages first_page .. the one of the last row (first_page: the one of the first key of the tile's first row)
     const int first_page = first_key(pos0 + tile * BM) / PAGE;
     const int n_pages = (pos0 + tile * BM + rows - 1) / PAGE + 1 - first_page;
+    // some key of the page lies after some row (or, with chunks or a window, before the first key of some row)
+    const int c_last = first_key(pos0 + tile * BM + BM - 1);
+    auto partly_seen = [&](int key0) { return key0 + PAGE - 1 > pos0 + tile * BM || (CAPPED && key0 < c_last); };
 
     const uint32_t base = smem_u32(smem_raw);
     if (base & 1023u) {                                  // the swizzled tiles need 1024-byte alignment
@@ -193,6 +292,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const uint32_t bar_v_full = bar_k_empty + 8 * K_STAGES, bar_v_empty = bar_v_full + 8 * V_STAGES;
     const uint32_t bar_s_full = bar_v_empty + 8 * V_STAGES, bar_s_read = bar_s_full + 8, bar_p_full = bar_s_read + 8;
     const uint32_t bar_pv_done = bar_p_full + 8, tmem_slot = bar_pv_done + 8;
+    const ValueCheck values = {tmem_slot + 8, tmem_slot + 16, tmem_slot + 24, tmem_slot + 32};
 
     if (threadIdx.x == 0) {
         mbar_init(bar_q, 1);
@@ -208,6 +308,11 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         mbar_init(bar_s_read, 4);
         mbar_init(bar_p_full, 4);
         mbar_init(bar_pv_done, 1);
+        if constexpr (WIDE) {
+            mbar_init(values.bar_looked, 1);
+            mbar_init(values.bar_added, 4);
+            st_shared(values.started, 0);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -238,15 +343,48 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         }
     } else if (warp == 6) {
         // ------------------------------------------------ TMA producer: the V panels
-        if (lane == 0) {
-            for (int j = 0; j < n_pages; ++j) {
-                const int s = j % V_STAGES;
-                if (!mbar_wait(bar_v_empty + 8 * s, ((uint32_t)(j / V_STAGES) & 1u) ^ 1u)) { atomicExch(status, 19); break; }
-                const uint32_t dst = v_smem + s * V_PANEL_BYTES;
-                const int row = (pages[first_page + j] * nkv + kvh) * PAGE;
-                mbar_expect_tx(bar_v_full + 8 * s, V_PANEL_BYTES);
+        auto load_values = [&](int j) {
+            const int s = j % V_STAGES;
+            const uint32_t dst = v_smem + s * V_PANEL_BYTES;
+            const int row = (pages[first_page + j] * nkv + kvh) * PAGE;
+            mbar_expect_tx(bar_v_full + 8 * s, V_PANEL_BYTES);
 #pragma unroll
-                for (int h = 0; h < V_HALVES; ++h) tma_load_2d(dst + h * PAGE * 128, &map_v, bar_v_full + 8 * s, h * 64, row);
+            for (int h = 0; h < V_HALVES; ++h) tma_load_2d(dst + h * PAGE * 128, &map_v, bar_v_full + 8 * s, h * 64, row);
+        };
+        auto stage_free = [&](int j) { return mbar_wait(bar_v_empty + 8 * (j % V_STAGES), ((uint32_t)(j / V_STAGES) & 1u) ^ 1u); };
+        if constexpr (WIDE) {
+            // Page j - 1 is looked through when page j is asked for, that is, after the product of page j - 2 (which is also waited for behind
+            // the last page): nobody is still at the page looked through before, and the product of page j - 1 waits for this.
+            for (int j = 0; j <= n_pages; ++j) {
+                if (!__all_sync(0xffffffffu, stage_free(j))) {
+                    if (lane == 0) atomicExch(status, 19);
+                    break;
+                }
+                if (lane == 0 && j < n_pages) load_values(j);
+                __syncwarp();
+                if (j == 0 || !partly_seen((first_page + j - 1) * PAGE)) continue;
+                const uint32_t s = (uint32_t)(j - 1) % V_STAGES, v_page = v_smem + s * V_PANEL_BYTES;
+                if (!mbar_wait_warp(bar_v_full + 8 * s, ((uint32_t)(j - 1) / V_STAGES) & 1u)) {
+                    if (lane == 0) atomicExch(status, 20);
+                    break;
+                }
+                uint32_t any = 0;
+#pragma unroll 4
+                for (int i = lane; i < V_PANEL_BYTES / 16; i += 32) {
+                    const uint4 w = ld_shared_v4(v_page + i * 16);
+                    any |= no_numbers(w.x) | no_numbers(w.y) | no_numbers(w.z) | no_numbers(w.w);
+                }
+                const bool some = __any_sync(0xffffffffu, any != 0);
+                if (lane == 0) {
+                    st_shared(values.found, some ? 1u : 0u);
+                    mbar_arrive(values.bar_looked);
+                }
+                __syncwarp();
+            }
+        } else if (lane == 0) {
+            for (int j = 0; j < n_pages; ++j) {
+                if (!stage_free(j)) { atomicExch(status, 19); break; }
+                load_values(j);
             }
         }
     } else if (warp == 1) {
@@ -291,10 +429,11 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             tc_fence_after();
             const uint32_t s = (uint32_t)j % V_STAGES;
             const uint64_t v_src = v_desc + (uint64_t)(s * (V_PANEL_BYTES >> 4));
+            const bool begun = j > 0 || (WIDE && ld_shared(values.started) != 0);     // the output holds something
             if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < PAGE / 16; ++kk)
-                    tc_mma_ts(acc + COL_O, acc + COL_P + kk * 8, v_src + (uint64_t)(kk * 16 * 128 >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+                    tc_mma_ts(acc + COL_O, acc + COL_P + kk * 8, v_src + (uint64_t)(kk * 16 * 128 >> 4), idesc_pv, (begun || kk > 0) ? 1u : 0u);
                 if constexpr (CAPPED) {                                      // the low term of the weights on the same V
 #pragma unroll
                     for (int kk = 0; kk < PAGE / 16; ++kk)
@@ -313,8 +452,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         const uint32_t t_row = tmem + ((uint32_t)lane_base << 16);
         float m_run = -INFINITY, l_run = 0.0f;
         bool ok = true;
+        uint32_t turns = 0;                                                 // see settle_values
         // the capped form: the first key this row sees, and the constants of s -> cap * tanh(s * scale / cap) in log2 units
-        const int c_row = first_key(p_row), c_last = first_key(pos0 + tile * BM + BM - 1);
+        const int c_row = first_key(p_row);
         const float cap_l2 = capped.cap * 1.4426950408889634f;                       // the cap in log2 units
         const float tanh_k = capped.cap > 0.0f ? 2.0f * capped.scale * 1.4426950408889634f / capped.cap : 0.0f;
         const float sink_score = CAPPED && capped.sink_values != nullptr ? capped.sink_values[head] * 1.4426950408889634f : 0.0f;
@@ -333,8 +473,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_s_read);
             const int key0 = (first_page + j) * PAGE;
-            // some key of the page lies after some row (or, with chunks or a window, before the first key of some row)
-            const bool edge = key0 + PAGE - 1 > pos0 + tile * BM || (CAPPED && key0 < c_last);
+            const bool edge = partly_seen(key0);
             if (edge) {
 #pragma unroll
                 for (int c = 0; c < 64; ++c)
@@ -461,6 +600,14 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             }
             tc_st32(t_row + COL_P, p);
             if constexpr (CAPPED) tc_st32(t_row + COL_P_LO, p_lo);
+            if constexpr (WIDE) {
+                if (edge) {
+                    turns = settle_values(values, v_smem + ((uint32_t)j % V_STAGES) * V_PANEL_BYTES, t_row + COL_O, c_row - key0, p_row - key0,
+                                          j == 0, r, turns, status);
+                    ok = turns != GAVE_UP;
+                    if (!ok) break;
+                }
+            }
             tc_wait_st();
             tc_fence_before();
             __syncwarp();

@@ -115,6 +115,37 @@ def test_sinks_that_weigh_nothing(d, vd, window, chunk):
         assert not bool(excess.isnan().any()) and excess.max().item() <= 0, (i, excess.max().item())
 
 
+# Values that are no numbers, in pages of which some rows of a tile see other keys: behind the last token (slots nobody wrote), later than
+# some rows, before the window of others, in a tile's first page and in later ones, twice the same column.  They belong to the rows that see
+# them; all others are what they are without them.
+@pytest.mark.parametrize("d,vd,window", [(256, 192, None), (256, 192, 100), (192, 128, 64), (256, 256, 1)])
+@pytest.mark.parametrize("bad", [[(0, 5, 0, math.inf)], [(0, 130, 63, -math.inf), (0, 299, 40, math.nan)], [(1, 198, 17, math.inf), (1, 70, 33, math.nan)],
+                                 [(0, 64, 8, math.inf), (0, 65, 8, -math.inf), (1, 0, 1, math.nan)], [(0, 300, 2, math.nan), (1, 199, 60, math.inf)]])
+def test_values_that_are_no_numbers(d, vd, window, bad):
+    from qwen3_b200.csrc import ops
+    H, G, spans = 4, 2, [(0, 300), (70, 129)]
+    g = torch.Generator(device="cuda").manual_seed(d + vd + 1)
+    kp, vp, table, own = paged(spans, G, d, vd, g)
+    N = sum(b for _, b in spans)
+    q = torch.randn(N, H * d, generator=g, device="cuda").to(torch.bfloat16)
+    start, pos0 = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([0, 300, N], [0, 70]))
+    want = [exact(q[s:s + b].view(b, H, d), own(kp, i), own(vp, i), d ** -0.5, a, window, None) for i, (s, (a, b)) in enumerate(zip((0, 300), spans))]
+    touched = [torch.zeros_like(w, dtype=torch.bool) for w in want]
+    for seq, key, col, value in bad:                       # in the second kv head, whose queries are the heads 2 and 3
+        vp[table[seq, key // 64].item(), 1, key % 64, col] = value
+        a, b = spans[seq]
+        sees = torch.arange(a, a + b, device="cuda") - key
+        touched[seq][:, 2:, col] |= ((sees >= 0) & (sees < (window or 1 << 30)))[:, None]
+    out = torch.full((N, H * vd), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.attention_wide_prefill_tc(q, kp, vp, out, start, pos0, table, 2, 300, N, H, G, d, vd, d ** -0.5, window=window)
+    assert ops.tcgen05_status("cuda") == 0
+    for i, (s, (a, b)) in enumerate(zip((0, 300), spans)):
+        got = out[s:s + b].double().view(b, H, vd)
+        assert bool((~got[touched[i]].isfinite()).all()), "a value that a row sees is lost"
+        excess = (got - want[i]).abs() - (2.0 ** -8 * want[i].abs() + 4e-4)              # as above
+        assert bool((excess <= 0)[~touched[i]].all()), "a value reaches rows that do not see it"
+
+
 def test_sizes_that_stay_where_they_were():
     from qwen3_b200.csrc import ops
     assert [ops.attention_wide_prefill_tc_fits(d, v) for d, v in ((128, 128), (64, 128), (200, 128), (256, 100), (256, 320))] == [False] * 5
