@@ -743,7 +743,7 @@ __device__ __forceinline__ void store_rows(const uint32_t (&v)[64], bf16* Y, int
 template <int GATED, typename OutT, bool QKV = false, bool ROWS = false>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
-                         OutT* __restrict__ Y, int M, int N, int K, int tile, int* __restrict__ status, const QkvEpilogue qkv) {
+                         OutT* __restrict__ Y, int M, int N, int K, int tile, int ahead, int* __restrict__ status, const QkvEpilogue qkv) {
     extern __shared__ unsigned char smem_raw[];
     constexpr int BN = 256, STAGES = 6;
     constexpr int A_BYTES = BM * BK * 2, B_BYTES = (BN / 2) * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
@@ -790,9 +790,6 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
         // the whole warp walks and one elected thread copies, as with the products: 300 tokens gate/up 73 us against 69 and down 51 / 50,
         // 1,300 tokens down 134 / 114 and output 46 / 40
         pdl_wait();                                           // X is the output of the kernel before
-        // Few tiles of tokens: W comes from memory, and each K step's rows would wait for it; the lines of the step after next but six are
-        // asked into the L2 (527 tokens down 61 us against 58, output 22.7 / 22.1; from 1,000 tokens on no difference).
-        const int ahead = ROWS && tiles_m <= 4 ? 8 : nkb;
         uint32_t it = 0;
         bool ok = true;
         for (int i = first; i < tiles && ok; i += stride) {
@@ -812,7 +809,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                     if (rank == 0) mbar_expect_tx(bars + s * 8, 2 * (tile / 2 * BK * 2 + B_BYTES));   // both blocks' bytes
                     tma_load_2d_pair(a, &map_x, full_in_leader, kb * BK, m0);
                     tma_load_2d_pair(b, &map_w, full_in_leader, kb * BK, n0);
-                    if (kb % 2 == 0 && kb + ahead < nkb) tma_prefetch_2d(&map_w, (kb + ahead) * BK, n0);      // a line holds two K steps
+                    if (ahead != 0 && kb % 2 == 0 && kb + ahead < nkb) tma_prefetch_2d(&map_w, (kb + ahead) * BK, n0);
                 }
                 __syncwarp();
             }
@@ -1237,10 +1234,15 @@ int launch_pair_form(const bf16* X, const bf16* W, OutT* Y, int M, int N, int K,
     }
     CUtensorMap map_x, map_w;
     if (!make_map(&map_x, X, M, K, tile / 2) || !make_map(&map_w, W, N, K, 128)) return Q3_ERR_BAD_SIZE;
-    const int tiles = ((M + tile - 1) / tile) * ((N + 255) / 256);
+    const int tiles_m = (M + tile - 1) / tile, tiles = tiles_m * ((N + 255) / 256);
     const int pairs = tiles < sm_count() / 2 ? tiles : sm_count() / 2;
+    // Few tiles of tokens: W comes from memory, and each K step's rows would wait for it, so they are asked into the L2 eight K steps ahead, two
+    // at a time, as a line of 256 bytes holds two.  Where rows of W do not begin at such lines every step would bring in two lines a row
+    // of which it needs one.  (With / without: 300 tokens, N 4,096, K 4,096 18.9 / 19.9 us, K 12,288 44.3 / 47.5, K 4,104 29.5 / 26.2, K 12,296
+    // 82 / 69; K 4,160 equal; 527 tokens K 4,096 19.3 / 20.0, N 24,576 K 4,104 153 / 129; from 700 tokens on no difference.)
+    const int ahead = ROWS && tiles_m <= 4 && K % 128 == 0 && (reinterpret_cast<uintptr_t>(W) & 255u) == 0 ? 8 : 0;
     return (int)q3_launch_cluster(kernel, dim3(2 * pairs), dim3(PAIR_THREADS), (size_t)SMEM, stream, dim3(2, 1, 1), map_x, map_w, Y, M, N, K,
-                                  tile, status, qkv);
+                                  tile, ahead, status, qkv);
 }
 
 template <int GATED, typename OutT, bool QKV = false>
