@@ -1346,9 +1346,33 @@ Q3_EXPORT int q3_gemm_tcgen05_pair_bf16(const void* X, const void* W, void* Y, i
                       : launch_pair<0, bf16>(x, w, (bf16*)Y, M, N, K, status, stream);
 }
 
-// Microseconds that q3_gemm_tcgen05_pair_bf16 without a split of K should take (`may_row`: bfloat16 output, aligned).
+// The same in tiles of `tile` tokens (32 to 256 in steps of 32) with W as the 256-row operand, whatever the estimate says: what that form can
+// take alone, bfloat16 in rows of whole 16-byte packets, `gated` 0 to 2.
+Q3_EXPORT int q3_gemm_tcgen05_pair_rows_bf16(const void* X, const void* W, void* Y, int M, int N, int K, int gated, int tile, int* status,
+                                             void* stream_) {
+    if (M <= 0 || N <= 0) return 0;
+    if (K <= 0 || K % 8 != 0 || gated < 0 || gated > 2 || (gated && N % 16 != 0) || N % 8 != 0 || tile < 32 || tile > 256 || tile % 32 != 0)
+        return Q3_ERR_BAD_SIZE;
+    if (!aligned16(X) || !aligned16(W) || !aligned16(Y)) return Q3_ERR_MISALIGNED;
+    cudaStream_t stream = (cudaStream_t)stream_;
+    const bf16* x = (const bf16*)X;
+    const bf16* w = (const bf16*)W;
+    const QkvEpilogue none = {};
+    if (gated == 2) return launch_pair_form<2, bf16, false, true>(x, w, (bf16*)Y, M, N, K, tile, status, stream, none);
+    if (gated) return launch_pair_form<1, bf16, false, true>(x, w, (bf16*)Y, M, N, K, tile, status, stream, none);
+    return launch_pair_form<0, bf16, false, true>(x, w, (bf16*)Y, M, N, K, tile, status, stream, none);
+}
+
+// Microseconds that q3_gemm_tcgen05_pair_bf16 without a split of K should take (`may_row`: an output that the rows form can take).
 Q3_EXPORT float q3_gemm_tcgen05_pair_us(int M, int N, int K, int may_row) {
     return M > 0 && N > 0 && K > 0 ? pair_form(M, N, K, may_row && N % 8 == 0).us : 0.0f;
+}
+
+// The tokens of a tile with W as the 256-row operand that it would take; 0: tokens first in tiles of 256.
+Q3_EXPORT int q3_gemm_tcgen05_pair_tile(int M, int N, int K, int may_row) {
+    if (M <= 0 || N <= 0 || K <= 0) return 0;
+    const PairForm f = pair_form(M, N, K, may_row && N % 8 == 0);
+    return f.rows ? f.tile : 0;
 }
 
 // Pairs of SMs that run at once when K is split over `splits` pairs of a cluster (0: the device cannot place it).

@@ -1513,9 +1513,10 @@ def gemm_tcgen05_prompt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, til
 
 
 def gemm_tcgen05_pair(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool = False,
-                      splits: int = 1, activation: str = "silu") -> torch.Tensor:
+                      splits: int = 1, activation: str = "silu", tile: int = 0) -> torch.Tensor:
     """The prompt product on pairs of SMs (tcgen05 cta_group::2): tiles of 256 tokens by 256 rows of w, each
-    block of a pair loading its own tokens and half of the w tile.  `gated`: w holds gate and up rows
+    block of a pair loading its own tokens and half of the w tile, or of 256 rows of w by equal numbers of tokens (`tile`, 32 to 256 in
+    steps of 32; 0: as the kernel's estimate says, `gemm_tcgen05_pair_tile`).  `gated`: w holds gate and up rows
     interleaved in blocks of eight and out is [M, N/2] = round(act(g)) * u, act being SiLU or (`activation`) the tanh
     form of GELU.  `splits` (1..4): K split over
     that many pairs of one cluster, whose partial tiles are summed over distributed shared memory in a fixed
@@ -1528,6 +1529,14 @@ def gemm_tcgen05_pair(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated
         raise KernelError("gemm_tcgen05_pair: output must be bfloat16 (or float32 when not gated)")
     if not 1 <= splits <= PAIR_MAX_SPLITS:
         raise KernelError(f"gemm_tcgen05_pair: 1 to {PAIR_MAX_SPLITS} K ranges, not {splits}")
+    if tile:
+        if splits != 1 or out.dtype != torch.bfloat16:
+            raise KernelError("gemm_tcgen05_pair: tiles of equal tokens are for bfloat16 outputs and no split of K")
+        fn = _fn("gemm_tcgen05.cu", "q3_gemm_tcgen05_pair_rows_bf16",
+                 [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+        _check(fn(_dev(x, "x", torch.bfloat16), _dev(w, "w", torch.bfloat16), _dev(out, "out"), M, N, K,
+                  ACTIVATIONS[activation] + 1 if gated else 0, int(tile), _status_word(x.device).data_ptr(), _stream()), "gemm_tcgen05_pair")
+        return out
     fn = _fn("gemm_tcgen05.cu", "q3_gemm_tcgen05_pair_bf16",
              [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
     _check(fn(_dev(x, "x", torch.bfloat16), _dev(w, "w", torch.bfloat16), _dev(out, "out"), M, N, K,
@@ -1546,11 +1555,17 @@ def gemm_tcgen05_pair_capacity(splits: int) -> int:
     return int(fn(int(splits)))
 
 
-def gemm_tcgen05_pair_us(M: int, N: int, K: int, out_bf16: bool = True) -> float:
-    """Microseconds that `gemm_tcgen05_pair` without a split of K should take, in the tiles it would choose."""
+def gemm_tcgen05_pair_us(M: int, N: int, K: int, may_row: bool = True) -> float:
+    """Microseconds that `gemm_tcgen05_pair` without a split of K should take, in the tiles it would choose; `may_row`: of equal tokens,
+    too (bfloat16 outputs, plain or gated)."""
     fn = _fn_untimed("gemm_tcgen05.cu", "q3_gemm_tcgen05_pair_us", [c_int, c_int, c_int, c_int])
     fn.restype = c_float
-    return float(fn(int(M), int(N), int(K), int(bool(out_bf16))))
+    return float(fn(int(M), int(N), int(K), int(bool(may_row))))
+
+
+def gemm_tcgen05_pair_tile(M: int, N: int, K: int, may_row: bool = True) -> int:
+    """The tokens of a tile where `gemm_tcgen05_pair` takes W as the 256-row operand, 0 where it takes tiles of 256 tokens."""
+    return int(_fn_untimed("gemm_tcgen05.cu", "q3_gemm_tcgen05_pair_tile", [c_int, c_int, c_int, c_int])(int(M), int(N), int(K), int(bool(may_row))))
 
 
 PAIR_QKV_HEAD_DIMS = (64, 128, 256)

@@ -258,8 +258,13 @@ int q3_gemm_tcgen05_pair_qkv_bf16(const void* X, const void* W, int M, int K, vo
 int q3_gemm_tcgen05_pair_bf16(const void* X, const void* W, void* Y, int M, int N, int K, int out_is_f32, int gated, int splits,
                               int* status, void* stream);
 int q3_gemm_tcgen05_pair_capacity(int splits);
-/* microseconds that q3_gemm_tcgen05_pair_bf16 with splits 1 should take; may_row: bfloat16 output, aligned to 16 bytes */
+/* the same in tiles of `tile` tokens (32 to 256 in steps of 32) with W as the 256-row operand: bfloat16, gated 0 to 2 */
+int q3_gemm_tcgen05_pair_rows_bf16(const void* X, const void* W, void* Y, int M, int N, int K, int gated, int tile, int* status,
+                                   void* stream);
+/* microseconds that q3_gemm_tcgen05_pair_bf16 with splits 1 should take, and the tokens of its tiles where W is the 256-row operand (0: it is
+   not); may_row: it may be (a bfloat16 output aligned to 16 bytes, gated 0 to 2) */
 float q3_gemm_tcgen05_pair_us(int M, int N, int K, int may_row);
+int q3_gemm_tcgen05_pair_tile(int M, int N, int K, int may_row);
 
 /* ---- hyper.cu: a hidden state of several streams per token, float32 [token, streams, hidden] ------------------ */
 /* out[t] = `copies` times table[ids[t]] * scale side by side */
