@@ -1137,6 +1137,21 @@ int mid_splits(int N, int K, int token_tiles) {
     return s;
 }
 
+// Up to eight rows, where this kernel stands against the weight-streaming one: as many ranges as above, but three quarters of them where not all
+// clusters would run at once.  The SMs come in groups, and a group whose places are no multiple of a cluster leaves some empty: at two blocks
+// an SM 71 clusters of four run together and not 72, 33 of eight and not 34.  (In fours / threes / the other kernel: 9,088 rows of W, K 4,096
+// 14.7 / 14.5 / 16.5 us, 9,216 19.2 / 14.7 / 16.8, 9,472 19.5 / 15.0 / 17.0 and with K 8,192 33.3 / 27.0 / 31.4; in eights / sixes: 4,224 rows,
+// K 17,984 26.7 / 26.7 / 28.2, 4,352 rows, K 17,472 34.5 / 27.0 / 28.7.)
+int few_row_splits(int N, int K) {
+    const int s = mid_splits(N, K, 0), blocks = (N + BM - 1) / BM * s, places = 2 * sm_count();
+    if (blocks > places) return s;                            // the variant with three blocks an SM: places enough
+    return (s == 4 && blocks > places * 31 / 32) || (s == 8 && blocks > places * 9 / 10) ? s * 3 / 4 : s;
+}
+
+int mid_splits_for(int M, int N, int K) {
+    return M <= 8 ? few_row_splits(N, K) : mid_splits(N, K, M <= 128 ? 0 : (M + 255) / 256);
+}
+
 template <int MT, int STAGES, int MINB, int GATED, typename OutT>
 int launch_mid(const bf16* X, const bf16* W, OutT* Y, int M, int N, int K, int splits, int* status, cudaStream_t stream) {
     constexpr int RING = STAGES * (BM * BK * 2 + MT * BK * 2), PART = (MT * PART_LD * 4 + 1023) / 1024 * 1024;
@@ -1426,7 +1441,7 @@ Q3_EXPORT int q3_gemm_tcgen05_mid_bf16(const void* X, const void* W, void* Y, in
     cudaStream_t stream = (cudaStream_t)stream_;
     const bf16* x = (const bf16*)X;
     const bf16* w = (const bf16*)W;
-    if (splits == 0) splits = mid_splits(N, K, M <= 128 ? 0 : (M + 255) / 256);
+    if (splits == 0) splits = mid_splits_for(M, N, K);
     if (splits > (K + BK - 1) / BK) splits = (K + BK - 1) / BK;
     if (gated == 3) return dispatch_mid<3, bf16>(x, w, (bf16*)Y, M, N, K, splits, status, stream);
     if (gated == 2)
@@ -1439,4 +1454,4 @@ Q3_EXPORT int q3_gemm_tcgen05_mid_bf16(const void* X, const void* W, void* Y, in
                       : dispatch_mid<0, bf16>(x, w, (bf16*)Y, M, N, K, splits, status, stream);
 }
 
-Q3_EXPORT int q3_gemm_tcgen05_mid_splits(int N, int K, int M) { return mid_splits(N, K, M <= 128 ? 0 : (M + 255) / 256); }
+Q3_EXPORT int q3_gemm_tcgen05_mid_splits(int N, int K, int M) { return mid_splits_for(M, N, K); }
