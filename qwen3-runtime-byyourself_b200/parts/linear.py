@@ -85,14 +85,21 @@ def tcgen05_form(M: int, N: int, K: int, gated: bool = False, out_bf16: bool = T
     return min(cost, key=cost.get)
 
 
+@functools.lru_cache(maxsize=4096)
 def few_rows_weights_first(M: int, N: int, K: int) -> bool:
-    """Whether the weights-first kernel reads W [N, K] sooner than the weight-streaming one even for M <= `skinny_rows` rows: the
-    largest matrices from four rows on (gate and up of the 8B shape, 201 MB, 32.7 us against 35.7 at 8 rows, 32.5 against 34.7 at 4; of
-    the 14B shape 53.7 against 57.1; its 178 MB down 30.0 against 32.9; the vocabulary's 182 against 184, in 32 bits, stays), and rows of W
-    that make little more than one wave of the other kernel's blocks (7,168 x 5,120 14.1 against 17.6).  Smaller ones are slower (4,096 x
-    4,096 8.7 against 7.5, 4,096 x 12,288 18.3 against 17.9); of one row the largest gained 2 us in one place and lost 2 in another."""
-    wave = 444                                    # three blocks of 16 rows an SM
-    return M >= 4 and 2 * N * K >= 150_000_000 and N <= 65536 or K >= 4096 and wave < -(-N // 16) <= wave * 4 // 3
+    """Whether the weights-first kernel reads W [N, K] sooner than the weight-streaming one even for M <= `skinny_rows` rows, plain or gated.
+
+    The largest matrices from four rows on, up to what three blocks of 128 rows of W an SM hold at once (that / the streaming kernel, us, at 8
+    rows: gate and up of the 8B shape, 201 MB, 33.7 / 36.2, of the 14B shape 55.2 / 58.1, its 178 MB down 30.2 / 34.2, 40,960 x 8,192 103 / 111,
+    56,832 x 4,096 72.4 / 73.1; one block more, 56,960 x 4,096, 81.8 / 75.0, and 57,344 x 8,192 160 / 154; at 4 rows between 28,672 and 49,152 x
+    4,096 the two are within 2 %).  Of one row the largest gained 2 us in one place and lost 2 in another.
+
+    And rows of W that make little more than one wave of the streaming kernel's blocks, three of 16 rows an SM, which it begins anew for a few
+    (K 4,096 and 8,192 at 1 row: 7,104 rows of W, one wave, 12.0 / 11.3; 7,168 12.1 / 14.4 and 20.6 / 27.1; 8,192 13.5 / 15.6 and 23.3 / 29.7;
+    9,472 14.8 / 16.9 and 26.5 / 31.4; gated 1 us more on both sides).  With K of 2,048 the two are level.  Smaller matrices are slower
+    (4,096 x 4,096 8.7 against 7.5, 4,096 x 12,288 18.3 against 17.9)."""
+    wave = 3 * torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    return M >= 4 and 2 * N * K >= 150_000_000 and -(-N // 128) <= wave or K >= 4096 and wave < -(-N // 16) <= wave * 4 // 3
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
