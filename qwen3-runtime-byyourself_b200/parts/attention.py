@@ -492,8 +492,8 @@ def _projection_pair_kernel(part, x, cache, q, ctx, table, q_norm_w, k_norm_w, e
         return False
     if cos is not None and 2 * cos.shape[-1] != d:
         return False
-    if linear_module.set_bf16_kernel_active() or linear_module.tcgen05_form(N, (nq + 2 * nkv) * d, K) != "pair" \
-            or linear_module.pair_plan(N, (nq + 2 * nkv) * d, K)[1] != 1:
+    if linear_module.set_bf16_kernel_active() or linear_module.tcgen05_form(N, (nq + 2 * nkv) * d, K, may_row=False) != "pair" \
+            or linear_module.pair_plan(N, (nq + 2 * nkv) * d, K, may_row=False)[1] != 1:
         return False
     ops.gemm_tcgen05_pair_qkv(x, part.w_qkv, q, cache.keys, cache.values, q_norm_w, k_norm_w, cos, sin, eps, ctx.token_seq,
                               ctx.token_pos, table, N, nq, nkv, d, write_kv=not cache.shared)

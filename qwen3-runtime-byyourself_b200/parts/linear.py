@@ -45,11 +45,12 @@ _WEIGHTS_FIRST_SPLIT_US = 7.0
 
 
 @functools.lru_cache(maxsize=4096)
-def pair_plan(M: int, N: int, K: int, out_bf16: bool = True) -> tuple:
+def pair_plan(M: int, N: int, K: int, may_row: bool = True) -> tuple:
     """(estimated microseconds, K ranges) of the pairs-of-SMs form: the number of K ranges per tile (1 = persistent
-    pairs, no split, in the tiles that the kernel chooses) whose waves of tiles x K steps cost least."""
+    pairs, no split, in the tiles that the kernel chooses) whose waves of tiles x K steps cost least.  `may_row`: the product may
+    have tiles of equal tokens (bfloat16 output, plain or gated; not the squared relu, nor the q/k/v product with its epilogue)."""
     nkb, tiles = -(-K // 64), -(-M // 256) * -(-N // 256)
-    best = (ops.gemm_tcgen05_pair_us(M, N, K, out_bf16), 1)
+    best = (ops.gemm_tcgen05_pair_us(M, N, K, may_row), 1)
     for splits in range(2, ops.PAIR_MAX_SPLITS + 1):
         capacity = ops.gemm_tcgen05_pair_capacity(splits)
         if capacity <= 0 or splits > nkb or tiles > 65535:
@@ -62,11 +63,11 @@ def pair_plan(M: int, N: int, K: int, out_bf16: bool = True) -> tuple:
 
 
 @functools.lru_cache(maxsize=4096)
-def tcgen05_form(M: int, N: int, K: int, gated: bool = False, out_bf16: bool = True) -> str:
+def tcgen05_form(M: int, N: int, K: int, gated: bool = False, may_row: bool = True) -> str:
     """Which form of the tcgen05 product takes M rows (M > skinny_rows, K a multiple of 8): weights first
     (K split over a cluster; the only form that fills the GPU when M and N give few tiles), or tokens first
-    and persistent, on single SMs with 128 x 128 tiles or on pairs of SMs with 256 x 256 tiles.  A small
-    cost model: waves of blocks times K steps."""
+    and persistent, on single SMs with 128 x 128 tiles or on pairs of SMs with 256 x 256 tiles or (`may_row`, as above) tiles of
+    equal tokens by 256 rows of W.  A small cost model: waves of blocks times K steps."""
     if M <= 128:
         return "weights_first"
     sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
@@ -75,7 +76,7 @@ def tcgen05_form(M: int, N: int, K: int, gated: bool = False, out_bf16: bool = T
     def waves(blocks, slots):
         return -(-blocks // slots)
 
-    cost = {"pair": pair_plan(M, N, K, out_bf16)[0]}
+    cost = {"pair": pair_plan(M, N, K, may_row)[0]}
     if not gated:                                        # the gated epilogue exists for the 256-row tiles
         cost["prompt128"] = waves(-(-M // 128) * -(-N // 128), sms) * nkb * _STEP_US["prompt128"] + _BLOCK_US["prompt128"]
     if M <= 1024:
@@ -121,10 +122,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         if out.dtype == torch.bfloat16 and few_rows_weights_first(M, w.shape[0], K):
             return ops.gemm_tcgen05_mid(x, w, out)
         return ops.gemm_skinny(x, w, out)
-    out_bf16 = out.dtype == torch.bfloat16
-    form = tcgen05_form(M, w.shape[0], K, out_bf16=out_bf16)
+    may_row = out.dtype == torch.bfloat16
+    form = tcgen05_form(M, w.shape[0], K, may_row=may_row)
     if form == "weights_first":
         return ops.gemm_tcgen05_mid(x, w, out)
     if form == "pair":
-        return ops.gemm_tcgen05_pair(x, w, out, splits=pair_plan(M, w.shape[0], K, out_bf16)[1])
+        return ops.gemm_tcgen05_pair(x, w, out, splits=pair_plan(M, w.shape[0], K, may_row)[1])
     return ops.gemm_tcgen05_prompt(x, w, out, tile_n=128)

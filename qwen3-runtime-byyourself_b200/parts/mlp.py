@@ -101,10 +101,10 @@ class DenseMLP(Part):
             M, I, K = N, self.intermediate_size, self.hidden_size          # the square in the product's epilogue
             if M <= linear_module.skinny_rows:
                 ops.gemm_relu2(x, self.w_up, act, "skinny")
-            elif linear_module.tcgen05_form(M, I, K, gated=True) == "weights_first":
+            elif linear_module.tcgen05_form(M, I, K, gated=True, may_row=False) == "weights_first":
                 ops.gemm_relu2(x, self.w_up, act, "mid")
             else:
-                ops.gemm_relu2(x, self.w_up, act, "pair", splits=linear_module.pair_plan(M, I, K)[1])
+                ops.gemm_relu2(x, self.w_up, act, "pair", splits=linear_module.pair_plan(M, I, K, may_row=False)[1])
         else:
             linear(x, self.w_up, act)
             ops.activation(act, act, self.activation)
