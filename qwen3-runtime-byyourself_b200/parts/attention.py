@@ -463,14 +463,18 @@ def _decode_fused_kernel(part, qkv, cache, out, ctx, table, q_norm_w, k_norm_w, 
         # two: 54.7 with 12 against 64.8; at 2,048 keys 11.8 against 11.1)
         wide = min(splits, max(8, wide_cluster_blocks // (ctx.n_tokens * nkv)), ops.attention_decode_fused_max_splits(d, ctx.device))
         splits = wide if ctx.max_context > long_context_keys else 8
-    elif splits in (6, 7):
-        # a cluster of six or seven blocks leaves SMs empty where four fit (8 kv heads, contexts of 300 to 3,000 tokens: five sequences
-        # 14.6 us in fours against 22.6 in sevens, six 13.8 against 20.2; of 4,000 tokens 23.8 / 34.1 and 24.7 / 36.7)
+    elif splits in (6, 7) and d > 64:
+        # a cluster of six or seven blocks leaves SMs empty where four fit (8 kv heads of 128, contexts of 300 to 3,000 tokens: five sequences
+        # 14.6 us in fours against 22.6 in sevens, six 13.8 against 20.2; of 4,000 tokens 23.8 / 34.1 and 24.7 / 36.7; 1, 2, 4 and 16 kv heads and
+        # head sizes 96, 192 and 256 alike).  The small blocks of heads up to 64 do fit (four / six or seven: 15.8 / 14.5 and 15.9 / 15.5 with
+        # 64, 15.1 / 12.7 with 32, at 4,000 tokens), and so do fives (seven sequences 26.9 in both, of 100 to 3,000 tokens 19.3 against 21.0).
         splits = 4
     parts = counters = None
-    # rows (sequences x kv heads) that the form below cannot split any more, or in three: parts of equal length instead (twelve sequences of
-    # 100 to 3,000 tokens 19.7 us against 23.2 in threes, of 100 to 300 10.6 against 17.0)
-    shared_out = splits == 3 or ctx.n_tokens * nkv > shared_out_rows_per_sm * _sm_count(ctx.device)
+    # rows (sequences x kv heads) that the form below cannot split any more, or in three: parts of equal length instead (96 rows of 1 to 16 kv
+    # heads of 128, contexts of 100 to 300 / 100 to 3,000 / 3,500 to 4,000 tokens: 9.4-10.3 / 20-21 / 39-45 us against 18 / 28-33 / 56-57 in threes,
+    # where not all clusters run at once; 80 rows 9 / 19 / 35-38 against 11 / 24 / 35-36).  Threes of heads of 64 do run at once: 23.4-26.3 against
+    # 22.7-23.5 at 4,000 tokens, 12.4-13.4 against 14.8-17.1 where contexts differ.
+    shared_out = (splits == 3 and d > 64) or ctx.n_tokens * nkv > shared_out_rows_per_sm * _sm_count(ctx.device)
     if shared_out and ops.attention_decode_flat_fits(d, nq // nkv):
         parts = ctx.scratch.get("attn.decode_parts", (ops.attention_decode_flat_parts(d, nq // nkv),), torch.float32)
         counters = ctx.scratch.counters("attn.decode_counters", ctx.n_tokens * nkv)
