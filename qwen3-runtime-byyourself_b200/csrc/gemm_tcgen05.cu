@@ -736,10 +736,11 @@ __device__ __forceinline__ void store_rows(const uint32_t (&v)[64], bf16* Y, int
 // ROWS: W is the 256-row operand instead and the tokens are the other one, of which a tile may have any multiple of 32 (`tile`; 256
 // without ROWS): a few hundred tokens are cut into equal tiles instead of whole 256s.  A thread of the drain then owns a row of W.
 // The eight drain warps take their share of an accumulator (32 lanes by half of its columns) into registers at once, rounded and two a
-// register, and give it back before they finish and store.  Measured for an 8B-sized layer, launches back to back (before, with
-// whole 256s and four drain warps / now / cuBLAS, us): 527 tokens gate/up 117 / 90 / 78, down 73 / 56 / 49, q/k/v 31 / 25 / 22, output
-// 27 / 21 / 18; 1,300 tokens 255 / 200 / 203, 149 / 111 / 94, 62 / 53 / 52, 52 / 43 / 35; 2,048 tokens (whole 256s now, too) 333 / 303 / 341,
-// 158 / 149 / 151, 85 / 79 / 82, 56 / 54 / 54; 7,000 tokens 1,094 / 970 / 1,204, 553 / 533 / 545, 280 / 261 / 277, 188 / 179 / 195.
+// register, and give it back before they finish and store.  Measured for an 8B-sized layer, W from memory, all in one call in short runs at full
+// clocks (before, with whole 256s, four drain warps and copies and products from one lane / now / cuBLAS, without the gate, us): 300 tokens gate/up
+// 114 / 68 / 53, down 63 / 46 / 31, q/k/v 28 / 21 / 17, output 25.5 / 19 / 13; 527 tokens 140 / 99 / 78, 65 / 50 / 46, 29 / 24 / 20, 27 / 20 / 17;
+// 1,300 tokens 272 / 202 / 178, 125 / 101 / 92, 52 / 46 / 44, 45.5 / 35 / 32; 2,048 tokens (whole 256s now, too) 368 / 278 / 279, 145 / 142 / 134,
+// 73 / 70 / 70, 48.6 / 47.2 / 46; 7,000 tokens 1,285 / 915 / 945, 528 / 494 / 477, 251 / 235 / 232, 171 / 161 / 161.
 template <int GATED, typename OutT, bool QKV = false, bool ROWS = false>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
@@ -787,8 +788,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot) : "memory");
 
     if (warp == 0) {
-        // the whole warp walks and one elected thread copies, as with the products: 300 tokens gate/up 73 us against 69 and down 51 / 50,
-        // 1,300 tokens down 134 / 114 and output 46 / 40
+        // the whole warp walks and one elected thread copies, as with the products (from one lane / so, us, nothing else changed: 300 tokens
+        // gate/up 73.3 / 67.6, down 57.9 / 45.6, q/k/v 24.8 / 20.9, output 23.6 / 19.2; 1,300 tokens 204 / 202, 120 / 101, 47.8 / 46.3, 43.6 / 34.7; from
+        // 2,048 tokens on, in whole 256s, gate/up gains 1.5 % and the others nothing)
         pdl_wait();                                           // X is the output of the kernel before
         uint32_t it = 0;
         bool ok = true;

@@ -604,8 +604,8 @@ shared_out_rows_per_sm = 1
 wide_cluster_blocks = 200 # blocks of a decode step with clusters beyond the portable size
 tc_prefill_rows = 128     # from this many new tokens of the longest sequence on, the tcgen05 kernel runs
 # From this many tokens in a step on, the q/k/v product does norm, rotation and cache write in its epilogue: with
-# several tiles per pair of SMs the longer epilogue hides under the next tile's K steps (measured: 8,192 tokens
-# 321-338 us against 381-412 for product + qkv_prepare, 2,048 tokens 83.5 against 86, 512 tokens 41 against 34).
+# several tiles per pair of SMs the longer epilogue hides under the next tile's K steps (whole prompt steps of 12 layers of the 8B
+# shape, fused / product + qkv_prepare: 300 tokens 2.54 / 2.46 ms, 700 and 1,024 equal, 4,096 16.9 / 17.5, 24,000 142.3 / 144.0).
 fused_projection_rows = 2048
 
 DECODE_KERNELS.append(_decode_split_kernel)
