@@ -36,12 +36,15 @@ def set_bf16_kernel_active() -> bool:
 # Microseconds per 64-wide K step of a tile and per block for its start and end, measured on B200 (the unsplit pairs form
 # gives its own estimate, of the tiles it would take).
 _STEP_US = {"pair": 0.33, "prompt128": 0.29, "weights_first": 0.40}
-_BLOCK_US = {"prompt128": 5.0}
+_BLOCK_US = {"prompt128": 4.0}
 # A tile with K split over the pairs of a cluster is not persistent: every wave pays the start of the stream and the
 # meeting of the partial tiles over distributed shared memory, and the launch a little more.  (K 4,096 and 12,288: two ranges
-# 18.3 and 39.7 us, three 16.2 and 29.5; the weights-first form with a range per block of a cluster 13.4 and 26.4 with four, 19.7 with two.)
+# 18.3 and 39.7 us, three 16.2 and 29.5; the weights-first form with a range per block of a cluster 13.4 and 26.4 with four, 19.7 with two,
+# whose blocks have twice as many tokens to add up and write.)  With K up to 2,048 these decide: 300 tokens of 4,096 x 2,048 in 32 bits weights
+# first 16.4, single SMs 11.0, pairs with two ranges 14.2; 600 tokens of 2,048 x 1,024 pairs 8.7, single SMs 6.2; 256 tokens of 3,072 x 4,096
+# weights first in four ranges 14.9, pairs in four 15.6, single SMs 16.6; 600 of them 21.9 (two ranges) against 20.2 on pairs without a split.
 _PAIR_SPLIT_WAVE_US, _PAIR_SPLIT_LAUNCH_US = 6.0, 2.5
-_WEIGHTS_FIRST_SPLIT_US = 7.0
+_WEIGHTS_FIRST_US = {1: 5.0, 2: 9.0, 4: 7.0, 8: 7.0}      # a block's start and end, by the ranges of K
 
 
 @functools.lru_cache(maxsize=4096)
@@ -82,7 +85,7 @@ def tcgen05_form(M: int, N: int, K: int, gated: bool = False, may_row: bool = Tr
     if M <= 1024:
         splits = ops.gemm_tcgen05_mid_splits(M, N, K)
         blocks = -(-N // 128) * -(-M // 256) * splits
-        cost["weights_first"] = waves(blocks, sms) * (-(-nkb // splits) * _STEP_US["weights_first"] + (_WEIGHTS_FIRST_SPLIT_US if splits > 1 else 5.0))
+        cost["weights_first"] = waves(blocks, sms) * (-(-nkb // splits) * _STEP_US["weights_first"] + _WEIGHTS_FIRST_US[splits])
     return min(cost, key=cost.get)
 
 
