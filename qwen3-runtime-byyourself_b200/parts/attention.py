@@ -42,6 +42,7 @@ values of its own (no tensors of them) and reads another layer's cache.
 """
 from __future__ import annotations
 
+import functools
 from fractions import Fraction
 from typing import List, Optional
 
@@ -560,11 +561,50 @@ def _prefill_capped_tcgen05_kernel(part, q, cache, out, ctx, table) -> bool:
     return True
 
 
+# Microseconds that a block of 64 rows on `mma.sync` tiles takes for a page, by the sizes of keys and values.
+_TILES_PAGE_US = {(192, 64): 1.84, (192, 128): 2.23, (192, 192): 3.1, (192, 256): 4.2, (256, 64): 3.0, (256, 128): 2.46, (256, 192): 3.7, (256, 256): 4.5}
+
+
+@functools.lru_cache(maxsize=256)
+def wide_prefill_pays(pos0: tuple, n_new: tuple, heads: int, d: int, vd: int, window: int, sms: int) -> bool:
+    """Whether the tcgen05 kernel for wide heads takes a step's prompts sooner than the `mma.sync` tiles: sequences of `n_new` tokens after `pos0`, a
+    window (0: none).
+
+    One block of 128 rows an SM against blocks of 64 rows: it takes 5 to 8 us to start and end a block, 1.3 us a page and 1 more where some row
+    does not see all of it, the other 1 to 3 and 1.8 to 4.5 a page (with one block an SM, that is with more than 400 values a key, a third more when
+    these fill the GPU).  So short spans and many short sequences - a prompt beside single tokens - stay with the
+    tiles.  The two sums below are within 7 and 12 % (rms) of 7,900 measured steps of 1 to 32 heads and 1 to 32 sequences; tcgen05 / tiles, 16 heads of
+    192 over 64, us: 512 tokens 18.8 / 20.1, behind a window of 128 14.9 / 11.1; 130 tokens beside 15 single ones behind a window of 128 23 / 15;
+    of 256 over 192: 512 tokens 21.4 / 39.6, behind a window of 128 19.0 / 19.5; 2,000 tokens beside 31 single ones behind 64 1.4 times the tiles'."""
+    if not window and max(n_new) >= 1024:
+        return True
+
+    def cost(rows: int, block: float, page: float, edge: float, busy: float) -> float:
+        longest = total = 0.0
+        for p, n in zip(pos0, n_new):
+            for first in range(p, p + n, rows):
+                start = max(0, first - window + 1) if window else 0              # the first key that the tile's first row sees, and its last row
+                full = max(0, first + rows - window) if window else 0
+                pages = (min(first + rows, p + n) - 1) // ops.PAGE_TOKENS + 1 - start // ops.PAGE_TOKENS
+                whole = max(0, (first + 1) // ops.PAGE_TOKENS - -(-full // ops.PAGE_TOKENS)) if edge else 0
+                one = block + page * pages + edge * (pages - whole)
+                longest, total = max(longest, one), total + block + busy * page * pages + edge * (pages - whole)
+        return max(longest, heads * total / sms)
+
+    tiles = sum(-(-n // 128) for n in n_new)
+    empty = heads * (len(n_new) * -(-max(n_new) // 128) - tiles)                # blocks of the grid that find no rows
+    wide = 1.5 + cost(128, 4.3 + 0.0155 * vd, 1.27, 0.5 + 0.003 * vd, 1.0) + 0.65 * empty / sms
+    return wide < 5.2 + cost(64, 1.3 + 0.008 * max(0, d + vd - 320), _TILES_PAGE_US[d, vd], 0.0, 1.37 if d + vd > 400 else 1.0)
+
+
 def _prefill_wide_tcgen05_kernel(part, q, cache, out, ctx, table) -> bool:
     """Heads of up to 256 with values of their own size (latent attention), a window and a sink on tcgen05."""
     if part.plain or part.keep_first or part.shared_values or part.softcap or part.chunk or part.bias_table is not None \
             or part.pooled(ctx, cache) is not None or part.value_heads != part.num_kv_heads or out.dtype != torch.bfloat16 \
             or not ops.attention_wide_prefill_tc_fits(part.head_dim, part.value_dim) or ctx.max_new < tc_prefill_rows or part.scale <= 0:
+        return False
+    spans = (tuple(ctx.host_pos0), tuple(ctx.host_n_new)) if ctx.host_n_new else ((ctx.max_context - ctx.max_new,), (ctx.max_new,))
+    if not wide_prefill_pays(*spans, part.num_heads, part.head_dim, part.value_dim, int(part.window or 0), _sm_count(ctx.device)):
         return False
     ops.attention_wide_prefill_tc(q[:ctx.n_tokens], cache.keys, cache.values, out, ctx.seq_start, ctx.seq_pos0, table, ctx.n_seqs, ctx.max_new,
                                   ctx.n_tokens, part.num_heads, part.num_kv_heads, part.head_dim, part.value_dim, part.scale,
